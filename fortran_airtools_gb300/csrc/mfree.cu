@@ -346,12 +346,17 @@ __device__ __forceinline__ void bp_angle(const MfAngle &A, long long D, int p,
     }
 }
 
-template <typename YT, typename ACC, int MODE, int PB, class Epi>
+// SPLIT: block row s sums its share of the angles into part (n values per
+// share) and k_mf_finish adds the shares.
+template <typename YT, typename ACC, int MODE, int PB, bool SPLIT, class Epi>
 __global__ void __launch_bounds__(128) k_mf_backproject(const MfAngle *__restrict__ ang,
                                                         int nth, int p, int N,
-                                                        const YT *__restrict__ y, Epi epi) {
+                                                        const YT *__restrict__ y, ACC *part,
+                                                        Epi epi) {
     const int groups = (N + PB - 1) / PB;  // pixel groups per image column
     const int64_t ngr = (int64_t)N * groups;
+    const int i0 = SPLIT ? (int)((int64_t)nth * blockIdx.y / gridDim.y) : 0;
+    const int i1 = SPLIT ? (int)((int64_t)nth * (blockIdx.y + 1) / gridDim.y) : nth;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ngr;
          t += (int64_t)gridDim.x * blockDim.x) {
         const int ix = (int)(t / groups), k = (int)(t - (int64_t)ix * groups);
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(128) k_mf_backproject(const MfAngle *__restric
         ACC acc[PB];
 #pragma unroll
         for (int b = 0; b < PB; ++b) acc[b] = 0;
-        for (int i = 0; i < nth; ++i) {
+        for (int i = i0; i < i1; ++i) {
             const MfAngle A = mf_load<ACC>(ang + i);
             const YT *__restrict__ yi = y + (int64_t)i * p;
             const long long D = (long long)ix * A.C + (long long)iy0 * A.S + A.K;
@@ -368,15 +373,32 @@ __global__ void __launch_bounds__(128) k_mf_backproject(const MfAngle *__restric
         }
         const int64_t q0 = (int64_t)ix * N + PB * k;
 #pragma unroll
-        for (int b = 0; b < PB; ++b)
-            if (iy0 - b >= 0) epi(q0 + b, acc[b]);
+        for (int b = 0; b < PB; ++b) {
+            if (iy0 - b < 0) continue;
+            if (SPLIT) part[(int64_t)blockIdx.y * N * N + q0 + b] = acc[b];
+            else epi(q0 + b, acc[b]);
+        }
+    }
+}
+
+// The shares of the angles added per pixel, in order, then the epilogue.
+template <typename ACC, class Epi>
+__global__ void __launch_bounds__(256) k_mf_finish(const ACC *__restrict__ part, int shares,
+                                                   int64_t n, Epi epi) {
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        ACC acc = part[q];
+        for (int s = 1; s < shares; ++s) acc += part[(int64_t)s * n + q];
+        epi(q, acc);
     }
 }
 
 // Per angle of a fan: the source P and the unit direction u0 towards the
-// origin (floats, for the candidate search only).
+// origin (floats, for the candidate search only), and whether one of its rays
+// is axis-aligned.
 struct MfFanAngle {
     float px, py, ux, uy;
+    int tie, pad[3];
 };
 
 // The sorted bin angles oms and, for a uniform grid of L cells over
@@ -390,6 +412,10 @@ struct MfBins {
     const int *tab;
     float om0, inv_cell;
     int L;
+    // the sorted keys [ua, ub) that pixels of the image can reach, where those
+    // are evenly spaced (ub > ua): key k is ukey + (k - ua) / uinv
+    int ua, ub;
+    float ukey, uinv;
     // the first k with oms[k] >= lo
     __device__ __forceinline__ int first(float lo, int p) const {
         const float t = (lo - om0) * inv_cell;
@@ -398,69 +424,311 @@ struct MfBins {
         while (a < p && __ldg(oms + a) < lo) ++a;
         return a;
     }
+    // the first k with oms[k] > hi
+    __device__ __forceinline__ int past(float hi, int p) const {
+        int a = first(hi, p);
+        while (a < p && __ldg(oms + a) <= hi) ++a;
+        return a;
+    }
 };
 
-// The rays of angle i through pixel (ix, iy): bin angles within the pixel's
-// angular half-width of its centre's angle from the source (oms sorted, omj
-// their bins), each tested with the exact fixed-point distance. TANK: the
-// keys are tan(bin angle) (a source at least 1.42 N from the centre: every
-// pixel lies within 30 degrees of the central ray, where tan is monotone), and
-// the window is the tangent of the angle window, t = tan(alpha) = cross/dot
-// and tan(de) = 0.7072/sqrt(|v|^2 - 0.7072^2) + 2.5e-4 combined by the
-// tangent addition formula -- no arctangent or arcsine.
-template <typename YT, typename ACC, int MODE, bool TANK>
-__device__ __forceinline__ void bp_fan_rays(const MfAngle *__restrict__ rays, const MfFanAngle &F,
-                                            const MfBins &B, int i, int p, int ix, int iy, float cx,
-                                            float cy, const YT *__restrict__ y, ACC &acc) {
-    const float vx = cx - F.px, vy = cy - F.py;
-    const float cr = fmaf(F.ux, vy, -F.uy * vx), dt = fmaf(F.ux, vx, F.uy * vy);
-    float lo, hi;
-    if constexpr (TANK) {
-        const float t = __fdividef(cr, dt);
-        const float tau = 0.7072f * rsqrtf(fmaf(vx, vx, fmaf(vy, vy, -0.50014f))) + 2.5e-4f;
-        lo = __fdividef(t - tau, fmaf(t, tau, 1.f));
-        hi = __fdividef(t + tau, fmaf(-t, tau, 1.f));
-    } else {
-        const float al = atan2f(cr, dt);
-        const float de = asinf(fminf(1.f, 0.7072f * rsqrtf(fmaf(vx, vx, vy * vy)))) + 2e-4f;
-        lo = al - de;
-        hi = al + de;
+// Fan backprojector. A block takes a tile of 32 pixel rows (a warp's lanes) by
+// 16 image columns (kFanPB per warp) and walks its share of the angles, two
+// at a time: it stages the rays that can meet the tile -- their records,
+// distances at the tile's origin and y -- in shared memory, the next angles'
+// loads in flight while these are used, and every pixel meets its candidates
+// there. (One thread per two pixels that read each candidate's 96-byte record
+// from global memory was bound by those scattered, dependent loads.)
+constexpr int kFanThreads = 128;        // 4 warps
+constexpr int kFanPB = 4;               // image columns per warp
+constexpr int kFanCap = kFanThreads / 2;  // most rays of an angle staged at once
+constexpr int kFanPad = 4;              // records of weight 0 on either side of them
+// A staged ray (48 or 80 bytes: the lanes' 16-byte reads of neighbouring
+// records fall in different banks).
+template <typename ACC> struct FanRay;
+template <> struct __align__(16) FanRay<float> {
+    longlong2 cs;          // C, -S
+    int H2s;               // H2 at 30 bits
+    float inv_c, ramp, y;
+    long long d0, H2;      // the distance at the tile's origin pixel; H2
+    __device__ __forceinline__ void put(const MfAngle &A, long long d, float v) {
+        cs = longlong2{A.C, -A.S};
+        H2s = A.H2s;
+        inv_c = A.inv_c;
+        ramp = A.ramp30;
+        y = v;
+        d0 = d;
+        H2 = A.H2;
     }
-    for (int k = B.first(lo, p); k < p && __ldg(B.oms + k) <= hi; ++k) {
-        const int j = __ldg(B.omj + k);
-        const int64_t r = (int64_t)i * p + j;
-        const MfAngle A = mf_load<ACC>(rays + r);
-        const long long d = (long long)ix * A.C + (long long)iy * A.S + A.K;
-        const ACC w = Chord<ACC>::of(A, d);
-        if (w > (ACC)0) {
-            if (MODE == 0) acc += w * (ACC)__ldg(y + r);
-            else acc += w;
-        }
+    __device__ __forceinline__ void none() {
+        cs = longlong2{0, 0};
+        H2s = 0;
+        inv_c = 0.f;
+        ramp = 0.f;
+        y = 0.f;
+        d0 = H2 = 0;
     }
+    // acc += a_rq y_r at distance d: the same entry, from the same exact
+    // distance, as the projector's. TIE: the ray may be axis-aligned (tie its
+    // side), FAR: more than two pixels away.
+    template <int MODE, bool TIE, bool FAR>
+    __device__ __forceinline__ void add(long long d, int tie, float &acc) const {
+        const long long ad = d < 0 ? -d : d;
+        float w = inv_c * __saturatef((float)(H2s - (int)(ad >> 16)) * ramp);
+        if (TIE && tie != 0) w = ad < H2 || (ad == H2 && tie == (d > 0 ? 1 : -1)) ? inv_c : 0.f;
+        if (FAR && (ad >> 47) != 0) w = 0.f;
+        if (w > 0.f) acc += MODE == 0 ? w * y : w;
+    }
+};
+template <> struct __align__(16) FanRay<double> {
+    longlong2 cs;
+    long long d0, H2;
+    long long H1, Hcut;
+    double inv_c, ramp;
+    double y, pad;
+    __device__ __forceinline__ void put(const MfAngle &A, long long d, double v) {
+        cs = longlong2{A.C, -A.S};
+        d0 = d;
+        H2 = A.H2;
+        H1 = A.H1;
+        Hcut = A.Hcut;
+        inv_c = A.inv_c64;
+        ramp = A.scale_ramp64;
+        y = v;
+    }
+    __device__ __forceinline__ void none() {
+        cs = longlong2{0, 0};
+        d0 = 0;
+        Hcut = -1;
+    }
+    // below Hcut every entry is positive; an axis-aligned ray (Hcut = H1 = H2)
+    // also keeps |d| = H2 on its positive side
+    template <int MODE, bool TIE, bool FAR>
+    __device__ __forceinline__ void add(long long d, int tie, double &acc) const {
+        const long long ad = d < 0 ? -d : d;
+        if (ad >= Hcut && !(TIE && tie != 0 && ad == Hcut && tie == (d > 0 ? 1 : -1))) return;
+        const double w = ad <= H1 ? inv_c : (double)(H2 - ad) * ramp;
+        acc += MODE == 0 ? w * y : w;
+    }
+};
+template <typename ACC> struct FanRays {
+    FanRay<ACC> ray[kFanCap + 2 * kFanPad];
+    float key[kFanCap];
+    int tie[kFanCap];
+};
+
+// d + l C for a small l >= 0.
+__device__ __forceinline__ long long mad_small(long long d, unsigned l, long long C) {
+    unsigned long long r = (unsigned long long)d + (unsigned long long)l * (unsigned)C;
+    r += (unsigned long long)(l * (unsigned)((unsigned long long)C >> 32)) << 32;
+    return (long long)r;
 }
 
-template <typename YT, typename ACC, int MODE, bool TANK, class Epi>
-__global__ void __launch_bounds__(128) k_mf_backproject_fan(
+// TANK: the keys are tan(bin angle) (a source at least 1.42 N from the
+// centre: every pixel lies within 30 degrees of the central ray, where tan is
+// monotone); a pixel's window is the tangent of its angle window, t =
+// tan(alpha) = cross/dot and tan(de) combined by the tangent addition formula
+// -- no arctangent or arcsine. UNI (N >= 16): the keys the image can reach are
+// evenly spaced, so a pixel's candidates are the indices in f -+ w: f from t,
+// w from the half-width H2/|v| of a pixel square along its own direction, H2 =
+// (|cos| + |sin|)/2 of v, bounded once per tile and angle. With at most
+// kFanPad candidates every lane tests the same number (a ray that misses the
+// pixel has entry 0), so the loop has no branch on the lane.
+// N = 512, 720 angles, 728 bins, FP32: 3.12 ms (a thread per two pixels, records
+// from global memory) -> 0.81 ms; bound by shared-memory reads (75% of the
+// wavefront rate: 40 bytes per candidate) and issue (64%).
+template <typename YT, typename ACC, int MODE, bool TANK, bool UNI, class Epi>
+__global__ void __launch_bounds__(kFanThreads, 7) k_mf_backproject_fan(
         const MfAngle *__restrict__ rays, const MfFanAngle *__restrict__ fa, MfBins B, int nth,
-        int p, int N, const YT *__restrict__ y, Epi epi) {
-    const int half = (N + 1) / 2;  // pixel pairs per image column
-    const int64_t npairs = (int64_t)N * half;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < npairs;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int ix = (int)(t / half), k = (int)(t - (int64_t)ix * half);
-        const int iy0 = N - 1 - 2 * k;  // pixel q0 = ix*N + 2k
-        const bool two = iy0 >= 1;      // and q0 + 1 (iy0 - 1) when it exists
-        const float cx = (float)ix + 0.5f - 0.5f * (float)N;
-        const float cy0 = (float)iy0 + 0.5f - 0.5f * (float)N;
-        ACC acc0 = 0, acc1 = 0;
-        for (int i = 0; i < nth; ++i) {
-            const MfFanAngle F = fa[i];
-            bp_fan_rays<YT, ACC, MODE, TANK>(rays, F, B, i, p, ix, iy0, cx, cy0, y, acc0);
-            if (two) bp_fan_rays<YT, ACC, MODE, TANK>(rays, F, B, i, p, ix, iy0 - 1, cx, cy0 - 1.f, y, acc1);
+        int p, int N, const YT *__restrict__ y, ACC *part, Epi epi) {
+    constexpr int PB = kFanPB, CAP = kFanCap, PAD = kFanPad, NA = kFanThreads;
+    __shared__ FanRays<ACC> W[2][2];
+    __shared__ int2 win[NA];     // per angle: the sorted keys [x, y) that can meet the tile
+    __shared__ float4 fs[NA];    // P, u0
+    __shared__ float2 wt[NA];    // w (UNI), axis-aligned rays
+    const int t = threadIdx.x, lane = t & 31, wc = (t >> 5) * PB;
+    const int half_id = t / CAP, ts = t % CAP;  // this thread stages ray ts of piece half_id
+    const int tiles_k = (N + 31) >> 5;
+    const int k0 = (int)(blockIdx.x % tiles_k) * 32, ix0 = (int)(blockIdx.x / tiles_k) * 4 * PB;
+    // pixel (ix0 + lx, iyT - lane) is element (ix0 + lx) N + k0 + lane
+    const int iyT = N - 1 - k0;
+    const float half = 0.5f * (float)N - 0.5f;
+    const float cy = (float)(iyT - lane) - half, cx0 = (float)(ix0 + wc) - half;
+    const int a0 = (int)((int64_t)nth * blockIdx.y / gridDim.y);
+    const int a1 = (int)((int64_t)nth * (blockIdx.y + 1) / gridDim.y);
+    ACC acc[PB];
+#pragma unroll
+    for (int c = 0; c < PB; ++c) acc[c] = 0;
+    if (t < 4 * PAD) W[t / (2 * PAD)][t / PAD & 1].ray[t % PAD].none();  // the records before a window
+
+    for (int i0 = a0; i0 < a1; i0 += NA) {
+        const int na = min(NA, a1 - i0);
+        if (t < na) {
+            // the tile's centre and the radius that covers its pixels
+            const int cols = min(4 * PB, N - ix0), rows = min(32, N - k0);
+            const float tx = (float)ix0 + 0.5f * (float)(cols - 1) - half;
+            const float ty = (float)iyT - 0.5f * (float)(rows - 1) - half;
+            const float rho = 0.5f * sqrtf((float)((cols - 1) * (cols - 1) + (rows - 1) * (rows - 1))) + 0.75f;
+            const MfFanAngle F = fa[i0 + t];
+            const float vx = tx - F.px, vy = ty - F.py, vv = fmaf(vx, vx, vy * vy);
+            const float cr = fmaf(F.ux, vy, -F.uy * vx), dt = fmaf(F.ux, vx, F.uy * vy);
+            bool all = vv <= 1.05f * rho * rho;
+            float lo = 0.f, hi = 0.f, w = 1e9f;
+            if (TANK) {
+                const float tt = cr / dt, tau = rho * rsqrtf(fmaxf(vv - rho * rho, 1e-6f)) * 1.001f + 1e-4f;
+                all = all || dt <= 0.f || fabsf(tt) * tau > 0.9f;
+                lo = (tt - tau) / (1.f + tt * tau);
+                hi = (tt + tau) / (1.f - tt * tau);
+            } else {
+                const float al = atan2f(cr, dt), de = asinf(fminf(1.f, rho * rsqrtf(vv))) + 1e-3f;
+                lo = al - de;
+                hi = al + de;
+                all = all || lo < -3.14f || hi > 3.14f;
+            }
+            int ka = 0, kb = p;
+            if (!all) {
+                ka = B.first(lo, p);
+                kb = B.past(hi, p);
+            }
+            if (UNI) {
+                ka = max(ka, B.ua);
+                kb = min(kb, B.ub);
+                if (!all) {
+                    const float av = sqrtf(vv), rm = 1.f / (av - rho);  // 1/|v| of any pixel of the tile
+                    const float h = fminf(0.7072f, 0.5f * (fabsf(vx) + fabsf(vy)) / av + rm * (0.71f * rho + 0.75f));
+                    const float tm = fmaxf(fabsf(lo), fabsf(hi));
+                    const float tau = h * rm * (1.f + 0.5f * rm * rm) + 8e-6f;  // >= tan(de) for |v| >= 2
+                    if (rm > 0.f && tm * tau < 0.5f)
+                        w = B.uinv * tau * (1.f + tm * tm) / (1.f - tm * tau) + 0.011f;
+                }
+            }
+            fs[t] = make_float4(F.px, F.py, F.ux, F.uy);
+            wt[t] = make_float2(w, F.tie != 0 ? 1.f : 0.f);
+            win[t] = make_int2(ka, kb);
         }
-        const int64_t q0 = (int64_t)ix * N + 2 * k;
-        epi(q0, acc0);
-        if (two) epi(q0 + 1, acc1);
+        __syncthreads();
+        // the windows in pieces of at most CAP rays: angle .x, first key .y;
+        // .x = na past the last
+        auto next = [&](int2 c, int by) {
+            c.y += by;
+            while (c.x < na && c.y >= win[c.x].y)
+                if (++c.x < na) c.y = win[c.x].x;
+            return c;
+        };
+        MfAngle R;
+        YT yv = 0;
+        float key = 0.f;
+        int have = 0;  // 1: a ray of the piece; 2: past its end
+        auto load = [&](int2 c) {  // this thread's ray of piece c
+            have = c.x >= na ? 0 : (c.y + ts < win[c.x].y ? 1 : 2);
+            if (have != 1) return;
+            const int64_t r = (int64_t)(i0 + c.x) * p + __ldg(B.omj + c.y + ts);
+            R = mf_load<ACC>(rays + r);
+            if (MODE == 0) yv = __ldg(y + r);
+            if (!UNI) key = __ldg(B.oms + c.y + ts);
+        };
+        auto store = [&](int b) {
+            FanRays<ACC> &V = W[b][half_id];
+            if (have == 1) {
+                V.ray[PAD + ts].put(R, mad_small(mad_small(R.K, (unsigned)ix0, R.C), (unsigned)iyT, R.S), (ACC)yv);
+                V.tie[ts] = R.tie;
+                if (!UNI) V.key[ts] = key;
+            } else if (have == 2) {
+                V.ray[PAD + ts].none();
+            }
+            if (UNI && have != 0 && ts < PAD) V.ray[PAD + CAP + ts].none();
+        };
+        int buf = 0;
+        int2 c0 = next(make_int2(0, win[0].x), 0), c1 = next(c0, CAP);
+        load(half_id ? c1 : c0);
+        store(buf);
+        __syncthreads();
+        while (c0.x < na) {
+            const int2 n0 = next(c1, CAP), n1 = next(n0, CAP);
+            load(half_id ? n1 : n0);
+#pragma unroll 1
+            for (int hh = 0; hh < 2; ++hh) {
+                const int2 cur = hh ? c1 : c0;
+                if (cur.x >= na) break;
+                const int len = min(CAP, win[cur.x].y - cur.y);
+                const FanRays<ACC> &V = W[buf][hh];
+                const float4 F = fs[cur.x];
+                const float2 wf = wt[cur.x];
+                const float vy = cy - F.y, vx0 = cx0 - F.x;
+                float cr = fmaf(F.z, vy, -F.w * vx0), dt = fmaf(F.z, vx0, F.w * vy);
+                const float w = wf.x, off = (float)(B.ua - cur.y);
+                const int nc = (int)floorf(2.f * w) + 1;  // candidates of a pixel
+                if (UNI && nc <= PAD && wf.y == 0.f) {
+#pragma unroll
+                    for (int c = 0; c < PB; ++c) {
+                        const float f = fmaf(__fdividef(cr, dt) - B.ukey, B.uinv, off);
+                        const int kl = min(max((int)ceilf(f - w), -PAD), len);
+                        const FanRay<ACC> *r = V.ray + (PAD + kl);
+#pragma unroll
+                        for (int e = 0; e < PAD; ++e)
+                            if (e < nc) {
+                                const long long d = mad_small(mad_small(r[e].d0, (unsigned)(wc + c), r[e].cs.x),
+                                                              (unsigned)lane, r[e].cs.y);
+                                r[e].template add<MODE, false, true>(d, 0, acc[c]);
+                            }
+                        cr -= F.w;
+                        dt += F.z;
+                    }
+                    continue;
+                }
+#pragma unroll
+                for (int c = 0; c < PB; ++c) {
+                    auto entry = [&](int k) {
+                        const FanRay<ACC> &r = V.ray[PAD + k];
+                        const long long d = mad_small(mad_small(r.d0, (unsigned)(wc + c), r.cs.x),
+                                                      (unsigned)lane, r.cs.y);
+                        r.template add<MODE, true, true>(d, V.tie[k], acc[c]);
+                    };
+                    const float tt = __fdividef(cr, dt);
+                    if constexpr (UNI) {
+                        const float f = fmaf(tt - B.ukey, B.uinv, off);
+                        const int kl = max(0, (int)ceilf(f - w)), kh = min(len - 1, (int)floorf(f + w));
+                        for (int k = kl; k <= kh; ++k) entry(k);
+                    } else {
+                        float lo, hi;
+                        const float vx = vx0 + (float)c;
+                        if constexpr (TANK) {
+                            const float tau = 0.7072f * rsqrtf(fmaf(vx, vx, fmaf(vy, vy, -0.50014f))) + 2.5e-4f;
+                            lo = __fdividef(tt - tau, fmaf(tt, tau, 1.f));
+                            hi = __fdividef(tt + tau, fmaf(-tt, tau, 1.f));
+                        } else {
+                            const float al = atan2f(cr, dt);
+                            const float de = asinf(fminf(1.f, 0.7072f * rsqrtf(fmaf(vx, vx, vy * vy)))) + 2e-4f;
+                            lo = al - de;
+                            hi = al + de;
+                        }
+                        // the first staged key >= lo: a guess by interpolation, then steps
+                        const float f = V.key[0], l = V.key[len - 1];
+                        int k = l > f ? (int)((lo - f) * __fdividef((float)(len - 1), l - f)) : 0;
+                        k = max(0, min(len, k));
+                        while (k > 0 && V.key[k - 1] >= lo) --k;
+                        while (k < len && V.key[k] < lo) ++k;
+                        for (; k < len && V.key[k] <= hi; ++k) entry(k);
+                    }
+                    cr -= F.w;
+                    dt += F.z;
+                }
+            }
+            buf ^= 1;
+            store(buf);
+            c0 = n0;
+            c1 = n1;
+            __syncthreads();
+        }
+    }
+    const int k = k0 + lane;
+#pragma unroll
+    for (int c = 0; c < PB; ++c) {
+        const int ix = ix0 + wc + c;
+        if (ix >= N || k >= N) continue;
+        const int64_t q = (int64_t)ix * N + k;
+        if (gridDim.y > 1) part[(int64_t)blockIdx.y * N * N + q] = acc[c];
+        else epi(q, acc[c]);
     }
 }
 
@@ -487,6 +755,9 @@ struct fair_mf_s {
     float om0 = 0.f, om_inv = 0.f;     // the grid: start, 1 / cell width, cells
     int om_L = 1;
     bool tan_keys = false;             // oms holds tan(bin angle) (the backprojector's TANK)
+    int uni_a = 0, uni_b = 0;          // evenly spaced reachable keys (MfBins), none: uni_b = 0
+    float uni_key = 0.f, uni_inv = 0.f;
+    fair::DevBuf part;                 // the backprojector's sums per share of the angles
     fair::DevBuf w_in, w_out;          // host-call staging (FP64)
     fair::DevBuf xt;                   // the projector's transposed copy of x
     fair::DevBuf v_a, v_b;             // reduced-precision staging
@@ -527,22 +798,48 @@ void mf_project(fair_mf A, const XT *x, Epi epi, cudaStream_t s) {
     else
         k_mf_project<XT, ACC, MODE, false><<<grid_for(m, 128), 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, epi);
 }
+// Blocks of the backprojector over the image, and the shares its angles are
+// cut into so that a small image still fills the GPU: about 8 blocks of 4
+// warps per SM, at least 8 angles each.
+int64_t mf_bp_blocks(fair_mf A) {
+    const int64_t N = A->N;
+    if (A->kind == 1) return ((N + 31) / 32) * ((N + 4 * kFanPB - 1) / (4 * kFanPB));
+    return (N * ((N + kMfPB - 1) / kMfPB) + 127) / 128;
+}
+int mf_bp_shares(fair_mf A) {
+    const int64_t want = ((int64_t)sm_count() * 8) / mf_bp_blocks(A);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min(A->nth / 8, 32)));
+}
 template <typename YT, typename ACC, int MODE, class Epi>
-void mf_backproject(fair_mf A, const YT *y, Epi epi, cudaStream_t s) {
+int mf_backproject(fair_mf A, const YT *y, Epi epi, cudaStream_t s) {
     const int64_t n = (int64_t)A->N * A->N;
     const MfAngle *ang = A->ang.as<MfAngle>();
+    const int shares = mf_bp_shares(A);
+    if (shares > 1) FAIR_TRY(A->part.grow(sizeof(ACC) * (size_t)shares * n));
+    ACC *part = A->part.as<ACC>();
     if (A->kind == 1) {
-        const MfBins B{A->oms.as<float>(), A->omj.as<int>(), A->omt.as<int>(), A->om0, A->om_inv, A->om_L};
-        if (A->tan_keys)
-            k_mf_backproject_fan<YT, ACC, MODE, true><<<grid_for(n / 2 + 1, 128), 128, 0, s>>>(
-                ang, A->fang.as<MfFanAngle>(), B, A->nth, A->p, A->N, y, epi);
+        const MfBins B{A->oms.as<float>(), A->omj.as<int>(), A->omt.as<int>(), A->om0, A->om_inv, A->om_L,
+                       A->uni_a, A->uni_b, A->uni_key, A->uni_inv};
+        const dim3 g((unsigned)mf_bp_blocks(A), shares);
+        const MfFanAngle *fa = A->fang.as<MfFanAngle>();
+        if (A->tan_keys && A->uni_b > A->uni_a)
+            k_mf_backproject_fan<YT, ACC, MODE, true, true><<<g, kFanThreads, 0, s>>>(
+                ang, fa, B, A->nth, A->p, A->N, y, part, epi);
+        else if (A->tan_keys)
+            k_mf_backproject_fan<YT, ACC, MODE, true, false><<<g, kFanThreads, 0, s>>>(
+                ang, fa, B, A->nth, A->p, A->N, y, part, epi);
         else
-            k_mf_backproject_fan<YT, ACC, MODE, false><<<grid_for(n / 2 + 1, 128), 128, 0, s>>>(
-                ang, A->fang.as<MfFanAngle>(), B, A->nth, A->p, A->N, y, epi);
+            k_mf_backproject_fan<YT, ACC, MODE, false, false><<<g, kFanThreads, 0, s>>>(
+                ang, fa, B, A->nth, A->p, A->N, y, part, epi);
+    } else {
+        const dim3 g((unsigned)std::min<int64_t>(mf_bp_blocks(A), (int64_t)sm_count() * 32), shares);
+        if (shares > 1)
+            k_mf_backproject<YT, ACC, MODE, kMfPB, true><<<g, 128, 0, s>>>(ang, A->nth, A->p, A->N, y, part, epi);
+        else
+            k_mf_backproject<YT, ACC, MODE, kMfPB, false><<<g, 128, 0, s>>>(ang, A->nth, A->p, A->N, y, part, epi);
     }
-    else
-        k_mf_backproject<YT, ACC, MODE, kMfPB><<<grid_for(n / kMfPB + A->N, 128), 128, 0, s>>>(
-            ang, A->nth, A->p, A->N, y, epi);
+    if (shares > 1) k_mf_finish<ACC><<<grid_for(n, 256), 256, 0, s>>>(part, shares, n, epi);
+    return FAIR_OK;
 }
 
 int mf_weights(fair_mf A, bool sart, cudaStream_t s) {
@@ -553,7 +850,7 @@ int mf_weights(fair_mf A, bool sart, cudaStream_t s) {
         EpiStore<double> e1{A->M_sart.as<double>()};
         mf_project<double, double, 1>(A, (const double *)nullptr, e1, s);
         EpiStore<double> e2{A->D.as<double>()};
-        mf_backproject<double, double, 1>(A, (const double *)nullptr, e2, s);
+        FAIR_TRY((mf_backproject<double, double, 1>(A, (const double *)nullptr, e2, s)));
         FAIR_CUDA(cudaGetLastError());
         FAIR_TRY(vec_reciprocal(A->M_sart.as<double>(), m, s));  // the epilogues multiply
         FAIR_TRY(vec_reciprocal(A->D.as<double>(), n, s));
@@ -571,7 +868,7 @@ int mf_weights(fair_mf A, bool sart, cudaStream_t s) {
 }
 
 // One projector / backprojector pass of a SIRT iteration.
-void mf_pass(fair_mf A, int pass, const double *d_b, double *d_x, cudaStream_t s) {
+int mf_pass(fair_mf A, int pass, const double *d_b, double *d_x, cudaStream_t s) {
     const double *M = A->sart ? A->M_sart.as<double>() : A->M_cim.as<double>();
     const double *D = A->sart ? A->D.as<double>() : nullptr;
     if (A->prec == FAIR_PREC_F64) {
@@ -580,7 +877,7 @@ void mf_pass(fair_mf A, int pass, const double *d_b, double *d_x, cudaStream_t s
             mf_project<double, double, 0>(A, (const double *)d_x, e, s);
         } else {
             EpiUpdateF64 e{D, d_x, A->omg, A->lb, A->ub, A->bmode};
-            mf_backproject<double, double, 0>(A, (const double *)A->r.as<double>(), e, s);
+            return mf_backproject<double, double, 0>(A, (const double *)A->r.as<double>(), e, s);
         }
     } else {
         if (pass == 1) {
@@ -588,9 +885,10 @@ void mf_pass(fair_mf A, int pass, const double *d_b, double *d_x, cudaStream_t s
             mf_project<float, float, 0>(A, (const float *)A->x32.as<float>(), e, s);
         } else {
             EpiUpdateLP e{D, d_x, A->x32.as<float>(), A->omg, A->lb, A->ub, A->bmode, 1.0};
-            mf_backproject<float, float, 0>(A, (const float *)A->r.as<float>(), e, s);
+            return mf_backproject<float, float, 0>(A, (const float *)A->r.as<float>(), e, s);
         }
     }
+    return FAIR_OK;
 }
 
 }  // namespace
@@ -746,7 +1044,7 @@ int fair_mf_create_fan(fair_mf *out, const fair_data *dat, int32_t geometry_fix,
         const double c = cos(dat->theta[i]), s = sin(dat->theta[i]);
         const double x0th = c * 0.0 - s * R, y0th = s * 0.0 + c * R;
         const double ath = -x0th / R, bth = -y0th / R;
-        fa[i] = fair::MfFanAngle{(float)x0th, (float)y0th, (float)ath, (float)bth};
+        fa[i] = fair::MfFanAngle{(float)x0th, (float)y0th, (float)ath, (float)bth, 0, {0, 0, 0}};
         for (int j = 0; j < p; ++j) {
             // the ray direction of the reference's tracer (:163-166)
             const double a = com[j] * ath - som[j] * bth;
@@ -755,6 +1053,7 @@ int fair_mf_create_fan(fair_mf *out, const fair_data *dat, int32_t geometry_fix,
             const double C = b / nu, S = -a / nu;  // unit normal
             const double K = C * (0.5 - 0.5 * N - x0th) + S * (0.5 - 0.5 * N - y0th);
             fair::mf_line(C, S, K, rays[(size_t)i * p + j]);
+            if (rays[(size_t)i * p + j].tie != 0) fa[i].tie = 1;
         }
     }
     // the bin angles sorted (the odd-p angles of :122 are not monotone in j)
@@ -770,6 +1069,27 @@ int fair_mf_create_fan(fair_mf *out, const fair_data *dat, int32_t geometry_fix,
     A->tan_keys = tk;
     std::vector<float> oms(p);
     for (int k = 0; k < p; ++k) oms[k] = (float)(tk ? std::tan(omega[order[k]]) : omega[order[k]]);
+    // the sorted keys that a pixel of the image can reach, and whether they are
+    // evenly spaced (a flat detector's tangents are; the odd-p angles of :122
+    // lie past them)
+    if (tk && N >= 16) {
+        const double amax = asin(std::min(1.0, 0.7072 * (N + 2) / R)) + 2e-3;
+        int ua = 0, ub = p;
+        while (ua < p && atan((double)oms[ua]) < -amax) ++ua;
+        while (ub > ua && atan((double)oms[ub - 1]) > amax) --ub;
+        if (ub - ua >= 2) {
+            const double step = ((double)oms[ub - 1] - (double)oms[ua]) / (ub - 1 - ua);
+            bool even = step > 0;
+            for (int k = ua; k < ub; ++k)
+                even = even && std::fabs((double)oms[k] - ((double)oms[ua] + (k - ua) * step)) <= 2e-3 * step;
+            if (even) {
+                A->uni_a = ua;
+                A->uni_b = ub;
+                A->uni_key = oms[ua];
+                A->uni_inv = (float)(1.0 / step);
+            }
+        }
+    }
     // a grid of 4p cells over the sorted angles; tab[c] = first k with oms[k] >=
     // om0 + c / inv (the device starts one cell early and steps forward)
     const int L = 4 * p;
@@ -799,7 +1119,7 @@ int fair_mf_destroy(fair_mf A) {
     cudaStreamSynchronize(A->stream);
     for (fair::DevBuf *d : {&A->ang, &A->fang, &A->oms, &A->omj, &A->omt, &A->w_in, &A->w_out, &A->v_a,
                             &A->v_b, &A->M_sart, &A->M_cim, &A->D, &A->x32, &A->r, &A->w_b,
-                            &A->w_x, &A->xt})
+                            &A->w_x, &A->xt, &A->part})
         d->release();
     if (A->own_stream) cudaStreamDestroy(A->stream);
     delete A;
@@ -842,7 +1162,7 @@ static int mf_apply(fair_mf A, bool back, const double *in, double *out) {
     if (A->prec == FAIR_PREC_F64) {
         fair::EpiStore<double> e{A->w_out.as<double>()};
         const double *vin = A->w_in.as<double>();
-        if (back) fair::mf_backproject<double, double, 0>(A, vin, e, s);
+        if (back) FAIR_TRY((fair::mf_backproject<double, double, 0>(A, vin, e, s)));
         else fair::mf_project<double, double, 0>(A, vin, e, s);
         FAIR_CUDA(cudaGetLastError());
     } else {
@@ -851,7 +1171,7 @@ static int mf_apply(fair_mf A, bool back, const double *in, double *out) {
         FAIR_TRY(fair::vec_to_f32(A->w_in.as<double>(), nin, A->v_a.as<float>(), s));
         fair::EpiStore<float> e{A->v_b.as<float>()};
         const float *vin = A->v_a.as<float>();
-        if (back) fair::mf_backproject<float, float, 0>(A, vin, e, s);
+        if (back) FAIR_TRY((fair::mf_backproject<float, float, 0>(A, vin, e, s)));
         else fair::mf_project<float, float, 0>(A, vin, e, s);
         FAIR_CUDA(cudaGetLastError());
         FAIR_TRY(fair::vec_to_f64(A->v_b.as<float>(), nout, A->w_out.as<double>(), s));
@@ -905,6 +1225,8 @@ int fair_mf_sirt_prepare(fair_mf A, const char *sirt_method, const fair_opts *op
     if (red) FAIR_TRY(A->x32.grow(sizeof(float) * (n + 1)));
     FAIR_TRY(fair::mf_grow_xt(A));
     FAIR_TRY(fair::mf_weights(A, sart, A->stream));
+    const int shares = fair::mf_bp_shares(A);
+    if (shares > 1) FAIR_TRY(A->part.grow((red ? sizeof(float) : sizeof(double)) * (size_t)shares * n));
     FAIR_CUDA(cudaStreamSynchronize(A->stream));
     A->ready = true;
     return FAIR_OK;
@@ -928,9 +1250,10 @@ static int mf_iterations(fair_mf A, const double *d_b, double *d_x, int32_t K, f
     int st = FAIR_OK;
     for (int it = 0; it < K; ++it) {
         if (ms1) cudaEventRecord(ev[0], s);
-        fair::mf_pass(A, 1, d_b, d_x, s);
+        st = fair::mf_pass(A, 1, d_b, d_x, s);
         if (ms1) cudaEventRecord(ev[1], s);
-        fair::mf_pass(A, 2, d_b, d_x, s);
+        if (st == FAIR_OK) st = fair::mf_pass(A, 2, d_b, d_x, s);
+        if (st != FAIR_OK) break;
         if (ms1) {
             cudaEventRecord(ev[2], s);
             cudaError_t e = cudaEventSynchronize(ev[2]);
