@@ -15,13 +15,18 @@
 // is reversed, so memory is O(sqrt(K)) vectors and work is three forward
 // sweeps of products.
 //
-// Vectors of the batch are interleaved ([row][NR]) so that one gather loads
-// every right-hand side of a column; the multi-vector row engine follows the
-// chunk layout of rows.cuh (32 rows per warp chunk, G lanes per row, results
-// moved to lane row mod 32 for a coalesced epilogue).
+// Vectors of the batch are interleaved ([row][NR], NR = 1, 4, 8 or 16) so that
+// one gather loads every right-hand side of a column. Matrices whose columns
+// (A) or rows (A') are an image run on the tiled copies (tl_multi_partials,
+// tiled.cu: the gathered vectors staged in shared memory per tile) followed
+// by row sums with the epilogue; others on the multi-vector row engine below.
+// N = 256, 360 angles, 362 bins, 16 right-hand sides, FP32: a product takes
+// 134 + 19 us (the row engine: 280 us); 101 x 101 fan, 180 angles, 3
+// right-hand sides, FP64: 30 + 7 us (82 / 62).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "fair_gpu_ext.h"
@@ -90,7 +95,7 @@ __device__ __forceinline__ void chunk_rows_multi(const int64_t *__restrict__ row
     finish_chunks(sched, nwarps, lane);
 }
 
-// The same products with the right-hand sides across the lanes (NR = 4 or
+// The same products with the right-hand sides across the lanes (NR = 4, 8 or
 // 16): lane l handles right-hand side l % NR of entry slot l / NR, so a warp
 // step covers E = 32 / NR entries of one row and each entry's NR values of x
 // are one contiguous run of NR x sizeof(T) bytes. The warp reads a row's
@@ -106,7 +111,7 @@ __device__ __forceinline__ void chunk_rows_rhs(const int64_t *__restrict__ rowpt
                                                const int32_t *__restrict__ col,
                                                const T *__restrict__ val, const T *__restrict__ x,
                                                const Epi &epi, unsigned *sched) {
-    static_assert(NR == 4 || NR == 16, "4 or 16 right-hand sides");
+    static_assert(NR == 4 || NR == 8 || NR == 16, "4, 8 or 16 right-hand sides");
     constexpr int E = 32 / NR, STEPS = 32 / E, NA = 4, CR = kRhsRows;
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, slot = lane / NR, c = lane % NR;
@@ -160,12 +165,14 @@ __device__ __forceinline__ T boxT(T t, int bmode, T lb, T ub) {
     return t;
 }
 
+// The weights arrive as reciprocals (1/0 = Inf): an FP64 division is a
+// sequence of FP64-pipe instructions, 64 cycles each per warp.
 // forward pass 1: r = (b - A x) / M
 template <typename T, int NR>
 struct EpiFwdResid {
-    const T *b, *M;
+    const T *b, *Mi;
     T *r;
-    __device__ void one(int64_t i, int c, T v) const { r[i * NR + c] = (b[i * NR + c] - v) / M[i]; }
+    __device__ void one(int64_t i, int c, T v) const { r[i * NR + c] = (b[i * NR + c] - v) * Mi[i]; }
     __device__ void operator()(int64_t i, const T (&acc)[NR]) const {
 #pragma unroll
         for (int c = 0; c < NR; ++c) one(i, c, acc[c]);
@@ -174,13 +181,13 @@ struct EpiFwdResid {
 // forward pass 2: g = A' r (kept when recording), x = P(x + lam g / D)
 template <typename T, int NR>
 struct EpiFwdUpdate {
-    const T *D, *lam;
+    const T *Di, *lam;
     T *x, *gsave;
     T lb, ub;
     int bmode;
     __device__ void one(int64_t j, int c, T v) const {
         T u = lam[c] * v;
-        if (D) u = u / D[j];
+        if (Di) u = u * Di[j];
         if (gsave) gsave[j * NR + c] = v;
         x[j * NR + c] = boxT<T>(x[j * NR + c] + u, bmode, lb, ub);
     }
@@ -192,10 +199,11 @@ struct EpiFwdUpdate {
 // reverse, over A: w = (A t) / M (0 on empty rows), gb += lam w
 template <typename T, int NR>
 struct EpiAdjA {
-    const T *M, *lam;
+    const T *Mi, *lam;
     T *w, *gb;
     __device__ void one(int64_t i, int c, T v) const {
-        T wi = M[i] != (T)0 ? v / M[i] : (T)0;
+        const T mi = Mi[i];
+        T wi = isinf(mi) ? (T)0 : v * mi;
         w[i * NR + c] = wi;
         gb[i * NR + c] += lam[c] * wi;
     }
@@ -228,10 +236,41 @@ __global__ void __launch_bounds__(256, 4) k_multi(const int64_t *rowptr, int32_t
         chunk_rows_rhs<T, NR>(rowptr, m, col, val, x, epi, sched);
 }
 
+// Row sums of the tiled products' partials (in row order) and the epilogue: a
+// thread per row and 16 bytes of its NR values.
+template <typename T, int NR, class Epi>
+__global__ void __launch_bounds__(256) k_multi_rows(int32_t m, const int64_t *__restrict__ segbase,
+                                                    const T *__restrict__ part, Epi epi) {
+    constexpr int V = NR * sizeof(T) >= 16 ? 16 / (int)sizeof(T) : NR, L = NR / V;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)m * L;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = e / L;
+        const int c0 = (int)(e % L) * V;
+        T acc[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[k] = 0;
+        const int64_t k1 = segbase[i + 1];
+        for (int64_t k = segbase[i]; k < k1; ++k) {
+            const T *p = part + (size_t)k * NR + c0;
+            if constexpr (V == 4) {
+                const float4 u = __ldcs(reinterpret_cast<const float4 *>(p));
+                acc[0] += u.x; acc[1] += u.y; acc[2] += u.z; acc[3] += u.w;
+            } else if constexpr (V == 2) {
+                const double2 u = __ldcs(reinterpret_cast<const double2 *>(p));
+                acc[0] += u.x; acc[1] += u.y;
+            } else {
+                acc[0] += __ldcs(p);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < V; ++k) epi.one(i, c0 + k, acc[k]);
+    }
+}
+
 // Elementwise reverse step: gz = gx * [P does not clamp z], t = gz / D,
 // per-block partial sums of gz * g / D for every column (FP64).
 template <typename T, int NR>
-__global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T *gk, const T *D,
+__global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T *gk, const T *Di,
                                                   const T *lam, const T *gx, T *gz, T *t, int bmode,
                                                   T lb, T ub, double *partials) {
     __shared__ double sh[NR][8];
@@ -245,8 +284,8 @@ __global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T
         const int c = (int)(e % NR);
         T g = gk[e];
         T u = lam[c] * g;
-        T d = D ? D[j] : (T)1;
-        if (D) u = u / d;
+        T d = Di ? Di[j] : (T)1;
+        if (Di) u = u * d;
         T z = x[e] + u;
         bool pass = true;
         T zc = z;
@@ -254,8 +293,8 @@ __global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T
         if (bmode & 2) pass = pass && (zc > lb);
         T gzv = pass ? gx[e] : (T)0;
         gz[e] = gzv;
-        t[e] = D ? gzv / d : gzv;
-        part += (double)gzv * (double)(D ? g / d : g);
+        t[e] = Di ? gzv * d : gzv;
+        part += (double)gzv * (double)(Di ? g * d : g);
     }
     // reduce over the threads sharing a column: lanes c, c+NR, ... then warps
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -316,135 +355,130 @@ int mgrid(K kernel, int64_t m, int nr) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count() * occ, need));
 }
 
-struct AdjBufs {
-    DevBuf b, x, r, gk_seg, x_seg, cp, gx, gz, t, w, gb, lam, M, D, part;
-};
+// The handle's buffers (w_adj): kept between calls, each grown to what a call needs.
+enum AdjBuf { AB_B, AB_X, AB_R, AB_GSEG, AB_XSEG, AB_CP, AB_GX, AB_GZ, AB_T, AB_W, AB_GB, AB_LAM, AB_MI,
+              AB_DI, AB_PART, AB_STAGE, AB_SUM, AB_COUNT };
 
 template <typename T, int NR>
-int run_group(const DevCSR &A, const DevCSR &AT, const T *vA, const T *vAT, bool sart,
-              const double *h_b, const double *h_x0, const double *h_gx, const double *h_lam,
-              int nrhs, int c0, int ncols, int K, int bmode, double lb, double ub,
-              const double *d_M64, const double *d_D64, unsigned *sched, cudaStream_t s,
-              double *h_xK, double *h_gb, double *h_gx0, double *h_glam) {
+int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_b,
+              const double *h_x0, const double *h_gx, const double *h_lam, int nrhs, int c0,
+              int ncols, int K, int bmode, double lb, double ub, const double *d_Mi64,
+              const double *d_Di64, double *h_xK, double *h_gb, double *h_gx0, double *h_glam) {
+    DevCSR &A = h->A, &AT = h->AT;
+    cudaStream_t s = h->stream;
+    unsigned *sched = h->w_sched.as<unsigned>();
+    constexpr int prec = sizeof(T) == 8 ? FAIR_PREC_F64 : FAIR_PREC_F32;
     const int64_t m = A.m, n = A.n;
     const int C = K > 0 ? (int)std::ceil(std::sqrt((double)K)) : 1;
     const int nseg = K > 0 ? (K + C - 1) / C : 0;
-    AdjBufs B;
-    FAIR_TRY(B.b.grow(sizeof(T) * m * NR));
-    FAIR_TRY(B.r.grow(sizeof(T) * m * NR));
-    FAIR_TRY(B.w.grow(sizeof(T) * m * NR));
-    FAIR_TRY(B.gb.grow(sizeof(T) * m * NR));
-    FAIR_TRY(B.x.grow(sizeof(T) * n * NR));
-    FAIR_TRY(B.gx.grow(sizeof(T) * n * NR));
-    FAIR_TRY(B.gz.grow(sizeof(T) * n * NR));
-    FAIR_TRY(B.t.grow(sizeof(T) * n * NR));
-    FAIR_TRY(B.cp.grow(sizeof(T) * n * NR * (size_t)(nseg + 1)));
-    FAIR_TRY(B.x_seg.grow(sizeof(T) * n * NR * (size_t)C));
-    FAIR_TRY(B.gk_seg.grow(sizeof(T) * n * NR * (size_t)C));
-    FAIR_TRY(B.lam.grow(sizeof(T) * NR));
-    FAIR_TRY(B.M.grow(sizeof(T) * m));
-    FAIR_TRY(B.D.grow(sizeof(T) * n));
+    static_assert(AB_COUNT <= sizeof(h->w_adj) / sizeof(h->w_adj[0]), "adjoint buffers");
+    DevBuf *W = h->w_adj;
+    const bool tiled1 = tl_multi_ready(A, prec, 1), tiled2 = tl_multi_ready(AT, prec, 2);
     const int ge = egrid(n * NR);
-    FAIR_TRY(B.part.grow(sizeof(double) * (size_t)ge * NR));
-    // inputs
-    DevBuf stage;
-    FAIR_TRY(stage.grow(sizeof(double) * std::max<int64_t>(m, n) * ncols));
-    FAIR_CUDA(cudaMemcpyAsync(stage.p, h_b + (size_t)c0 * m, sizeof(double) * m * ncols,
-                              cudaMemcpyHostToDevice, s));
-    k_interleave<T><<<egrid(m * NR), 256, 0, s>>>(stage.as<double>(), m, ncols, NR, 0, B.b.as<T>());
-    if (h_x0) {
-        FAIR_CUDA(cudaMemcpyAsync(stage.p, h_x0 + (size_t)c0 * n, sizeof(double) * n * ncols,
-                                  cudaMemcpyHostToDevice, s));
-        k_interleave<T><<<egrid(n * NR), 256, 0, s>>>(stage.as<double>(), n, ncols, NR, 0, B.x.as<T>());
-    } else {
-        k_interleave<T><<<egrid(n * NR), 256, 0, s>>>(nullptr, n, ncols, NR, 0, B.x.as<T>());
-    }
-    FAIR_CUDA(cudaStreamSynchronize(s));  // stage reused below
-    FAIR_CUDA(cudaMemcpyAsync(stage.p, h_gx + (size_t)c0 * n, sizeof(double) * n * ncols,
-                              cudaMemcpyHostToDevice, s));
-    k_interleave<T><<<egrid(n * NR), 256, 0, s>>>(stage.as<double>(), n, ncols, NR, 0, B.gx.as<T>());
+    for (int q : {AB_B, AB_R, AB_W, AB_GB}) FAIR_TRY(W[q].grow(sizeof(T) * m * NR));
+    for (int q : {AB_X, AB_GX, AB_GZ, AB_T}) FAIR_TRY(W[q].grow(sizeof(T) * n * NR));
+    FAIR_TRY(W[AB_CP].grow(sizeof(T) * n * NR * (size_t)(nseg + 1)));
+    FAIR_TRY(W[AB_XSEG].grow(sizeof(T) * n * NR * (size_t)C));
+    FAIR_TRY(W[AB_GSEG].grow(sizeof(T) * n * NR * (size_t)C));
+    FAIR_TRY(W[AB_LAM].grow(sizeof(T) * NR));
+    FAIR_TRY(W[AB_MI].grow(sizeof(T) * m));
+    FAIR_TRY(W[AB_DI].grow(sizeof(T) * n));
+    FAIR_TRY(W[AB_SUM].grow(sizeof(double) * (size_t)ge * NR * (size_t)std::max(K, 1)));
+    const int64_t segs = std::max<int64_t>(tiled1 ? A.tlm.nseg : 0, tiled2 ? AT.tlm.nseg : 0);
+    FAIR_TRY(W[AB_PART].grow(sizeof(T) * NR * (size_t)segs));
+    FAIR_TRY(W[AB_STAGE].grow(sizeof(double) * std::max<int64_t>(m, n) * ncols));
+    T *b = W[AB_B].as<T>(), *x = W[AB_X].as<T>(), *r = W[AB_R].as<T>(), *gx = W[AB_GX].as<T>(),
+      *gz = W[AB_GZ].as<T>(), *t = W[AB_T].as<T>(), *w = W[AB_W].as<T>(), *gb = W[AB_GB].as<T>(),
+      *lam = W[AB_LAM].as<T>(), *Mi = W[AB_MI].as<T>();
+    double *stage = W[AB_STAGE].as<double>(), *sums = W[AB_SUM].as<double>();
+    const size_t nNR = (size_t)n * NR, vecb = sizeof(T) * nNR;
+    // inputs (stage is reused in stream order)
+    auto put = [&](const double *src, int64_t rows, T *dst) -> int {
+        if (src)
+            FAIR_CUDA(cudaMemcpyAsync(stage, src + (size_t)c0 * rows, sizeof(double) * rows * ncols,
+                                      cudaMemcpyHostToDevice, s));
+        k_interleave<T><<<egrid(rows * NR), 256, 0, s>>>(src ? stage : nullptr, rows, ncols, NR, 0, dst);
+        return FAIR_OK;
+    };
+    FAIR_TRY(put(h_b, m, b));
+    FAIR_TRY(put(h_x0, n, x));
+    FAIR_TRY(put(h_gx, n, gx));
     T lamh[NR];
     for (int c = 0; c < NR; ++c) lamh[c] = (T)(c < ncols ? h_lam[c0 + c] : 0.0);
-    FAIR_CUDA(cudaMemcpyAsync(B.lam.p, lamh, sizeof(lamh), cudaMemcpyHostToDevice, s));
-    k_cast<T><<<egrid(m), 256, 0, s>>>(d_M64, m, B.M.as<T>());
-    if (sart) k_cast<T><<<egrid(n), 256, 0, s>>>(d_D64, n, B.D.as<T>());
-    FAIR_CUDA(cudaMemsetAsync(B.gb.p, 0, sizeof(T) * m * NR, s));
+    FAIR_CUDA(cudaMemcpyAsync(lam, lamh, sizeof(lamh), cudaMemcpyHostToDevice, s));
+    k_cast<T><<<egrid(m), 256, 0, s>>>(d_Mi64, m, Mi);
+    if (sart) k_cast<T><<<egrid(n), 256, 0, s>>>(d_Di64, n, W[AB_DI].as<T>());
+    FAIR_CUDA(cudaMemsetAsync(gb, 0, sizeof(T) * m * NR, s));
     FAIR_CUDA(cudaGetLastError());
-    const T *D = sart ? B.D.as<T>() : nullptr;
+    const T *Di = sart ? W[AB_DI].as<T>() : nullptr;
     const T tlb = (T)lb, tub = (T)ub;
-    auto fwd_step = [&](T *gsave) -> int {
-        EpiFwdResid<T, NR> e1{B.b.as<T>(), B.M.as<T>(), B.r.as<T>()};
-        auto k1 = k_multi<T, NR, EpiFwdResid<T, NR>>;
-        k1<<<mgrid(k1, m, NR), 256, 0, s>>>(A.rowptr.as<int64_t>(), A.m, A.col.as<int32_t>(), vA,
-                                        B.x.as<T>(), e1, sched);
-        EpiFwdUpdate<T, NR> e2{D, B.lam.as<T>(), B.x.as<T>(), gsave, tlb, tub, bmode};
-        auto k2 = k_multi<T, NR, EpiFwdUpdate<T, NR>>;
-        k2<<<mgrid(k2, n, NR), 256, 0, s>>>(AT.rowptr.as<int64_t>(), AT.m, AT.col.as<int32_t>(), vAT,
-                                        B.r.as<T>(), e2, sched);
+    // epi(row, M v) over A (pass 1) or A' (pass 2)
+    auto product = [&](int pass, const T *v, const auto &epi) -> int {
+        using Epi = std::decay_t<decltype(epi)>;
+        DevCSR &M = pass == 1 ? A : AT;
+        if (pass == 1 ? tiled1 : tiled2) {
+            T *part = W[AB_PART].as<T>();
+            FAIR_TRY(tl_multi_partials(M, prec, NR, v, part, sched, s));
+            k_multi_rows<T, NR, Epi><<<egrid((int64_t)M.m * NR * 2), 256, 0, s>>>(
+                M.m, M.tlm.segbase.as<int64_t>(), part, epi);
+        } else {
+            auto k = k_multi<T, NR, Epi>;
+            k<<<mgrid(k, M.m, NR), 256, 0, s>>>(M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(),
+                                                pass == 1 ? vA : vAT, v, epi, sched);
+        }
         FAIR_CUDA(cudaGetLastError());
         return FAIR_OK;
     };
-    const size_t vecb = sizeof(T) * n * NR;
+    auto fwd_step = [&](T *gsave) -> int {
+        FAIR_TRY(product(1, x, EpiFwdResid<T, NR>{b, Mi, r}));
+        return product(2, r, EpiFwdUpdate<T, NR>{Di, lam, x, gsave, tlb, tub, bmode});
+    };
     // forward with checkpoints
     for (int k = 0; k < K; ++k) {
         if (k % C == 0)
-            FAIR_CUDA(cudaMemcpyAsync(B.cp.as<char>() + vecb * (k / C), B.x.p, vecb,
-                                      cudaMemcpyDeviceToDevice, s));
+            FAIR_CUDA(cudaMemcpyAsync(W[AB_CP].as<T>() + nNR * (k / C), x, vecb, cudaMemcpyDeviceToDevice, s));
         FAIR_TRY(fwd_step(nullptr));
     }
-    if (h_xK) {
-        k_deinterleave<T><<<egrid(n * ncols), 256, 0, s>>>(B.x.as<T>(), n, nrhs, NR, 0, ncols,
-                                                           stage.as<double>());
-        FAIR_CUDA(cudaMemcpyAsync(h_xK + (size_t)c0 * n, stage.p, sizeof(double) * n * ncols,
+    auto get = [&](const T *src, int64_t rows, double *dst) -> int {
+        k_deinterleave<T><<<egrid(rows * ncols), 256, 0, s>>>(src, rows, nrhs, NR, 0, ncols, stage);
+        FAIR_CUDA(cudaMemcpyAsync(dst + (size_t)c0 * rows, stage, sizeof(double) * rows * ncols,
                                   cudaMemcpyDeviceToHost, s));
         FAIR_CUDA(cudaStreamSynchronize(s));
-    }
-    // reverse, one segment at a time
-    std::vector<double> glam_acc(NR, 0.0), hpart((size_t)ge * NR);
+        return FAIR_OK;
+    };
+    if (h_xK) FAIR_TRY(get(x, n, h_xK));
+    // reverse, one segment at a time; the sums of glam stay on the device
     for (int seg = nseg - 1; seg >= 0; --seg) {
         const int k0 = seg * C, k1 = std::min(K, k0 + C);
-        FAIR_CUDA(cudaMemcpyAsync(B.x.p, B.cp.as<char>() + vecb * seg, vecb,
-                                  cudaMemcpyDeviceToDevice, s));
+        FAIR_CUDA(cudaMemcpyAsync(x, W[AB_CP].as<T>() + nNR * seg, vecb, cudaMemcpyDeviceToDevice, s));
         for (int k = k0; k < k1; ++k) {
-            FAIR_CUDA(cudaMemcpyAsync(B.x_seg.as<char>() + vecb * (k - k0), B.x.p, vecb,
+            FAIR_CUDA(cudaMemcpyAsync(W[AB_XSEG].as<T>() + nNR * (k - k0), x, vecb,
                                       cudaMemcpyDeviceToDevice, s));
-            FAIR_TRY(fwd_step((T *)(B.gk_seg.as<char>() + vecb * (k - k0))));
+            FAIR_TRY(fwd_step(W[AB_GSEG].as<T>() + nNR * (k - k0)));
         }
         for (int k = k1 - 1; k >= k0; --k) {
-            const T *xk = (const T *)(B.x_seg.as<char>() + vecb * (k - k0));
-            const T *gk = (const T *)(B.gk_seg.as<char>() + vecb * (k - k0));
-            k_adj_mask<T, NR><<<ge, 256, 0, s>>>(n, xk, gk, D, B.lam.as<T>(), B.gx.as<T>(),
-                                                 B.gz.as<T>(), B.t.as<T>(), bmode, tlb, tub,
-                                                 B.part.as<double>());
+            const T *xk = W[AB_XSEG].as<T>() + nNR * (k - k0);
+            const T *gk = W[AB_GSEG].as<T>() + nNR * (k - k0);
+            k_adj_mask<T, NR><<<ge, 256, 0, s>>>(n, xk, gk, Di, lam, gx, gz, t, bmode, tlb, tub,
+                                                 sums + (size_t)k * ge * NR);
             FAIR_CUDA(cudaGetLastError());
-            FAIR_CUDA(cudaMemcpyAsync(hpart.data(), B.part.p, sizeof(double) * ge * NR,
-                                      cudaMemcpyDeviceToHost, s));
-            EpiAdjA<T, NR> ea{B.M.as<T>(), B.lam.as<T>(), B.w.as<T>(), B.gb.as<T>()};
-            auto ka = k_multi<T, NR, EpiAdjA<T, NR>>;
-            ka<<<mgrid(ka, m, NR), 256, 0, s>>>(A.rowptr.as<int64_t>(), A.m, A.col.as<int32_t>(), vA,
-                                            B.t.as<T>(), ea, sched);
-            EpiAdjAT<T, NR> eb{B.gz.as<T>(), B.lam.as<T>(), B.gx.as<T>()};
-            auto kb = k_multi<T, NR, EpiAdjAT<T, NR>>;
-            kb<<<mgrid(kb, n, NR), 256, 0, s>>>(AT.rowptr.as<int64_t>(), AT.m, AT.col.as<int32_t>(),
-                                            vAT, B.w.as<T>(), eb, sched);
-            FAIR_CUDA(cudaGetLastError());
-            FAIR_CUDA(cudaStreamSynchronize(s));
-            for (int bl = 0; bl < ge; ++bl)
-                for (int c = 0; c < NR; ++c) glam_acc[c] += hpart[(size_t)bl * NR + c];
+            FAIR_TRY(product(1, t, EpiAdjA<T, NR>{Mi, lam, w, gb}));
+            FAIR_TRY(product(2, w, EpiAdjAT<T, NR>{gz, lam, gx}));
         }
     }
     // outputs
-    k_deinterleave<T><<<egrid(m * ncols), 256, 0, s>>>(B.gb.as<T>(), m, nrhs, NR, 0, ncols,
-                                                       stage.as<double>());
-    FAIR_CUDA(cudaMemcpyAsync(h_gb + (size_t)c0 * m, stage.p, sizeof(double) * m * ncols,
-                              cudaMemcpyDeviceToHost, s));
-    FAIR_CUDA(cudaStreamSynchronize(s));
-    k_deinterleave<T><<<egrid(n * ncols), 256, 0, s>>>(B.gx.as<T>(), n, nrhs, NR, 0, ncols,
-                                                       stage.as<double>());
-    FAIR_CUDA(cudaMemcpyAsync(h_gx0 + (size_t)c0 * n, stage.p, sizeof(double) * n * ncols,
-                              cudaMemcpyDeviceToHost, s));
-    FAIR_CUDA(cudaStreamSynchronize(s));
-    for (int c = 0; c < ncols; ++c) h_glam[c0 + c] = glam_acc[c];
+    FAIR_TRY(get(gb, m, h_gb));
+    FAIR_TRY(get(gx, n, h_gx0));
+    std::vector<double> hsum((size_t)ge * NR * K);
+    if (K > 0) {
+        FAIR_CUDA(cudaMemcpyAsync(hsum.data(), sums, sizeof(double) * hsum.size(), cudaMemcpyDeviceToHost, s));
+        FAIR_CUDA(cudaStreamSynchronize(s));
+    }
+    double acc[NR] = {};
+    for (int k = K - 1; k >= 0; --k)
+        for (int bl = 0; bl < ge; ++bl)
+            for (int c = 0; c < NR; ++c) acc[c] += hsum[((size_t)k * ge + bl) * NR + c];
+    for (int c = 0; c < ncols; ++c) h_glam[c0 + c] = acc[c];
     return FAIR_OK;
 }
 
@@ -457,30 +491,31 @@ int sirt_adjoint(fair_csr h, bool sart, int nrhs, const double *b, const double 
     cudaStream_t s = h->stream;
     FAIR_TRY(h->w_M.grow(sizeof(double) * ((size_t)A.m + 1)));
     FAIR_TRY(h->w_D.grow(sizeof(double) * ((size_t)A.n + 1)));
-    FAIR_TRY(sirt_weights(A, AT, sart, h->w_M.as<double>(), h->w_D.as<double>(), s));
+    FAIR_TRY(sirt_weights_recip(A, AT, sart, h->w_M.as<double>(), h->w_D.as<double>(), s));
     const bool f32 = h->prec == FAIR_PREC_F32;
     if (f32) {
         FAIR_TRY(csr_make_lowprec(A, FAIR_PREC_F32, s));
         FAIR_TRY(csr_make_lowprec(AT, FAIR_PREC_F32, s));
     }
-    unsigned *sched = h->w_sched.as<unsigned>();
+    // the tiled copies of the products (left unbuilt for matrices without an image)
+    FAIR_TRY(csr_make_tiled_multi(A, h->prec, 1, s));
+    FAIR_TRY(csr_make_tiled_multi(AT, h->prec, 2, s));
     for (int c0 = 0; c0 < nrhs; c0 += 16) {
         const int nc = std::min(16, nrhs - c0);
-        const int NRt = nc == 1 ? 1 : (nc <= 4 ? 4 : 16);
-#define FAIR_ADJ_GROUP(T, NRC, VA, VAT)                                                          \
-    run_group<T, NRC>(A, AT, VA, VAT, sart, b, x0, gx, lam, nrhs, c0, nc, K, bmode, lb, ub,      \
-                      h->w_M.as<double>(), h->w_D.as<double>(), sched, s, xK, gb, gx0, glam)
+        auto group = [&](auto nr) -> int {
+            constexpr int NR = decltype(nr)::value;
+            const double *Mi = h->w_M.as<double>(), *Di = h->w_D.as<double>();
+            if (f32)
+                return run_group<float, NR>(h, A.v32.as<float>(), AT.v32.as<float>(), sart, b, x0, gx, lam,
+                                            nrhs, c0, nc, K, bmode, lb, ub, Mi, Di, xK, gb, gx0, glam);
+            return run_group<double, NR>(h, A.v64.as<double>(), AT.v64.as<double>(), sart, b, x0, gx, lam,
+                                         nrhs, c0, nc, K, bmode, lb, ub, Mi, Di, xK, gb, gx0, glam);
+        };
         int st;
-        if (f32) {
-            const float *va = A.v32.as<float>(), *vt = AT.v32.as<float>();
-            st = NRt == 1 ? FAIR_ADJ_GROUP(float, 1, va, vt)
-                 : NRt == 4 ? FAIR_ADJ_GROUP(float, 4, va, vt) : FAIR_ADJ_GROUP(float, 16, va, vt);
-        } else {
-            const double *va = A.v64.as<double>(), *vt = AT.v64.as<double>();
-            st = NRt == 1 ? FAIR_ADJ_GROUP(double, 1, va, vt)
-                 : NRt == 4 ? FAIR_ADJ_GROUP(double, 4, va, vt) : FAIR_ADJ_GROUP(double, 16, va, vt);
-        }
-#undef FAIR_ADJ_GROUP
+        if (nc == 1) st = group(std::integral_constant<int, 1>());
+        else if (nc <= 4) st = group(std::integral_constant<int, 4>());
+        else if (nc <= 8) st = group(std::integral_constant<int, 8>());
+        else st = group(std::integral_constant<int, 16>());
         if (st) return st;
     }
     return FAIR_OK;

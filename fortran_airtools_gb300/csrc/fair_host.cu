@@ -76,6 +76,12 @@ void DevCSR::Tiled::release() {
     L6 = 5;
     nslots6 = nesc6 = 0;
     tried6 = built6 = has6_16 = has6_q = false;
+    for (MvUnits &m : mv) {
+        m.units.release();
+        m.n = 0;
+    }
+    hchunk.clear();
+    hsoff.clear();
     T = N = ntr = 0;
     nseg = nchunks = nslots = 0;
     nunits = 0;
@@ -95,6 +101,7 @@ void DevCSR::Delta::release() {
 void DevCSR::release() {
     drop_sliced();
     tl.release();
+    tlm.release();
     dl[0].release();
     dl[1].release();
     rowptr.release(); col.release(); v64.release(); v32.release(); v16.release(); vq.release();
@@ -315,6 +322,7 @@ int fair_csr_destroy(fair_csr h) {
                       &h->w_D, &h->w_xn, &h->w_tmp, &h->w_part, &h->w_flag, &h->w_ord,
                       &h->w_cumul, &h->w_nrA, &h->w_y, &h->s_M, &h->s_D, &h->s_r, &h->s_x32, &h->w_sched};
     for (DevBuf *b : bufs) b->release();
+    for (DevBuf &b : h->w_adj) b.release();
     h->w_sweep.release();
     if (h->own_stream) cudaStreamDestroy(h->stream);
     delete h;

@@ -140,9 +140,17 @@ struct DevCSR {
         bool has6_16 = false, has6_q = false;
         bool has_idx = false, has_v64 = false, has_v32 = false, has_r16 = false, has_rq = false;
         DevBuf part;      // partial sums [nseg] (8 bytes each)
+        // the multi-vector products' work units per lanes per entry (1, 2, 4, 8)
+        struct MvUnits {
+            DevBuf units;
+            int32_t n = 0;
+        } mv[4];
+        std::vector<int32_t> hchunk;  // first chunk of each tile (host)
+        std::vector<int64_t> hsoff;   // soff (host, read by mv_units)
         bool built() const { return T > 0; }
         void release();
     } tl;
+    Tiled tlm;  // the tiled copy of the multi-vector products (the adjoint)
     // Delta copies (sirt_delta.cu): the sliced layout with one lane per row
     // whose slots carry column steps from the row's previous entry instead of
     // columns (the row's first column is its anchor). dl[0]: 4 entries per
@@ -259,6 +267,13 @@ void sirt_pass(const SirtDev &S, int pass, cudaStream_t s);
 // an N x N image and whose columns rays of p bins per angle (p = its stride
 // hint). Does nothing for other matrices.
 int csr_make_tiled(DevCSR &A, int prec, int pass, cudaStream_t s);
+// The tiled copy of the products with nr interleaved vectors (adjoint.cu;
+// pass as above), and its partial sums: part[segment][nr] from x[column][nr],
+// nr = 1, 4, 8 or 16 (FP64 or FP32), segments in row order (M.tlm.segbase).
+int csr_make_tiled_multi(DevCSR &A, int prec, int pass, cudaStream_t s);
+bool tl_multi_ready(const DevCSR &M, int prec, int pass);
+int tl_multi_partials(DevCSR &M, int prec, int nr, const void *x, void *part, unsigned *ctr,
+                      cudaStream_t s);
 // The tile shape csr_make_tiled uses for M in `pass` (the request or the
 // default): tile side and (pass 2) residual cells per tile.
 void tiled_shape(const DevCSR &M, int pass, int *side, int *cells);
@@ -443,6 +458,7 @@ struct fair_csr_s {
     // work buffers reused across calls
     fair::DevBuf w_in, w_out, w_b, w_x, w_x32, w_r, w_M, w_D, w_xn, w_tmp, w_part, w_flag;
     fair::DevBuf w_ord, w_cumul, w_nrA, w_y;
+    fair::DevBuf w_adj[19];  // the adjoint's vectors, kept between calls
     fair::DevBuf w_sched;  // two zeroed counters for dynamic chunk scheduling
     fair::SweepWork w_sweep;  // Kaczmarz sweep buffers (released after each call)
     // state of fair_sirt_prepare (device-resident SIRT)

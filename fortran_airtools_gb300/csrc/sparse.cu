@@ -580,6 +580,7 @@ int csr_scale(DevCSR &A, double c, cudaStream_t s) {
     A.hassv64 = A.hassv32 = A.hassf16 = A.hassfq = false;
     A.tl.has_v64 = A.tl.has_v32 = A.tl.has_r16 = A.tl.has_rq = false;
     A.tl.has6_16 = A.tl.has6_q = false;
+    A.tlm.has_v64 = A.tlm.has_v32 = false;
     for (auto &d : A.dl) d.has_v64 = d.has_v32 = d.has_r16 = d.has_rq = false;
     return FAIR_OK;
 }

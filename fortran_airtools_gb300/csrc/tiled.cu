@@ -844,8 +844,7 @@ void launch_tl(const DevCSR &M, int code, const LD &ldr, const XT *x, const Epi 
 }
 
 // Index part of the 6-entry step records (after the tiled copy is built).
-int t6_build(DevCSR &A, cudaStream_t s) {
-    DevCSR::Tiled &tl = A.tl;
+int t6_build(DevCSR &A, DevCSR::Tiled &tl, cudaStream_t s) {
     const int64_t nch = tl.nchunks;
     TmpBuf cnt, esc;
     FAIR_TRY(cnt.grow(sizeof(int32_t) * (nch + 1)));
@@ -912,12 +911,23 @@ void tiled_shape(const DevCSR &M, int pass, int *side, int *cells) {
     *cells = pass == 1 ? 0 : (M.tile_req[1] > 0 ? M.tile_req[1] : kPixCells);
 }
 
+static int tl_make(DevCSR &A, DevCSR::Tiled &tl, int prec, int pass, int want_T, int want_cells,
+                   cudaStream_t s);
+
 int csr_make_tiled(DevCSR &A, int prec, int pass, cudaStream_t s) {
+    int T = 0, cells = 0;
+    tiled_shape(A, pass, &T, &cells);
+    FAIR_TRY(tl_make(A, A.tl, prec, pass, T, cells, s));
+    if (A.tl.built()) FAIR_TRY(A.tl.part.grow(sizeof(double) * A.tl.nseg));
+    return FAIR_OK;
+}
+
+// The tiled copy tl of A for `pass`, with tiles of side want_T and (pass 2)
+// at most want_cells cells.
+static int tl_make(DevCSR &A, DevCSR::Tiled &tl, int prec, int pass, int want_T, int want_cells,
+                   cudaStream_t s) {
     if (A.m == 0 || A.nnz == 0) return FAIR_OK;
-    DevCSR::Tiled &tl = A.tl;
     const int kind = pass == 1 ? 0 : 1;
-    int want_T = 0, want_cells = 0;
-    tiled_shape(A, pass, &want_T, &want_cells);
     if (tl.built() && (tl.kind != kind || tl.T != want_T || (kind == 1 && tl.cells_cap != want_cells)))
         tl.release();
     if (!tl.built()) {
@@ -1036,6 +1046,9 @@ int csr_make_tiled(DevCSR &A, int prec, int pass, cudaStream_t s) {
                 units.push_back(make_int4((int)t, (int)c, (int)std::min<int64_t>(c + per_unit, c1), 0));
             c0 = c1;
         }
+        tl.hchunk.assign((size_t)ntiles + 1, 0);
+        for (int64_t t = 0; t < ntiles; ++t)
+            tl.hchunk[t + 1] = tl.hchunk[t] + (int32_t)(((int64_t)ho[(t + 1) * LB] - (int64_t)ho[t * LB] + 31) / 32);
         // most work first: units of longer segments lead within a tile already
         const int64_t nch = (int64_t)chunks.size();
         TmpBuf dch, ccnt;
@@ -1072,7 +1085,6 @@ int csr_make_tiled(DevCSR &A, int prec, int pass, cudaStream_t s) {
             tl.send.as<int64_t>(), tl.srow.as<int32_t>(), A.col.as<int32_t>(), G, tl.idx.as<uint2>(),
             PutNone{});
         FAIR_CUDA(cudaGetLastError());
-        FAIR_TRY(tl.part.grow(sizeof(double) * S));
         tl.kind = G.kind;
         tl.T = G.T;
         tl.N = G.N;
@@ -1122,7 +1134,7 @@ int csr_make_tiled(DevCSR &A, int prec, int pass, cudaStream_t s) {
     if (prec == FAIR_PREC_F16 || prec == FAIR_PREC_Q16) {  // the 6-entry step records
         if (!tl.tried6) {
             tl.tried6 = true;
-            FAIR_TRY(t6_build(A, s));
+            FAIR_TRY(t6_build(A, tl, s));
         }
         const bool h = prec == FAIR_PREC_F16;
         if (tl.built6 && !(h ? tl.has6_16 : tl.has6_q)) {
@@ -1195,6 +1207,282 @@ bool sirt_pass_tiled(const SirtDev &S, const DevCSR &M, int pass, int code, cuda
     if (!tl.has_rq) return false;
     if (M.qsigned) return run(TlFused<int16_t>{tl.rq.as<uint4>()});
     return run(TlFused<uint16_t>{tl.rq.as<uint4>()});
+}
+
+// ---- several right-hand sides (the adjoint) -----------------------------------
+// The tiled copies with NR interleaved vectors: the tile's shared copy holds
+// NR values per cell, LPE lanes share a segment (16 bytes of a cell each, 16
+// contiguous bytes per lane and entry), so that a warp step works on 32 / LPE
+// segments of a chunk. Gathering the NR values of each entry from global
+// memory instead cost an L2 round trip of NR x sizeof(T) bytes per nonzero
+// (N = 256, 16 right-hand sides, FP32: 270-290 us per product, 7.5 TB/s out of
+// L2); here 134 us, bound by the shared-memory reads: 64 bytes per nonzero, 1.3
+// wavefronts per 128 bytes (two cells of one parity share banks). FP64 is
+// bound by its pipe (66% busy at 4 right-hand sides). 384 threads: 16-byte
+// shares leave 56 registers for 36 warps per SM (512 threads at 40 spilled).
+// The partials are NR values per segment, in row order.
+namespace {
+
+constexpr int kMvTile = 32;            // image tile and pixel tile side
+constexpr int kMvCells = 32 * 33;      // most residual cells of a tile of A'
+constexpr int kMvThreads = 384;
+
+template <typename T, int NR> struct MvCfg {
+    static constexpr int CB = NR * (int)sizeof(T);       // bytes per cell
+    static constexpr int LPE = CB > 16 ? CB / 16 : 1;    // lanes per entry
+    static constexpr int VPL = NR / LPE;                 // values per lane
+    static constexpr int SPW = 32 / LPE;                 // segments per warp step
+    static constexpr int CTAS = sizeof(T) == 8 ? 2 : 3;   // register budget: 80 or 56
+};
+
+template <typename T, int V> __device__ __forceinline__ void mv_load(const unsigned char *p, T (&o)[V]) {
+    if constexpr (V * sizeof(T) == 16) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(p);
+        if constexpr (sizeof(T) == 4) {
+            o[0] = __uint_as_float(u.x); o[1] = __uint_as_float(u.y);
+            o[2] = __uint_as_float(u.z); o[3] = __uint_as_float(u.w);
+        } else {
+            o[0] = __hiloint2double((int)u.y, (int)u.x);
+            o[1] = __hiloint2double((int)u.w, (int)u.z);
+        }
+    } else {
+        static_assert(V == 1, "16 bytes or one value per lane");
+        o[0] = *reinterpret_cast<const T *>(p);
+    }
+}
+
+__device__ __forceinline__ void cp_async16(unsigned dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+// The tile's copy: NR values per cell, 16 bytes per asynchronous copy.
+template <typename T, int NR>
+__device__ __forceinline__ void mv_fill_tile(const TlGeo &G, int4 U, const T *__restrict__ x,
+                                             unsigned char *xs) {
+    using C = MvCfg<T, NR>;
+    constexpr int CPC = C::CB / 16, VPC = 16 / (int)sizeof(T);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const unsigned base = (unsigned)__cvta_generic_to_shared(xs);
+    // `cells` consecutive cells from cell c0, the first `in` of them from src
+    auto run = [&](int c0, int cells, int in, const T *src) {
+        for (int e = lane; e < cells * CPC; e += 32) {
+            const unsigned d = (unsigned)(c0 * CPC + e) * 16u;
+            if (e < in * CPC) cp_async16(base + d, src + (size_t)e * VPC);
+            else *reinterpret_cast<uint4 *>(xs + d) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    if (G.kind == 0) {
+        const int tc = U.x / G.ntr, tr = U.x - tc * G.ntr, gr = tr * G.T;
+        for (int lc = wid; lc < G.T; lc += nw) {
+            const int gc = tc * G.T + lc;
+            const int in = gc < G.N ? max(0, min(G.T, G.N - gr)) : 0;
+            run(lc * (G.T + 1), G.T, in, x + ((size_t)gc * G.N + gr) * NR);
+        }
+    } else {
+        const int pt = U.x / G.nab, a0 = (U.x - pt * G.nab) * G.NA;
+        for (int ai = wid; ai < G.NA; ai += nw) {
+            const int a = a0 + ai;
+            const int b = a < G.nth ? __ldg(G.bmin + (int64_t)pt * G.nth + a) : 0;
+            const int in = a < G.nth ? max(0, min(G.W, G.p - b)) : 0;
+            run(ai * G.W, G.W, in, x + ((size_t)a * G.p + b) * NR);
+        }
+    }
+    if (threadIdx.x < CPC)  // the zero cell
+        *reinterpret_cast<uint4 *>(xs + ((size_t)G.cells() * CPC + threadIdx.x) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    cp_async_wait_all();
+}
+
+template <typename T, int NR>
+__global__ void __launch_bounds__(kMvThreads, (MvCfg<T, NR>::CTAS)) k_tlm_partials(
+        TlArgs P, const uint2 *__restrict__ idx, const T *__restrict__ val,
+        const T *__restrict__ x, T *__restrict__ part, unsigned *ctr) {
+    using C = MvCfg<T, NR>;
+    extern __shared__ __align__(16) unsigned char tl_smem[];
+    __shared__ int s_unit;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int sl = lane / C::LPE, sub = lane % C::LPE;  // segment of the step, lane of the segment
+    const unsigned char *xl = tl_smem + sub * 16;
+    struct Raw {
+        uint2 w;
+        VBlk<T> v;
+    };
+    auto load = [&](int64_t j) {
+        Raw r;
+        r.w = ld_stream(idx + j);
+        r.v.ld(val + 4 * j);
+        return r;
+    };
+    for (;;) {
+        if (threadIdx.x == 0) s_unit = (int)atomicAdd(ctr, 1u);
+        __syncthreads();
+        const int u = s_unit;
+        if (u >= P.nunits) break;
+        const int4 U = P.units[u];
+        if constexpr (C::CB >= 16) mv_fill_tile<T, NR>(P.G, U, x, tl_smem);
+        else tl_fill_tile(P.G, U, x, reinterpret_cast<T *>(tl_smem));
+        // items of the unit: (chunk, group of SPW of its segments)
+        const int nitems = (U.z - U.y) * C::LPE;
+        struct Item {
+            int64_t s0;
+            int len, ps;
+        };
+        auto item = [&](int it) {
+            Item r{0, 0, -1};
+            if (it < nitems) {
+                const int c = U.y + it / C::LPE, l = (it % C::LPE) * C::SPW + sl;
+                const int64_t o = __ldg(P.soff + c);
+                r.s0 = o + l;
+                r.len = (int)((__ldg(P.soff + c + 1) - o) >> 5);
+                r.ps = __ldg(P.pslot + (int64_t)c * 32 + l);
+            }
+            return r;
+        };
+        // two slots in flight: an item's first two are loaded during the one
+        // before (the first item's while the tile arrives)
+        Item cur = item(wid), nxt = item(wid + nw);
+        auto fetch = [&](Raw &r, int q) {  // slot q of cur, or past its end of nxt
+            if (q < cur.len) r = load(cur.s0 + 32 * (int64_t)q);
+            else if (q - cur.len < nxt.len) r = load(nxt.s0 + 32 * (int64_t)(q - cur.len));
+        };
+        Raw r0, r1;
+        if (0 < cur.len) r0 = load(cur.s0);
+        if (1 < cur.len) r1 = load(cur.s0 + 32);
+        __syncthreads();
+        for (int it = wid; it < nitems; it += nw) {
+            T acc[C::VPL];
+#pragma unroll
+            for (int k = 0; k < C::VPL; ++k) acc[k] = 0;
+            auto slot = [&](const Raw &w) {
+                const uint32_t li[4] = {w.w.x & 0xFFFFu, w.w.x >> 16, w.w.y & 0xFFFFu, w.w.y >> 16};
+                T v[4], xv[4][C::VPL];
+                w.v.to(v);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) mv_load<T, C::VPL>(xl + li[q] * (unsigned)C::CB, xv[q]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int k = 0; k < C::VPL; ++k) acc[k] += v[q] * xv[q][k];
+            };
+            int t = 0;
+            for (; t + 2 <= cur.len; t += 2) {
+                Raw w = r0;
+                fetch(r0, t + 2);
+                slot(w);
+                w = r1;
+                fetch(r1, t + 3);
+                slot(w);
+            }
+            if (t < cur.len) {  // an odd last slot: nxt's slot 0 is in r1
+                const Raw w = r0;
+                if (cur.len > 1) {
+                    r0 = r1;
+                    fetch(r1, t + 2);
+                } else {  // a single slot: nothing of nxt is loaded yet
+                    if (0 < nxt.len) r0 = load(nxt.s0);
+                    if (1 < nxt.len) r1 = load(nxt.s0 + 32);
+                }
+                slot(w);
+            }
+            const Item aft = item(it + 2 * nw);
+            if (cur.ps >= 0) {
+                T *o = part + (size_t)cur.ps * NR + sub * C::VPL;
+                if constexpr (C::VPL * sizeof(T) == 16 && sizeof(T) == 4)
+                    *reinterpret_cast<float4 *>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                else if constexpr (C::VPL * sizeof(T) == 16)
+                    *reinterpret_cast<double2 *>(o) = make_double2(acc[0], acc[1]);
+                else o[0] = acc[0];
+            }
+            cur = nxt;
+            nxt = aft;
+        }
+        __syncthreads();  // the tile is rewritten by the next unit
+    }
+    if (threadIdx.x == 0) {
+        const unsigned done = atomicAdd(ctr + 1, 1u);
+        if (done == gridDim.x - 1) {  // every CTA has stopped taking units
+            ctr[0] = 0u;
+            ctr[1] = 0u;
+        }
+    }
+}
+
+// The work units of the products with LPE lanes per entry: whole rounds of the
+// CTA's warps (one item each), about 6 units per resident CTA (fewer leaves a
+// tail, more reloads the tile too often: a fill costs about one chunk),
+// longest first.
+int mv_units(DevCSR::Tiled &tl, int lpe, int nctas, cudaStream_t s) {
+    DevCSR::Tiled::MvUnits &mu = tl.mv[lpe == 1 ? 0 : lpe == 2 ? 1 : lpe == 4 ? 2 : 3];
+    if (mu.n > 0) return FAIR_OK;
+    if (tl.hsoff.empty()) {
+        tl.hsoff.resize((size_t)tl.nchunks + 1);
+        FAIR_CUDA(cudaMemcpyAsync(tl.hsoff.data(), tl.soff.p, sizeof(int64_t) * (tl.nchunks + 1),
+                                  cudaMemcpyDeviceToHost, s));
+        FAIR_CUDA(cudaStreamSynchronize(s));
+    }
+    const int warps = kMvThreads / 32, round = std::max(1, warps / lpe);  // chunks of a round
+    int64_t per = tl.nchunks / ((int64_t)nctas * 6) / round * round;
+    per = std::max<int64_t>(round, std::min<int64_t>(per, round * 16));
+    std::vector<int4> units;
+    for (size_t t = 0; t + 1 < tl.hchunk.size(); ++t)
+        for (int64_t c = tl.hchunk[t]; c < tl.hchunk[t + 1]; c += per)
+            units.push_back(make_int4((int)t, (int)c, (int)std::min<int64_t>(c + per, tl.hchunk[t + 1]), 0));
+    std::stable_sort(units.begin(), units.end(), [&](const int4 &a, const int4 &b) {
+        return tl.hsoff[a.z] - tl.hsoff[a.y] > tl.hsoff[b.z] - tl.hsoff[b.y];
+    });
+    FAIR_TRY(mu.units.grow(sizeof(int4) * std::max<size_t>(units.size(), 1)));
+    FAIR_CUDA(cudaMemcpyAsync(mu.units.p, units.data(), sizeof(int4) * units.size(), cudaMemcpyHostToDevice, s));
+    FAIR_CUDA(cudaStreamSynchronize(s));
+    mu.n = (int32_t)units.size();
+    return FAIR_OK;
+}
+
+template <typename T, int NR>
+int mv_run(DevCSR::Tiled &tl, const T *val, const T *x, T *part, unsigned *ctr, cudaStream_t s) {
+    using C = MvCfg<T, NR>;
+    const TlGeo G = tl_geo(tl);
+    const size_t smem = ((size_t)G.cells() + 1) * C::CB;
+    auto kernel = k_tlm_partials<T, NR>;
+    FAIR_CUDA(smem_allow(reinterpret_cast<const void *>(kernel), smem));
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kMvThreads, smem);
+    const int nctas = sm_count() * std::max(occ, 1);
+    FAIR_TRY(mv_units(tl, C::LPE, nctas, s));
+    const DevCSR::Tiled::MvUnits &mu = tl.mv[C::LPE == 1 ? 0 : C::LPE == 2 ? 1 : C::LPE == 4 ? 2 : 3];
+    const TlArgs P{tl.soff.as<int64_t>(), tl.pslot.as<int32_t>(), mu.units.as<int4>(), mu.n, G};
+    kernel<<<std::max(1, std::min(nctas, (int)mu.n)), kMvThreads, smem, s>>>(P, tl.idx.as<uint2>(), val, x,
+                                                                            part, ctr);
+    FAIR_CUDA(cudaGetLastError());
+    return FAIR_OK;
+}
+
+template <typename T>
+int mv_dispatch(DevCSR::Tiled &tl, int nr, const T *val, const T *x, T *part, unsigned *ctr,
+                cudaStream_t s) {
+    switch (nr) {
+        case 1: return mv_run<T, 1>(tl, val, x, part, ctr, s);
+        case 4: return mv_run<T, 4>(tl, val, x, part, ctr, s);
+        case 8: return mv_run<T, 8>(tl, val, x, part, ctr, s);
+        default: return mv_run<T, 16>(tl, val, x, part, ctr, s);
+    }
+}
+
+}  // namespace
+
+int csr_make_tiled_multi(DevCSR &A, int prec, int pass, cudaStream_t s) {
+    return tl_make(A, A.tlm, prec, pass, kMvTile, kMvCells, s);
+}
+
+bool tl_multi_ready(const DevCSR &M, int prec, int pass) {
+    const DevCSR::Tiled &tl = M.tlm;
+    return tl.built() && tl.kind == (pass == 1 ? 0 : 1) && (prec == FAIR_PREC_F64 ? tl.has_v64 : tl.has_v32);
+}
+
+int tl_multi_partials(DevCSR &M, int prec, int nr, const void *x, void *part, unsigned *ctr,
+                      cudaStream_t s) {
+    DevCSR::Tiled &tl = M.tlm;
+    if (prec == FAIR_PREC_F64)
+        return mv_dispatch<double>(tl, nr, tl.v64.as<double>(), (const double *)x, (double *)part, ctr, s);
+    return mv_dispatch<float>(tl, nr, tl.v32.as<float>(), (const float *)x, (float *)part, ctr, s);
 }
 
 // ---- batches: the tiled passes of many problems in one launch ---------------
