@@ -18,6 +18,23 @@
 // Every product, sum and quotient on the ray uses explicit round-to-nearest
 // intrinsics so that no multiply-add is fused: the results then match the
 // reference's separately rounded operations bit for bit.
+//
+// This part runs 2 FP64 lanes per clock and SM, so the FP64 operations per
+// nonzero set the time (about 50 in each pass of the merge above). Almost
+// every ray stays clear of the grid's corners and lines, and on those the
+// integer units do the rest (the plain path):
+//  * the in-box crossings of both families are index intervals, so a ray's
+//    count is their number less one. The count pass checks in fixed point
+//    that every crossing of the ray's major axis is at least 2^-28 off the
+//    other family's lines; a ray that is not (or has a or b = 0) is listed
+//    and takes the merge (or exact) path in both passes;
+//  * the fill merges by integer comparison of the keys' bits, takes the
+//    columns from the cells' indices, and forms the quotient and the root with
+//    one and three FP64 operations, rounded correctly by their exact integer
+//    remainders: 13 FP64 operations per nonzero.
+// N = 256, 360 angles, 362 bins (33.4M nonzeros): count 3.2 -> 0.04 ms, fill
+// 3.8 -> 1.03 ms (FP64 pipe 83% busy), the listed rays 0.03 ms.
+#include <algorithm>
 #include <vector>
 
 #include "fair_internal.cuh"
@@ -285,20 +302,297 @@ __device__ int64_t trace_exact(const GeomDev &G, const Ray &r, RayScratch s, Sin
     return cnt;
 }
 
-__global__ void k_geom_count(GeomDev G, int32_t *counts, int32_t *special, int32_t *nspecial) {
-    int64_t m = (int64_t)G.nth * G.p;
+// ---- the plain path ----------------------------------------------------------
+__device__ __forceinline__ long long key_of(double t) {  // order-preserving for numbers
+    const long long b = __double_as_longlong(t);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+
+__device__ __noinline__ double div_slow(double n, double a) { return __ddiv_rn(n, a); }
+__device__ __noinline__ double sqrt_slow(double v) { return __dsqrt_rn(v); }
+
+// The cell of a segment by its midpoint (:200-203). Rare operations are calls:
+// inlined they would be predicated, and an FP64 instruction holds its pipe for
+// 64 cycles whether or not a lane executes it.
+__device__ __noinline__ int mid_cell(double p0, double p1, int N) {
+    return (int)floor(__dmul_rn(0.5, __dadd_rn(__dadd_rn(p0, p1), (double)N)));
+}
+
+// n / a rounded to nearest, y = 1/a rounded to nearest. q = n y is within 1.5
+// units in the last place (half a unit from the product, up to one from y);
+// the remainder n - a q in units of ulp(a) ulp(q) is below 2^55, so its low 64
+// bits give it exactly, and the quotient is the neighbour that leaves at most
+// |a|/2 (no quotient of two doubles lies half way between doubles). Zero, a
+// result at a power of two from below and exponents off the usual two go to
+// the division itself.
+__device__ __forceinline__ double div_by(double n, double a, double y) {
+    const unsigned long long M52 = 1ull << 52, mask = M52 - 1;
+    const double q = __dmul_rn(n, y);
+    const unsigned long long nb = __double_as_longlong(n), ab = __double_as_longlong(a),
+                             qb = __double_as_longlong(q);
+    const unsigned long long mn = (nb & mask) | M52, ma = (ab & mask) | M52, mq = (qb & mask) | M52;
+    const int en = (int)(nb >> 52) & 0x7ff, ea = (int)(ab >> 52) & 0x7ff, eq = (int)(qb >> 52) & 0x7ff;
+    const int sh = en - ea - eq + 1075;
+    const long long R = (long long)((mn << (sh & 63)) - ma * mq);
+    const long long R2 = 2 * R, A = (long long)ma;
+    if ((unsigned)(sh - 51) > 3u || eq == 0 || (mq == M52 && R < 0)) return div_slow(n, a);
+    const int k = (R2 > A ? 1 : 0) - (R2 < -A ? 1 : 0);
+    return __longlong_as_double((long long)qb + k);
+}
+
+// sqrt(v) rounded to nearest, s0 close to it (the difference of the ray
+// parameters): one Newton step with a 22-bit 1/(2 s0), then the neighbour whose
+// exact integer remainder v - s^2 lies in (-s, s] (units of ulp(s)^2). Short
+// segments, where s0 is not close enough, take the root itself.
+__device__ __forceinline__ double sqrt_near(double v, double s0) {
+    const unsigned long long M52 = 1ull << 52, mask = M52 - 1;
+    const double e = fma(-s0, s0, v);
+    const unsigned long long sb0 = __double_as_longlong(s0);
+    // s0 as a float (truncated) and its reciprocal back as a double, by the bits
+    const unsigned fb = (unsigned)((sb0 >> 29) - (896ull << 23));
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fb)));
+    const double h = __longlong_as_double((long long)(((unsigned long long)__float_as_uint(r) << 29) +
+                                                      ((896ull - 1) << 52)));  // r / 2
+    const double s = fma(e, h, s0);
+    const unsigned long long vb = __double_as_longlong(v), sb = __double_as_longlong(s);
+    const unsigned long long mv = (vb & mask) | M52, ms = (sb & mask) | M52;
+    const int ev = (int)(vb >> 52), es = (int)(sb >> 52);
+    const int sh = ev - 2 * es + 1075;  // v in units of ulp(s)^2
+    const long long R = (long long)((mv << (sh & 63)) - ms * ms), S = (long long)ms;
+    if ((int)(sb0 >> 52) < 1023 - 12 || (unsigned)(sh - 50) > 5u || R > 3 * S || R < -3 * S || (ms == M52 && R < 0))
+        return sqrt_slow(v);
+    const int k = (R > S ? 1 : 0) - (R <= -S ? 1 : 0);
+    return __longlong_as_double((long long)sb + k);
+}
+
+// Crossings as eval_x / eval_y, the quotient by div_by.
+__device__ __forceinline__ void cross(double line, double o0, double dir, double inv, double odir,
+                                      double oo0, double &t, double &other) {
+    t = div_by(__dsub_rn(line, o0), dir, inv);
+    other = __dadd_rn(__dmul_rn(odir, t), oo0);
+}
+
+// The in-box interval [k0, k1] of one family: lines g[0..N], the other
+// coordinate monotone in k and within [lo, hi] there.
+struct Span {
+    int k0, k1;
+};
+__device__ __forceinline__ Span in_box(const double *g, int N, double o0, double dir, double inv,
+                                       double odir, double oo0, long long klo, long long khi) {
+    auto at = [&](int k) {
+        double t, o;
+        cross(g[k], o0, dir, inv, odir, oo0, t, o);
+        return key_of(o);
+    };
+    const bool up = at(0) <= at(N);
+    // where the other coordinate meets lo / hi, from floats; the exact predicate decides
+    const float f = (float)dir / (float)odir, z = (float)o0 + 0.5f * (float)N, w = (float)oo0;
+    auto first = [&](float other, auto pred) {
+        const float kf = ceilf(fmaf(other - w, f, z));
+        const int k = kf >= 0.f && kf <= (float)(N + 1) ? (int)kf : (kf < 0.f ? 0 : N + 1);
+        // k is the first true when pred(k) (or none left) and not pred(k - 1)
+        for (int c = k - 1; c <= k + 1; ++c)
+            if (c >= 0 && c <= N + 1 && (c > N || pred(c)) && (c == 0 || !pred(c - 1))) return c;
+        return first_true(N, pred);
+    };
+    const float lo = -0.5f * (float)N, hi = 0.5f * (float)N;
+    Span s;
+    if (up) {
+        s.k0 = first(lo, [&](int k) { return at(k) >= klo; });
+        s.k1 = first(hi, [&](int k) { return at(k) > khi; }) - 1;
+    } else {
+        s.k0 = first(hi, [&](int k) { return at(k) <= khi; });
+        s.k1 = first(lo, [&](int k) { return at(k) < klo; }) - 1;
+    }
+    return s;
+}
+
+// True when a crossing of the ray's major axis (direction component d, in-box
+// lines s) comes within 2^-28 of a line of the other family: the other
+// coordinate o(k) in fixed point with 46 fractional bits (off by less than
+// 2^-35), lines of the other family at its integers.
+__device__ __forceinline__ bool near_line(const double *g, int N, double o0, double dir, double inv,
+                                          double odir, double oo0, Span s) {
+    if (s.k1 < s.k0) return false;
+    double t, o;
+    cross(g[s.k0], o0, dir, inv, odir, oo0, t, o);
+    const double one = 70368744177664.0;  // 2^46
+    long long Y = llrint((o + 0.5 * N) * one) + (1LL << 18);
+    const long long S = llrint(odir * inv * one);
+    unsigned bad = 0;
+    for (int k = s.k0; k <= s.k1; ++k) {
+        // bits 19..45 of Y all zero: within 2^18 units of an integer
+        const unsigned lo = (unsigned)Y, hi = (unsigned)((unsigned long long)Y >> 32);
+        bad |= ((lo >> 19) | (hi & 0x3fffu)) == 0u ? 1u : 0u;
+        Y += S;
+    }
+    return bad != 0;
+}
+
+// Count pass: spans[r] = the in-box lines of both families; rays off the
+// plain path are listed (their counts come from k_geom_count_list).
+__global__ void __launch_bounds__(128) k_geom_spans(GeomDev G, int32_t *counts, int4 *spans,
+                                                    int32_t *listed, int32_t *nlisted) {
+    const int64_t m = (int64_t)G.nth * G.p;
+    const int N = G.N;
+    const long long klo = key_of(-0.5 * N), khi = key_of(0.5 * N);
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m;
          r += (int64_t)gridDim.x * blockDim.x) {
-        int i = (int)(r / G.p), j = (int)(r % G.p);
-        Ray ray = ray_params(G, i, j);
-        CountSink cs;
-        int64_t c = trace_merge(G, ray, cs);
-        if (c < 0) {
-            int slot = atomicAdd(nspecial, 1);
-            special[slot] = (int32_t)r;
-            c = 0;
+        const Ray ray = ray_params(G, (int)(r / G.p), (int)(r % G.p));
+        int4 sp = make_int4(0, -1, 0, -1);
+        int c = 0;
+        if (!ray.excluded) {
+            // NaN positions (p = 1) and infinite ones leave the comparisons false; a
+            // direction component is 0 or large enough for finite parameters
+            const double fa = fabs(ray.a), fb = fabs(ray.b);
+            bool list = !((fa > 1e-30 || fa == 0.0) && (fb > 1e-30 || fb == 0.0) && fa + fb > 0.5 &&
+                          fabs(ray.x0th) < 1e15 && fabs(ray.y0th) < 1e15);
+            if (!list) {
+                const double ia = __drcp_rn(ray.a), ib = __drcp_rn(ray.b);
+                Span x{0, -1}, y{0, -1};
+                if (fa > 0.0) x = in_box(G.grid, N, ray.x0th, ray.a, ia, ray.b, ray.y0th, klo, khi);
+                if (fb > 0.0) y = in_box(G.grid, N, ray.y0th, ray.b, ib, ray.a, ray.x0th, klo, khi);
+                // (an axis-aligned ray on a line of the other family, where the reference
+                // divides 0 by 0, may lie on any of the N + 1: also outside the box's ends)
+                list = fa >= fb ? near_line(G.grid, N, ray.x0th, ray.a, ia, ray.b, ray.y0th, x)
+                                : near_line(G.grid, N, ray.y0th, ray.b, ib, ray.a, ray.x0th, y);
+                const int nx = max(0, x.k1 - x.k0 + 1), ny = max(0, y.k1 - y.k0 + 1);
+                c = max(0, nx + ny - 1);
+                sp = make_int4(x.k0, x.k1, y.k0, y.k1);
+            }
+            if (list) {
+                listed[atomicAdd(nlisted, 1)] = (int32_t)r;
+                sp = make_int4(0, -1, 0, -2);  // not the plain path's
+                c = 0;
+            }
         }
-        counts[r] = (int32_t)c;
+        spans[r] = sp;
+        counts[r] = c;
+    }
+}
+
+// A listed ray by a block: the merge of trace_merge with every crossing
+// evaluated at once, a point's place its own index plus the number of the
+// other family's points before it. Returns the nonzero count, or -1 for the
+// exact path. (One thread per listed ray took 0.8 ms for the few hundred rays
+// that meet corners at 30 and 60 degrees; a block takes ~10 us.)
+constexpr int kListThreads = 128;
+template <class Sink>
+__device__ int64_t trace_block(const GeomDev &G, const Ray &r, unsigned char *smem, Sink &sink) {
+    const int N = G.N, t = threadIdx.x;
+    const double *g = G.grid;
+    double *T = reinterpret_cast<double *>(smem);       // tX [N+1], tY [N+1]
+    double *O = T + 2 * (N + 1);                        // yX, xY
+    int *place = reinterpret_cast<int *>(O + 2 * (N + 1));  // merged point -> point
+    __shared__ int s_scan[kListThreads / 32];
+    if (r.excluded) return 0;
+    const double lo = -0.5 * N, hi = 0.5 * N;
+    int k0[2] = {0, 0}, cnt[2] = {0, 0};
+    const double dir[2] = {r.a, r.b}, org[2] = {r.x0th, r.y0th};
+    bool special = false;
+    for (int f = 0; f < 2; ++f) {
+        if (dir[f] == 0.0) {
+            for (int k = t; k <= N; k += kListThreads) special |= g[k] == org[f];  // 0/0 = NaN key
+            continue;
+        }
+        auto other = [&](int k) {
+            double tt, px, py;
+            if (f == 0) eval_x(g, r, k, tt, px, py); else eval_y(g, r, k, tt, px, py);
+            return f == 0 ? py : px;
+        };
+        int a, b;
+        if (other(0) <= other(N)) {
+            a = first_true(N, [&](int k) { return other(k) >= lo; });
+            b = first_true(N, [&](int k) { return other(k) > hi; }) - 1;
+        } else {
+            a = first_true(N, [&](int k) { return other(k) <= hi; });
+            b = first_true(N, [&](int k) { return other(k) < lo; }) - 1;
+        }
+        k0[f] = dir[f] > 0.0 ? a : b;  // first in ray order
+        cnt[f] = b >= a ? b - a + 1 : 0;
+    }
+    for (int f = 0; f < 2; ++f)
+        for (int i = t; i < cnt[f]; i += kListThreads) {
+            const int k = k0[f] + (dir[f] > 0.0 ? i : -i);
+            double tt, px, py;
+            if (f == 0) eval_x(g, r, k, tt, px, py); else eval_y(g, r, k, tt, px, py);
+            T[f * (N + 1) + i] = tt;
+            O[f * (N + 1) + i] = f == 0 ? py : px;
+        }
+    __syncthreads();
+    for (int f = 0; f < 2; ++f) {
+        const double *A = T + f * (N + 1), *B = T + (1 - f) * (N + 1);
+        const int nb = cnt[1 - f];
+        for (int i = t; i < cnt[f]; i += kListThreads) {
+            const double v = A[i];
+            int L = 0, R = nb;
+            while (L < R) {
+                const int mid = (L + R) >> 1;
+                if (B[mid] < v) L = mid + 1; else R = mid;
+            }
+            special |= L < nb && B[L] == v;  // unstable-sort tie
+            place[i + L] = f * (N + 1) + i;
+        }
+    }
+    if (__syncthreads_or(special)) return -1;
+    const int n = cnt[0] + cnt[1];
+    auto point = [&](int q, double &px, double &py) {
+        const int u = place[q], f = u > N, i = u - f * (N + 1);
+        const double line = g[k0[f] + (dir[f] > 0.0 ? i : -i)];
+        px = f ? O[u] : line;
+        py = f ? line : O[u];
+    };
+    int64_t total = 0;
+    for (int base = 0; base + 1 < n; base += kListThreads) {
+        const int q = base + t;
+        double x0 = 0, y0 = 0, x1 = 0, y1 = 0;
+        bool keep = false;
+        if (q + 1 < n) {
+            point(q, x0, y0);
+            point(q + 1, x1, y1);
+            CountSink cs;
+            int64_t c = 0;
+            segment(N, x0, y0, x1, y1, c, cs);
+            keep = c > 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if ((t & 31) == 0) s_scan[t >> 5] = __popc(m);
+        __syncthreads();
+        int64_t at = total + __popc(m & ((1u << (t & 31)) - 1u));
+        for (int w = 0; w < kListThreads / 32; ++w) {
+            if (w < t >> 5) at += s_scan[w];
+            total += s_scan[w];
+        }
+        if (keep) segment(N, x0, y0, x1, y1, at, sink);
+        __syncthreads();
+    }
+    return total;
+}
+size_t list_smem(int N) { return (size_t)(N + 1) * (4 * sizeof(double) + 2 * sizeof(int)); }
+constexpr size_t kListSmem = 200 * 1024;  // N <= 5119; longer rays take the merge, one thread each
+
+// The listed rays; those neither can order go on to the exact path.
+__global__ void __launch_bounds__(kListThreads) k_geom_count_list(GeomDev G, const int32_t *listed,
+                                                                  int32_t nlisted, int32_t *counts,
+                                                                  int32_t *special, int32_t *nspecial,
+                                                                  bool block) {
+    extern __shared__ __align__(16) unsigned char list_smem_buf[];
+    for (int q = blockIdx.x; q < nlisted; q += gridDim.x) {
+        const int32_t r = listed[q];
+        const Ray ray = ray_params(G, r / G.p, r % G.p);
+        CountSink cs;
+        int64_t c = 0;
+        if (block) c = trace_block(G, ray, list_smem_buf, cs);
+        else if (threadIdx.x == 0) c = trace_merge(G, ray, cs);
+        if (threadIdx.x == 0) {
+            if (c < 0) {
+                special[atomicAdd(nspecial, 1)] = r;
+                c = 0;
+            }
+            counts[r] = (int32_t)c;
+        }
+        __syncthreads();
     }
 }
 
@@ -315,17 +609,139 @@ __global__ void k_geom_count_exact(GeomDev G, const int32_t *special, int32_t ns
     counts[r] = (int32_t)trace_exact(G, ray, s, cs);
 }
 
-__global__ void k_geom_fill(GeomDev G, const int64_t *rowptr, int32_t *col, double *val,
-                            int32_t ncols, int *err) {
-    int64_t m = (int64_t)G.nth * G.p;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m;
-         r += (int64_t)gridDim.x * blockDim.x) {
-        int i = (int)(r / G.p), j = (int)(r % G.p);
-        Ray ray = ray_params(G, i, j);
-        int64_t s0 = rowptr[r], cap = rowptr[r + 1] - s0;
+// Fill pass of the plain path. A ray's crossings are cut into parts of
+// kPart lines of its major axis, one lane per ray and part (a warp: the same
+// part of 32 neighbouring rays), so that the warps' work is even; a part
+// starts at a major crossing, whose place in the row is its own index plus
+// the minor lines before it (the cell it lies in tells them).
+constexpr int kPart = 64;
+__global__ void __launch_bounds__(128) k_geom_fill(GeomDev G, const int4 *spans, const int64_t *rowptr,
+                                                   int32_t *col, double *val, int parts, int *err) {
+    const int64_t m = (int64_t)G.nth * G.p;
+    const int N = G.N, lane = threadIdx.x & 31;
+    const double *g = G.grid;
+    const long long never = 0x7fffffffffffffffLL;
+    const int64_t items = ((m + 31) >> 5) * parts;
+    for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < items;
+         w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        const int64_t r = (w / parts) * 32 + lane;
+        const int part = (int)(w % parts);
+        if (r >= m) continue;
+        const int4 sp = spans[r];
+        if (sp.w == -2) continue;  // listed
+        const Ray ray = ray_params(G, (int)(r / G.p), (int)(r % G.p));
+        const bool xm = fabs(ray.a) >= fabs(ray.b);  // the major axis
+        const double dm = xm ? ray.a : ray.b, dn = xm ? ray.b : ray.a;
+        const double om = xm ? ray.x0th : ray.y0th, on = xm ? ray.y0th : ray.x0th;
+        const int m0 = xm ? sp.x : sp.z, m1 = xm ? sp.y : sp.w, n0 = xm ? sp.z : sp.x, n1 = xm ? sp.w : sp.y;
+        const int nm = max(0, m1 - m0 + 1), nn = max(0, n1 - n0 + 1);
+        if (part > 0 ? part * kPart >= nm : nm + nn < 2) continue;
+        const int stop = (part + 1) * kPart < nm ? (part + 1) * kPart : -1;  // major crossing it ends at
+        const double im = __drcp_rn(dm), in = __drcp_rn(dn);
+        // line numbers grow along the ray when its direction component is positive
+        const int sm = dm > 0.0 ? 1 : -1, sn = dn > 0.0 ? 1 : -1;
+        int q = part * kPart, c = 0;  // major and minor crossings passed
+        int km = sm > 0 ? m0 + q : m1 - q, kn = sn > 0 ? n0 : n1;
+        double tm = 0, om1 = 0, gm = 0, tn = 0, on1 = 0, gn = 0;
+        long long Km = never, Kn = never;
+        double pt = 0, pm = 0, pn = 0;
+        int cm = -1, cn = -1;  // the cell behind the last crossing, -1: not known yet
+        int64_t o = rowptr[r];
+        const int64_t end = rowptr[r + 1];
+        bool have = false;
+        if (q < nm) {
+            gm = g[km];
+            cross(gm, om, dm, im, dn, on, tm, om1);
+            Km = key_of(tm);
+        }
+        if (part > 0) {  // start at that crossing
+            pt = tm; pm = gm; pn = om1;
+            have = true;
+            cm = sm > 0 ? km : km - 1;
+            cn = (int)floor(__dadd_rn(om1, 0.5 * N));
+            c = max(0, min(nn, sn > 0 ? cn - n0 + 1 : n1 - cn));
+            kn += sn * c;
+            o += q + c;
+            ++q;
+            km += sm;
+            Km = never;
+            if (q < nm) {
+                gm = g[km];
+                cross(gm, om, dm, im, dn, on, tm, om1);
+                Km = key_of(tm);
+            }
+        }
+        if (c < nn) {
+            gn = g[kn];
+            cross(gn, on, dn, in, dm, om, tn, on1);
+            Kn = key_of(tn);
+        }
+        while (q < nm || c < nn) {
+            const bool maj = Km < Kn;
+            const double ct = maj ? tm : tn, vm = maj ? gm : on1, vn = maj ? om1 : gn;
+            if (have) {
+                const double d1 = __dsub_rn(pm, vm), d2 = __dsub_rn(pn, vn);
+                const double v = __dadd_rn(__dmul_rn(d1, d1), __dmul_rn(d2, d2));
+                const double s0 = __longlong_as_double(
+                    __double_as_longlong(__dsub_rn(ct, pt)) & 0x7fffffffffffffffLL);
+                const double d = sqrt_near(v, s0);
+                if (cm < 0) cm = mid_cell(pm, vm, N);  // the first segment's
+                if (cn < 0) cn = mid_cell(pn, vn, N);
+                const int ix = xm ? cm : cn, iy = xm ? cn : cm;
+                if ((unsigned)ix >= (unsigned)N || (unsigned)iy >= (unsigned)N) atomicOr(err, 1);
+                else if (o < end) {
+                    col[o] = ix * N + (N - 1 - iy);
+                    val[o] = d;
+                }
+                ++o;
+            }
+            have = true;
+            pt = ct; pm = vm; pn = vn;
+            // the next crossing of the family just passed: selects around one
+            // evaluation (in a branch per family a warp would evaluate both)
+            if (maj && q == stop) break;
+            int mj = maj ? 1 : 0;
+            asm volatile("" : "+r"(mj));
+            cm = mj ? (sm > 0 ? km : km - 1) : cm;
+            cn = mj ? cn : (sn > 0 ? kn : kn - 1);
+            km += mj ? sm : 0;
+            kn += mj ? 0 : sn;
+            q += mj;
+            c += 1 - mj;
+            const bool more = mj ? q < nm : c < nn;
+            const double line = g[more ? (mj ? km : kn) : 0];
+            double t1, o1;
+            cross(line, mj ? om : on, mj ? dm : dn, mj ? im : in, mj ? dn : dm, mj ? on : om, t1, o1);
+            const long long K1 = more ? key_of(t1) : never;
+            tm = mj ? t1 : tm;
+            om1 = mj ? o1 : om1;
+            gm = mj ? line : gm;
+            Km = mj ? K1 : Km;
+            tn = mj ? tn : t1;
+            on1 = mj ? on1 : o1;
+            gn = mj ? gn : line;
+            Kn = mj ? Kn : K1;
+        }
+        if (stop < 0 && o != end) atomicOr(err, 2);  // "Didn't hit all elements" (:304)
+    }
+}
+
+// The listed rays' fill.
+__global__ void __launch_bounds__(kListThreads) k_geom_fill_list(GeomDev G, const int32_t *listed,
+                                                                 int32_t nlisted, const int64_t *rowptr,
+                                                                 int32_t *col, double *val, int32_t ncols,
+                                                                 int *err, bool block) {
+    extern __shared__ __align__(16) unsigned char list_smem_buf[];
+    for (int q = blockIdx.x; q < nlisted; q += gridDim.x) {
+        const int32_t r = listed[q];
+        const Ray ray = ray_params(G, r / G.p, r % G.p);
+        const int64_t s0 = rowptr[r], cap = rowptr[r + 1] - s0;
         WriteSink ws{col + s0, val + s0, cap, ncols, err};
-        int64_t c = trace_merge(G, ray, ws);
-        if (c >= 0 && c != cap) atomicOr(err, 2);  // "Didn't hit all elements" (:304)
+        int64_t c = -1;
+        if (block) c = trace_block(G, ray, list_smem_buf, ws);
+        else if (threadIdx.x == 0) c = trace_merge(G, ray, ws);
+        if (threadIdx.x == 0 && c >= 0 && c != cap) atomicOr(err, 2);
+        __syncthreads();
     }
 }
 
@@ -362,33 +778,52 @@ constexpr int kExactBatch = 2048;  // special rays traced per launch (scratch bo
 }  // namespace
 
 namespace {
-// The count pass (k_geom_count, then the exact path for the rays whose keys
-// need the quicksort replay): entries per ray into counts [m]; the special
-// rays, their number and the exact path's scratch stay for the fill.
+// The count pass (k_geom_spans, the listed rays through the merge, then the
+// exact path for those whose keys need the quicksort replay): entries per ray
+// into counts [m]; the spans, the lists and the exact path's scratch stay for
+// the fill.
 struct GeomCount {
-    DevBuf counts, special, nsp, scr_d, scr_i;
-    int32_t h_nsp = 0, batch = 0;
+    DevBuf counts, spans, listed, special, nsp, scr_d, scr_i;
+    int32_t h_listed = 0, h_nsp = 0, batch = 0;
     int blocks = 1;
     static constexpr int threads = 128;
+    // a block per listed ray, its crossings in shared memory where they fit
+    bool in_blocks(int N) const { return list_smem(N) <= kListSmem; }
+    int list_blocks() const { return h_listed < 4096 ? h_listed : 4096; }
+    size_t smem(int N) const { return in_blocks(N) ? list_smem(N) : 0; }
     void release() {
-        counts.release(); special.release(); nsp.release(); scr_d.release(); scr_i.release();
+        counts.release(); spans.release(); listed.release(); special.release(); nsp.release();
+        scr_d.release(); scr_i.release();
     }
 };
 
 int geometry_count(const GeomTables &T, const GeomDev &G, GeomCount &C, cudaStream_t s) {
     const int64_t m = (int64_t)T.nth * T.p;
     FAIR_TRY(C.counts.grow(sizeof(int32_t) * (m > 0 ? m : 1)));
-    FAIR_TRY(C.special.grow(sizeof(int32_t) * (m > 0 ? m : 1)));
-    FAIR_TRY(C.nsp.grow(sizeof(int32_t)));
-    FAIR_CUDA(cudaMemsetAsync(C.nsp.p, 0, sizeof(int32_t), s));
+    FAIR_TRY(C.spans.grow(sizeof(int4) * (m > 0 ? m : 1)));
+    FAIR_TRY(C.listed.grow(sizeof(int32_t) * (m > 0 ? m : 1)));
+    FAIR_TRY(C.nsp.grow(2 * sizeof(int32_t)));
+    FAIR_CUDA(cudaMemsetAsync(C.nsp.p, 0, 2 * sizeof(int32_t), s));
     int64_t blocks64 = (m + C.threads - 1) / C.threads;
     C.blocks = (int)(blocks64 < (int64_t)sm_count() * 64 ? (blocks64 > 0 ? blocks64 : 1)
                                                          : (int64_t)sm_count() * 64);
-    k_geom_count<<<C.blocks, C.threads, 0, s>>>(G, C.counts.as<int32_t>(), C.special.as<int32_t>(),
-                                                C.nsp.as<int32_t>());
+    k_geom_spans<<<C.blocks, C.threads, 0, s>>>(G, C.counts.as<int32_t>(), C.spans.as<int4>(),
+                                                C.listed.as<int32_t>(), C.nsp.as<int32_t>());
     FAIR_CUDA(cudaGetLastError());
-    FAIR_CUDA(cudaMemcpyAsync(&C.h_nsp, C.nsp.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    FAIR_CUDA(cudaMemcpyAsync(&C.h_listed, C.nsp.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     FAIR_CUDA(cudaStreamSynchronize(s));
+    if (C.h_listed > 0) {
+        FAIR_TRY(C.special.grow(sizeof(int32_t) * (size_t)C.h_listed));
+        FAIR_CUDA(cudaFuncSetAttribute(k_geom_count_list, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kListSmem));
+        k_geom_count_list<<<C.list_blocks(), kListThreads, C.smem(T.N), s>>>(
+            G, C.listed.as<int32_t>(), C.h_listed, C.counts.as<int32_t>(), C.special.as<int32_t>(),
+            C.nsp.as<int32_t>() + 1, C.in_blocks(T.N));
+        FAIR_CUDA(cudaGetLastError());
+        FAIR_CUDA(cudaMemcpyAsync(&C.h_nsp, C.nsp.as<int32_t>() + 1, sizeof(int32_t),
+                                  cudaMemcpyDeviceToHost, s));
+        FAIR_CUDA(cudaStreamSynchronize(s));
+    }
     // Scratch for the exact path: keys, two coordinate arrays, permutation.
     const int nt = 2 * T.N + 2;
     C.batch = C.h_nsp < kExactBatch ? C.h_nsp : kExactBatch;
@@ -438,7 +873,6 @@ int build_geometry(const GeomTables &T, DevCSR &A, cudaStream_t s) {
     FAIR_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
     DevBuf &counts = C.counts, &special = C.special, &scr_d = C.scr_d, &scr_i = C.scr_i;
     const int32_t h_nsp = C.h_nsp, batch = C.batch;
-    const int blocks = C.blocks, threads = C.threads;
 
     FAIR_TRY(A.rowptr.grow(sizeof(int64_t) * (m + 1)));
     FAIR_TRY(scan_counts(counts.as<int32_t>(), m, A.rowptr.as<int64_t>(), s));
@@ -449,9 +883,20 @@ int build_geometry(const GeomTables &T, DevCSR &A, cudaStream_t s) {
     A.nnz = nnz;
     FAIR_TRY(A.alloc_entries(nnz, s));
 
-    k_geom_fill<<<blocks, threads, 0, s>>>(G, A.rowptr.as<int64_t>(), A.col.as<int32_t>(),
-                                           A.v64.as<double>(), ncols, err.as<int>());
+    const int parts = T.N / kPart + 1;  // of up to N + 1 major lines
+    const int64_t items = (m + 31) / 32 * parts;
+    k_geom_fill<<<(unsigned)std::min<int64_t>((items + 3) / 4, 1 << 20), 128, 0, s>>>(
+        G, C.spans.as<int4>(), A.rowptr.as<int64_t>(), A.col.as<int32_t>(), A.v64.as<double>(), parts,
+        err.as<int>());
     FAIR_CUDA(cudaGetLastError());
+    if (C.h_listed > 0) {
+        FAIR_CUDA(cudaFuncSetAttribute(k_geom_fill_list, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kListSmem));
+        k_geom_fill_list<<<C.list_blocks(), kListThreads, C.smem(T.N), s>>>(
+            G, C.listed.as<int32_t>(), C.h_listed, A.rowptr.as<int64_t>(), A.col.as<int32_t>(),
+            A.v64.as<double>(), ncols, err.as<int>(), C.in_blocks(T.N));
+        FAIR_CUDA(cudaGetLastError());
+    }
     for (int32_t q0 = 0; q0 < h_nsp; q0 += batch) {
         int32_t nq = h_nsp - q0 < batch ? h_nsp - q0 : batch;
         k_geom_fill_exact<<<(nq + 63) / 64, 64, 0, s>>>(
