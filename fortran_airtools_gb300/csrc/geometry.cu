@@ -490,6 +490,7 @@ __device__ int64_t trace_block(const GeomDev &G, const Ray &r, unsigned char *sm
     const double lo = -0.5 * N, hi = 0.5 * N;
     int k0[2] = {0, 0}, cnt[2] = {0, 0};
     const double dir[2] = {r.a, r.b}, org[2] = {r.x0th, r.y0th};
+    const bool usual = fabs(r.a) > 1e-30 && fabs(r.b) > 1e-30 && fabs(r.x0th) < 1e15 && fabs(r.y0th) < 1e15;
     bool special = false;
     for (int f = 0; f < 2; ++f) {
         if (dir[f] == 0.0) {
@@ -502,7 +503,12 @@ __device__ int64_t trace_block(const GeomDev &G, const Ray &r, unsigned char *sm
             return f == 0 ? py : px;
         };
         int a, b;
-        if (other(0) <= other(N)) {
+        if (usual) {
+            const Span sp = in_box(g, N, org[f], dir[f], __drcp_rn(dir[f]), dir[1 - f], org[1 - f],
+                                   key_of(lo), key_of(hi));
+            a = sp.k0;
+            b = sp.k1;
+        } else if (other(0) <= other(N)) {
             a = first_true(N, [&](int k) { return other(k) >= lo; });
             b = first_true(N, [&](int k) { return other(k) > hi; }) - 1;
         } else {
