@@ -1,17 +1,20 @@
 // rows.cuh -- the row-product engine shared by every CSR pass.
 //
-// A warp owns chunks of 32 consecutive rows (rays of one angle, or pixels of
-// one image column for the transposed matrix, so the rows of a chunk have
-// similar lengths). Within a chunk it works on 32/G rows at a time with G
+// A warp owns chunks of up to 32 consecutive rows (rays of one angle, or
+// pixels of one image column for the transposed matrix, so the rows of a chunk
+// have similar lengths). Within a chunk it works on 32/G rows at a time with G
 // lanes per row; every lane reads 4 consecutive entries per step with one
 // 128-bit load of column indices and one vector load of values, from the
-// 16-byte-aligned window around the row, masking entries outside the row, and
-// prefetches its next step before gathering x for the current one. The row
-// sums are reduced over the G lanes and moved to lane (row mod 32), so the
-// epilogue of a chunk runs once for its 32 rows with coalesced loads and
-// stores: FP64 epilogue work (division, bounds) costs one warp instruction per
-// 32 rows instead of one per row, which matters on a part whose FP64 pipe
-// issues two lanes per clock.
+// 16-byte-aligned window around the row, and prefetches its next step before
+// gathering x for the current one; the next rows' first step is loaded during
+// the lane sums and the epilogue. Entries outside the row
+// are zeroed by integer selects: an FP64 instruction holds its pipe for 64
+// cycles also when predicated off, and masked multiply-adds in a branch of
+// their own cost every first and last step of a row twice. The row sums are
+// reduced over the G lanes and moved to one lane per row, so that the epilogue
+// of a chunk runs once, with coalesced loads and stores. A matrix with few
+// rows takes smaller chunks (down to the 32/G rows of one round), so that more
+// warps work on it: the same arithmetic per row, the same results.
 //
 // Column/value arrays are allocated with 4 spare entries so that the aligned
 // window never reads past the allocation.
@@ -169,120 +172,192 @@ template <> struct VLoad<int16_t, float> {
     }
 };
 
-// Row sums of one chunk (rows base..base+31): returns, in lane l, the sum of
-// row base+l. All lanes of the warp call it together.
-// VT: stored value type; XT: gathered vector type; ACC: accumulator type.
-// The sum of row `row` (0 past m) by the G lanes of its group, gl the lane's
-// place in the group: each lane takes the 4-entry groups at (s & ~3) + 4 gl,
-// then every 4 G entries, adding each group's products in order; the group's
-// butterfly leaves the sum in every lane of the group.
-template <typename VT, typename XT, typename ACC, int G>
-__device__ __forceinline__ ACC csr_row_sum(const int64_t *__restrict__ rowptr, int32_t m,
-                                           const int32_t *__restrict__ col,
-                                           const VT *__restrict__ val,
-                                           const XT *__restrict__ x, int64_t row, int gl) {
-    int64_t s = 0, e = 0;
-    if (row < m) {
-        s = __ldg(rowptr + row);
-        e = __ldg(rowptr + row + 1);
-    }
-    ACC acc = 0;
-    int64_t k = (s & ~(int64_t)3) + 4 * gl;
-    int4 cc = make_int4(0, 0, 0, 0);
-    ACC vv[4] = {0, 0, 0, 0};
-    if (k < e) {
-        cc = ld_stream(reinterpret_cast<const int4 *>(col + k));
-        VLoad<VT, ACC>::ld(val + k, vv);
-    }
-    while (k < e) {
-        const int64_t kn = k + 4 * G;
-        int4 cn = make_int4(0, 0, 0, 0);
-        ACC vn[4] = {0, 0, 0, 0};
-        if (kn < e) {
-            cn = ld_stream(reinterpret_cast<const int4 *>(col + kn));
-            VLoad<VT, ACC>::ld(val + kn, vn);
+// Programmatic dependent launch (launch_rows, solvers.cu): a kernel may start
+// while the one before it on the stream still runs; what it reads of that
+// kernel's results it reads after pdl_wait (a no-op in an ordinary launch),
+// with ordinary loads: the read-only path need not see them.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// The CSR as a source of row steps: a lane's step is 4 entries from offset k
+// of the row (multiples of 4 from the aligned window's start, k may be -3..-1).
+template <typename VT, typename XT, typename ACC, int G> struct CsrSteps {
+    const int64_t *off;
+    const int32_t *col;
+    const VT *val;
+    static constexpr int STEP = 4 * G;
+    struct Raw {
+        int4 c;
+        ACC v[4];
+    };
+    __device__ __forceinline__ int first(int64_t s, int gl) const { return 4 * gl - (int)(s & 3); }
+    __device__ __forceinline__ void load(Raw &r, int64_t s, int k, int len) const {
+        if (k < len) {
+            r.c = ld_stream(reinterpret_cast<const int4 *>(col + s + k));
+            VLoad<VT, ACC>::ld(val + s + k, r.v);
         }
-        if (k >= s && k + 3 < e) {
-            acc += (ACC)__ldg(x + cc.x) * vv[0];
-            acc += (ACC)__ldg(x + cc.y) * vv[1];
-            acc += (ACC)__ldg(x + cc.z) * vv[2];
-            acc += (ACC)__ldg(x + cc.w) * vv[3];
-        } else {
-            if (k >= s && k < e) acc += (ACC)__ldg(x + cc.x) * vv[0];
-            if (k + 1 >= s && k + 1 < e) acc += (ACC)__ldg(x + cc.y) * vv[1];
-            if (k + 2 >= s && k + 2 < e) acc += (ACC)__ldg(x + cc.z) * vv[2];
-            if (k + 3 >= s && k + 3 < e) acc += (ACC)__ldg(x + cc.w) * vv[3];
-        }
-        cc = cn;
+    }
+    static constexpr int N = 4;
+    __device__ __forceinline__ void gather(const Raw &r, int k, int len, const XT *x, ACC (&xv)[N],
+                                           ACC (&vv)[N]) const {
+        const int c[4] = {r.c.x, r.c.y, r.c.z, r.c.w};
 #pragma unroll
-        for (int t = 0; t < 4; ++t) vv[t] = vn[t];
-        k = kn;
+        for (int t = 0; t < 4; ++t) {
+            const bool in = (unsigned)(k + t) < (unsigned)len;
+            xv[t] = in ? (ACC)x[c[t]] : (ACC)0;
+            vv[t] = in ? r.v[t] : (ACC)0;
+        }
     }
+};
+
+// This lane's part of the sum of a row of len entries from s (gl the lane's
+// place among the row's G), its first steps already loaded (r0; r1 in FP64):
+// its entries in order. FP64 gathers a step's x values while the step before
+// is added and loads entries two steps ahead (its 12 multiply-adds a step leave
+// time for both, and 24 warps per SM fit); the reduced forms, bound by the
+// gathers' L1 wavefronts, load one step ahead and keep 40 warps.
+template <typename XT, typename ACC, class ST>
+__device__ __forceinline__ ACC steps_part(const ST &st, int64_t s, int len, int gl, typename ST::Raw &r0,
+                                          typename ST::Raw &r1, const XT *x) {
+    ACC acc = 0;
+    ACC xv[ST::N], vv[ST::N];
+    int k = st.first(s, gl);
+    if constexpr (sizeof(ACC) == 8) {
+        st.gather(r0, k, len, x, xv, vv);
+        while (k < len) {
+            st.load(r0, s, k + 2 * ST::STEP, len);
+            ACC xn[ST::N], vn[ST::N];
+            st.gather(r1, k + ST::STEP, len, x, xn, vn);
+#pragma unroll
+            for (int t = 0; t < ST::N; ++t) acc += xv[t] * vv[t];
+#pragma unroll
+            for (int t = 0; t < ST::N; ++t) {
+                xv[t] = xn[t];
+                vv[t] = vn[t];
+            }
+            r1 = r0;
+            k += ST::STEP;
+        }
+    } else {
+        while (k < len) {
+            r1 = r0;
+            st.load(r0, s, k + ST::STEP, len);
+            st.gather(r1, k, len, x, xv, vv);
+#pragma unroll
+            for (int t = 0; t < ST::N; ++t) acc += xv[t] * vv[t];
+            k += ST::STEP;
+        }
+    }
+    return acc;
+}
+// The parts of the G lanes of every group added: the sum in every lane of the group.
+template <typename ACC, int G> __device__ __forceinline__ ACC group_sum(ACC acc) {
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     return acc;
 }
 
-// The sums of the 32 rows of a chunk, row base + lane in lane `lane`: 32/G
-// rows at a time, one per group of G lanes.
-template <typename VT, typename XT, typename ACC, int G>
-__device__ __forceinline__ ACC csr_chunk_sums(const int64_t *__restrict__ rowptr, int32_t m,
-                                              const int32_t *__restrict__ col,
-                                              const VT *__restrict__ val,
-                                              const XT *__restrict__ x, int64_t base) {
+// Row sums of one chunk (rows base..base+31): returns, in lane l, the sum of
+// row base+l, 32/G rows at a time, one per group of G lanes. All lanes of the
+// warp call it together.
+template <typename XT, typename ACC, int G, class ST>
+__device__ __forceinline__ ACC steps_chunk_sums(const ST &st, int32_t m, const XT *__restrict__ x,
+                                                int64_t base) {
     constexpr int R = 32 / G;
     const int lane = threadIdx.x & 31, g = lane / G, gl = lane % G;
     ACC mine = 0;
 #pragma unroll 1
     for (int sub = 0; sub < 32; sub += R) {
-        const ACC acc = csr_row_sum<VT, XT, ACC, G>(rowptr, m, col, val, x, base + sub + g, gl);
-        ACC r = __shfl_sync(0xffffffffu, acc, ((lane - sub) & (R - 1)) * G);
+        const int64_t row = base + sub + g;
+        int64_t s = 0;
+        int len = 0;
+        if (row < m) {
+            s = __ldg(st.off + row);
+            len = (int)(__ldg(st.off + row + 1) - s);
+        }
+        typename ST::Raw r0 = {}, r1 = {};
+        st.load(r0, s, st.first(s, gl), len);
+        if constexpr (sizeof(ACC) == 8) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
+        const ACC acc = group_sum<ACC, G>(steps_part<XT, ACC>(st, s, len, gl, r0, r1, x));
+        const ACC r = __shfl_sync(0xffffffffu, acc, ((lane - sub) & (R - 1)) * G);
         if (lane >= sub && lane < sub + R) mine = r;
     }
     return mine;
 }
+// VT: stored value type; XT: gathered vector type; ACC: accumulator type.
+template <typename VT, typename XT, typename ACC, int G>
+__device__ __forceinline__ ACC csr_chunk_sums(const int64_t *__restrict__ rowptr, int32_t m,
+                                              const int32_t *__restrict__ col,
+                                              const VT *__restrict__ val,
+                                              const XT *__restrict__ x, int64_t base) {
+    return steps_chunk_sums<XT, ACC, G>(CsrSteps<VT, XT, ACC, G>{rowptr, col, val}, m, x, base);
+}
 
 // Sum over the rows of every chunk owned by this warp; calls epi(row, sum)
-// from the lane that owns `row` (all lanes of the warp call epi together).
-template <typename VT, typename XT, typename ACC, int G, class Epi>
-__device__ __forceinline__ void chunk_rows(const int64_t *__restrict__ rowptr, int32_t m,
-                                           const int32_t *__restrict__ col,
-                                           const VT *__restrict__ val,
-                                           const XT *__restrict__ x, Epi &epi,
-                                           unsigned *sched = nullptr) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t nchunks = ((int64_t)m + 31) >> 5;
-    for (int64_t ch = sched ? next_chunk(sched, 0, nwarps, lane) : warp; ch < nchunks;
-         ch = next_chunk(sched, ch, nwarps, lane)) {
-        const int64_t base = ch << 5;
-        const ACC mine = csr_chunk_sums<VT, XT, ACC, G>(rowptr, m, col, val, x, base);
-        const int64_t row = base + lane;
-        if (row < m) epi(row, mine);
+// from the lane that owns `row`. A chunk is `subs` rounds of 32/G rows (at
+// most 32 rows). A warp's first chunk is its own number, so that its offsets
+// and first entries can be read before pdl_wait; later ones are claimed
+// (sched) or strided.
+template <typename XT, typename ACC, int G, class ST, class Epi>
+__device__ __forceinline__ void rows_stream(const ST &st, int32_t m, const XT *x, Epi &epi,
+                                            unsigned *sched, int subs) {
+    constexpr int R = 32 / G;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, g = lane / G, gl = lane % G, CR = subs * R;
+    const int warp = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+    const int nwarps = (int)(((int64_t)gridDim.x * blockDim.x) >> 5);
+    const int nchunks = (int)(((int64_t)m + CR - 1) / CR);
+    int64_t hs = 0;  // lane l: row l of the chunk in hand
+    int hl = 0;
+    auto head = [&](int ch) {
+        const int64_t row = (int64_t)ch * CR + lane;
+        hs = 0;
+        hl = 0;
+        if (ch < nchunks && lane < CR && row < m) {
+            hs = __ldg(st.off + row);
+            hl = (int)(__ldg(st.off + row + 1) - hs);
+        }
+    };
+    pdl_trigger();
+    int ch = warp;
+    head(ch);
+    int64_t s = __shfl_sync(FULL, hs, g);
+    int len = __shfl_sync(FULL, hl, g);
+    typename ST::Raw r0 = {}, r1 = {};
+    st.load(r0, s, st.first(s, gl), len);
+    if constexpr (sizeof(ACC) == 8) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
+    pdl_wait();
+    while (ch < nchunks) {
+        const int next = sched ? (int)next_chunk(sched, ch, nwarps, lane) + nwarps : ch + nwarps;
+        ACC mine = 0;
+#pragma unroll 1
+        for (int sub = 0; sub < CR; sub += R) {
+            ACC acc = steps_part<XT, ACC>(st, s, len, gl, r0, r1, x);
+            // the next rows' first steps are in flight during the lane sums and the epilogue
+            if (sub + R >= CR) head(next);
+            const int from = sub + R >= CR ? g : sub + R + g;
+            s = __shfl_sync(FULL, hs, from);
+            len = __shfl_sync(FULL, hl, from);
+            st.load(r0, s, st.first(s, gl), len);
+            if constexpr (sizeof(ACC) == 8) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
+            acc = group_sum<ACC, G>(acc);
+            const ACC r = __shfl_sync(FULL, acc, ((lane - sub) & (R - 1)) * G);
+            if (lane >= sub && lane < sub + R) mine = r;
+        }
+        const int64_t row = (int64_t)ch * CR + lane;
+        if (lane < CR && row < m) epi(row, mine);
+        ch = next;
     }
     finish_chunks(sched, nwarps, lane);
 }
 
-// The same row sums with each warp taking one group of 32/G consecutive rows
-// at a time instead of a chunk of 32: G times the warps for the same rows, the
-// same arithmetic per row (csr_row_sum), so the same results bit for bit.
-// For matrices with too few 32-row chunks to fill the GPU.
 template <typename VT, typename XT, typename ACC, int G, class Epi>
-__device__ __forceinline__ void rows_by_group(const int64_t *__restrict__ rowptr, int32_t m,
-                                              const int32_t *__restrict__ col,
-                                              const VT *__restrict__ val,
-                                              const XT *__restrict__ x, Epi &epi) {
-    constexpr int R = 32 / G;
-    const int lane = threadIdx.x & 31, g = lane / G, gl = lane % G;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t nunits = ((int64_t)m + R - 1) / R;
-    for (int64_t u = warp; u < nunits; u += nwarps) {
-        const int64_t row = u * R + g;
-        const ACC acc = csr_row_sum<VT, XT, ACC, G>(rowptr, m, col, val, x, row, gl);
-        if (gl == 0 && row < m) epi(row, acc);
-    }
+__device__ __forceinline__ void chunk_rows(const int64_t *__restrict__ rowptr, int32_t m,
+                                           const int32_t *__restrict__ col,
+                                           const VT *__restrict__ val,
+                                           const XT *x, Epi &epi,
+                                           unsigned *sched = nullptr, int subs = G) {
+    rows_stream<XT, ACC, G>(CsrSteps<VT, XT, ACC, G>{rowptr, col, val}, m, x, epi, sched, subs);
 }
 
 // ---- packed index stream ------------------------------------------------------
@@ -351,85 +426,55 @@ template <typename VT> struct FusedLoad {
     }
 };
 
-// Row sums of one chunk over the packed index stream: every lane takes NG
-// groups (4*NG entries) per step through the loader and issues the 4*NG
-// gathers of a step together.
-template <typename XT, typename ACC, int G, int NG, class LD>
-__device__ __forceinline__ ACC pk_chunk_sums_ld(const int64_t *__restrict__ prow, int32_t m,
-                                                const LD &ldr, const int4 *__restrict__ gside,
-                                                int S, int L, const XT *__restrict__ x,
-                                                int64_t base) {
-    constexpr int R = 32 / G;
-    const int lane = threadIdx.x & 31, g = lane / G, gl = lane % G;
-    ACC mine = 0;
-#pragma unroll 1
-    for (int sub = 0; sub < 32; sub += R) {
-        const int64_t row = base + sub + g;
-        int64_t g0 = 0;
-        int ng = 0;  // groups in the row
-        if (row < m) {
-            g0 = __ldg(prow + row);
-            ng = (int)(__ldg(prow + row + 1) - g0);
-        }
-        ACC acc = 0;
+// The packed stream as a source of row steps: a lane's step is NG groups
+// (4*NG entries) through the loader, their 4*NG gathers issued together.
+template <typename XT, typename ACC, int G, int NG, class LD> struct PkSteps {
+    const int64_t *off;
+    LD ldr;
+    const int4 *gside;
+    int S, L;
+    static constexpr int STEP = NG * G;
+    struct Raw {
         uint2 w[NG];
-        ACC vv[NG][4];
+        ACC v[NG][4];
+    };
+    __device__ __forceinline__ int first(int64_t, int gl) const { return gl; }
+    __device__ __forceinline__ void load(Raw &r, int64_t s, int k, int len) const {
 #pragma unroll
         for (int q = 0; q < NG; ++q) {
-            const int j = gl + q * G;
-            w[q] = make_uint2(0u, 0u);
-            vv[q][0] = vv[q][1] = vv[q][2] = vv[q][3] = 0;
-            if (j < ng) ldr.ld(g0 + j, w[q], vv[q]);
+            r.w[q] = make_uint2(0u, 0u);
+            r.v[q][0] = r.v[q][1] = r.v[q][2] = r.v[q][3] = 0;
+            if (k + q * G < len) ldr.ld(s + k + q * G, r.w[q], r.v[q]);
         }
-        for (int j = gl; j < ng; j += NG * G) {
-            const int jn = j + NG * G;
-            uint2 wn[NG];
-            ACC vn[NG][4];
-#pragma unroll
-            for (int q = 0; q < NG; ++q) {
-                wn[q] = make_uint2(0u, 0u);
-                vn[q][0] = vn[q][1] = vn[q][2] = vn[q][3] = 0;
-                if (jn + q * G < ng) ldr.ld(g0 + jn + q * G, wn[q], vn[q]);
-            }
-            int c[NG][4];
-            ACC xv[NG][4];
-#pragma unroll
-            for (int q = 0; q < NG; ++q) {
-                pk_decode(w[q], gside, S, L, c[q]);
-                // entries past the group's count (and groups past the row)
-                // read nothing and add zero
-                const int cnt = j + q * G < ng ? (int)((w[q].y >> 24) & 3u) : -1;
-#pragma unroll
-                for (int t = 0; t < 4; ++t) xv[q][t] = t <= cnt ? (ACC)__ldg(x + c[q][t]) : (ACC)0;
-            }
-#pragma unroll
-            for (int q = 0; q < NG; ++q)
-#pragma unroll
-                for (int t = 0; t < 4; ++t) acc += xv[q][t] * vv[q][t];
-#pragma unroll
-            for (int q = 0; q < NG; ++q) {
-                w[q] = wn[q];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) vv[q][t] = vn[q][t];
-            }
-        }
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        ACC r = __shfl_sync(0xffffffffu, acc, ((lane - sub) & (R - 1)) * G);
-        if (lane >= sub && lane < sub + R) mine = r;
     }
-    return mine;
-}
+    static constexpr int N = 4 * NG;
+    __device__ __forceinline__ void gather(const Raw &r, int k, int len, const XT *x, ACC (&xv)[N],
+                                           ACC (&vv)[N]) const {
+        int c[NG][4];
+#pragma unroll
+        for (int q = 0; q < NG; ++q) {
+            pk_decode(r.w[q], gside, S, L, c[q]);
+            // entries past the group's count (and groups past the row)
+            // read nothing and add zero
+            const int cnt = k + q * G < len ? (int)((r.w[q].y >> 24) & 3u) : -1;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                xv[4 * q + t] = t <= cnt ? (ACC)x[c[q][t]] : (ACC)0;
+                vv[4 * q + t] = r.v[q][t];
+            }
+        }
+    }
+};
 
-// The split layout (index array + padded values).
+// The split layout (index array + padded values): the sums of a chunk's rows.
 template <typename VT, typename XT, typename ACC, int G, int NG>
 __device__ __forceinline__ ACC pk_chunk_sums(const int64_t *__restrict__ prow, int32_t m,
                                              const uint2 *__restrict__ gidx,
                                              const int4 *__restrict__ gside, int S, int L,
                                              const VT *__restrict__ val,
                                              const XT *__restrict__ x, int64_t base) {
-    const SplitLoad<VT, ACC> ldr{gidx, val};
-    return pk_chunk_sums_ld<XT, ACC, G, NG>(prow, m, ldr, gside, S, L, x, base);
+    const PkSteps<XT, ACC, G, NG, SplitLoad<VT, ACC>> st{prow, {gidx, val}, gside, S, L};
+    return steps_chunk_sums<XT, ACC, G>(st, m, x, base);
 }
 
 // chunk_rows over the fused 16-byte records (2-byte values).
@@ -437,21 +482,10 @@ template <typename VT, int G, int NG, class Epi>
 __device__ __forceinline__ void chunk_rows_pkf(const int64_t *__restrict__ prow, int32_t m,
                                                const uint4 *__restrict__ rec,
                                                const int4 *__restrict__ gside, int S, int L,
-                                               const float *__restrict__ x, Epi &epi,
-                                               unsigned *sched) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t nchunks = ((int64_t)m + 31) >> 5;
-    const FusedLoad<VT> ldr{rec};
-    for (int64_t ch = sched ? next_chunk(sched, 0, nwarps, lane) : warp; ch < nchunks;
-         ch = next_chunk(sched, ch, nwarps, lane)) {
-        const int64_t base = ch << 5;
-        const float mine = pk_chunk_sums_ld<float, float, G, NG>(prow, m, ldr, gside, S, L, x, base);
-        const int64_t row = base + lane;
-        if (row < m) epi(row, mine);
-    }
-    finish_chunks(sched, nwarps, lane);
+                                               const float *x, Epi &epi,
+                                               unsigned *sched, int subs) {
+    const PkSteps<float, float, G, NG, FusedLoad<VT>> st{prow, {rec}, gside, S, L};
+    rows_stream<float, float, G>(st, m, x, epi, sched, subs);
 }
 
 // chunk_rows over the packed index stream.
@@ -460,20 +494,10 @@ __device__ __forceinline__ void chunk_rows_pk(const int64_t *__restrict__ prow, 
                                               const uint2 *__restrict__ gidx,
                                               const int4 *__restrict__ gside, int S, int L,
                                               const VT *__restrict__ val,
-                                              const XT *__restrict__ x, Epi &epi,
-                                              unsigned *sched) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t nchunks = ((int64_t)m + 31) >> 5;
-    for (int64_t ch = sched ? next_chunk(sched, 0, nwarps, lane) : warp; ch < nchunks;
-         ch = next_chunk(sched, ch, nwarps, lane)) {
-        const int64_t base = ch << 5;
-        const ACC mine = pk_chunk_sums<VT, XT, ACC, G, NG>(prow, m, gidx, gside, S, L, val, x, base);
-        const int64_t row = base + lane;
-        if (row < m) epi(row, mine);
-    }
-    finish_chunks(sched, nwarps, lane);
+                                              const XT *x, Epi &epi,
+                                              unsigned *sched, int subs) {
+    const PkSteps<XT, ACC, G, NG, SplitLoad<VT, ACC>> st{prow, {gidx, val}, gside, S, L};
+    rows_stream<XT, ACC, G>(st, m, x, epi, sched, subs);
 }
 
 // ---- sliced copy of the packed stream --------------------------------------

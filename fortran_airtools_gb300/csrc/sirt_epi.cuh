@@ -7,10 +7,21 @@
 
 namespace fair {
 
+// Order of two doubles by their bits (-0 equal to 0; NaN not ordered).
+__device__ __forceinline__ long long ord_key(double t) {
+    const long long b = __double_as_longlong(t);
+    const long long k = b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+    return k + (k == -1);
+}
+__device__ __forceinline__ bool is_nan(double t) {
+    return (__double_as_longlong(t) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+
+// AIRMs.f90:1093-1100: upper bound first, then lower bound; fmin_f / fmax_f with
+// the comparisons on the integer units (each FP64 one holds its pipe for 64 cycles).
 __device__ __forceinline__ double sirt_box(double t, int bmode, double lb, double ub) {
-    // AIRMs.f90:1093-1100: upper bound first, then lower bound
-    if (bmode & 1) t = fmin_f(t, ub);
-    if (bmode & 2) t = fmax_f(t, lb);
+    if (bmode & 1) t = (!is_nan(ub) && ord_key(ub) < ord_key(t)) || is_nan(t) ? ub : t;
+    if (bmode & 2) t = (!is_nan(lb) && ord_key(lb) > ord_key(t)) || is_nan(t) ? lb : t;
     return t;
 }
 

@@ -73,28 +73,27 @@ struct EpiStoreSq {  // y = Ax, partial sum of y^2
     }
 };
 
+// Blocks of 8 warps per SM the row engine's kernels are compiled for: 80
+// registers hold the FP64 pipeline (steps_part, rows.cuh), 48 the reduced forms'.
+// Fan N = 128 / parallel N = 256 / N = 363 iterations in us, FP64: 3 blocks 42 /
+// 159 / 295, 4 blocks 42 / 164 / 305, 2 blocks 41 / 181 / 344; N = 363 FP32: 5
+// blocks 177, 6 blocks 183, 4 blocks 184.
+constexpr int kOcc64 = 3, kOccLP = 5;
+
 // ---- kernels --------------------------------------------------------------------
 template <int G>
-__global__ void __launch_bounds__(256) k_sirt_resid_f64(const int64_t *rowptr, int32_t m,
+__global__ void __launch_bounds__(256, kOcc64) k_sirt_resid_f64(const int64_t *rowptr, int32_t m,
                                                         const int32_t *col, const double *v,
                                                         const double *x, EpiResidF64 epi,
-                                                        unsigned *sched) {
-    chunk_rows<double, double, double, G>(rowptr, m, col, v, x, epi, sched);
-}
-// Matrices with few rows: a group of 32/G rows per warp (rows_by_group, the
-// same per-row arithmetic as the chunked kernels above).
-template <int G, class Epi>
-__global__ void __launch_bounds__(256) k_sirt_rows_f64(const int64_t *rowptr, int32_t m,
-                                                       const int32_t *col, const double *v,
-                                                       const double *x, Epi epi) {
-    rows_by_group<double, double, double, G>(rowptr, m, col, v, x, epi);
+                                                        unsigned *sched, int subs) {
+    chunk_rows<double, double, double, G>(rowptr, m, col, v, x, epi, sched, subs);
 }
 template <typename VT, int G>
-__global__ void __launch_bounds__(256) k_sirt_resid_lp(const int64_t *rowptr, int32_t m,
+__global__ void __launch_bounds__(256, kOccLP) k_sirt_resid_lp(const int64_t *rowptr, int32_t m,
                                                        const int32_t *col, const VT *v,
                                                        const float *x, EpiResidLP epi,
-                                                       unsigned *sched) {
-    chunk_rows<VT, float, float, G>(rowptr, m, col, v, x, epi, sched);
+                                                       unsigned *sched, int subs) {
+    chunk_rows<VT, float, float, G>(rowptr, m, col, v, x, epi, sched, subs);
 }
 // Packed index stream (rows.cuh) with padded values.
 struct PkArgs {
@@ -104,56 +103,54 @@ struct PkArgs {
     int S, L;
 };
 template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256) k_sirt_resid_pk(PkArgs P, int32_t m, const VT *v,
+__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_resid_pk(PkArgs P, int32_t m, const VT *v,
                                                        const float *x, EpiResidLP epi,
-                                                       unsigned *sched) {
-    chunk_rows_pk<VT, float, float, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, x, epi, sched);
+                                                       unsigned *sched, int subs) {
+    chunk_rows_pk<VT, float, float, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, x, epi, sched, subs);
 }
 template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256) k_sirt_update_pk(PkArgs P, int32_t m, const VT *v,
+__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_update_pk(PkArgs P, int32_t m, const VT *v,
                                                         const float *r, EpiUpdateLP epi,
-                                                        unsigned *sched) {
-    chunk_rows_pk<VT, float, float, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, r, epi, sched);
+                                                        unsigned *sched, int subs) {
+    chunk_rows_pk<VT, float, float, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, r, epi, sched, subs);
 }
 template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256) k_sirt_resid_pkf(PkArgs P, int32_t m, const uint4 *rec,
+__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_resid_pkf(PkArgs P, int32_t m, const uint4 *rec,
                                                         const float *x, EpiResidLP epi,
-                                                        unsigned *sched) {
-    chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, x, epi, sched);
+                                                        unsigned *sched, int subs) {
+    chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, x, epi, sched, subs);
 }
 template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256) k_sirt_update_pkf(PkArgs P, int32_t m, const uint4 *rec,
+__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_update_pkf(PkArgs P, int32_t m, const uint4 *rec,
                                                          const float *r, EpiUpdateLP epi,
-                                                         unsigned *sched) {
-    chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, r, epi, sched);
+                                                         unsigned *sched, int subs) {
+    chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, r, epi, sched, subs);
 }
 template <int G, int NG>
-__global__ void __launch_bounds__(256) k_sirt_resid_pk64(PkArgs P, int32_t m, const double *v,
+__global__ void __launch_bounds__(256, kOcc64) k_sirt_resid_pk64(PkArgs P, int32_t m, const double *v,
                                                          const double *x, EpiResidF64 epi,
-                                                         unsigned *sched) {
-    chunk_rows_pk<double, double, double, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, x, epi,
-                                                 sched);
+                                                         unsigned *sched, int subs) {
+    chunk_rows_pk<double, double, double, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, x, epi, sched, subs);
 }
 template <int G, int NG>
-__global__ void __launch_bounds__(256) k_sirt_update_pk64(PkArgs P, int32_t m, const double *v,
+__global__ void __launch_bounds__(256, kOcc64) k_sirt_update_pk64(PkArgs P, int32_t m, const double *v,
                                                           const double *r, EpiUpdateF64 epi,
-                                                          unsigned *sched) {
-    chunk_rows_pk<double, double, double, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, r, epi,
-                                                 sched);
+                                                          unsigned *sched, int subs) {
+    chunk_rows_pk<double, double, double, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, r, epi, sched, subs);
 }
 template <int G>
-__global__ void __launch_bounds__(256) k_sirt_update_f64(const int64_t *rowptr, int32_t m,
+__global__ void __launch_bounds__(256, kOcc64) k_sirt_update_f64(const int64_t *rowptr, int32_t m,
                                                          const int32_t *col, const double *v,
                                                          const double *r, EpiUpdateF64 epi,
-                                                         unsigned *sched) {
-    chunk_rows<double, double, double, G>(rowptr, m, col, v, r, epi, sched);
+                                                         unsigned *sched, int subs) {
+    chunk_rows<double, double, double, G>(rowptr, m, col, v, r, epi, sched, subs);
 }
 template <typename VT, int G>
-__global__ void __launch_bounds__(256) k_sirt_update_lp(const int64_t *rowptr, int32_t m,
+__global__ void __launch_bounds__(256, kOccLP) k_sirt_update_lp(const int64_t *rowptr, int32_t m,
                                                         const int32_t *col, const VT *v,
                                                         const float *r, EpiUpdateLP epi,
-                                                        unsigned *sched) {
-    chunk_rows<VT, float, float, G>(rowptr, m, col, v, r, epi, sched);
+                                                        unsigned *sched, int subs) {
+    chunk_rows<VT, float, float, G>(rowptr, m, col, v, r, epi, sched, subs);
 }
 template <int G>
 __global__ void __launch_bounds__(256) k_gd_update(const int64_t *rowptr, int32_t m,
@@ -183,13 +180,6 @@ __global__ void __launch_bounds__(256) k_pm_spmv(const int64_t *rowptr, int32_t 
     if (flag && flag[0]) return;
     chunk_rows<double, double, double, G>(rowptr, m, col, v, x, epi);
     if (partials) block_partial(epi.part, partials);
-}
-
-__global__ void k_cimmino_M(double *M, int32_t m) {
-    // AIRMs.f90:1072: Mdiag = m * row_norms(2)**2
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
-         i += (int64_t)gridDim.x * blockDim.x)
-        M[i] = __dmul_rn((double)m, __dmul_rn(M[i], M[i]));
 }
 
 __global__ void k_to_f32v(const double *a, int64_t n, float *o) {
@@ -313,20 +303,6 @@ int elem_grid(int64_t n) {
 }  // namespace
 
 // ------------------------------------------------------------------ host ----
-int sirt_weights(const DevCSR &A, const DevCSR &AT, bool sart, double *d_M, double *d_D,
-                 cudaStream_t s) {
-    if (!sart) {
-        FAIR_TRY(csr_row_norms(A, 2, d_M, s));
-        if (A.m > 0) k_cimmino_M<<<elem_grid(A.m), 256, 0, s>>>(d_M, A.m);
-        FAIR_CUDA(cudaGetLastError());
-    } else {
-        // AIRMs.f90:1076-1079: row 1-norms, column 1-norms (via the transpose)
-        FAIR_TRY(csr_row_norms(A, 1, d_M, s));
-        FAIR_TRY(csr_row_norms(AT, 1, d_D, s));
-    }
-    return FAIR_OK;
-}
-
 __global__ void k_reciprocal(double *v, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -342,10 +318,11 @@ int vec_reciprocal(double *v, int64_t n, cudaStream_t s) {
 
 int sirt_weights_recip(const DevCSR &A, const DevCSR &AT, bool sart, double *d_Mi, double *d_Di,
                        cudaStream_t s) {
-    FAIR_TRY(sirt_weights(A, AT, sart, d_Mi, d_Di, s));
-    FAIR_TRY(vec_reciprocal(d_Mi, A.m, s));
-    if (sart) FAIR_TRY(vec_reciprocal(d_Di, A.n, s));
-    return FAIR_OK;
+    if (sart) {  // AIRMs.f90:1076-1079: row 1-norms, column 1-norms (via the transpose)
+        FAIR_TRY(csr_row_weights(A, 1, ROW_RECIP, d_Mi, s));
+        return csr_row_weights(AT, 1, ROW_RECIP, d_Di, s);
+    }
+    return csr_row_weights(A, 2, ROW_CIMMINO, d_Mi, s);  // :1072: M = m * row_norms(2)**2
 }
 
 int sirt_prepare_shadow(const SirtDev &S, cudaStream_t s) {
@@ -354,6 +331,38 @@ int sirt_prepare_shadow(const SirtDev &S, cudaStream_t s) {
         FAIR_CUDA(cudaGetLastError());
     }
     return FAIR_OK;
+}
+
+// A pass on the row engine (rows.cuh), kernel K, chunks of one round (32/G
+// rows): chunks of 32 rows left one per warp on images up to N = 400, and a pass
+// took as long as 8 rounds in series (N = 363, FP32, us per iteration: 274
+// against 177; N = 1024: 2783 against 2606). FAIR_ROWS_BY_GROUP=0: 32 rows, the
+// same results.
+// S.chained: the launch follows another pass of the same call, so it may start
+// (and read its matrix entries) while that one still runs (7 us of the 47 an
+// iteration took at fan N = 128).
+template <auto K, class... A>
+static void launch_rows(const SirtDev &S, int64_t m, int G, cudaStream_t s, A... args) {
+    static const int occ = [] {
+        int o = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, K, 256, 0);
+        return std::max(o, 1);
+    }();
+    const int64_t blocks = (int64_t)sm_count() * occ;
+    const int R = 32 / G;
+    const char *bg = getenv("FAIR_ROWS_BY_GROUP");
+    const int subs = bg && bg[0] == '0' ? G : 1;
+    const int64_t chunks = (m + subs * R - 1) / (subs * R);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((chunks + 7) / 8, blocks)));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = S.chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, K, args..., S.sched, subs);  // errors: the caller's cudaGetLastError
 }
 
 // One reduced-precision pass on the layout `code` selects (0 the CSR; 1, 2
@@ -389,20 +398,15 @@ static void lp_pass(const SirtDev &S, const DevCSR &M, int pass, const VT *vals,
         switch (code) {
             case 4:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (k_sirt_resid_pkf<VT, g_, 2><<<chunk_grid(k_sirt_resid_pkf<VT, g_, 2>, M.m), 256, 0, s>>>(
-                                           P, M.m, fused, S.x32, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 2>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
                 break;
             case 3:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (k_sirt_resid_pkf<VT, g_, 1><<<chunk_grid(k_sirt_resid_pkf<VT, g_, 1>, M.m), 256, 0, s>>>(
-                                           P, M.m, fused, S.x32, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 1>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
                 break;
-            case 2: FAIR_G_DISPATCH(G, (k_sirt_resid_pk<VT, g_, 2><<<chunk_grid(k_sirt_resid_pk<VT, g_, 2>, M.m), 256, 0, s>>>(
-                                           P, M.m, pvals, S.x32, e, S.sched))) break;
-            case 1: FAIR_G_DISPATCH(G, (k_sirt_resid_pk<VT, g_, 1><<<chunk_grid(k_sirt_resid_pk<VT, g_, 1>, M.m), 256, 0, s>>>(
-                                           P, M.m, pvals, S.x32, e, S.sched))) break;
-            default: FAIR_G_DISPATCH(G, (k_sirt_resid_lp<VT, g_><<<chunk_grid(k_sirt_resid_lp<VT, g_>, M.m), 256, 0, s>>>(
-                                            M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(), vals, S.x32, e, S.sched))) break;
+            case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 2>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
+            case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 1>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
+            default: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_lp<VT, g_>>(S, M.m, g_, s, M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(), vals, S.x32, e))) break;
         }
     } else {
         EpiUpdateLP e{S.D, S.x, S.x32, S.omg, S.lb, S.ub, S.bmode, scale};
@@ -410,20 +414,15 @@ static void lp_pass(const SirtDev &S, const DevCSR &M, int pass, const VT *vals,
         switch (code) {
             case 4:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (k_sirt_update_pkf<VT, g_, 2><<<chunk_grid(k_sirt_update_pkf<VT, g_, 2>, M.m), 256, 0, s>>>(
-                                           P, M.m, fused, r, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 2>>(S, M.m, g_, s, P, M.m, fused, r, e)))
                 break;
             case 3:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (k_sirt_update_pkf<VT, g_, 1><<<chunk_grid(k_sirt_update_pkf<VT, g_, 1>, M.m), 256, 0, s>>>(
-                                           P, M.m, fused, r, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 1>>(S, M.m, g_, s, P, M.m, fused, r, e)))
                 break;
-            case 2: FAIR_G_DISPATCH(G, (k_sirt_update_pk<VT, g_, 2><<<chunk_grid(k_sirt_update_pk<VT, g_, 2>, M.m), 256, 0, s>>>(
-                                           P, M.m, pvals, r, e, S.sched))) break;
-            case 1: FAIR_G_DISPATCH(G, (k_sirt_update_pk<VT, g_, 1><<<chunk_grid(k_sirt_update_pk<VT, g_, 1>, M.m), 256, 0, s>>>(
-                                           P, M.m, pvals, r, e, S.sched))) break;
-            default: FAIR_G_DISPATCH(G, (k_sirt_update_lp<VT, g_><<<chunk_grid(k_sirt_update_lp<VT, g_>, M.m), 256, 0, s>>>(
-                                            M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(), vals, r, e, S.sched))) break;
+            case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 2>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
+            case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 1>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
+            default: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_lp<VT, g_>>(S, M.m, g_, s, M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(), vals, r, e))) break;
         }
     }
 }
@@ -448,52 +447,26 @@ void sirt_pass(const SirtDev &S, int pass, cudaStream_t s) {
             if (pass == 1) {
                 EpiResidF64 e{S.b, S.Minv, (double *)S.r};
                 if (NG == 2)
-                    FAIR_G_DISPATCH(G, (k_sirt_resid_pk64<g_, 2><<<chunk_grid(k_sirt_resid_pk64<g_, 2>, M.m), 256, 0, s>>>(
-                                           P, M.m, pv, S.x, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk64<g_, 2>>(S, M.m, g_, s, P, M.m, pv, S.x, e)))
                 else
-                    FAIR_G_DISPATCH(G, (k_sirt_resid_pk64<g_, 1><<<chunk_grid(k_sirt_resid_pk64<g_, 1>, M.m), 256, 0, s>>>(
-                                           P, M.m, pv, S.x, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk64<g_, 1>>(S, M.m, g_, s, P, M.m, pv, S.x, e)))
             } else {
                 EpiUpdateF64 e{S.D, S.x, S.omg, S.lb, S.ub, S.bmode};
                 if (NG == 2)
-                    FAIR_G_DISPATCH(G, (k_sirt_update_pk64<g_, 2><<<chunk_grid(k_sirt_update_pk64<g_, 2>, M.m), 256, 0, s>>>(
-                                           P, M.m, pv, (const double *)S.r, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk64<g_, 2>>(S, M.m, g_, s, P, M.m, pv, (const double *)S.r, e)))
                 else
-                    FAIR_G_DISPATCH(G, (k_sirt_update_pk64<g_, 1><<<chunk_grid(k_sirt_update_pk64<g_, 1>, M.m), 256, 0, s>>>(
-                                           P, M.m, pv, (const double *)S.r, e, S.sched)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk64<g_, 1>>(S, M.m, g_, s, P, M.m, pv, (const double *)S.r, e)))
             }
             return;
         }
         const int64_t *rp = M.rowptr.as<int64_t>();
         const int32_t *cl = M.col.as<int32_t>();
-        // fewer 32-row chunks than 16 warps per SM: a group of rows per warp
-        // (FAIR_ROWS_BY_GROUP=0: the chunked engine for every matrix)
-        const char *bg = getenv("FAIR_ROWS_BY_GROUP");
-        if (!(bg && bg[0] == '0') && ((int64_t)M.m + 31) / 32 < (int64_t)sm_count() * 16) {
-            auto go = [&](auto kern, const double *xv, const auto &e) {
-                int occ = 0;
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, 0);
-                const int64_t units = ((int64_t)M.m * G + 31) / 32;  // groups of 32/G rows
-                const int64_t blocks = std::min<int64_t>((units + 7) / 8, (int64_t)sm_count() * std::max(occ, 1));
-                kern<<<(int)std::max<int64_t>(blocks, 1), 256, 0, s>>>(rp, M.m, cl, M.v64.as<double>(), xv, e);
-            };
-            if (pass == 1) {
-                const EpiResidF64 e{S.b, S.Minv, (double *)S.r};
-                FAIR_G_DISPATCH(G, go(k_sirt_rows_f64<g_, EpiResidF64>, S.x, e));
-            } else {
-                const EpiUpdateF64 e{S.D, S.x, S.omg, S.lb, S.ub, S.bmode};
-                FAIR_G_DISPATCH(G, go(k_sirt_rows_f64<g_, EpiUpdateF64>, (const double *)S.r, e));
-            }
-            return;
-        }
         if (pass == 1) {
             EpiResidF64 e{S.b, S.Minv, (double *)S.r};
-            FAIR_G_DISPATCH(G, (k_sirt_resid_f64<g_><<<chunk_grid(k_sirt_resid_f64<g_>, M.m), 256, 0, s>>>(
-                                                  rp, M.m, cl, M.v64.as<double>(), S.x, e, S.sched)));
+            FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_f64<g_>>(S, M.m, g_, s, rp, M.m, cl, M.v64.as<double>(), S.x, e)));
         } else {
             EpiUpdateF64 e{S.D, S.x, S.omg, S.lb, S.ub, S.bmode};
-            FAIR_G_DISPATCH(G, (k_sirt_update_f64<g_><<<chunk_grid(k_sirt_update_f64<g_>, M.m), 256, 0, s>>>(
-                                                  rp, M.m, cl, M.v64.as<double>(), (const double *)S.r, e, S.sched)));
+            FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_f64<g_>>(S, M.m, g_, s, rp, M.m, cl, M.v64.as<double>(), (const double *)S.r, e)));
         }
         return;
     }
@@ -551,9 +524,11 @@ int sirt_make_forms(DevCSR &A, DevCSR &AT, int prec, cudaStream_t s, bool all, b
 
 int sirt_iterations(const SirtDev &S, int K, cudaStream_t s) {
     FAIR_TRY(sirt_make_forms(const_cast<DevCSR &>(*S.A), const_cast<DevCSR &>(*S.AT), S.prec, s));
+    SirtDev P = S;
     for (int it = 0; it < K; ++it) {
-        sirt_pass(S, 1, s);
-        sirt_pass(S, 2, s);
+        sirt_pass(P, 1, s);
+        P.chained = true;
+        sirt_pass(P, 2, s);
         FAIR_CUDA(cudaGetLastError());
     }
     return FAIR_OK;
