@@ -137,7 +137,7 @@ __device__ __forceinline__ long long fx_of(double v, int E) {
     const long long f = sh < 64 ? (m >> sh) : 0LL;
     return b < 0 ? -f : f;
 }
-__device__ __forceinline__ long long fx_warp_sum(long long F) {  // |F| < 2^55 per lane
+__device__ __forceinline__ long long fx_warp_sum(long long F) {  // |F| < 2^60 per lane
     const unsigned l0 = __reduce_add_sync(0xffffffffu, (unsigned)(F & 0x3FFFFFF));
     const unsigned l1 = __reduce_add_sync(0xffffffffu, (unsigned)((F >> 26) & 0x3FFFFFF));
     const int l2 = __reduce_add_sync(0xffffffffu, (int)(F >> 52));
@@ -376,7 +376,8 @@ int sweep_warps() {
 // previous angle that cross its pixels, so about 30 (fan beam N=128) to 80
 // (N=512) steps share a level.
 //
-// The levels are exact, computed per sweep order in windows of 32 steps:
+// The levels are exact, computed per sweep order in windows of WR = 128 steps
+// (64 or 32 where a window's entries would not fit shared memory):
 //   k_lvl_setup (every SM, windows in parallel): each entry swaps a stamp
 //     into its column's cell of the block's table; a stamp of an earlier step
 //     of the window makes the entry "shared" and that step a predecessor; the
@@ -388,7 +389,10 @@ int sweep_warps() {
 //     shared memory, on a 16-block cluster), windows in order: a step's level
 //     is the largest, over the steps a of its window with a path to it, of
 //     base(a) + the path's length, base(a) = 1 + the table's level over a's
-//     first-touch columns; the last touches write the levels into the table;
+//     first-touch columns; the last touches write the levels into the table
+//     (a window costs two barriers and two rounds of scattered table accesses
+//     whatever it holds: fan N=512, 243,328 steps, 32.5 ms in windows of 32,
+//     13.9 ms in windows of 128);
 //   counting sort of the steps by level (level pointers, steps in level order).
 // The sweep (k_lvl_sweep) runs a group of G warps per step, the steps of a
 // level spread over the groups, on one thread-block cluster (a cluster barrier
@@ -403,7 +407,6 @@ struct WinRow {
 };
 static_assert(sizeof(WinRow) == 24, "WinRow layout");
 
-constexpr int kWinRows = 32;      // steps per window (one predecessor bit each)
 constexpr int kMinStepsPerLevel = 4;
 constexpr int kSetupThreads = 512;
 constexpr int kSetupWarps = kSetupThreads / 32;
@@ -432,8 +435,13 @@ __device__ __forceinline__ double fx_to_double_fast(long long total, int E) {
         return __longlong_as_double(bits + ((long long)(E - 1075) << 52));
     return fx_to_double(total, E);
 }
-__device__ __forceinline__ double fx_part_double(const FxPart &p) {
-    return p.e >= 0x7FF ? p.d : fx_to_double_fast(p.s, p.e);
+
+// The FP64 sum of the parts that hold an Inf or NaN term.
+__device__ __noinline__ double fx_special(const FxPart *parts, int G) {
+    double d = 0.0;
+    for (int w = 0; w < G; ++w)
+        if (parts[w].e >= 0x7FF) d += parts[w].d;
+    return d;
 }
 
 __device__ __forceinline__ void cluster_barrier() {
@@ -500,24 +508,25 @@ __global__ void k_step_lengths(const RowStep *__restrict__ steps, int32_t nord,
 // row repeats a column: *err is set and the single-block kernel applies the
 // sweep's updates in order instead. From the predecessors, the longest path
 // between every two steps of the window (dpath: 32 bytes per step).
+template <int WR>
 __global__ void __launch_bounds__(kSetupThreads) k_lvl_setup(
         const RowStep *__restrict__ steps, const int64_t *__restrict__ eoff, int32_t nord,
         const int32_t *__restrict__ col, unsigned long long *__restrict__ tabs, int32_t n,
         unsigned long long id0, int32_t *__restrict__ oidx, WinRow *__restrict__ rec,
-        signed char *__restrict__ dpath, int *err) {
+        unsigned char *__restrict__ dpath, int *err) {
     extern __shared__ __align__(16) unsigned char fl[];  // [entries of a window]
-    __shared__ int rb[kWinRows + 1];
-    __shared__ uint32_t msk[kWinRows];              // predecessor steps in the window
-    __shared__ signed char dps[kWinRows][kWinRows];  // longest path a -> r, -1: none
+    __shared__ int rb[WR + 1];
+    __shared__ uint32_t msk[WR][WR / 32];  // predecessor steps in the window
+    __shared__ uint32_t dps[WR][WR / 4];   // 1 + longest path a -> r, 0: none (a byte per a)
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     unsigned long long *tab = tabs + (size_t)blockIdx.x * (size_t)n;
-    const int nwin = (nord + kWinRows - 1) / kWinRows;
+    const int nwin = (nord + WR - 1) / WR;
     for (int q = blockIdx.x; q < nwin; q += gridDim.x) {
-        const int k0 = q * kWinRows, nr = min(kWinRows, nord - k0);
+        const int k0 = q * WR, nr = min(WR, nord - k0);
         const int64_t wbase = eoff[k0];
-        if (tid < kWinRows) {
+        if (tid < WR) {
             rb[tid + 1] = tid < nr ? (int)(eoff[k0 + tid + 1] - wbase) : 0;
-            msk[tid] = 0;
+            for (int w = 0; w < WR / 32; ++w) msk[tid][w] = 0;
             if (tid == 0) rb[0] = 0;
         }
         __syncthreads();
@@ -537,24 +546,29 @@ __global__ void __launch_bounds__(kSetupThreads) k_lvl_setup(
                     } else {
                         f = 2;
                         fl[old & ((1ull << kStampPosBits) - 1ull)] |= 1;  // its one writer
-                        atomicOr(&msk[r], 1u << orow);
+                        atomicOr(&msk[r][orow >> 5], 1u << (orow & 31));
                     }
                 }
                 fl[pos] = f;
             }
             __syncthreads();
         }
-        if (wid == 0) {  // longest paths within the window (rows in order)
+        if (wid == 0 && lane < WR / 4) {  // longest paths within the window (rows in order),
+                                          // four steps a per lane
+            constexpr unsigned LANES = WR / 4 == 32 ? 0xffffffffu : (1u << (WR / 4)) - 1u;
             for (int r = 0; r < nr; ++r) {
-                int v = lane == r ? 0 : -1;
-                for (uint32_t bits = msk[r]; bits; bits &= bits - 1u) {
-                    const int d = dps[__ffs(bits) - 1][lane];
-                    if (d >= 0) v = max(v, d + 1);
-                }
-                dps[r][lane] = (signed char)v;
-                __syncwarp();
+                uint32_t v = lane == r >> 2 ? 1u << (8 * (r & 3)) : 0u;
+#pragma unroll
+                for (int w = 0; w < WR / 32; ++w)
+                    for (uint32_t bits = msk[r][w]; bits; bits &= bits - 1u) {
+                        const uint32_t d = dps[32 * w + __ffs(bits) - 1][lane];
+                        v = __vmaxu4(v, __vaddus4(d, 0x01010101u) & __vcmpne4(d, 0u));
+                    }
+                dps[r][lane] = v;
+                __syncwarp(LANES);
             }
-            for (int r = 0; r < nr; ++r) dpath[(size_t)(k0 + r) * kWinRows + lane] = dps[r][lane];
+            for (int r = 0; r < nr; ++r)
+                reinterpret_cast<uint32_t *>(dpath + (size_t)(k0 + r) * WR)[lane] = dps[r][lane];
         }
         const unsigned lt = (1u << lane) - 1u;
         for (int r = wid; r < nr; r += kSetupWarps) {
@@ -595,86 +609,93 @@ __global__ void __launch_bounds__(kSetupThreads) k_lvl_setup(
     }
 }
 
-// The steps' levels, windows in order (one block of 1024 threads). lv: the
-// last level written into each column (shared memory when it fits, else
-// global memory, zeroed by the caller). A step's level is the largest, over
-// the steps a of its window with a path to it, of base(a) + the path's length,
-// where base(a) = 1 + the table's level over a's first-touch columns. The next
-// window's records are loaded while a window runs.
-template <bool SMEM>
+// The steps' levels, windows in order (one block of 1024 threads, warp w the
+// steps w, w + 32, ... of a window). lv: the last level written into each
+// column (shared memory when it fits, else global memory, zeroed by the
+// caller). A step's level is the largest, over the steps a of its window with a
+// path to it, of base(a) + the path's length, where base(a) = 1 + the table's
+// level over a's first-touch columns. The next window's records are loaded
+// while a window runs.
+template <int WR, bool SMEM>
 __global__ void __launch_bounds__(1024, 1) k_lvl_levels(
-        const WinRow *__restrict__ rec, const signed char *__restrict__ dpath,
+        const WinRow *__restrict__ rec, const unsigned char *__restrict__ dpath,
         const int32_t *__restrict__ oidx, int32_t nord, int32_t *lvg, int32_t n,
         int32_t *__restrict__ lvl, int *__restrict__ nlev) {
+    constexpr int SW = WR / 32;  // steps per warp
     extern __shared__ int32_t lvs[];
-    __shared__ int32_t base[kWinRows], lvw[kWinRows];
+    __shared__ int32_t base[WR];
+    __shared__ int s_top[32];
     int32_t *lv = SMEM ? lvs : lvg;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (SMEM)
         for (int32_t j = tid; j < n; j += 1024) lvs[j] = 0;
     const WinRow none{0, 0, 0, 0, 0};
-    const int nwin = (nord + kWinRows - 1) / kWinRows;
-    int nr1 = min(kWinRows, nord);
-    WinRow wn = wid < nr1 ? rec[wid] : none;
-    uint4 dn0 = make_uint4(0, 0, 0, 0), dn1 = dn0;
-    if (wid == 0 && lane < nr1) {
-        const uint4 *d = reinterpret_cast<const uint4 *>(dpath + (size_t)lane * kWinRows);
-        dn0 = d[0];
-        dn1 = d[1];
-    }
+    const int nwin = (nord + WR - 1) / WR;
+    WinRow wn[SW];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < SW; ++i) {
+            const int k = k0 + wid + 32 * i;
+            wn[i] = k < nord ? rec[k] : none;
+        }
+    };
+    fetch(0);
     __syncthreads();
     int top = 0;
     for (int q = 0; q < nwin; ++q) {
-        const int k0 = q * kWinRows, nr = nr1;
-        const WinRow w = wn;
-        const uint4 d0 = dn0, d1 = dn1;
-        if (q + 1 < nwin) {
-            nr1 = min(kWinRows, nord - k0 - kWinRows);
-            wn = wid < nr1 ? rec[k0 + kWinRows + wid] : none;
-            if (wid == 0 && lane < nr1) {
-                const uint4 *d = reinterpret_cast<const uint4 *>(
-                    dpath + (size_t)(k0 + kWinRows + lane) * kWinRows);
-                dn0 = d[0];
-                dn1 = d[1];
+        const int k0 = q * WR, nr = min(WR, nord - k0);
+        WinRow w[SW];
+        uint32_t d[SW];  // dpath of the warp's steps: step a = SW lane + j in byte j
+#pragma unroll
+        for (int i = 0; i < SW; ++i) {
+            w[i] = wn[i];
+            const int r = wid + 32 * i;
+            d[i] = 0;
+            if (r < nr) {
+                const unsigned char *p = dpath + (size_t)(k0 + r) * WR + SW * lane;
+                if constexpr (SW == 4) d[i] = *reinterpret_cast<const uint32_t *>(p);
+                else if constexpr (SW == 2) d[i] = *reinterpret_cast<const uint16_t *>(p);
+                else d[i] = *p;
             }
         }
-        if (wid < nr) {  // 1 + the table's level over the step's first-touch columns
+        if (q + 1 < nwin) fetch(k0 + WR);
+#pragma unroll
+        for (int i = 0; i < SW; ++i) {  // 1 + the table's level over the step's first-touch columns
+            const int r = wid + 32 * i;
+            if (r >= nr) break;
             int m = 0;
-            for (int e0 = lane; e0 < w.c2; e0 += 32 * 8) {  // 8 independent loads per lane
+            for (int e0 = lane; e0 < w[i].c2; e0 += 32 * 8) {  // 8 independent loads per lane
                 int32_t j[8];
 #pragma unroll
-                for (int t = 0; t < 8; ++t) j[t] = e0 + 32 * t < w.c2 ? oidx[w.off + e0 + 32 * t] : -1;
+                for (int t = 0; t < 8; ++t) j[t] = e0 + 32 * t < w[i].c2 ? oidx[w[i].off + e0 + 32 * t] : -1;
 #pragma unroll
                 for (int t = 0; t < 8; ++t)
                     if (j[t] >= 0) m = max(m, SMEM ? lvs[j[t]] : __ldcg(lvg + j[t]));
             }
             m = (int)__reduce_max_sync(0xffffffffu, (unsigned)m);
-            if (lane == 0) base[wid] = m + 1;
+            if (lane == 0) base[r] = m + 1;
         }
         __syncthreads();
-        if (wid == 0) {  // the longest paths within the window
-            const uint32_t dw[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-            int L = 0;
 #pragma unroll
-            for (int a = 0; a < kWinRows; ++a) {
-                const int dv = (int)(signed char)(dw[a >> 2] >> (8 * (a & 3)));
-                if (a < nr && dv >= 0) L = max(L, base[a] + dv);
+        for (int i = 0; i < SW; ++i) {
+            const int r = wid + 32 * i;
+            if (r >= nr) break;
+            unsigned v = 0;  // the longest path to the step (a path has length d - 1)
+#pragma unroll
+            for (int j = 0; j < SW; ++j) {
+                const unsigned dj = d[i] >> (8 * j) & 255u;
+                if (dj > 0) v = max(v, (unsigned)base[SW * lane + j] + dj - 1u);
             }
-            if (lane < nr) {
-                lvw[lane] = L;
-                lvl[k0 + lane] = L;
-            }
-            top = max(top, (int)__reduce_max_sync(0xffffffffu, lane < nr ? (unsigned)L : 0u));
-        }
-        __syncthreads();
-        if (wid < nr) {  // the last touches of the window write the step's level
-            const int L = lvw[wid];
-            for (int e0 = lane; e0 < w.len; e0 += 32 * 8) {
+            const int L = (int)__reduce_max_sync(0xffffffffu, v);
+            if (lane == 0) lvl[k0 + r] = L;
+            top = max(top, L);
+            // the last touches of the window write the step's level
+            for (int e0 = lane; e0 < w[i].len; e0 += 32 * 8) {
                 int32_t j[8];
 #pragma unroll
                 for (int t = 0; t < 8; ++t) {
                     const int e = e0 + 32 * t;
-                    j[t] = e < w.len && (e < w.c1 || e >= w.c3) ? oidx[w.off + e] : -1;
+                    j[t] = e < w[i].len && (e < w[i].c1 || e >= w[i].c3) ? oidx[w[i].off + e] : -1;
                 }
 #pragma unroll
                 for (int t = 0; t < 8; ++t)
@@ -683,31 +704,37 @@ __global__ void __launch_bounds__(1024, 1) k_lvl_levels(
         }
         __syncthreads();
     }
-    if (tid == 0) *nlev = top;
+    if (lane == 0) s_top[wid] = top;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < 32; ++w) top = max(top, s_top[w]);
+        *nlev = top;
+    }
 }
 
 // The same on a cluster of CS blocks (512 threads each), for a level table
 // in global memory: block c takes the steps c, c + CS, ... of every window
-// (16 * CS / 32 warps per step), so the scattered table reads and writes are
+// (16 * CS / WR warps per step), so the scattered table reads and writes are
 // spread over CS SMs. The steps' bases meet in distributed shared memory; a
 // cluster barrier after the bases and one after the table writes keep the
 // windows in order. *nlev must be zero at the start.
-template <int CS>
+template <int WR, int CS>
 __global__ void __launch_bounds__(512, 1) k_lvl_levels_cluster(
-        const WinRow *__restrict__ rec, const signed char *__restrict__ dpath,
+        const WinRow *__restrict__ rec, const unsigned char *__restrict__ dpath,
         const int32_t *__restrict__ oidx, int32_t nord, int32_t *lv, int32_t *__restrict__ lvl,
         int *__restrict__ nlev) {
-    constexpr int RW = (kWinRows + CS - 1) / CS;  // steps per block and window
-    constexpr int WPR = 16 / RW;                  // warps per step
-    static_assert(WPR >= 1 && RW * WPR <= 16, "cluster shape");
+    constexpr int RW = WR / CS;   // steps per block and window
+    constexpr int WPR = 16 / RW;  // warps per step
+    static_assert(CS == 16 && RW >= 2 && WPR >= 1 && RW * WPR == 16, "cluster shape");
     __shared__ int32_t base[RW], lvw[RW];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int rank = (int)cluster_rank();
     const int i = wid / WPR, sw = wid - i * WPR;  // the warp's step slot, warp in the step
     const WinRow none{0, 0, 0, 0, 0};
-    const int nwin = (nord + kWinRows - 1) / kWinRows;
+    const int nwin = (nord + WR - 1) / WR;
     int top = 0;
-    // distributed shared memory address of the base of step `lane` of a window
+    // distributed shared memory address of the base of step `lane` of a window;
+    // step lane + 32 j lies 2 j slots further in the same block
     uint32_t lane_base;
     {
         const uint32_t a = (uint32_t)__cvta_generic_to_shared(base);
@@ -715,52 +742,52 @@ __global__ void __launch_bounds__(512, 1) k_lvl_levels_cluster(
             : "=r"(lane_base)
             : "r"(a + 4u * (uint32_t)(lane / CS)), "r"((uint32_t)(lane % CS)));
     }
+    const int r = rank + CS * i;  // this warp's step in every window
+    WinRow wn = r < nord ? rec[r] : none;
     for (int q = 0; q < nwin; ++q) {
-        const int k0 = q * kWinRows, nr = min(kWinRows, nord - k0);
-        const int r = rank + CS * i;  // this warp's step in the window
-        const bool mine = i < RW && r < nr;
-        const WinRow w = mine ? rec[k0 + r] : none;
-        if (sw == 0 && lane == 0 && i < RW) base[i] = 0;
-        if (q + 1 < nwin && mine) {  // the next window's step of this warp: its columns into L2
-            const int r1 = r;
-            if (k0 + kWinRows + r1 < nord) {
-                const WinRow wn = rec[k0 + kWinRows + r1];
-                const char *c0 = reinterpret_cast<const char *>(oidx + wn.off);
-                const int nl = (wn.len * 4 + 127) >> 7;
-                for (int l = sw * 32 + lane; l < nl; l += 32 * WPR)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + ((size_t)l << 7)));
-            }
+        const int k0 = q * WR, nr = min(WR, nord - k0);
+        const bool mine = r < nr;
+        const WinRow w = mine ? wn : none;
+        if (sw == 0 && lane == 0) base[i] = 0;
+        if (k0 + WR + r < nord) {  // the next window's step of this warp: its columns into L2
+            wn = rec[k0 + WR + r];
+            const char *c0 = reinterpret_cast<const char *>(oidx + wn.off);
+            const int nl = (wn.len * 4 + 127) >> 7;
+            for (int l = sw * 32 + lane; l < nl; l += 32 * WPR)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + ((size_t)l << 7)));
         }
+        unsigned char d[WR / 32];
+        if (mine && sw == 0)
+#pragma unroll
+            for (int j = 0; j < WR / 32; ++j) d[j] = dpath[(size_t)(k0 + r) * WR + 32 * j + lane];
         __syncthreads();
         if (mine) {  // 1 + the table's level over the step's first-touch columns
             int m = 0;
-            for (int e0 = sw * 32 + lane; e0 < w.c2; e0 += 32 * WPR * 4) {
-                int32_t j[4];
+            for (int e0 = sw * 32 + lane; e0 < w.c2; e0 += 32 * WPR * 8) {
+                int32_t j[8];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
+                for (int t = 0; t < 8; ++t) {
                     const int e = e0 + 32 * WPR * t;
                     j[t] = e < w.c2 ? oidx[w.off + e] : -1;
                 }
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
+                for (int t = 0; t < 8; ++t)
                     if (j[t] >= 0) m = max(m, __ldcg(lv + j[t]));
             }
             m = (int)__reduce_max_sync(0xffffffffu, (unsigned)m);
             if (lane == 0) atomicMax(&base[i], m + 1);
         }
         cluster_barrier();
-        if (mine && sw == 0) {  // the longest paths within the window
-            const uint4 *dp = reinterpret_cast<const uint4 *>(dpath + (size_t)(k0 + r) * kWinRows);
-            const uint4 d0 = dp[0], d1 = dp[1];
-            const uint32_t dw[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-            int dv = 0;
+        if (mine && sw == 0) {  // the longest paths within the window (of length d - 1)
+            unsigned v = 0;
 #pragma unroll
-            for (int a = 0; a < kWinRows; ++a)
-                if (a == lane) dv = (int)(signed char)(dw[a >> 2] >> (8 * (a & 3)));
-            int bv = 0;
-            if (lane < nr && dv >= 0)
-                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bv) : "r"(lane_base));
-            const int L = (int)__reduce_max_sync(0xffffffffu, (lane < nr && dv >= 0) ? (unsigned)(bv + dv) : 0u);
+            for (int j = 0; j < WR / 32; ++j) {
+                int bv = 0;
+                if (d[j] > 0)
+                    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bv) : "r"(lane_base + 8u * j));
+                if (d[j] > 0) v = max(v, (unsigned)(bv + d[j] - 1));
+            }
+            const int L = (int)__reduce_max_sync(0xffffffffu, v);
             if (lane == 0) {
                 lvw[i] = L;
                 lvl[k0 + r] = L;
@@ -770,15 +797,15 @@ __global__ void __launch_bounds__(512, 1) k_lvl_levels_cluster(
         __syncthreads();
         if (mine) {  // the last touches of the window write the step's level
             const int L = lvw[i];
-            for (int e0 = sw * 32 + lane; e0 < w.len; e0 += 32 * WPR * 4) {
-                int32_t j[4];
+            for (int e0 = sw * 32 + lane; e0 < w.len; e0 += 32 * WPR * 8) {
+                int32_t j[8];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
+                for (int t = 0; t < 8; ++t) {
                     const int e = e0 + 32 * WPR * t;
                     j[t] = e < w.len && (e < w.c1 || e >= w.c3) ? oidx[w.off + e] : -1;
                 }
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
+                for (int t = 0; t < 8; ++t)
                     if (j[t] >= 0) lv[j[t]] = L;
             }
         }
@@ -801,6 +828,19 @@ __global__ void k_lvl_scatter(const RowStep *__restrict__ steps, const int32_t *
     }
 }
 
+
+// The schedule of the opposite direction: the levels and their steps in
+// reverse (a step's level is above those of the earlier steps it shares a
+// column with, so in reverse they come after it).
+__global__ void k_lvl_reverse(const RowStep *__restrict__ sched, const int64_t *__restrict__ lptr,
+                              const int *__restrict__ nlev, int32_t nord, RowStep *__restrict__ rsched,
+                              int64_t *__restrict__ rlptr, int *__restrict__ rnlev) {
+    const int L = *nlev;
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t k = t0; k < nord; k += nt) rsched[k] = sched[nord - 1 - k];
+    for (int64_t l = t0; l <= L; l += nt) rlptr[l] = nord - lptr[L - l];
+    if (t0 == 0) *rnlev = L;
+}
 
 // Where the level sweep keeps x: global memory read past L1 (XG), the
 // block's shared memory (XS, one block), or the cluster's distributed shared
@@ -882,7 +922,7 @@ template <int XM, int CACHE>
 __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__restrict__ col,
                                         const double *__restrict__ val, const XAcc<XM> &X,
                                         const Box &box, int lane, int G, int wg, FxPart *parts,
-                                        int bar, const LvlChunks<CACHE> &pre) {
+                                        double *coef, int bar, const LvlChunks<CACHE> &pre) {
     using R = typename XAcc<XM>::R;
     constexpr int B = 4;  // chunks per batch beyond the cached ones
     R cr[CACHE];
@@ -935,28 +975,34 @@ __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__rest
         }
     }
     const FxPart part = fx_warp_part(p0, p1, (wg == 0 && lane == 0) ? -st.b : 0.0);
-    double resid;
+    double c;
     if (G > 1) {
+        // the coefficient, by one warp of the group for all: the G parts one per
+        // lane, aligned and added by warp reductions. All 16 warps of a block
+        // at it (the conversion and the product are 64 cycles each of a
+        // sub-partition's FP64 pipe, and about 200 integer instructions where
+        // they are done without it) took 730 of a level's 5650 cycles at fan N=128
+        // and 1410 of 8800 at N=512 (sweeps 3.22 and 13.2 ms; one warp: 2.72 and
+        // 12.6 ms); groups take warps of different sub-partitions.
         if (lane == 0) parts[wg] = part;
         asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * G) : "memory");
-        int E = 0;
-        for (int w = 0; w < G; ++w) E = max(E, parts[w].e);
-        if (E >= 0x7FF) {
-            resid = 0.0;
-            for (int w = 0; w < G; ++w)
-                if (parts[w].e >= 0x7FF) resid += parts[w].d;
-        } else {
-            long long t = 0;
-            for (int w = 0; w < G; ++w) {
-                const int sh = E - parts[w].e;
-                if (sh < 64) t += parts[w].s >> sh;
+        if (wg == (bar & (G - 1))) {
+            const int e = lane < G ? parts[lane].e : 0;
+            const int E = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
+            double r;
+            if (E >= 0x7FF) {
+                r = fx_special(parts, G);
+            } else {
+                const int sh = E - e;
+                r = fx_to_double_fast(fx_warp_sum(lane < G && sh < 64 ? parts[lane].s >> sh : 0ll), E);
             }
-            resid = fx_to_double_fast(t, E);
+            if (lane == 0) *coef = __dmul_rn(-r, st.w);
         }
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * G) : "memory");
+        c = *(volatile double *)coef;
     } else {
-        resid = fx_part_double(part);
+        c = __dmul_rn(-(part.e >= 0x7FF ? part.d : fx_to_double_fast(part.s, part.e)), st.w);
     }
-    const double c = __dmul_rn(-resid, st.w);
 #pragma unroll
     for (int i = 0; i < CACHE; ++i) {
         if (i >= nmine) break;
@@ -985,42 +1031,35 @@ __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__rest
 }
 
 
-// The levels in order on one cluster of gridDim.x blocks (CLUSTER) or one
-// block. Groups of G consecutive warps take the steps of a level in turn; each
-// group's first step of a level is known two levels ahead and its first
-// chunks are loaded one level ahead (in registers). With x in
-// (distributed) shared memory (XM = XS or XD, cb = log2 of a block's part), x
-// is loaded at the start and written back at the end.
 // A barrier of all blocks of a cooperative launch on one counter, gbar[0]
 // (zero at the launch): block 0 adds 2^31 - (blocks - 1), every other block
 // 1, so the counter's top bit flips exactly when the last block arrives -- one
-// atomic per block and nothing to reset (the counter wraps). The arrival
-// follows a fence (the block's writes of the level are visible first); the
-// waiting thread reads the counter with acquire semantics. A block that waits
-// more than kGridSpinLimit polls, or sees *gerr set (checked every 1024
-// polls), sets *gerr and returns false; the sweep then stops, and the host
-// reports the error.
+// reduction per block, nothing to reset (the counter wraps) and, the barriers
+// being counted (phase: the top bit before this one), no value to wait for.
+// The arrival releases the block's writes of the level; the waiting thread
+// reads the counter with acquire semantics. A block that waits more than
+// kGridSpinLimit polls, or sees *gerr set (checked every 1024 polls), sets
+// *gerr and returns false; the sweep then stops, and the host reports the
+// error.
 constexpr unsigned long long kGridSpinLimit = 1ull << 26;
 enum { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
 
-__device__ __forceinline__ bool grid_barrier(unsigned *gbar, int *gerr) {
+__device__ __forceinline__ bool grid_barrier(unsigned *gbar, int *gerr, unsigned phase) {
     __shared__ int ok_s;
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u;
         int ok = 1;
-        __threadfence();
-        const unsigned old = atomicAdd(gbar, add);
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(gbar), "r"(add) : "memory");
         for (unsigned long long it = 1;; ++it) {
             unsigned cur;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(gbar) : "memory");
-            if ((cur ^ old) & 0x80000000u) break;
+            if ((cur >> 31) != phase) break;
             if ((it & 1023u) == 0 && (it > kGridSpinLimit || *(volatile int *)gerr)) {
                 atomicExch(gerr, 1);
                 ok = 0;
                 break;
             }
-            __nanosleep(32);
         }
         ok_s = ok;
     }
@@ -1028,6 +1067,12 @@ __device__ __forceinline__ bool grid_barrier(unsigned *gbar, int *gerr) {
     return ok_s != 0;
 }
 
+// The levels in order on one cluster of gridDim.x blocks (CLUSTER) or one
+// block. Groups of G consecutive warps take the steps of a level in turn; each
+// group's first step of a level is known two levels ahead and its first
+// chunks are loaded one level ahead (in registers). With x in
+// (distributed) shared memory (XM = XS or XD, cb = log2 of a block's part), x
+// is loaded at the start and written back at the end.
 template <int SYNC, int XM, int CACHE, int NT>
 __global__ void __launch_bounds__(NT, 1) k_lvl_sweep(
         const RowStep *__restrict__ sched, const int64_t *__restrict__ lptr,
@@ -1038,6 +1083,7 @@ __global__ void __launch_bounds__(NT, 1) k_lvl_sweep(
     constexpr bool CLUSTER = SYNC == SYNC_CLUSTER;
     extern __shared__ __align__(16) double xsm[];
     __shared__ FxPart parts[2][NW];  // per group: two rows' parts (by parity), G each
+    __shared__ double coef[2][NW];
     if (*err) return;
     const int nlev = *nlevp;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1084,12 +1130,12 @@ __global__ void __launch_bounds__(NT, 1) k_lvl_sweep(
         int par = 0;
         for (int64_t k = a0 + grp; k < a1; k += NG, par ^= 1) {
             if (k == a0 + grp) {
-                lvl_row<XM, CACHE>(cur, col, val, X, box, lane, G, wg, parts[par] + gl * G, bar, pc);
+                lvl_row<XM, CACHE>(cur, col, val, X, box, lane, G, wg, parts[par] + gl * G, &coef[par][gl], bar, pc);
             } else {
                 const RowStep st = sched[k];
                 LvlChunks<CACHE> pk;
                 lvl_load_chunks<CACHE>(st, col, val, lane, G, wg, pk);
-                lvl_row<XM, CACHE>(st, col, val, X, box, lane, G, wg, parts[par] + gl * G, bar, pk);
+                lvl_row<XM, CACHE>(st, col, val, X, box, lane, G, wg, parts[par] + gl * G, &coef[par][gl], bar, pk);
             }
         }
         if (nxt.len > 32 * G * CACHE) {  // the rest of the next level's first step: into L2
@@ -1103,7 +1149,7 @@ __global__ void __launch_bounds__(NT, 1) k_lvl_sweep(
         }
         if (SYNC == SYNC_CLUSTER) cluster_barrier();
         else if (SYNC == SYNC_GRID) {
-            if (!grid_barrier(gbar, gerr)) return;
+            if (!grid_barrier(gbar, gerr, (unsigned)l & 1u)) return;
         } else {
             __syncthreads();
         }
@@ -1315,9 +1361,10 @@ int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, con
 // The levels on a 16-block cluster (the level table in global memory);
 // false when no such cluster can be had (FAIR_SWEEP_CLUSTER below 16 also
 // keeps the single block).
+template <int WR>
 bool lvl_levels_cluster(SweepWork &W, int32_t nord, int *nlev, cudaStream_t s) {
     if (env_int("FAIR_SWEEP_CLUSTER", 16) < 16) return false;
-    auto kern = k_lvl_levels_cluster<16>;
+    auto kern = k_lvl_levels_cluster<WR, 16>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -1340,13 +1387,67 @@ bool lvl_levels_cluster(SweepWork &W, int32_t nord, int *nlev, cudaStream_t s) {
     }
     if (cudaMemsetAsync(nlev, 0, sizeof(int), s) != cudaSuccess ||
         cudaLaunchKernelEx(&cfg, kern, (const WinRow *)W.rec.as<WinRow>(),
-                           (const signed char *)W.dpath.as<signed char>(),
+                           (const unsigned char *)W.dpath.as<unsigned char>(),
                            (const int32_t *)W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(),
                            W.lvl.as<int32_t>(), nlev) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     return true;
+}
+
+// Set-up and levels in windows of WR steps. *built = false (and FAIR_OK) when
+// a buffer cannot be had.
+template <int WR>
+int lvl_build(const SweepDev &S, SweepWork &W, SweepWork::Levels &C, const RowStep *steps, size_t setup_smem,
+              size_t optin, bool want, bool *built, cudaStream_t s) {
+    const DevCSR &A = *S.A;
+    const int32_t nord = S.nord;
+    const int nwin = (nord + WR - 1) / WR;
+    const size_t tab_row = (size_t)std::max<int32_t>(A.n, 1) * sizeof(unsigned long long);
+    int blocks = std::min(nwin, 2 * sm_count());
+    blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)blocks, ((size_t)2 << 30) / tab_row));
+    *built = false;
+    if (W.dpath.grow((size_t)WR * ((size_t)nord + WR))) return FAIR_OK;
+    if (W.tab_n != A.n || W.tab_blocks < blocks || W.uid + (uint64_t)nwin >= kStampIdLimit) {
+        W.tabs.release();
+        W.tab_n = 0;
+        W.tab_blocks = 0;
+        if (W.tabs.grow(tab_row * (size_t)blocks)) return FAIR_OK;
+        FAIR_CUDA(cudaMemsetAsync(W.tabs.p, 0xFF, tab_row * (size_t)blocks, s));
+        W.tab_n = A.n;
+        W.tab_blocks = blocks;
+        W.uid = 0;
+    }
+    FAIR_CUDA(cudaFuncSetAttribute(k_lvl_setup<WR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)setup_smem));
+    k_lvl_setup<WR><<<blocks, kSetupThreads, setup_smem, s>>>(
+        steps, W.eoff.as<int64_t>(), nord, A.col.as<int32_t>(), W.tabs.as<unsigned long long>(), A.n, W.uid,
+        W.idx.as<int32_t>(), W.rec.as<WinRow>(), W.dpath.as<unsigned char>(), W.err.as<int>());
+    FAIR_CUDA(cudaGetLastError());
+    W.err_valid = true;
+    W.uid += (uint64_t)nwin;
+    *built = true;
+    if (!want) return FAIR_OK;
+    // on a cluster with the table in global memory; else in one block, the table
+    // in its shared memory where it fits
+    const size_t lv_bytes = 4 * (size_t)std::max<int32_t>(A.n, 1);
+    if (W.lvtab.grow(lv_bytes)) {
+        *built = false;
+        return FAIR_OK;
+    }
+    FAIR_CUDA(cudaMemsetAsync(W.lvtab.p, 0, lv_bytes, s));
+    if (!lvl_levels_cluster<WR>(W, nord, C.dnlev.as<int>(), s)) {
+        const bool smem = lv_bytes + 4096 <= optin;
+        auto kern = smem ? k_lvl_levels<WR, true> : k_lvl_levels<WR, false>;
+        if (smem)
+            FAIR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lv_bytes));
+        kern<<<1, 1024, smem ? lv_bytes : 0, s>>>(W.rec.as<WinRow>(), W.dpath.as<unsigned char>(),
+                                                  W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(), A.n,
+                                                  W.lvl.as<int32_t>(), C.dnlev.as<int>());
+    }
+    FAIR_CUDA(cudaGetLastError());
+    return FAIR_OK;
 }
 
 // Builds (or takes from the cache of this sweep order) the level schedule and
@@ -1368,72 +1469,56 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
     if (!cached) {
         C.key = 0;
         const int32_t nord = S.nord;
-        const int nwin = (nord + kWinRows - 1) / kWinRows;
-        const size_t tab_row = (size_t)std::max<int32_t>(A.n, 1) * sizeof(unsigned long long);
-        int blocks = std::min(nwin, 2 * sm_count());
-        blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)blocks, ((size_t)2 << 30) / tab_row));
-        const int64_t max_win = (int64_t)kWinRows * std::max(A.max_row, 1);
-        if (max_win >= (1 << kStampPosBits)) return FAIR_OK;
-        // the entries of this sweep: an upper bound from the longest row
-        const size_t ent = (size_t)nord * (size_t)std::max(A.max_row, 1);
-        if (W.lens.grow(4 * ((size_t)nord + 1)) || W.eoff.grow(8 * ((size_t)nord + 1)) ||
-            W.idx.grow(4 * ent) || W.rec.grow(sizeof(WinRow) * (size_t)nord) ||
-            W.dpath.grow((size_t)kWinRows * ((size_t)nord + kWinRows)) || W.lvl.grow(4 * (size_t)nord) ||
-            W.cnt.grow(4 * ((size_t)nord + 1)) || W.err.grow(sizeof(int)) ||
-            C.sched.grow(sizeof(RowStep) * (size_t)nord) || C.lptr.grow(8 * ((size_t)nord + 2)) ||
-            C.dnlev.grow(sizeof(int))) {
-            W.release();
-            return FAIR_OK;
+        const int g = (int)std::min<int64_t>((nord + 255) / 256, (int64_t)sm_count() * 4);
+        // the other direction's schedule of the same order, reversed
+        const SweepWork::Levels &O = W.lev[1 - slot];
+        if (S.order_key != 0 && O.key == S.order_key && O.nord == nord && W.err_valid) {
+            if (O.use) {
+                if (C.sched.grow(sizeof(RowStep) * (size_t)nord) || C.lptr.grow(8 * ((size_t)nord + 2)) ||
+                    C.dnlev.grow(sizeof(int)))
+                    return FAIR_OK;
+                k_lvl_reverse<<<g, 256, 0, s>>>(O.sched.as<RowStep>(), O.lptr.as<int64_t>(), O.dnlev.as<int>(),
+                                                nord, C.sched.as<RowStep>(), C.lptr.as<int64_t>(),
+                                                C.dnlev.as<int>());
+                FAIR_CUDA(cudaGetLastError());
+            }
+            C.nlev = O.nlev;
+            C.entries = O.entries;
+            C.use = O.use;
+            C.key = S.order_key;
+            C.nord = nord;
         }
-        if (W.tab_n != A.n || W.tab_blocks < blocks || W.uid + (uint64_t)nwin >= kStampIdLimit) {
-            W.tabs.release();
-            W.tab_n = 0;
-            W.tab_blocks = 0;
-            if (W.tabs.grow(tab_row * (size_t)blocks)) return FAIR_OK;
-            FAIR_CUDA(cudaMemsetAsync(W.tabs.p, 0xFF, tab_row * (size_t)blocks, s));
-            W.tab_n = A.n;
-            W.tab_blocks = blocks;
-            W.uid = 0;
-        }
+    }
+    if (S.order_key == 0 || C.key != S.order_key || C.nord != S.nord) {
+        const int32_t nord = S.nord;
+        const int g = (int)std::min<int64_t>((nord + 255) / 256, (int64_t)sm_count() * 4);
         int dev = 0, optin = 0;
         FAIR_CUDA(cudaGetDevice(&dev));
         FAIR_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        const int g = (int)std::min<int64_t>((nord + 255) / 256, (int64_t)sm_count() * 4);
+        // the widest window whose entries (a byte each) and stamps fit
+        const int64_t row_max = std::max(A.max_row, 1);
+        auto fits = [&](int wr) {
+            return wr * row_max < (1 << kStampPosBits) && wr * row_max + wr * wr + 24 * wr + 1024 <= optin;
+        };
+        const int wr = fits(128) ? 128 : fits(64) ? 64 : 32;
+        if (!fits(wr)) return FAIR_OK;
+        // the entries of this sweep: an upper bound from the longest row
+        const size_t ent = (size_t)nord * (size_t)row_max;
+        if (W.lens.grow(4 * ((size_t)nord + 1)) || W.eoff.grow(8 * ((size_t)nord + 1)) ||
+            W.idx.grow(4 * ent) || W.rec.grow(sizeof(WinRow) * (size_t)nord) || W.lvl.grow(4 * (size_t)nord) ||
+            W.cnt.grow(4 * ((size_t)nord + 1)) || W.err.grow(sizeof(int)) ||
+            C.sched.grow(sizeof(RowStep) * (size_t)nord) || C.lptr.grow(8 * ((size_t)nord + 2)) ||
+            C.dnlev.grow(sizeof(int)))
+            return FAIR_OK;
         k_step_lengths<<<g, 256, 0, s>>>(steps, nord, W.lens.as<int32_t>());
         k_scan_excl<<<1, 1024, 0, s>>>(W.lens.as<int32_t>(), nord, nullptr, W.eoff.as<int64_t>());
         FAIR_CUDA(cudaMemsetAsync(W.err.p, 0, sizeof(int), s));
-        const size_t setup_smem = (size_t)max_win;
-        if (setup_smem + 1024 > (size_t)optin) return FAIR_OK;
-        FAIR_CUDA(cudaFuncSetAttribute(k_lvl_setup, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)setup_smem));
-        k_lvl_setup<<<blocks, kSetupThreads, setup_smem, s>>>(
-            steps, W.eoff.as<int64_t>(), nord, A.col.as<int32_t>(), W.tabs.as<unsigned long long>(),
-            A.n, W.uid, W.idx.as<int32_t>(), W.rec.as<WinRow>(), W.dpath.as<signed char>(),
-            W.err.as<int>());
-        FAIR_CUDA(cudaGetLastError());
-        W.err_valid = true;
-        W.uid += (uint64_t)nwin;
-        if (!want) return FAIR_OK;
-        const size_t lv_bytes = 4 * (size_t)std::max<int32_t>(A.n, 1);
-        if (lv_bytes + 2048 <= (size_t)optin) {
-            FAIR_CUDA(cudaFuncSetAttribute(k_lvl_levels<true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lv_bytes));
-            k_lvl_levels<true><<<1, 1024, lv_bytes, s>>>(W.rec.as<WinRow>(), W.dpath.as<signed char>(),
-                                                        W.idx.as<int32_t>(), nord, nullptr, A.n,
-                                                        W.lvl.as<int32_t>(), C.dnlev.as<int>());
-        } else {
-            if (W.lvtab.grow(lv_bytes)) {
-                W.release();
-                return FAIR_OK;
-            }
-            FAIR_CUDA(cudaMemsetAsync(W.lvtab.p, 0, lv_bytes, s));
-            if (!lvl_levels_cluster(W, nord, C.dnlev.as<int>(), s))
-                k_lvl_levels<false><<<1, 1024, 0, s>>>(W.rec.as<WinRow>(), W.dpath.as<signed char>(),
-                                                      W.idx.as<int32_t>(), nord,
-                                                      W.lvtab.as<int32_t>(), A.n,
-                                                      W.lvl.as<int32_t>(), C.dnlev.as<int>());
-        }
-        FAIR_CUDA(cudaGetLastError());
+        const size_t smem = (size_t)(wr * row_max);
+        bool built = false;
+        if (wr == 128) FAIR_TRY(lvl_build<128>(S, W, C, steps, smem, optin, want, &built, s));
+        else if (wr == 64) FAIR_TRY(lvl_build<64>(S, W, C, steps, smem, optin, want, &built, s));
+        else FAIR_TRY(lvl_build<32>(S, W, C, steps, smem, optin, want, &built, s));
+        if (!built || !want) return FAIR_OK;
         FAIR_CUDA(cudaMemsetAsync(W.cnt.p, 0, 4 * ((size_t)nord + 1), s));
         k_lvl_count<<<g, 256, 0, s>>>(W.lvl.as<int32_t>(), nord, W.cnt.as<int32_t>());
         k_scan_excl<<<1, 1024, 0, s>>>(W.cnt.as<int32_t>(), 0, C.dnlev.as<int>(), C.lptr.as<int64_t>());
