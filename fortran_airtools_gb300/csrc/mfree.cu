@@ -22,14 +22,16 @@
 // evaluated in 64-bit fixed point with 46 fractional bits (N <= 8192 and
 // p <= 16384 keep every term below 2^60): exact integer
 // arithmetic, so every kernel computes bit-identical entries whatever the
-// order it meets the (ray, pixel) pairs in. The projector runs one thread
-// per ray and walks the image along the ray's faster axis (per column when
-// |sin| >= |cos|, else per row); at each step the only pixels within H2 of
-// the ray are the two that bracket its crossing, which the walk tracks
-// exactly with one 64-bit add per step. The backprojector runs one thread per
-// 4 pixels of an image column and, per angle, evaluates the two rays whose
-// offsets bracket each pixel's. Both keep only pairs with L > 0, so they sum
-// the same entries: an exact adjoint pair, deterministic, without atomics.
+// order it meets the (ray, pixel) pairs in. The projector walks the image
+// along each ray's faster axis (per column when |sin| >= |cos|, else per row);
+// at each step the only pixels within H2 of the ray are the two that bracket
+// its crossing, which the walk tracks exactly with one 64-bit add per step
+// (FP32: a warp walks 32 adjacent rays in step; FP64: a thread a ray). The
+// backprojector evaluates, per pixel and angle, the two rays whose offsets
+// bracket the pixel's (FP32: tiles of 32 x 32 pixels, their bins staged in
+// shared memory; FP64: a thread per 4 pixels of a column). Both keep only pairs
+// with L > 0, so they sum the same entries: an exact adjoint pair,
+// deterministic, without atomics.
 //
 // Fan beam (fanlineartomo, system_generation.f90:79-307): ray (i, j) is the
 // line through the rotated source P_i with direction u_ij = R(omega_j) u0_i,
@@ -38,17 +40,16 @@
 // K_ij = n . ((1/2 - N/2, 1/2 - N/2) - P_i) give d = ix*n_x + iy*n_y + K_ij,
 // the same fixed-point form, one record per ray. The projector walks each ray
 // as above (and the rays that walk image rows read a transposed copy of x, so
-// that a warp's rays gather adjacent addresses); the backprojector finds, per
-// pixel and angle, the rays whose bin
-// angle omega_j lies within asin(0.7072/|c - P_i|) (+ 2e-4) of the angle of
-// the pixel centre c seen from the source (a binary search over the bin
-// angles, sorted once: the reference's odd-p angles are not monotone in j),
-// and tests them with the exact distance.
+// that a warp's rays gather adjacent addresses); the backprojector stages, per
+// tile and angle, the rays whose bin angles the tile can see from the source
+// (the reference's odd-p angles are not monotone in j: they are sorted once),
+// and every pixel tests those within its own window with the exact distance.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "fair_internal.cuh"
@@ -67,9 +68,9 @@ constexpr double kOne = 70368744177664.0;  // 2^46
 struct __align__(16) MfAngle {
     long long C, S;      // cos, sin in fixed point
     long long K, H2;     // K_i; (c + s)/2 in fixed point
-    int H2s;             // H2 truncated to 30 fractional bits (FP32 entries)
+    int H2s;             // H2 cut to 31 fractional bits (FP32 entries)
     float inv_c;         // 1/c
-    float ramp30;        // 2^-30 / s (0 when s = 0)
+    float ramp;          // 2^-31 / s (0 on axis-aligned lines)
     int tie;             // s = 0: +1 / -1 = sign of d that keeps |d| = 1/2; 0 otherwise
     long long H1;        // (c - s)/2 in fixed point
     long long Hcut;      // |d| >= Hcut leaves a segment of at most 1e-10: dropped
@@ -93,7 +94,7 @@ __device__ __forceinline__ MfAngle mf_load(const MfAngle *p) {
     A.H2 = ll(b.z, b.w);
     A.H2s = c.x;
     A.inv_c = __int_as_float(c.y);
-    A.ramp30 = __int_as_float(c.z);
+    A.ramp = __int_as_float(c.z);
     A.tie = c.w;
     if constexpr (sizeof(T) == 8) {
         const int4 d = __ldg(q + 3), e = __ldg(q + 4);
@@ -108,29 +109,16 @@ __device__ __forceinline__ MfAngle mf_load(const MfAngle *p) {
 template <typename T> struct Chord;
 // The chord of a unit pixel at |d| = ad < 2^47 from the line: ramp() for s > 0,
 // tied() for an axis-aligned line (s = 0), where tu = H2 when a ray on the
-// pixel's edge, on this side of it, keeps the pixel (else -1); at() picks one.
-// FP32 entries evaluate the ramp on the exact distance truncated to 30
-// fractional bits, as (1/c) sat((H2 - |d|) / s) with sat() the clamp to
-// [0, 1] (two multiplies on the FMA pipe; the cut of segments below 1e-10 is
-// left to the FP64 entries); every kernel evaluates the same expression on
-// the same exact value, so they agree bit for bit.
-template <> struct Chord<float> {
-    static __device__ __forceinline__ float ramp(const MfAngle &A, long long ad) {
-        const int u = (int)(ad >> 16);
-        return A.inv_c * __saturatef((float)(A.H2s - u) * A.ramp30);
-    }
-    static __device__ __forceinline__ float tied(const MfAngle &A, long long ad, long long tu) {
-        return ad < A.H2 || ad == tu ? A.inv_c : 0.f;
-    }
-    static __device__ __forceinline__ float at(const MfAngle &A, long long ad, long long tu) {
-        return A.tie != 0 ? tied(A, ad, tu) : ramp(A, ad);
-    }
-    static __device__ __forceinline__ float of(const MfAngle &A, long long d) {
-        const long long ad = d < 0 ? -d : d;
-        if (ad >= (1LL << 47)) return 0.f;  // more than two pixels away
-        return at(A, ad, A.tie == (d > 0 ? 1 : -1) ? A.H2 : -1);
-    }
-};
+// pixel's edge, on this side of it, keeps the pixel (else -1).
+//
+// FP32 entries are (1/c) sat((H2 - u) / s), sat() the clamp to [0, 1], on the
+// exact distance cut to 31 fractional bits: u = floor(d) for d >= 0 and
+// -floor(d) - 1 (a one's complement: no negation, no carry) for d < 0, in units
+// of 2^-31. H2 - u is exact in 32 bits, so an entry is one integer subtraction,
+// one conversion and one saturated multiply-add (an axis-aligned ray has ramp 0
+// and its entry, 0 or 1, as the addend); the cut of segments below 1e-10 is left
+// to the FP64 entries. Every kernel evaluates the same expression on the same
+// exact value, so they agree bit for bit.
 template <> struct Chord<double> {
     static __device__ __forceinline__ double ramp(const MfAngle &A, long long ad) {
         const double w = ad <= A.H1 ? A.inv_c64 : (double)(A.H2 - ad) * A.scale_ramp64;
@@ -138,13 +126,6 @@ template <> struct Chord<double> {
     }
     static __device__ __forceinline__ double tied(const MfAngle &A, long long ad, long long tu) {
         return ad < A.H2 || ad == tu ? A.inv_c64 : 0.0;
-    }
-    static __device__ __forceinline__ double at(const MfAngle &A, long long ad, long long tu) {
-        return A.tie != 0 ? tied(A, ad, tu) : ramp(A, ad);
-    }
-    static __device__ __forceinline__ double of(const MfAngle &A, long long d) {
-        const long long ad = d < 0 ? -d : d;
-        return at(A, ad, A.tie == (d > 0 ? 1 : -1) ? A.H2 : -1);
     }
 };
 
@@ -302,20 +283,369 @@ __global__ void __launch_bounds__(128) k_mf_project(const MfAngle *__restrict__ 
 }
 
 // xt = the transpose of x viewed as an N x N array (32 x 32 tiles through
-// shared memory, both sides coalesced).
+// shared memory, both sides coalesced). *nonfinite becomes epoch (the pass's
+// number, larger than any before) if x holds an Inf or NaN.
 template <typename T>
 __global__ void __launch_bounds__(256) k_mf_transpose(const T *__restrict__ x, T *__restrict__ xt,
-                                                      int N) {
+                                                      int N, unsigned *nonfinite, unsigned epoch) {
     __shared__ T tile[32][33];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
         const int r = r0 + k, c = c0 + threadIdx.x;
-        if (r < N && c < N) tile[k][threadIdx.x] = x[(int64_t)r * N + c];
+        if (r < N && c < N) {
+            const T v = x[(int64_t)r * N + c];
+            tile[k][threadIdx.x] = v;
+            if (sizeof(T) == 4 && !isfinite(v)) atomicMax(nonfinite, epoch);
+        }
     }
     __syncthreads();
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
         const int r = c0 + k, c = r0 + threadIdx.x;
         if (r < N && c < N) xt[(int64_t)r * N + c] = tile[threadIdx.x][k];
+    }
+}
+
+// FP32 projector. A warp takes 32 adjacent rays of one angle and walks their
+// image columns (or rows) in step, over the union of the rays' ranges, so that
+// its lanes always gather neighbouring pixels. A ray's distance at its lower
+// candidate, E in [0, Qa), is kept in units of 2^-63: the high word is the
+// entry's u, and one 64-bit add forms H2 - u of the upper candidate (Cb + E).
+// (sq = 1: the lower candidate lies at d = -E, and E - 1 is kept, whose high
+// word is the one's complement rule's u; E = 0 is then the upper candidate of
+// the pixel below, at d = 0.) Steps on which both candidates of all 32 rays
+// lie in the image -- nearly all -- run without bounds checks, and without the
+// test for entries 0 when x is finite (0 x adds nothing); the ends, and any x
+// with Inf or NaN, take the checked step, which reads x only at positive
+// entries, as a stored matrix does.
+// Bound by integer issue. N = 1024, 720 angles, 1448 bins: 1.23 ms with every
+// ray walking from its own start (47 instructions and 12 L1 wavefronts per warp
+// step) -> 0.59 ms (25 and 3); fan beam N = 512, 720 angles: 0.33 -> 0.21 ms.
+// Eight steps' loads in flight and 7 blocks per SM: 592 us, four 608 (8 blocks)
+// and 643 (9); the checked steps one at a time cost another 110 us.
+constexpr int kWalkUnroll = 8;  // interior steps whose loads are in flight together
+struct Walk32 {
+    long long E, Fw, Qa, Cb;  // E (see above); what a step takes off it; Qa; the upper candidate's constant
+    int H2s;
+    float ramp, aa, ab;       // entry = sat((H2s - u) ramp + a)
+    int ua;
+};
+template <bool COL>
+__device__ __forceinline__ float mf_walk32(Walk32 w, bool on, const float *__restrict__ x, int qt, int dqt,
+                                           int N, int steps, int k0, int k1) {
+    constexpr int su = COL ? -1 : 1;
+    float s0 = 0.f, s1 = 0.f;
+    auto entries = [&](float &wa, float &wb) {
+        wa = __saturatef(fmaf((float)(w.H2s - (int)(w.E >> 32)), w.ramp, w.aa));
+        wb = __saturatef(fmaf((float)(int)((w.Cb + w.E) >> 32), w.ramp, w.ab));
+    };
+    auto advance = [&] {
+        w.E -= w.Fw;
+        if (w.E < 0) {
+            w.E += w.Qa;
+            --w.ua;
+        }
+        qt += dqt;
+    };
+    auto checked = [&](int n) {  // four steps' loads in flight together
+#pragma unroll 1
+        for (; n > 0; n -= 4) {
+            float wa[4], wb[4], xa[4], xb[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                entries(wa[t], wb[t]);
+                const int q = qt + w.ua * su;
+                const bool h = on && t < n;
+                xa[t] = h && (unsigned)w.ua < (unsigned)N && wa[t] > 0.f ? __ldg(x + q) : 0.f;
+                xb[t] = h && (unsigned)(w.ua + 1) < (unsigned)N && wb[t] > 0.f ? __ldg(x + q + su) : 0.f;
+                if (t < n) advance();
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                s0 = fmaf(wa[t], xa[t], s0);
+                s1 = fmaf(wb[t], xb[t], s1);
+            }
+        }
+    };
+    checked(k0);
+    unsigned q = 4u * (unsigned)(qt + w.ua * su);
+    const unsigned dq = 4u * (unsigned)dqt;
+    const char *xc = reinterpret_cast<const char *>(x);
+#pragma unroll kWalkUnroll
+    for (int n = k1 - k0; n > 0; --n) {
+        float wa, wb;
+        entries(wa, wb);
+        const float *px = reinterpret_cast<const float *>(xc + q);
+        s0 = fmaf(wa, __ldg(px), s0);
+        s1 = fmaf(wb, __ldg(px + su), s1);
+        w.E -= w.Fw;
+        q += dq;
+        if (w.E < 0) {
+            w.E += w.Qa;
+            q -= 4u * (unsigned)su;
+        }
+    }
+    qt += (k1 - k0) * dqt;
+    w.ua = (((int)q >> 2) - qt) * su;  // (q may be -4 here: one before the image)
+    checked(steps - k1);
+    return s0 + s1;
+}
+
+template <bool FAN, class Epi>
+__global__ void __launch_bounds__(128, 7) k_mf_project32(const MfAngle *__restrict__ ang, int nth, int p,
+                                                      int N, const float *__restrict__ x,
+                                                      const float *__restrict__ xt,
+                                                      const unsigned *__restrict__ nonfinite, unsigned epoch,
+                                                      Epi epi) {
+    const int lane = threadIdx.x & 31, wpa = (p + 31) / 32;
+    const int64_t nw = (int64_t)nth * wpa;
+    const bool guard = *nonfinite == epoch;
+    for (int64_t g = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); g < nw;
+         g += (int64_t)gridDim.x * (blockDim.x >> 5)) {
+        const int i = (int)(g / wpa), j = (int)(g - (int64_t)i * wpa) * 32 + lane;
+        const bool ray = j < p;
+        const int64_t r = (int64_t)i * p + (ray ? j : p - 1);
+        const MfAngle &A = ang[FAN ? r : i];
+        const long long K = FAN ? A.K : A.K - ((long long)j << kFix);
+        const float Kf = FAN ? A.Kf : A.Kf - (float)j;
+        const bool col = A.by_column != 0;
+        const long long F = col ? A.C : A.S, Q = col ? A.S : A.C;
+        const float Ff = col ? A.Cf : A.Sf, Qf = col ? A.Sf : A.Cf;
+        const int sq = Q > 0 ? 1 : -1;
+        const long long Qa = Q > 0 ? Q : -Q, Fp = sq * F, Gk = sq * K;
+        const float Qaf = fabsf(Qf), Fpf = sq * Ff, Gkf = sq * Kf;
+        // steps with u* in [-1, N): -N Qa < t Fp + Gk <= Qa (widened by 0.05)
+        const float lo = -(float)N * Qaf - 0.05f - Gkf, hi = Qaf + 0.05f - Gkf;
+        float ta = 0.f, tb = (float)(N - 1);
+        if (Fpf > 0.f) {
+            ta = fmaxf(ta, lo / Fpf);
+            tb = fminf(tb, hi / Fpf);
+        } else if (Fpf < 0.f) {
+            ta = fmaxf(ta, hi / Fpf);
+            tb = fminf(tb, lo / Fpf);
+        } else if (!(lo < 0.f && hi >= 0.f)) {
+            tb = -1.f;
+        }
+        const int t0 = max(0, (int)floorf(ta)), t1 = min(N - 1, (int)ceilf(tb));
+        const bool live = ray && t0 <= t1;
+        const bool up = Fp >= 0;
+        const int kind = (col ? 2 : 0) + (up ? 1 : 0);  // one per parallel angle, up to four in a fan's warp
+        float acc = 0.f;
+        unsigned todo = __ballot_sync(0xffffffffu, live);
+        while (todo) {
+            const int kd = __shfl_sync(0xffffffffu, kind, __ffs(todo) - 1);
+            const bool on = live && kind == kd;
+            todo &= ~__ballot_sync(0xffffffffu, on);
+            const int T0 = __reduce_min_sync(0xffffffffu, on ? t0 : N);
+            const int T1 = __reduce_max_sync(0xffffffffu, on ? t1 : -1);
+            const bool kup = (kd & 1) != 0, kcol = (kd & 2) != 0;
+            const int ts = kup ? T0 : T1, dir = kup ? 1 : -1, steps = T1 - T0 + 1;
+            Walk32 w{0, 0, 0, 0, 0, 0.f, 0.f, 0.f, 0};
+            int k0 = 0, k1 = steps;
+            if (on) {
+                const long long G = (long long)ts * Fp + Gk, Fw = up ? Fp : -Fp;
+                w.ua = (int)floorf(-(float)G / (float)Qa);
+                long long e = G + (long long)w.ua * Qa;
+                while (e > 0) { --w.ua; e -= Qa; }
+                while (e <= -Qa) { ++w.ua; e += Qa; }
+                w.E = -e;  // in [0, Qa)
+                if (A.tie != 0) {  // Fw = 0: the same two entries on every step
+                    const long long tua = A.tie == -sq ? A.H2 : -1, tub = A.tie == sq ? A.H2 : -1;
+                    w.aa = w.E < A.H2 || w.E == tua ? 1.f : 0.f;
+                    w.ab = Qa - w.E < A.H2 || Qa - w.E == tub ? 1.f : 0.f;
+                    w.E = 0;
+                } else {
+                    w.Qa = Qa << 17;
+                    w.Fw = Fw << 17;
+                    w.E = (w.E << 17) - (sq > 0 ? 1 : 0);
+                    if (w.E < 0) {
+                        w.E += w.Qa;
+                        --w.ua;
+                    }
+                    w.H2s = A.H2s;
+                    w.ramp = A.ramp;
+                    w.Cb = (((long long)A.H2s << 32) | 0xFFFFFFFFLL) - w.Qa + 1;
+                }
+                // steps with both candidates inside for sure: -(G + k Fw)/Qa in [0.1, N - 2.1]
+                const float Gf = (float)G, qf = (float)Qa, ff = (float)Fw, kmax = (float)steps;
+                const float a = -((float)N - 2.1f) * qf - Gf, b = -0.1f * qf - Gf;
+                float f0, f1;
+                if (Fw > 0) {
+                    f0 = ceilf(a / ff);
+                    f1 = floorf(b / ff) + 1.f;
+                } else {
+                    f0 = a <= 0.f ? 0.f : kmax;
+                    f1 = b >= 0.f ? kmax : 0.f;
+                }
+                k0 = (int)fminf(fmaxf(f0, 0.f), kmax);
+                k1 = (int)fminf(fmaxf(f1, 0.f), kmax);
+            }
+            k0 = __reduce_max_sync(0xffffffffu, k0);
+            k1 = __reduce_min_sync(0xffffffffu, k1);
+            if (guard || k1 <= k0) k0 = k1 = 0;
+            float v;
+            // pixel (t, u): element qt + u su of x (columns) or xt (rows)
+            if (kcol) v = mf_walk32<true>(w, on, x, ts * N + N - 1, dir * N, N, steps, k0, k1);
+            else v = mf_walk32<false>(w, on, xt, (N - 1 - ts) * N, -dir * N, N, steps, k0, k1);
+            if (on) acc = v * A.inv_c;
+        }
+        if (ray) epi(r, acc);
+    }
+}
+
+// FP32 backprojector, parallel beam. A block takes a tile of 32 pixel rows (a
+// warp's lanes) by 32 image columns (8 per warp) and walks its share of the
+// angles in batches of kBpBatch, the next batch's loads in flight: the at most
+// 46 bins of an angle that meet the tile are staged in shared memory as pairs
+// (y_j, y_{j+1}) / c, so that a pixel reads its two rays' values with one load
+// and no bounds check. A thread's distance D = jh + dl is kept as three words
+// (jh relative to the tile's first bin, 32 bits of dl, the rest), stepped by
+// cos from column to column with one three-word add: no shifts or masks but
+// the one that cuts dl to 31 bits. A batch with an Inf or NaN in its staged
+// values reads y itself, only where the entry is positive, as a stored
+// matrix does.
+// Bound by integer issue. N = 1024, 720 angles, 1448 bins: 0.92 ms with a
+// thread per 4 pixels reading y from L1, 35 instructions per pixel and angle ->
+// 0.46 ms, 19 of them (4 shares of the angles, their sums added by k_mf_finish).
+constexpr int kBpBatch = 8;   // angles staged at once (half a warp each)
+constexpr int kBpOcc = 7;     // resident blocks per SM (72 registers; 8 of 64: 4% slower)
+constexpr int kBpBins = 48;   // bins of an angle that meet a tile: 31 (|cos| + |sin|) + 2 at most
+struct __align__(16) BpAngle {
+    unsigned c_lo, c_mid;     // cos as three words (the fraction's bits 46.. at the top of c_mid)
+    int c_hi, H2s;
+    int Hc;                   // H2s - (2^31 - 1): entry of the second ray from u of the first
+    float ramp, a0, a1;       // entries sat((H2s - u) ramp + a0), sat((Hc + u) ramp + a1)
+    long long S;
+    int jlo;                  // first staged bin
+    float inv_c;
+    long long Dw[4];          // distance at the warps' first pixels, from bin jlo
+};
+template <class Epi>
+__global__ void __launch_bounds__(128, kBpOcc) k_mf_backproject32(const MfAngle *__restrict__ ang, int nth, int p,
+                                                             int N, const float *__restrict__ y, float *part,
+                                                             Epi epi) {
+    __shared__ BpAngle cs[2][kBpBatch];
+    __shared__ float2 ys[2][kBpBatch][kBpBins];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int nt = (N + 31) / 32, tx = blockIdx.x / nt, ty = blockIdx.x - tx * nt;
+    const int nb = (nth + kBpBatch - 1) / kBpBatch;  // the share's angles: whole batches
+    const int i0 = (int)((int64_t)nb * blockIdx.y / gridDim.y) * kBpBatch;
+    const int i1 = min(nth, (int)((int64_t)nb * (blockIdx.y + 1) / gridDim.y) * kBpBatch);
+    const int ix0 = tx * 32, iy0 = N - 1 - ty * 32;  // the tile's first pixel; lane l is iy0 - l
+    const int sa = threadIdx.x >> 4, hl = threadIdx.x & 15;  // staging: angle of the batch, lane of 16
+    float acc[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) acc[b] = 0.f;
+    MfAngle R;
+    float yv[3];
+    auto load_angle = [&](int ib) {  // this thread's angle of the batch from ib (none: weight 0)
+        if (ib + sa < i1) R = mf_load<float>(ang + ib + sa);
+        else R = MfAngle{};
+    };
+    auto put_angle = [&](int ib, int buf) {  // its constants to shared memory, its bins' loads
+        const long long base = ix0 * R.C + iy0 * R.S + R.K;
+        const long long mn = base + min(0LL, 31 * R.C) + min(0LL, -31 * R.S);
+        const int jlo = (int)(mn >> kFix);
+        const long long Dr = base - ((long long)jlo << kFix);
+        BpAngle &B = cs[buf][sa];
+        if (hl < 4) B.Dw[hl] = Dr + hl * 8 * R.C;
+        if (hl == 0) {
+            B.c_lo = (unsigned)(R.C << 18);
+            B.c_mid = (unsigned)(R.C >> 14);
+            B.c_hi = (int)(R.C >> kFix);
+            B.H2s = R.H2s;
+            B.Hc = R.H2s - 0x7FFFFFFF;
+            B.ramp = R.ramp;
+            B.a0 = B.a1 = 0.f;
+            if (R.tie != 0) {  // every pixel at the same fraction of a bin: entries 0 or 1
+                const long long dl = R.K & ((1LL << kFix) - 1), dr = (1LL << kFix) - dl;
+                B.a0 = dl < R.H2 || (R.tie == 1 && dl == R.H2) ? 1.f : 0.f;
+                B.a1 = dr < R.H2 || (R.tie == -1 && dr == R.H2) ? 1.f : 0.f;
+            }
+            B.S = R.S;
+            B.jlo = jlo;
+            B.inv_c = R.inv_c;
+        }
+        const float *yi = y + (int64_t)(ib + sa) * p;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const int j = jlo + hl + 16 * e;
+            yv[e] = ib + sa < i1 && (unsigned)j < (unsigned)p ? __ldg(yi + j) : 0.f;
+        }
+    };
+    auto put_bins = [&](float inv_c, int buf) {
+        bool bad = false;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const int k = hl + 16 * e;
+            const float v = yv[e] * inv_c;
+            bad |= !isfinite(v);
+            ys[buf][sa][k].x = v;
+            if (k > 0) ys[buf][sa][k - 1].y = v;
+        }
+        return bad;
+    };
+    load_angle(i0);
+    put_angle(i0, 0);
+    float inv_c = R.inv_c;
+    load_angle(i0 + kBpBatch);
+    bool bad = __syncthreads_or(put_bins(inv_c, 0));
+    int buf = 0;
+    for (int ib = i0; ib < i1; ib += kBpBatch) {
+        const bool more = ib + kBpBatch < i1;
+        if (more) {
+            put_angle(ib + kBpBatch, buf ^ 1);
+            inv_c = R.inv_c;
+            load_angle(ib + 2 * kBpBatch);
+        }
+#pragma unroll 1
+        for (int a = 0; a < kBpBatch; ++a) {
+            const BpAngle &B = cs[buf][a];
+            const unsigned c_lo = B.c_lo, c_mid = B.c_mid;
+            const int c_hi = B.c_hi, H2s = B.H2s, Hc = B.Hc;
+            const float ramp = B.ramp, a0 = B.a0, a1 = B.a1;
+            const long long D = B.Dw[wid] - lane * B.S;
+            unsigned lo = (unsigned)(D << 18), mid = (unsigned)(D >> 14);
+            int hi = (int)(D >> kFix);
+            auto pixels = [&](auto guard) {
+#pragma unroll
+                for (int b = 0; b < 8; ++b) {
+                    const int u = (int)(mid >> 1);
+                    const float w0 = __saturatef(fmaf((float)(H2s - u), ramp, a0));
+                    const float w1 = __saturatef(fmaf((float)(Hc + u), ramp, a1));
+                    if constexpr (decltype(guard)::value) {
+                        const int j = B.jlo + hi;
+                        const float *yi = y + (int64_t)(ib + a) * p;
+                        if (w0 > 0.f && (unsigned)j < (unsigned)p) acc[b] += B.inv_c * w0 * __ldg(yi + j);
+                        if (w1 > 0.f && (unsigned)(j + 1) < (unsigned)p) acc[b] += B.inv_c * w1 * __ldg(yi + j + 1);
+                    } else {
+                        const float2 v = ys[buf][a][hi];
+                        acc[b] = fmaf(w0, v.x, acc[b]);
+                        acc[b] = fmaf(w1, v.y, acc[b]);
+                    }
+                    asm("add.cc.u32 %0, %0, %3; addc.cc.u32 %1, %1, %4; addc.u32 %2, %2, %5;"
+                        : "+r"(lo), "+r"(mid), "+r"(hi)
+                        : "r"(c_lo), "r"(c_mid), "r"(c_hi));
+                }
+            };
+            if (bad) {
+                if (ib + a < i1) pixels(std::true_type{});
+            } else {
+                pixels(std::false_type{});
+            }
+        }
+        bool nb = false;
+        if (more) nb = put_bins(inv_c, buf ^ 1);
+        bad = __syncthreads_or(nb);
+        buf ^= 1;
+    }
+    const int k = ty * 32 + lane;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const int ix = ix0 + wid * 8 + b;
+        if (ix >= N || k >= N) continue;
+        const int64_t q = (int64_t)ix * N + k;
+        if (gridDim.y > 1) part[(int64_t)blockIdx.y * N * N + q] = acc[b];
+        else epi(q, acc[b]);
     }
 }
 
@@ -448,14 +778,14 @@ constexpr int kFanPad = 4;              // records of weight 0 on either side of
 template <typename ACC> struct FanRay;
 template <> struct __align__(16) FanRay<float> {
     longlong2 cs;          // C, -S
-    int H2s;               // H2 at 30 bits
+    int H2s;               // H2 at 31 bits
     float inv_c, ramp, y;
     long long d0, H2;      // the distance at the tile's origin pixel; H2
     __device__ __forceinline__ void put(const MfAngle &A, long long d, float v) {
         cs = longlong2{A.C, -A.S};
         H2s = A.H2s;
         inv_c = A.inv_c;
-        ramp = A.ramp30;
+        ramp = A.ramp;
         y = v;
         d0 = d;
         H2 = A.H2;
@@ -470,13 +800,16 @@ template <> struct __align__(16) FanRay<float> {
     }
     // acc += a_rq y_r at distance d: the same entry, from the same exact
     // distance, as the projector's. TIE: the ray may be axis-aligned (tie its
-    // side), FAR: more than two pixels away.
+    // side), FAR: the pixel may be a pixel's width away or more.
     template <int MODE, bool TIE, bool FAR>
     __device__ __forceinline__ void add(long long d, int tie, float &acc) const {
-        const long long ad = d < 0 ? -d : d;
-        float w = inv_c * __saturatef((float)(H2s - (int)(ad >> 16)) * ramp);
-        if (TIE && tie != 0) w = ad < H2 || (ad == H2 && tie == (d > 0 ? 1 : -1)) ? inv_c : 0.f;
-        if (FAR && (ad >> 47) != 0) w = 0.f;
+        const long long ud = d ^ (d >> 63);
+        float w = inv_c * __saturatef((float)(H2s - (int)(ud >> 15)) * ramp);
+        if (TIE && tie != 0) {
+            const long long ad = d < 0 ? -d : d;
+            w = ad < H2 || (ad == H2 && tie == (d > 0 ? 1 : -1)) ? inv_c : 0.f;
+        }
+        if (FAR && (ud >> 46) != 0) w = 0.f;
         if (w > 0.f) acc += MODE == 0 ? w * y : w;
     }
 };
@@ -760,6 +1093,8 @@ struct fair_mf_s {
     fair::DevBuf part;                 // the backprojector's sums per share of the angles
     fair::DevBuf w_in, w_out;          // host-call staging (FP64)
     fair::DevBuf xt;                   // the projector's transposed copy of x
+    fair::DevBuf nonfinite;            // the last pass whose x held an Inf or NaN
+    unsigned epoch = 0;                // passes of the projector
     fair::DevBuf v_a, v_b;             // reduced-precision staging
     // SIRT state
     bool ready = false, sart = false;
@@ -779,6 +1114,10 @@ namespace {
 // operator's precision), grown before a pass that reads x.
 int mf_grow_xt(fair_mf A) {
     const size_t es = A->prec == FAIR_PREC_F64 ? sizeof(double) : sizeof(float);
+    if (!A->nonfinite.p) {
+        FAIR_TRY(A->nonfinite.grow(sizeof(unsigned)));
+        FAIR_CUDA(cudaMemsetAsync(A->nonfinite.p, 0, sizeof(unsigned), A->stream));
+    }
     return A->xt.grow(es * (size_t)A->N * A->N);
 }
 
@@ -788,39 +1127,69 @@ void mf_project(fair_mf A, const XT *x, Epi epi, cudaStream_t s) {
     const int N = A->N;
     const MfAngle *ang = A->ang.as<MfAngle>();
     const XT *xt = nullptr;
+    unsigned *nf = A->nonfinite.as<unsigned>();
     if (MODE == 0) {  // the rays that walk rows read the transpose (mf_grow_xt)
         const int nb = (N + 31) / 32;
-        k_mf_transpose<XT><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(x, A->xt.as<XT>(), N);
+        ++A->epoch;
+        k_mf_transpose<XT><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(x, A->xt.as<XT>(), N, nf, A->epoch);
         xt = A->xt.as<XT>();
     }
-    if (A->kind == 1)
+    if constexpr (std::is_same<ACC, float>::value) {
+        static_assert(MODE == 0, "FP32 passes read x");
+        const int g = grid_for((int64_t)A->nth * ((A->p + 31) / 32) * 32, 128);
+        if (A->kind == 1)
+            k_mf_project32<true><<<g, 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, nf, A->epoch, epi);
+        else
+            k_mf_project32<false><<<g, 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, nf, A->epoch, epi);
+    } else if (A->kind == 1) {
         k_mf_project<XT, ACC, MODE, true><<<grid_for(m, 128), 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, epi);
-    else
+    } else {
         k_mf_project<XT, ACC, MODE, false><<<grid_for(m, 128), 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, epi);
+    }
 }
 // Blocks of the backprojector over the image, and the shares its angles are
 // cut into so that a small image still fills the GPU: about 8 blocks of 4
 // warps per SM, at least 8 angles each.
-int64_t mf_bp_blocks(fair_mf A) {
+int64_t mf_bp_blocks(fair_mf A, bool f32) {
     const int64_t N = A->N;
+    if (A->kind == 0 && f32) return ((N + 31) / 32) * ((N + 31) / 32);
     if (A->kind == 1) return ((N + 31) / 32) * ((N + 4 * kFanPB - 1) / (4 * kFanPB));
     return (N * ((N + kMfPB - 1) / kMfPB) + 127) / 128;
 }
-int mf_bp_shares(fair_mf A) {
-    const int64_t want = ((int64_t)sm_count() * 8) / mf_bp_blocks(A);
+int mf_bp_shares(fair_mf A, bool f32) {
+    const int64_t blocks = mf_bp_blocks(A, f32);
+    if (A->kind == 0 && f32) {
+        // k_mf_backproject32: 4 waves of blocks where a share keeps at least 12
+        // batches of angles, 2 waves where it keeps 4, else one (the last wave's
+        // idle SMs against the shares' first, unoverlapped loads and the pass that
+        // adds them: N = 1024, 720 angles: 1, 2, 4 shares 518, 515, 477 us; N =
+        // 512, 360 angles: 4, 9, 19 shares 89, 78, 89 us); whole batches each
+        const int64_t nb = (A->nth + kBpBatch - 1) / kBpBatch;
+        for (int waves = 4; waves >= 1; waves >>= 1) {
+            const int64_t sh = std::min<int64_t>((int64_t)waves * kBpOcc * sm_count() / blocks, 32);
+            if (sh <= 1) break;
+            const int64_t keep = waves == 4 ? 12 : (waves == 2 ? 4 : 1);
+            if (nb < sh * keep && waves > 1) continue;
+            const int64_t per = (nb + sh - 1) / sh;  // batches per share
+            return (int)((nb + per - 1) / per);
+        }
+        return 1;
+    }
+    const int64_t want = ((int64_t)sm_count() * 8) / blocks;
     return (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min(A->nth / 8, 32)));
 }
 template <typename YT, typename ACC, int MODE, class Epi>
 int mf_backproject(fair_mf A, const YT *y, Epi epi, cudaStream_t s) {
     const int64_t n = (int64_t)A->N * A->N;
     const MfAngle *ang = A->ang.as<MfAngle>();
-    const int shares = mf_bp_shares(A);
+    constexpr bool f32 = std::is_same<ACC, float>::value;
+    const int shares = mf_bp_shares(A, f32);
     if (shares > 1) FAIR_TRY(A->part.grow(sizeof(ACC) * (size_t)shares * n));
     ACC *part = A->part.as<ACC>();
     if (A->kind == 1) {
         const MfBins B{A->oms.as<float>(), A->omj.as<int>(), A->omt.as<int>(), A->om0, A->om_inv, A->om_L,
                        A->uni_a, A->uni_b, A->uni_key, A->uni_inv};
-        const dim3 g((unsigned)mf_bp_blocks(A), shares);
+        const dim3 g((unsigned)mf_bp_blocks(A, f32), shares);
         const MfFanAngle *fa = A->fang.as<MfFanAngle>();
         if (A->tan_keys && A->uni_b > A->uni_a)
             k_mf_backproject_fan<YT, ACC, MODE, true, true><<<g, kFanThreads, 0, s>>>(
@@ -831,8 +1200,11 @@ int mf_backproject(fair_mf A, const YT *y, Epi epi, cudaStream_t s) {
         else
             k_mf_backproject_fan<YT, ACC, MODE, false, false><<<g, kFanThreads, 0, s>>>(
                 ang, fa, B, A->nth, A->p, A->N, y, part, epi);
+    } else if constexpr (f32) {
+        const dim3 g((unsigned)mf_bp_blocks(A, f32), shares);
+        k_mf_backproject32<<<g, 128, 0, s>>>(ang, A->nth, A->p, A->N, y, part, epi);
     } else {
-        const dim3 g((unsigned)std::min<int64_t>(mf_bp_blocks(A), (int64_t)sm_count() * 32), shares);
+        const dim3 g((unsigned)std::min<int64_t>(mf_bp_blocks(A, f32), (int64_t)sm_count() * 32), shares);
         if (shares > 1)
             k_mf_backproject<YT, ACC, MODE, kMfPB, true><<<g, 128, 0, s>>>(ang, A->nth, A->p, A->N, y, part, epi);
         else
@@ -931,8 +1303,8 @@ void mf_line(double C, double S, double K, MfAngle &a) {
     // segments of 1e-10 or less are dropped, as the ray tracer does
     // (system_generation.f90:393-394)
     a.Hcut = a.tie != 0 ? a.H2 : a.H2 - (long long)floor(1e-10 * c * s * kOne);
-    a.H2s = (int)(a.H2 >> 16);
-    a.ramp30 = s > 0 ? (float)(1.0 / (1073741824.0 * s)) : 0.f;
+    a.H2s = (int)(a.H2 >> 15);
+    a.ramp = a.tie == 0 ? (float)(1.0 / (2147483648.0 * s)) : 0.f;
 }
 
 // A new operator handle with its own stream, or a status.
@@ -1119,7 +1491,7 @@ int fair_mf_destroy(fair_mf A) {
     cudaStreamSynchronize(A->stream);
     for (fair::DevBuf *d : {&A->ang, &A->fang, &A->oms, &A->omj, &A->omt, &A->w_in, &A->w_out, &A->v_a,
                             &A->v_b, &A->M_sart, &A->M_cim, &A->D, &A->x32, &A->r, &A->w_b,
-                            &A->w_x, &A->xt, &A->part})
+                            &A->w_x, &A->xt, &A->part, &A->nonfinite})
         d->release();
     if (A->own_stream) cudaStreamDestroy(A->stream);
     delete A;
@@ -1225,7 +1597,7 @@ int fair_mf_sirt_prepare(fair_mf A, const char *sirt_method, const fair_opts *op
     if (red) FAIR_TRY(A->x32.grow(sizeof(float) * (n + 1)));
     FAIR_TRY(fair::mf_grow_xt(A));
     FAIR_TRY(fair::mf_weights(A, sart, A->stream));
-    const int shares = fair::mf_bp_shares(A);
+    const int shares = fair::mf_bp_shares(A, red);
     if (shares > 1) FAIR_TRY(A->part.grow((red ? sizeof(float) : sizeof(double)) * (size_t)shares * n));
     FAIR_CUDA(cudaStreamSynchronize(A->stream));
     A->ready = true;
