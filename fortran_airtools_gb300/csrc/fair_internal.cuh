@@ -297,12 +297,12 @@ struct TlBatchProb {
     float *x32;
 };
 struct TlBatch {
-    DevBuf desc, uoff, roff;  // per-problem descriptors, unit and row offsets
+    DevBuf desc, ulist, roff;  // per-problem descriptors, work units of all, row offsets
     int np = 0;
     int64_t units = 0, rows = 0;
     size_t smem = 0;          // shared memory of the largest tile
     void release() {
-        desc.release(); uoff.release(); roff.release();
+        desc.release(); ulist.release(); roff.release();
         np = 0; units = rows = 0; smem = 0;
     }
 };

@@ -1523,27 +1523,25 @@ template <typename VT> struct TlbMake<TlFused<VT>> {
     __device__ static TlFused<VT> make(const TlbDesc &d) { return TlFused<VT>{(const uint4 *)d.idx}; }
 };
 
-// The units of all problems numbered consecutively (uoff): a CTA takes the
-// next unit, finds its problem and runs the single-problem unit body on it, so
-// problems of any sizes share the GPU without tails.
+// The units of all problems in one list (.w: the problem), longest first: a CTA
+// takes the next unit and runs the single-problem unit body on it, so problems
+// of any sizes share the GPU without tails.
 template <class LD, typename XT, typename ACC>
 __global__ void __launch_bounds__(kTlThreads, LD::CTAS) k_tlb_partials(const TlbDesc *__restrict__ desc,
-                                                             const int64_t *__restrict__ uoff, int np,
+                                                             const int4 *__restrict__ units, int64_t total,
                                                              unsigned *ctr) {
     extern __shared__ __align__(16) unsigned char tl_smem[];
     XT *xs = reinterpret_cast<XT *>(tl_smem);
     __shared__ int s_unit, s_chunk;
-    const int64_t total = __ldg(uoff + np);
     for (;;) {
         if (threadIdx.x == 0) s_unit = (int)atomicAdd(ctr, 1u);
         __syncthreads();
         const int64_t u = s_unit;
         if (u >= total) break;
-        const int p = tlb_owner(uoff, np, u);
-        const TlbDesc &d = desc[p];
-        const TlArgs P = d.P;
-        tl_unit<LD, XT, ACC, 2, true>(P, TlbMake<LD>::make(d), (const XT *)d.x, (ACC *)d.part,
-                                      P.units[u - __ldg(uoff + p)], xs, s_chunk);
+        const int4 U = units[u];
+        const TlbDesc &d = desc[U.w];
+        tl_unit<LD, XT, ACC, 2, true>(d.P, TlbMake<LD>::make(d), (const XT *)d.x, (ACC *)d.part, U, xs,
+                                      s_chunk);
     }
     if (threadIdx.x == 0) {
         const unsigned done = atomicAdd(ctr + 1, 1u);
@@ -1620,7 +1618,7 @@ int tlb_run(const TlBatch &T, int pass, double omg, double lb, double ub, int bm
     if (dry) return FAIR_OK;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count() * occ, T.units));
     const TlbDesc *d = T.desc.as<TlbDesc>();
-    kernel<<<grid, kTlThreads, T.smem, s>>>(d, T.uoff.as<int64_t>(), T.np, ctr);
+    kernel<<<grid, kTlThreads, T.smem, s>>>(d, T.ulist.as<int4>(), T.units, ctr);
     if (pass == 1)
         k_tlb_rows<1, ACC><<<tl_grid(T.rows), 256, 0, s>>>(d, T.roff.as<int64_t>(), T.np, omg, lb, ub, bmode);
     else
@@ -1656,8 +1654,8 @@ void tl_drop_build(DevCSR &M) {
 int tl_batch_bind(TlBatch &T, int prec, const std::vector<TlBatchProb> &probs) {
     const int np = (int)probs.size();
     std::vector<TlbDesc> d(np);
-    std::vector<int64_t> uo(np + 1, 0), ro(np + 1, 0);
-    int64_t cells = 1;
+    std::vector<int64_t> ro(np + 1, 0);
+    int64_t cells = 1, chunks = 0;
     for (int p = 0; p < np; ++p) {
         const DevCSR &M = *probs[p].M;
         const DevCSR::Tiled &tl = M.tl;
@@ -1683,19 +1681,42 @@ int tl_batch_bind(TlBatch &T, int prec, const std::vector<TlBatchProb> &probs) {
         e.x64 = probs[p].x;
         e.x32 = probs[p].x32;
         e.scale = prec == FAIR_PREC_Q16 ? M.qscale : 1.0;
-        uo[p + 1] = uo[p] + tl.nunits;
         ro[p + 1] = ro[p] + M.m;
         cells = std::max<int64_t>(cells, (int64_t)e.P.G.cells() + 1);
+        chunks += tl.nchunks;
     }
+    // The units, cut for the batch: whole rounds of the CTA's warps (one chunk
+    // each), about 6 units per resident CTA (3 per SM), longest first. A problem's
+    // own units, cut to fill the GPU alone, hold 8 chunks here: half the warps of
+    // a CTA waited at its barriers (24 fan-beam problems of N <= 352, FP32: 528 us a pass,
+    // 4.5 TB/s; cut together 394 us, 6.1 TB/s).
+    constexpr int round = kTlThreads / 32;
+    int64_t per = chunks / ((int64_t)sm_count() * 3 * 6) / round * round;
+    per = std::max<int64_t>(round, std::min<int64_t>(per, kUnitChunks));
+    std::vector<std::pair<int64_t, int4>> ul;  // slots, unit
+    std::vector<int64_t> so;
+    for (int p = 0; p < np; ++p) {
+        const DevCSR::Tiled &tl = probs[p].M->tl;
+        so.resize((size_t)tl.nchunks + 1);
+        FAIR_CUDA(cudaMemcpy(so.data(), tl.soff.p, sizeof(int64_t) * so.size(), cudaMemcpyDeviceToHost));
+        for (size_t t = 0; t + 1 < tl.hchunk.size(); ++t)
+            for (int64_t c = tl.hchunk[t]; c < tl.hchunk[t + 1]; c += per) {
+                const int64_t e = std::min<int64_t>(c + per, tl.hchunk[t + 1]);
+                ul.emplace_back(so[e] - so[c], make_int4((int)t, (int)c, (int)e, p));
+            }
+    }
+    std::stable_sort(ul.begin(), ul.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+    std::vector<int4> units(ul.size());
+    for (size_t i = 0; i < ul.size(); ++i) units[i] = ul[i].second;
     FAIR_TRY(T.desc.grow(sizeof(TlbDesc) * std::max(np, 1)));
-    FAIR_TRY(T.uoff.grow(sizeof(int64_t) * (np + 1)));
+    FAIR_TRY(T.ulist.grow(sizeof(int4) * std::max<size_t>(units.size(), 1)));
     FAIR_TRY(T.roff.grow(sizeof(int64_t) * (np + 1)));
     // synchronous copies: the host tables go out of scope on return
     FAIR_CUDA(cudaMemcpy(T.desc.p, d.data(), sizeof(TlbDesc) * np, cudaMemcpyHostToDevice));
-    FAIR_CUDA(cudaMemcpy(T.uoff.p, uo.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice));
+    FAIR_CUDA(cudaMemcpy(T.ulist.p, units.data(), sizeof(int4) * units.size(), cudaMemcpyHostToDevice));
     FAIR_CUDA(cudaMemcpy(T.roff.p, ro.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice));
     T.np = np;
-    T.units = uo[np];
+    T.units = (int64_t)units.size();
     T.rows = ro[np];
     T.smem = (size_t)cells * (prec == FAIR_PREC_F64 ? sizeof(double) : sizeof(float));
     return FAIR_OK;
