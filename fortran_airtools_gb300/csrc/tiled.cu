@@ -463,23 +463,26 @@ template <typename VT, int LB> struct TlStep6 {  // 6-entry step records
     __device__ __forceinline__ static Raw none() { return make_uint4(0u, 0u, 0u, 0u); }
     __device__ __forceinline__ void open(const Raw &r, State &st, uint32_t (&li)[6], float (&v)[6]) const {
         const uint32_t w = r.x;
+        int d[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) d[q] = step(w, q);
+        // running sums in a tree of depth 3 instead of a chain of 6
+        const int s01 = d[0] + d[1], s23 = d[2] + d[3], s45 = d[4] + d[5];
+        const int b1 = st.li + s01, b3 = b1 + s23;
+        li[0] = (uint32_t)(st.li + d[0]);
+        li[1] = (uint32_t)b1;
+        li[2] = (uint32_t)(b1 + d[2]);
+        li[3] = (uint32_t)b3;
+        li[4] = (uint32_t)(b3 + d[4]);
+        li[5] = (uint32_t)(b3 + s45);
+        // a slot without codes: its indices from the side table, over the decoded
+        // ones (N = 1024, 720 angles, Q16: the decode as the other branch 607 and
+        // 564 us a pass, this 581 and 550; with the inner slots' plain fetch, 560
+        // and 532)
         if (w & kStepEsc) {
             const int4 a = __ldg(side + 2 * (int64_t)(w & kStepSlot));
             const int4 b = __ldg(side + 2 * (int64_t)(w & kStepSlot) + 1);
             li[0] = a.x; li[1] = a.y; li[2] = a.z; li[3] = a.w; li[4] = b.x; li[5] = b.y;
-        } else {
-            int d[6];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) d[q] = step(w, q);
-            // running sums in a tree of depth 3 instead of a chain of 6
-            const int s01 = d[0] + d[1], s23 = d[2] + d[3], s45 = d[4] + d[5];
-            const int b1 = st.li + s01, b3 = b1 + s23;
-            li[0] = (uint32_t)(st.li + d[0]);
-            li[1] = (uint32_t)b1;
-            li[2] = (uint32_t)(b1 + d[2]);
-            li[3] = (uint32_t)b3;
-            li[4] = (uint32_t)(b3 + d[4]);
-            li[5] = (uint32_t)(b3 + s45);
         }
         st.li = (int)li[5];
         Conv2B<VT>::two(r.y, v[0], v[1]);
@@ -654,7 +657,24 @@ __device__ __forceinline__ void tl_stream_chunks(const TlArgs &P, const LD &ldr,
     while (c < U.z) {
         ACC acc[KC] = {};
         int t = 0;
-        for (; t + 2 <= cur.len; t += 2) {  // slot pairs: both slots' work interleaves
+        // slot pairs (both slots' work interleaves). In the 6-entry form, whose pass is
+        // bound by issue, first those whose loads stay in the chunk, without the
+        // window's tests (the other forms' registers would spill)
+        if constexpr (E == 6) {
+            for (int64_t j = cur.s0 + 64; t + 4 <= cur.len; t += 2, j += 64) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const typename LD::Raw r = ring[k];
+                    ring[k] = ldr.load(j + 32 * k);
+                    uint32_t li[E];
+                    ACC v[E];
+                    ldr.open(r, cur.st, li, v);
+#pragma unroll
+                    for (int q = 0; q < E; ++q) acc[k % KC] += (ACC)xs[li[q]] * v[q];
+                }
+            }
+        }
+        for (; t + 2 <= cur.len; t += 2) {
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const typename LD::Raw r = ring[k];
