@@ -363,7 +363,12 @@ struct SweepWork {
     // column level table (large images), the fallback flag, the blocks' stamp
     // tables
     DevBuf lens, eoff, idx, rec, dpath, lvl, cnt, lvtab, err, tabs;
-    DevBuf gsync;                      // grid barrier of the cooperative sweep {count, generation, error}
+    DevBuf gsync;                      // grid barrier of the cooperative sweep {count, unused, error}
+    // the sweep without barriers: values and tags of the entries in step order
+    // (beside idx), x as {value, level} pairs, and the direction they serve (-1: none)
+    DevBuf gval, tag, pairs;
+    DevBuf bases;                      // level set-up on a grid: the steps' bases of two windows
+    int flow_slot = -1;
     int32_t tab_n = 0, tab_blocks = 0;
     uint64_t uid = 0;                  // next window stamp (the tables hold older ones)
     bool err_valid = false;            // err holds the set-up's repeated-column flag
@@ -373,6 +378,7 @@ struct SweepWork {
         int32_t nord = 0, nlev = 0;    // steps, levels
         int64_t entries = 0;           // entries of all steps
         bool use = false;              // enough steps per level to run the levels
+        bool grouped = false;          // the steps' entries are idx and gval (else the matrix's)
         DevBuf sched, lptr, dnlev;     // steps in level order, level pointers, level count
     } lev[2];
     void release();

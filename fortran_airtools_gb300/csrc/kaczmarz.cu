@@ -52,7 +52,7 @@ namespace {
 struct RowStep {
     int64_t s;    // first entry of the row
     int32_t len;  // entries
-    int32_t pad;
+    int32_t level;  // in a level schedule: the step's level
     double b;     // b(ri)
     double w;     // omega / nrA(ri)
 };
@@ -390,16 +390,20 @@ int sweep_warps() {
 //     is the largest, over the steps a of its window with a path to it, of
 //     base(a) + the path's length, base(a) = 1 + the table's level over a's
 //     first-touch columns; the last touches write the levels into the table
-//     (a window costs two barriers and two rounds of scattered table accesses
-//     whatever it holds: fan N=512, 243,328 steps, 32.5 ms in windows of 32,
-//     13.9 ms in windows of 128);
+//     (a window costs two rounds of scattered table accesses and the exchanges
+//     between them whatever it holds: fan N=512, 243,328 steps, on a cluster
+//     32.5 ms in windows of 32, 13.9 ms in windows of 128);
 //   counting sort of the steps by level (level pointers, steps in level order).
-// The sweep (k_lvl_sweep) runs a group of G warps per step, the steps of a
+// The sweep in the direction the levels were built for runs without barriers
+// (k_flow_sweep): every x_j carries the level that updated it last, and a step
+// waits for its own columns only. The opposite direction takes the levels in
+// reverse (k_lvl_sweep): a group of G warps per step, the steps of a
 // level spread over the groups, on one thread-block cluster (a cluster barrier
 // between levels; x in the cluster's distributed shared memory when its parts
 // fit, else in global memory read past L1) or, when a level outgrows the
 // cluster, on a cooperative grid of up to one block per SM (a software grid
-// barrier between levels; x in global memory).
+// barrier between levels; x in global memory); so does a sweep for whose copies
+// of the entries there is no memory.
 
 struct WinRow {
     int64_t off;              // first entry of the step in the grouped column array
@@ -419,9 +423,10 @@ constexpr unsigned long long kStampIdLimit = (1ull << 36) - 1ull;
 __device__ __forceinline__ unsigned long long win_stamp(unsigned long long id, int r, int pos) {
     return (id << 28) | ((unsigned long long)r << kStampPosBits) | (unsigned long long)pos;
 }
-// group of an entry from its flags (bit 0: a later step has the column; bit 1: an earlier one)
+// group of an entry from its flags (bit 0: a later step of the window has the
+// column; bits 1-7: 1 + the last earlier step that has it, 0: none)
 __device__ __forceinline__ int win_group(unsigned f) {
-    return (f & 2u) ? ((f & 1u) ? 2 : 3) : (int)f;
+    return f > 1u ? ((f & 1u) ? 2 : 3) : (int)f;
 }
 
 // total * 2^(E - 1075), rounded once: the integer converted to double (round
@@ -513,7 +518,8 @@ __global__ void __launch_bounds__(kSetupThreads) k_lvl_setup(
         const RowStep *__restrict__ steps, const int64_t *__restrict__ eoff, int32_t nord,
         const int32_t *__restrict__ col, unsigned long long *__restrict__ tabs, int32_t n,
         unsigned long long id0, int32_t *__restrict__ oidx, WinRow *__restrict__ rec,
-        unsigned char *__restrict__ dpath, int *err) {
+        unsigned char *__restrict__ dpath, const double *__restrict__ val, double *__restrict__ oval,
+        int32_t *__restrict__ otag, int *err) {
     extern __shared__ __align__(16) unsigned char fl[];  // [entries of a window]
     __shared__ int rb[WR + 1];
     __shared__ uint32_t msk[WR][WR / 32];  // predecessor steps in the window
@@ -544,7 +550,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_lvl_setup(
                     if (orow == r) {
                         atomicExch(err, 1);
                     } else {
-                        f = 2;
+                        f = (unsigned char)((orow + 1) << 1);
                         fl[old & ((1ull << kStampPosBits) - 1ull)] |= 1;  // its one writer
                         atomicOr(&msk[r][orow >> 5], 1u << (orow & 31));
                     }
@@ -586,7 +592,8 @@ __global__ void __launch_bounds__(kSetupThreads) k_lvl_setup(
             const int64_t ro = wbase + base;
             for (int e0 = 0; e0 < len; e0 += 32) {
                 const int e = e0 + lane;
-                const int g = e < len ? win_group(fl[base + e]) : -1;
+                const unsigned f = e < len ? fl[base + e] : 0u;
+                const int g = e < len ? win_group(f) : -1;
                 const unsigned b0 = __ballot_sync(0xffffffffu, g == 0);
                 const unsigned b1 = __ballot_sync(0xffffffffu, g == 1);
                 const unsigned b2 = __ballot_sync(0xffffffffu, g == 2);
@@ -597,6 +604,10 @@ __global__ void __launch_bounds__(kSetupThreads) k_lvl_setup(
                                 : g == 2 ? o2 + __popc(b2 & lt)
                                          : o3 + __popc(b3 & lt);
                     oidx[ro + d] = col[s0 + e];
+                    if (otag) {
+                        oval[ro + d] = val[s0 + e];
+                        if (f > 1u) otag[ro + d] = -(int)(f >> 1);  // k_lvl_tags looks the step up
+                    }
                 }
                 o0 += __popc(b0);
                 o1 += __popc(b1);
@@ -620,7 +631,7 @@ template <int WR, bool SMEM>
 __global__ void __launch_bounds__(1024, 1) k_lvl_levels(
         const WinRow *__restrict__ rec, const unsigned char *__restrict__ dpath,
         const int32_t *__restrict__ oidx, int32_t nord, int32_t *lvg, int32_t n,
-        int32_t *__restrict__ lvl, int *__restrict__ nlev) {
+        int32_t *__restrict__ lvl, int32_t *__restrict__ otag, int *__restrict__ nlev) {
     constexpr int SW = WR / 32;  // steps per warp
     extern __shared__ int32_t lvs[];
     __shared__ int32_t base[WR];
@@ -670,7 +681,11 @@ __global__ void __launch_bounds__(1024, 1) k_lvl_levels(
                 for (int t = 0; t < 8; ++t) j[t] = e0 + 32 * t < w[i].c2 ? oidx[w[i].off + e0 + 32 * t] : -1;
 #pragma unroll
                 for (int t = 0; t < 8; ++t)
-                    if (j[t] >= 0) m = max(m, SMEM ? lvs[j[t]] : __ldcg(lvg + j[t]));
+                    if (j[t] >= 0) {
+                        const int32_t v = SMEM ? lvs[j[t]] : __ldcg(lvg + j[t]);
+                        m = max(m, v);
+                        if (otag) otag[w[i].off + e0 + 32 * t] = v;
+                    }
             }
             m = (int)__reduce_max_sync(0xffffffffu, (unsigned)m);
             if (lane == 0) base[r] = m + 1;
@@ -722,7 +737,7 @@ template <int WR, int CS>
 __global__ void __launch_bounds__(512, 1) k_lvl_levels_cluster(
         const WinRow *__restrict__ rec, const unsigned char *__restrict__ dpath,
         const int32_t *__restrict__ oidx, int32_t nord, int32_t *lv, int32_t *__restrict__ lvl,
-        int *__restrict__ nlev) {
+        int32_t *__restrict__ otag, int *__restrict__ nlev) {
     constexpr int RW = WR / CS;   // steps per block and window
     constexpr int WPR = 16 / RW;  // warps per step
     static_assert(CS == 16 && RW >= 2 && WPR >= 1 && RW * WPR == 16, "cluster shape");
@@ -772,7 +787,11 @@ __global__ void __launch_bounds__(512, 1) k_lvl_levels_cluster(
                 }
 #pragma unroll
                 for (int t = 0; t < 8; ++t)
-                    if (j[t] >= 0) m = max(m, __ldcg(lv + j[t]));
+                    if (j[t] >= 0) {
+                        const int32_t v = __ldcg(lv + j[t]);
+                        m = max(m, v);
+                        if (otag) otag[w.off + e0 + 32 * WPR * t] = v;
+                    }
             }
             m = (int)__reduce_max_sync(0xffffffffu, (unsigned)m);
             if (lane == 0) atomicMax(&base[i], m + 1);
@@ -814,17 +833,193 @@ __global__ void __launch_bounds__(512, 1) k_lvl_levels_cluster(
     if (lane == 0 && top > 0) atomicMax(nlev, top);
 }
 
+// A barrier of all blocks of a cooperative launch on one counter, gbar[0]
+// (zero at the launch): block 0 adds 2^31 - (blocks - 1), every other block
+// 1, so the counter's top bit flips exactly when the last block arrives -- one
+// reduction per block, nothing to reset (the counter wraps) and, the barriers
+// being counted (phase: the top bit before this one), no value to wait for.
+// The arrival releases the block's writes of the level; the waiting thread
+// reads the counter with acquire semantics. A block that waits more than
+// kGridSpinLimit polls, or sees *gerr set (checked every 1024 polls), sets
+// *gerr and returns false; the sweep then stops, and the host reports the
+// error.
+constexpr unsigned long long kGridSpinLimit = 1ull << 26;
+enum { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
+
+__device__ __forceinline__ bool grid_barrier(unsigned *gbar, int *gerr, unsigned phase) {
+    __shared__ int ok_s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u;
+        int ok = 1;
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(gbar), "r"(add) : "memory");
+        for (unsigned long long it = 1;; ++it) {
+            unsigned cur;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(gbar) : "memory");
+            if ((cur >> 31) != phase) break;
+            if ((it & 1023u) == 0 && (it > kGridSpinLimit || *(volatile int *)gerr)) {
+                atomicExch(gerr, 1);
+                ok = 0;
+                break;
+            }
+        }
+        ok_s = ok;
+    }
+    __syncthreads();
+    return ok_s != 0;
+}
+
+// The same on a cooperative grid, a step of the window per block: the scattered
+// table accesses are spread over up to WR SMs, and each thread's columns (the
+// next window's loaded while a window runs) serve both phases from registers.
+// The steps' bases are published as {window + 1, base} words that the blocks
+// that need them poll (no barrier between the phases); a grid barrier closes the
+// window. Fan N=512 (1901 windows of 128): 17.3 ms on the cluster, whose 16 SMs
+// are bound by the scattered accesses (tags written), 8.5 ms here; N=128 1.11 and
+// 0.79 ms.
+template <int WR>
+__global__ void __launch_bounds__(512, 1) k_lvl_levels_grid(
+        const WinRow *__restrict__ rec, const unsigned char *__restrict__ dpath,
+        const int32_t *__restrict__ oidx, int32_t nord, int32_t *lv, int32_t *__restrict__ lvl,
+        int32_t *__restrict__ otag, unsigned long long *bases, unsigned *gbar, int *gerr,
+        int *__restrict__ nlev) {
+    constexpr int JC = 2, SW = WR / 32;  // columns per thread in registers; bases per lane
+    __shared__ int s_max, s_level, s_ok;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int nwin = (nord + WR - 1) / WR;
+    const int r = blockIdx.x;  // gridDim.x = WR: this block's step of every window
+    const WinRow none{0, 0, 0, 0, 0};
+    auto fetch = [&](const WinRow &w, int32_t (&j)[JC]) {
+#pragma unroll
+        for (int t = 0; t < JC; ++t) j[t] = tid + 512 * t < w.len ? __ldg(oidx + w.off + tid + 512 * t) : -1;
+    };
+    auto paths = [&](int k, unsigned char (&d)[SW]) {
+#pragma unroll
+        for (int i = 0; i < SW; ++i)
+            d[i] = wid == 0 && k < nord ? __ldg(dpath + (size_t)k * WR + 32 * i + lane) : (unsigned char)0;
+    };
+    WinRow w = r < nord ? rec[r] : none, wn = WR + r < nord ? rec[WR + r] : none;
+    int32_t j[JC];
+    unsigned char d[SW];
+    fetch(w, j);
+    paths(r, d);
+    if (tid == 0) {
+        s_max = 0;
+        s_ok = 1;
+    }
+    __syncthreads();
+    int top = 0;
+    for (int q = 0; q < nwin; ++q) {
+        const int k = q * WR + r;
+        const WinRow wn2 = k + 2 * WR < nord ? rec[k + 2 * WR] : none;
+        int32_t jn[JC];
+        unsigned char dn[SW];
+        // 1 + the table's level over the step's first-touch columns
+        int m = 0;
+#pragma unroll
+        for (int t = 0; t < JC; ++t) {
+            const int e = tid + 512 * t;
+            if (e < w.c2) {
+                const int32_t v = __ldcg(lv + j[t]);
+                m = max(m, v);
+                if (otag) otag[w.off + e] = v;
+            }
+        }
+        for (int e = tid + 512 * JC; e < w.c2; e += 512) {
+            const int32_t v = __ldcg(lv + __ldg(oidx + w.off + e));
+            m = max(m, v);
+            if (otag) otag[w.off + e] = v;
+        }
+        fetch(wn, jn);
+        paths(k + WR, dn);
+        m = (int)__reduce_max_sync(0xffffffffu, (unsigned)m);
+        if (lane == 0 && m > 0) atomicMax(&s_max, m);
+        __syncthreads();
+        unsigned long long *bq = bases + (q & 1) * WR;
+        if (tid == 0 && k < nord) {
+            const unsigned long long b = (unsigned long long)(unsigned)(q + 1) << 32 | (unsigned)(s_max + 1);
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(bq + r), "l"(b) : "memory");
+        }
+        if (wid == 0 && k < nord) {  // the longest paths within the window (of length d - 1)
+            unsigned v = 0, need = 0;
+#pragma unroll
+            for (int i = 0; i < SW; ++i) need |= d[i] > 0 ? 1u << i : 0u;
+            for (unsigned long long it = 1;; ++it) {
+#pragma unroll
+                for (int i = 0; i < SW; ++i)
+                    if (need >> i & 1u) {
+                        unsigned long long b;
+                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(bq + 32 * i + lane) : "memory");
+                        if ((unsigned)(b >> 32) == (unsigned)(q + 1)) {
+                            v = max(v, (unsigned)b + d[i] - 1u);
+                            need &= ~(1u << i);
+                        }
+                    }
+                if (__all_sync(0xffffffffu, need == 0)) break;
+                if ((it & 1023u) == 0 && (it > kGridSpinLimit || *(volatile int *)gerr)) {
+                    atomicExch(gerr, 1);
+                    s_ok = 0;
+                    break;
+                }
+            }
+            const int L = (int)__reduce_max_sync(0xffffffffu, v);
+            if (lane == 0) {
+                s_level = L;
+                s_max = 0;
+                lvl[k] = L;
+            }
+            top = max(top, L);
+        }
+        __syncthreads();
+        if (!s_ok) return;
+        const int L = s_level;  // the last touches of the window write the step's level
+#pragma unroll
+        for (int t = 0; t < JC; ++t) {
+            const int e = tid + 512 * t;
+            if (e < w.len && (e < w.c1 || e >= w.c3)) lv[j[t]] = L;
+        }
+        for (int e = tid + 512 * JC; e < w.len; e += 512)
+            if (e < w.c1 || e >= w.c3) lv[__ldg(oidx + w.off + e)] = L;
+        if (!grid_barrier(gbar, gerr, (unsigned)q & 1u)) return;
+        w = wn;
+        wn = wn2;
+#pragma unroll
+        for (int t = 0; t < JC; ++t) j[t] = jn[t];
+#pragma unroll
+        for (int i = 0; i < SW; ++i) d[i] = dn[i];
+    }
+    if (tid == 0 && top > 0) atomicMax(nlev, top);
+}
+
 __global__ void k_lvl_count(const int32_t *__restrict__ lvl, int32_t nord, int32_t *cnt) {
     for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nord; k += gridDim.x * blockDim.x)
         atomicAdd(cnt + lvl[k] - 1, 1);
 }
-// steps in level order (any order within a level: its steps share no column)
+// steps in level order (any order within a level: its steps share no column),
+// their levels beside them; eoff (when given): their first entries in the
+// grouped arrays
 __global__ void k_lvl_scatter(const RowStep *__restrict__ steps, const int32_t *__restrict__ lvl,
                               int32_t nord, const int64_t *__restrict__ lptr, int32_t *cnt,
-                              RowStep *__restrict__ sched) {
+                              const int64_t *__restrict__ eoff, RowStep *__restrict__ sched) {
     for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nord; k += gridDim.x * blockDim.x) {
         const int l = lvl[k] - 1;
-        sched[lptr[l] + atomicSub(cnt + l, 1) - 1] = steps[k];
+        RowStep st = steps[k];
+        st.level = l + 1;
+        if (eoff) st.s = eoff[k];
+        sched[lptr[l] + atomicSub(cnt + l, 1) - 1] = st;
+    }
+}
+// Tags of the entries whose column an earlier step of their window has (a warp
+// per step): that step's level.
+template <int WR>
+__global__ void k_lvl_tags(const WinRow *__restrict__ rec, int32_t nord, const int32_t *__restrict__ lvl,
+                           int32_t *__restrict__ otag) {
+    const int lane = threadIdx.x & 31;
+    const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+    for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < nord; k += nw) {
+        const WinRow w = rec[k];
+        const int32_t *wl = lvl + k / WR * WR - 1;
+        for (int e = w.c2 + lane; e < w.len; e += 32) otag[w.off + e] = wl[-otag[w.off + e]];
     }
 }
 
@@ -918,6 +1113,37 @@ __device__ __forceinline__ void lvl_load_chunks(const RowStep &st, const int32_t
     }
 }
 
+// The coefficient -(a.x - b) (omega / nrA) of a group's step from its warps'
+// parts (of shared memory: parts, G each, and coef).
+__device__ __forceinline__ double step_coef(const FxPart &part, FxPart *parts, double *coef, int G, int wg,
+                                            int lane, int bar, double w) {
+    if (G > 1) {
+        // by one warp of the group for all: the G parts one per lane, aligned and added by warp reductions. All 16 warps of a block
+        // at it (the conversion and the product are 64 cycles each of a
+        // sub-partition's FP64 pipe, and about 200 integer instructions where
+        // they are done without it) took 730 of a level's 5650 cycles at fan N=128
+        // and 1410 of 8800 at N=512 (sweeps 3.22 and 13.2 ms; one warp: 2.72 and
+        // 12.6 ms); groups take warps of different sub-partitions.
+        if (lane == 0) parts[wg] = part;
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * G) : "memory");
+        if (wg == (bar & (G - 1))) {
+            const int e = lane < G ? parts[lane].e : 0;
+            const int E = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
+            double r;
+            if (E >= 0x7FF) {
+                r = fx_special(parts, G);
+            } else {
+                const int sh = E - e;
+                r = fx_to_double_fast(fx_warp_sum(lane < G && sh < 64 ? parts[lane].s >> sh : 0ll), E);
+            }
+            if (lane == 0) *coef = __dmul_rn(-r, w);
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * G) : "memory");
+        return *(volatile double *)coef;
+    }
+    return __dmul_rn(-(part.e >= 0x7FF ? part.d : fx_to_double_fast(part.s, part.e)), w);
+}
+
 template <int XM, int CACHE>
 __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__restrict__ col,
                                         const double *__restrict__ val, const XAcc<XM> &X,
@@ -975,34 +1201,7 @@ __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__rest
         }
     }
     const FxPart part = fx_warp_part(p0, p1, (wg == 0 && lane == 0) ? -st.b : 0.0);
-    double c;
-    if (G > 1) {
-        // the coefficient, by one warp of the group for all: the G parts one per
-        // lane, aligned and added by warp reductions. All 16 warps of a block
-        // at it (the conversion and the product are 64 cycles each of a
-        // sub-partition's FP64 pipe, and about 200 integer instructions where
-        // they are done without it) took 730 of a level's 5650 cycles at fan N=128
-        // and 1410 of 8800 at N=512 (sweeps 3.22 and 13.2 ms; one warp: 2.72 and
-        // 12.6 ms); groups take warps of different sub-partitions.
-        if (lane == 0) parts[wg] = part;
-        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * G) : "memory");
-        if (wg == (bar & (G - 1))) {
-            const int e = lane < G ? parts[lane].e : 0;
-            const int E = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
-            double r;
-            if (E >= 0x7FF) {
-                r = fx_special(parts, G);
-            } else {
-                const int sh = E - e;
-                r = fx_to_double_fast(fx_warp_sum(lane < G && sh < 64 ? parts[lane].s >> sh : 0ll), E);
-            }
-            if (lane == 0) *coef = __dmul_rn(-r, st.w);
-        }
-        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * G) : "memory");
-        c = *(volatile double *)coef;
-    } else {
-        c = __dmul_rn(-(part.e >= 0x7FF ? part.d : fx_to_double_fast(part.s, part.e)), st.w);
-    }
+    const double c = step_coef(part, parts, coef, G, wg, lane, bar, st.w);
 #pragma unroll
     for (int i = 0; i < CACHE; ++i) {
         if (i >= nmine) break;
@@ -1030,42 +1229,6 @@ __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__rest
     }
 }
 
-
-// A barrier of all blocks of a cooperative launch on one counter, gbar[0]
-// (zero at the launch): block 0 adds 2^31 - (blocks - 1), every other block
-// 1, so the counter's top bit flips exactly when the last block arrives -- one
-// reduction per block, nothing to reset (the counter wraps) and, the barriers
-// being counted (phase: the top bit before this one), no value to wait for.
-// The arrival releases the block's writes of the level; the waiting thread
-// reads the counter with acquire semantics. A block that waits more than
-// kGridSpinLimit polls, or sees *gerr set (checked every 1024 polls), sets
-// *gerr and returns false; the sweep then stops, and the host reports the
-// error.
-constexpr unsigned long long kGridSpinLimit = 1ull << 26;
-enum { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
-
-__device__ __forceinline__ bool grid_barrier(unsigned *gbar, int *gerr, unsigned phase) {
-    __shared__ int ok_s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u;
-        int ok = 1;
-        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(gbar), "r"(add) : "memory");
-        for (unsigned long long it = 1;; ++it) {
-            unsigned cur;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(gbar) : "memory");
-            if ((cur >> 31) != phase) break;
-            if ((it & 1023u) == 0 && (it > kGridSpinLimit || *(volatile int *)gerr)) {
-                atomicExch(gerr, 1);
-                ok = 0;
-                break;
-            }
-        }
-        ok_s = ok;
-    }
-    __syncthreads();
-    return ok_s != 0;
-}
 
 // The levels in order on one cluster of gridDim.x blocks (CLUSTER) or one
 // block. Groups of G consecutive warps take the steps of a level in turn; each
@@ -1164,6 +1327,164 @@ __global__ void __launch_bounds__(NT, 1) k_lvl_sweep(
     if constexpr (XM != XG) {
         for (int64_t i = threadIdx.x; i < plen; i += NT)
             if (part0 + i < n) x[part0 + i] = xsm[i];
+    }
+}
+
+// ---- the sweep without barriers -------------------------------------------------
+// Between two levels of a barrier sweep lie a release of the writes, a barrier
+// and the reads of x, each a round trip through L2, and every step waits for
+// the slowest of its level. Here each x_j is kept as a 16-byte pair {value,
+// level of the last step that updated it}, read and written whole (128-bit
+// relaxed accesses are single-copy atomic), and each entry carries the level
+// its column must have reached (its tag: the level of the column's last
+// earlier step, from the level set-up). A group of G warps takes the steps grp,
+// grp + groups, ... of the level schedule, polls its entries' pairs until
+// each shows its tag, and writes them back with the step's own level: the
+// value is its own signal, so a step starts as soon as its last column
+// arrives, one store and one load after its predecessor. Every toucher of a
+// column updates it, so no version is missed or overwritten before its one
+// reader has seen it.
+// The blocks are co-resident (a cooperative launch) and every group takes its
+// steps in schedule order, so the first unfinished step of the schedule always
+// finds its columns ready. A wait longer than kGridSpinLimit polls sets *gerr;
+// all waits then end (checked every 1024 polls), and the host reports the error.
+// Bound by the latency of one level's chain: a store and a poll through L2, the
+// row's FP64 products, the parts' exchange. Per sweep, fan N=128 (1019 levels)
+// 2.72 ms on the cluster with x in distributed shared memory, 1.79 ms here; N=512
+// (3018 levels) 12.6 ms on the grid with barriers, 9.1 ms here.
+struct __align__(16) XPair {
+    double v;
+    long long level;
+};
+__device__ __forceinline__ void pair_ld(const XPair *p, double &v, long long &level) {
+    long long b;
+    asm volatile("{\n.reg .b128 t;\nld.relaxed.gpu.global.b128 t, [%2];\nmov.b128 {%0, %1}, t;\n}"
+                 : "=l"(b), "=l"(level) : "l"(p) : "memory");
+    v = __longlong_as_double(b);
+}
+__device__ __forceinline__ void pair_st(XPair *p, double v, long long level) {
+    asm volatile("{\n.reg .b128 t;\nmov.b128 t, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], t;\n}"
+                 ::"l"(p), "l"(__double_as_longlong(v)), "l"(level) : "memory");
+}
+__global__ void k_flow_pack(const double *__restrict__ x, int32_t n, XPair *__restrict__ xt) {
+    for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+        xt[j] = XPair{x[j], 0};
+}
+__global__ void k_flow_unpack(const XPair *__restrict__ xt, int32_t n, double *__restrict__ x) {
+    for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) x[j] = xt[j].v;
+}
+
+template <int K> struct FlowChunks {  // entries of a warp's chunks: column (-1: none), value, tag
+    int32_t c[K], t[K];
+    double v[K];
+};
+template <int K>
+__device__ __forceinline__ void flow_load(const RowStep &st, const int32_t *__restrict__ col,
+                                          const double *__restrict__ val, const int32_t *__restrict__ tag,
+                                          int lane, int G, int q0, FlowChunks<K> &k) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        const int e = (q0 + G * i) * 32 + lane;
+        const bool h = e < st.len;
+        k.c[i] = h ? __ldg(col + st.s + e) : -1;
+        k.t[i] = h ? __ldg(tag + st.s + e) : 0;
+        k.v[i] = h ? __ldg(val + st.s + e) : 0.0;
+    }
+}
+// The values of the chunks' columns, each once it has its tag (dead: a wait has
+// run out, no more waiting).
+template <int K>
+__device__ __forceinline__ void flow_wait(const FlowChunks<K> &k, const XPair *xt, double (&xo)[K], bool &dead,
+                                          int *gerr) {
+    unsigned need = 0;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        xo[i] = 0.0;
+        if (k.c[i] >= 0) need |= 1u << i;
+    }
+    for (unsigned long long it = 1;; ++it) {
+        double v[K];
+        long long l[K];
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+            if (need >> i & 1u) pair_ld(xt + k.c[i], v[i], l[i]);
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+            if ((need >> i & 1u) && l[i] == (long long)k.t[i]) {
+                xo[i] = v[i];
+                need &= ~(1u << i);
+            }
+        if (__all_sync(0xffffffffu, need == 0) || dead) break;
+        if ((it & 1023u) == 0 && (it > kGridSpinLimit || *(volatile int *)gerr)) {
+            dead = true;
+            atomicExch(gerr, 1);
+        }
+    }
+}
+
+template <int CACHE, int NT>
+__global__ void __launch_bounds__(NT, 1) k_flow_sweep(
+        const RowStep *__restrict__ sched, int32_t nord, const int32_t *__restrict__ col,
+        const double *__restrict__ val, const int32_t *__restrict__ tag, XPair *xt, Box box, int G,
+        const int *__restrict__ err, int *gerr) {
+    constexpr int NW = NT / 32, B = 2;  // B: chunks per batch beyond the cached ones
+    __shared__ FxPart parts[2][NW];
+    __shared__ double coef[2][NW];
+    if (*err) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int gl = wid / G, wg = wid - gl * G, bar = 1 + gl;
+    // consecutive steps on different SMs
+    const int64_t grp = (int64_t)gl * gridDim.x + blockIdx.x, NG = (int64_t)gridDim.x * (NW / G);
+    const RowStep none{0, 0, 0, 0.0, 0.0};
+    bool dead = false;
+    RowStep cur = grp < nord ? sched[grp] : none, nxt = grp + NG < nord ? sched[grp + NG] : none;
+    FlowChunks<CACHE> pc;
+    flow_load<CACHE>(cur, col, val, tag, lane, G, wg, pc);
+    int par = 0;
+    for (int64_t k = grp; k < nord; k += NG, par ^= 1) {
+        const RowStep nxt2 = k + 2 * NG < nord ? sched[k + 2 * NG] : none;
+        FlowChunks<CACHE> pn;
+        flow_load<CACHE>(nxt, col, val, tag, lane, G, wg, pn);
+        const int nq = (cur.len + 31) >> 5;
+        double xo[CACHE];
+        flow_wait<CACHE>(pc, xt, xo, dead, gerr);
+        double p0 = 0.0, p1 = 0.0;
+#pragma unroll
+        for (int i = 0; i < CACHE; ++i) {
+            if (wg + G * i >= nq) break;
+            if (i & 1) p1 = fma(xo[i], pc.v[i], p1);
+            else p0 = fma(xo[i], pc.v[i], p0);
+        }
+        for (int q0 = wg + G * CACHE; q0 < nq; q0 += G * B) {
+            FlowChunks<B> f;
+            double x2[B];
+            flow_load<B>(cur, col, val, tag, lane, G, q0, f);
+            flow_wait<B>(f, xt, x2, dead, gerr);
+            p0 = fma(x2[0], f.v[0], p0);
+            p1 = fma(x2[1], f.v[1], p1);
+        }
+        const FxPart part = fx_warp_part(p0, p1, (wg == 0 && lane == 0) ? -cur.b : 0.0);
+        const double c = step_coef(part, parts[par] + gl * G, &coef[par][gl], G, wg, lane, bar, cur.w);
+#pragma unroll
+        for (int i = 0; i < CACHE; ++i) {
+            if (wg + G * i >= nq) break;
+            if (pc.c[i] >= 0) pair_st(xt + pc.c[i], box.apply(fma(c, pc.v[i], xo[i])), cur.level);
+        }
+        for (int q0 = wg + G * CACHE; q0 < nq; q0 += G * B) {
+            FlowChunks<B> f;
+            flow_load<B>(cur, col, val, tag, lane, G, q0, f);
+#pragma unroll
+            for (int i = 0; i < B; ++i)
+                if (f.c[i] >= 0) {  // this step's until it writes it
+                    double v;
+                    long long l;
+                    pair_ld(xt + f.c[i], v, l);
+                    pair_st(xt + f.c[i], box.apply(fma(c, f.v[i], v)), cur.level);
+                }
+        }
+        cur = nxt;
+        nxt = nxt2;
+        pc = pn;
     }
 }
 
@@ -1294,7 +1615,8 @@ int lvl_grid_blocks(double spl, int G, int cs) {
 
 template <int CACHE, int NT>
 int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, const int *nlev,
-               const Box &box, int G, const int *err, double spl, cudaStream_t s) {
+               const int32_t *col, const double *val, const Box &box, int G, const int *err, double spl,
+               cudaStream_t s) {
     // cluster sizes found per device, x placement and image size (host
     // threads may sweep on different handles at once)
     static struct { int32_t n = -1; int want = 0, cs = 0; } cache[128][2];
@@ -1305,8 +1627,6 @@ int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, con
     const int want = std::max(1, env_int("FAIR_SWEEP_CLUSTER", 16));
     const bool xmem = env_int("FAIR_SWEEP_XMEM", 1) != 0;
     const int32_t n = S.A->n;
-    const int32_t *col = S.A->col.as<int32_t>();
-    const double *val = S.A->v64.as<double>();
     const size_t room = (size_t)optin - 8192;  // beside the static parts
     auto cluster = [&](int xd) {
         std::lock_guard<std::mutex> lk(cache_mu);
@@ -1358,11 +1678,42 @@ int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, con
                                              err, s);
 }
 
+// The sweep without barriers on a cooperative grid of nb blocks; gsync: {unused, unused, error}.
+template <int CACHE, int NT>
+int flow_launch(int nb, const RowStep *sched, int32_t nord, const int32_t *col, const double *val,
+                const int32_t *tag, XPair *xt, double *x, int32_t n, const Box &box, int G, const int *err,
+                int *gsync, cudaStream_t s) {
+    auto kern = k_flow_sweep<CACHE, NT>;
+    FAIR_CUDA(cudaMemsetAsync(gsync, 0, 4 * sizeof(int), s));
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)sm_count() * 8));
+    k_flow_pack<<<g, 256, 0, s>>>(x, n, xt);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(NT);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    FAIR_CUDA(cudaLaunchKernelEx(&cfg, kern, sched, nord, col, val, tag, xt, box, G, err, gsync + 2));
+    k_flow_unpack<<<g, 256, 0, s>>>(xt, n, x);
+    FAIR_CUDA(cudaGetLastError());
+    int gerr = 0;
+    FAIR_CUDA(cudaMemcpyAsync(&gerr, gsync + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+    FAIR_CUDA(cudaStreamSynchronize(s));
+    if (gerr) {
+        set_detail("Kaczmarz sweep: a step waited too long for its columns");
+        return FAIR_ERR_CUDA;
+    }
+    return FAIR_OK;
+}
+
 // The levels on a 16-block cluster (the level table in global memory);
 // false when no such cluster can be had (FAIR_SWEEP_CLUSTER below 16 also
 // keeps the single block).
 template <int WR>
-bool lvl_levels_cluster(SweepWork &W, int32_t nord, int *nlev, cudaStream_t s) {
+bool lvl_levels_cluster(SweepWork &W, int32_t nord, int *nlev, int32_t *otag, cudaStream_t s) {
     if (env_int("FAIR_SWEEP_CLUSTER", 16) < 16) return false;
     auto kern = k_lvl_levels_cluster<WR, 16>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -1389,7 +1740,42 @@ bool lvl_levels_cluster(SweepWork &W, int32_t nord, int *nlev, cudaStream_t s) {
         cudaLaunchKernelEx(&cfg, kern, (const WinRow *)W.rec.as<WinRow>(),
                            (const unsigned char *)W.dpath.as<unsigned char>(),
                            (const int32_t *)W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(),
-                           W.lvl.as<int32_t>(), nlev) != cudaSuccess) {
+                           W.lvl.as<int32_t>(), otag, nlev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
+// The levels on a cooperative grid of WR blocks (a step of every window each);
+// false when the device cannot hold them at once (FAIR_SWEEP_CLUSTER also keeps
+// to the cluster). gsync: {barrier counter, unused, error}, read by the caller.
+template <int WR>
+bool lvl_levels_grid(SweepWork &W, int32_t nord, int *nlev, int32_t *otag, cudaStream_t s) {
+    if (getenv("FAIR_SWEEP_CLUSTER")) return false;
+    auto kern = k_lvl_levels_grid<WR>;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 512, 0) != cudaSuccess || occ * sm_count() < WR ||
+        W.bases.grow(2 * WR * sizeof(unsigned long long))) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(WR);
+    cfg.blockDim = dim3(512);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaMemsetAsync(nlev, 0, sizeof(int), s) != cudaSuccess ||
+        cudaMemsetAsync(W.bases.p, 0, 2 * WR * sizeof(unsigned long long), s) != cudaSuccess ||
+        cudaLaunchKernelEx(&cfg, kern, (const WinRow *)W.rec.as<WinRow>(),
+                           (const unsigned char *)W.dpath.as<unsigned char>(),
+                           (const int32_t *)W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(),
+                           W.lvl.as<int32_t>(), otag, W.bases.as<unsigned long long>(),
+                           W.gsync.as<unsigned>(), W.gsync.as<int>() + 2, nlev) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -1400,13 +1786,14 @@ bool lvl_levels_cluster(SweepWork &W, int32_t nord, int *nlev, cudaStream_t s) {
 // a buffer cannot be had.
 template <int WR>
 int lvl_build(const SweepDev &S, SweepWork &W, SweepWork::Levels &C, const RowStep *steps, size_t setup_smem,
-              size_t optin, bool want, bool *built, cudaStream_t s) {
+              size_t optin, bool want, bool flow, bool *built, cudaStream_t s) {
     const DevCSR &A = *S.A;
     const int32_t nord = S.nord;
     const int nwin = (nord + WR - 1) / WR;
     const size_t tab_row = (size_t)std::max<int32_t>(A.n, 1) * sizeof(unsigned long long);
     int blocks = std::min(nwin, 2 * sm_count());
     blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)blocks, ((size_t)2 << 30) / tab_row));
+    int32_t *otag = flow ? W.tag.as<int32_t>() : nullptr;
     *built = false;
     if (W.dpath.grow((size_t)WR * ((size_t)nord + WR))) return FAIR_OK;
     if (W.tab_n != A.n || W.tab_blocks < blocks || W.uid + (uint64_t)nwin >= kStampIdLimit) {
@@ -1423,7 +1810,8 @@ int lvl_build(const SweepDev &S, SweepWork &W, SweepWork::Levels &C, const RowSt
                                    (int)setup_smem));
     k_lvl_setup<WR><<<blocks, kSetupThreads, setup_smem, s>>>(
         steps, W.eoff.as<int64_t>(), nord, A.col.as<int32_t>(), W.tabs.as<unsigned long long>(), A.n, W.uid,
-        W.idx.as<int32_t>(), W.rec.as<WinRow>(), W.dpath.as<unsigned char>(), W.err.as<int>());
+        W.idx.as<int32_t>(), W.rec.as<WinRow>(), W.dpath.as<unsigned char>(), A.v64.as<double>(),
+        W.gval.as<double>(), otag, W.err.as<int>());
     FAIR_CUDA(cudaGetLastError());
     W.err_valid = true;
     W.uid += (uint64_t)nwin;
@@ -1437,15 +1825,18 @@ int lvl_build(const SweepDev &S, SweepWork &W, SweepWork::Levels &C, const RowSt
         return FAIR_OK;
     }
     FAIR_CUDA(cudaMemsetAsync(W.lvtab.p, 0, lv_bytes, s));
-    if (!lvl_levels_cluster<WR>(W, nord, C.dnlev.as<int>(), s)) {
+    if (!lvl_levels_grid<WR>(W, nord, C.dnlev.as<int>(), otag, s) &&
+        !lvl_levels_cluster<WR>(W, nord, C.dnlev.as<int>(), otag, s)) {
         const bool smem = lv_bytes + 4096 <= optin;
         auto kern = smem ? k_lvl_levels<WR, true> : k_lvl_levels<WR, false>;
         if (smem)
             FAIR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lv_bytes));
         kern<<<1, 1024, smem ? lv_bytes : 0, s>>>(W.rec.as<WinRow>(), W.dpath.as<unsigned char>(),
                                                   W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(), A.n,
-                                                  W.lvl.as<int32_t>(), C.dnlev.as<int>());
+                                                  W.lvl.as<int32_t>(), otag, C.dnlev.as<int>());
     }
+    if (flow)
+        k_lvl_tags<WR><<<sm_count() * 8, 256, 0, s>>>(W.rec.as<WinRow>(), nord, W.lvl.as<int32_t>(), otag);
     FAIR_CUDA(cudaGetLastError());
     return FAIR_OK;
 }
@@ -1485,6 +1876,7 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
             C.nlev = O.nlev;
             C.entries = O.entries;
             C.use = O.use;
+            C.grouped = O.grouped;
             C.key = S.order_key;
             C.nord = nord;
         }
@@ -1502,36 +1894,54 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
         };
         const int wr = fits(128) ? 128 : fits(64) ? 64 : 32;
         if (!fits(wr)) return FAIR_OK;
-        // the entries of this sweep: an upper bound from the longest row
-        const size_t ent = (size_t)nord * (size_t)row_max;
         if (W.lens.grow(4 * ((size_t)nord + 1)) || W.eoff.grow(8 * ((size_t)nord + 1)) ||
-            W.idx.grow(4 * ent) || W.rec.grow(sizeof(WinRow) * (size_t)nord) || W.lvl.grow(4 * (size_t)nord) ||
+            W.rec.grow(sizeof(WinRow) * (size_t)nord) || W.lvl.grow(4 * (size_t)nord) ||
             W.cnt.grow(4 * ((size_t)nord + 1)) || W.err.grow(sizeof(int)) ||
             C.sched.grow(sizeof(RowStep) * (size_t)nord) || C.lptr.grow(8 * ((size_t)nord + 2)) ||
-            C.dnlev.grow(sizeof(int)))
+            C.dnlev.grow(sizeof(int)) || W.gsync.grow(4 * sizeof(int)))
             return FAIR_OK;
+        FAIR_CUDA(cudaMemsetAsync(W.gsync.p, 0, 4 * sizeof(int), s));
         k_step_lengths<<<g, 256, 0, s>>>(steps, nord, W.lens.as<int32_t>());
         k_scan_excl<<<1, 1024, 0, s>>>(W.lens.as<int32_t>(), nord, nullptr, W.eoff.as<int64_t>());
         FAIR_CUDA(cudaMemsetAsync(W.err.p, 0, sizeof(int), s));
+        FAIR_CUDA(cudaMemcpyAsync(&C.entries, W.eoff.as<int64_t>() + nord, sizeof(int64_t),
+                                  cudaMemcpyDeviceToHost, s));
+        FAIR_CUDA(cudaStreamSynchronize(s));
+        const size_t ent = (size_t)C.entries;
+        if (W.idx.grow(4 * std::max<size_t>(ent, 1))) return FAIR_OK;
+        // the sweep without barriers needs a copy of the entries in step order with
+        // their tags; the variables that pick a barrier sweep keep to it
+        const bool flow = want && S.order_key != 0 && env_int("FAIR_SWEEP_FLOW", 1) && !getenv("FAIR_SWEEP_CLUSTER") &&
+                          !getenv("FAIR_SWEEP_GRID") && !getenv("FAIR_SWEEP_XMEM") &&
+                          !W.gval.grow(8 * std::max<size_t>(ent, 1)) && !W.tag.grow(4 * std::max<size_t>(ent, 1)) &&
+                          !W.pairs.grow(sizeof(XPair) * (size_t)std::max<int32_t>(A.n, 1));
+        W.flow_slot = -1;
         const size_t smem = (size_t)(wr * row_max);
         bool built = false;
-        if (wr == 128) FAIR_TRY(lvl_build<128>(S, W, C, steps, smem, optin, want, &built, s));
-        else if (wr == 64) FAIR_TRY(lvl_build<64>(S, W, C, steps, smem, optin, want, &built, s));
-        else FAIR_TRY(lvl_build<32>(S, W, C, steps, smem, optin, want, &built, s));
+        if (wr == 128) FAIR_TRY(lvl_build<128>(S, W, C, steps, smem, optin, want, flow, &built, s));
+        else if (wr == 64) FAIR_TRY(lvl_build<64>(S, W, C, steps, smem, optin, want, flow, &built, s));
+        else FAIR_TRY(lvl_build<32>(S, W, C, steps, smem, optin, want, flow, &built, s));
         if (!built || !want) return FAIR_OK;
         FAIR_CUDA(cudaMemsetAsync(W.cnt.p, 0, 4 * ((size_t)nord + 1), s));
         k_lvl_count<<<g, 256, 0, s>>>(W.lvl.as<int32_t>(), nord, W.cnt.as<int32_t>());
         k_scan_excl<<<1, 1024, 0, s>>>(W.cnt.as<int32_t>(), 0, C.dnlev.as<int>(), C.lptr.as<int64_t>());
         k_lvl_scatter<<<g, 256, 0, s>>>(steps, W.lvl.as<int32_t>(), nord, C.lptr.as<int64_t>(),
-                                        W.cnt.as<int32_t>(), C.sched.as<RowStep>());
+                                        W.cnt.as<int32_t>(), flow ? W.eoff.as<int64_t>() : nullptr,
+                                        C.sched.as<RowStep>());
         FAIR_CUDA(cudaGetLastError());
         // levels pay when they hold several steps each (the ray orders: 30-80);
         // an order whose steps nearly all depend on the one before runs on the
         // single-block kernel
+        int gerr = 0;
+        FAIR_CUDA(cudaMemcpyAsync(&gerr, W.gsync.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
         FAIR_CUDA(cudaMemcpyAsync(&C.nlev, C.dnlev.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-        FAIR_CUDA(cudaMemcpyAsync(&C.entries, W.eoff.as<int64_t>() + nord, sizeof(int64_t),
-                                  cudaMemcpyDeviceToHost, s));
         FAIR_CUDA(cudaStreamSynchronize(s));
+        if (gerr) {
+            set_detail("Kaczmarz level set-up: a grid barrier timed out");
+            return FAIR_ERR_CUDA;
+        }
+        if (flow) W.flow_slot = slot;
+        C.grouped = flow;
         C.use = (int64_t)nord >= (int64_t)kMinStepsPerLevel * std::max(C.nlev, 1) ||
                 env_int("FAIR_SWEEP_LEVELS_ALWAYS", 0);
         C.key = S.order_key;
@@ -1557,7 +1967,29 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
     if (Ge == 1 || Ge == 2 || Ge == 4 || Ge == 8 || Ge == 16) G = Ge;
     if (W.gsync.grow(4 * sizeof(int))) return FAIR_OK;
     const double spl = C.nlev > 0 ? (double)S.nord / C.nlev : 1.0;
-    FAIR_TRY((lvl_launch<2, 512>(S, sched, lptr, nlev, box, G, err, spl, s)));
+    const int32_t *col = C.grouped ? W.idx.as<int32_t>() : A.col.as<int32_t>();
+    const double *val = C.grouped ? W.gval.as<double>() : A.v64.as<double>();
+    if (C.grouped && W.flow_slot == slot) {
+        // twice the warps of the barrier sweep: a warp's FP64 products lie on every
+        // level's chain (G = 4, 8, 16: fan N=128 21.3, 20.3, 20.5 ms; N=512 108, 92,
+        // 73 ms, two of its four sweeps with barriers)
+        const int Gf = Ge == 1 || Ge == 2 || Ge == 4 || Ge == 8 || Ge == 16 ? Ge : std::min(16, 2 * G);
+        int occ = 0;
+        auto kern = k_flow_sweep<2, 512>;
+        const int nb0 = env_int("FAIR_SWEEP_GRID_BLOCKS", 0);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 512, 0) == cudaSuccess && occ >= 1) {
+            // room for two levels' steps in flight: more groups only poll (10 sweeps of fan
+            // N=128, G = 8: 32 blocks 20.3 ms, 64 20.9, 152 22.0)
+            const int room = (int)std::ceil(spl * 2.0 * Gf / 16.0);
+            const int nb = std::min(nb0 > 0 ? nb0 : std::max(room, 1), occ * sm_count());
+            FAIR_TRY((flow_launch<2, 512>(nb, sched, S.nord, col, val, W.tag.as<int32_t>(), W.pairs.as<XPair>(), S.x,
+                                          A.n, box, Gf, err, W.gsync.as<int>(), s)));
+            *done = true;
+            return FAIR_OK;
+        }
+        cudaGetLastError();
+    }
+    FAIR_TRY((lvl_launch<2, 512>(S, sched, lptr, nlev, col, val, box, G, err, spl, s)));
     *done = true;
     return FAIR_OK;
 }
@@ -1577,6 +2009,11 @@ void SweepWork::release() {
     err.release();
     tabs.release();
     gsync.release();
+    gval.release();
+    tag.release();
+    pairs.release();
+    bases.release();
+    flow_slot = -1;
     for (Levels &L : lev) {
         L.sched.release();
         L.lptr.release();
@@ -1584,7 +2021,7 @@ void SweepWork::release() {
         L.key = 0;
         L.nord = L.nlev = 0;
         L.entries = 0;
-        L.use = false;
+        L.use = L.grouped = false;
     }
     tab_n = tab_blocks = 0;
     uid = 0;

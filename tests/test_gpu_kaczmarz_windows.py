@@ -23,12 +23,13 @@ def both(fair, oracle, A, R, b, method, K, order=None, **kw):
     return rel_err(X, Xr)
 
 
-@pytest.mark.parametrize("cluster", ["1", "16"])
+@pytest.mark.parametrize("cluster", ["", "1", "16"])
 @pytest.mark.parametrize("steps", [1, 2, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257])
 def test_window_edges(fair, oracle, monkeypatch, steps, cluster):
     """Sweeps of `steps` rows in a shuffled order, forwards and back."""
     monkeypatch.setenv("FAIR_SWEEP_LEVELS_ALWAYS", "1")
-    monkeypatch.setenv("FAIR_SWEEP_CLUSTER", cluster)
+    if cluster:  # unset: the sweep without barriers, levels on a grid
+        monkeypatch.setenv("FAIR_SWEEP_CLUSTER", cluster)
     n, nth, p = 24, 9, 34
     th = oracle.linspace(0.0, np.pi, nth)
     A = fair.paralleltomo(fair.Data(n=n, p=p, nth=nth, theta=th))
@@ -41,13 +42,14 @@ def test_window_edges(fair, oracle, monkeypatch, steps, cluster):
         assert both(fair, oracle, A, R, b, method, [2], order, relaxpar=0.7, lbound=0.0) < TOL64
 
 
-@pytest.mark.parametrize("cluster", ["1", "16"])
+@pytest.mark.parametrize("cluster", ["", "1", "16"])
 @pytest.mark.parametrize("longest", [1655, 1656, 3528, 3529, 7200, 7201])
 def test_window_widths(fair, oracle, monkeypatch, longest, cluster):
     """Longest rows on both sides of each window width's limit of shared
     memory (past the last, the sweep runs without levels)."""
     monkeypatch.setenv("FAIR_SWEEP_LEVELS_ALWAYS", "1")
-    monkeypatch.setenv("FAIR_SWEEP_CLUSTER", cluster)
+    if cluster:  # unset: the sweep without barriers, levels on a grid
+        monkeypatch.setenv("FAIR_SWEEP_CLUSTER", cluster)
     rng = np.random.default_rng(longest)
     m, n = 140, 8000
     lens = rng.integers(1, 60, m)
