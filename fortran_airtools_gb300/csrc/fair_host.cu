@@ -729,8 +729,22 @@ int fair_sirt(double *xout, const char *sirt_method, fair_csr h, const double *b
     S.ub = o.ub;
     S.sched = h->w_sched.as<unsigned>();
     FAIR_TRY(sirt_prepare_shadow(S, s));
-    FAIR_TRY(sirt_iterations(S, maxits, s));
-    return download<double>(xout, h->w_x.p, (size_t)n, s);
+    bool resident = false;
+    unsigned *gbar = h->w_sched.as<unsigned>() + 2;
+    FAIR_TRY(sirt_resident(S, maxits, gbar, s, &resident));
+    if (!resident) {
+        FAIR_TRY(sirt_iterations(S, maxits, s));
+        return download<double>(xout, h->w_x.p, (size_t)n, s);
+    }
+    unsigned gerr = 0;
+    FAIR_CUDA(cudaMemcpyAsync(&gerr, gbar + 1, sizeof(gerr), cudaMemcpyDeviceToHost, s));
+    FAIR_TRY(download<double>(xout, h->w_x.p, (size_t)n, s));
+    if (gerr) {
+        FAIR_CUDA(cudaMemsetAsync(gbar, 0, 2 * sizeof(unsigned), s));
+        set_detail("SIRT: a grid barrier timed out");
+        return FAIR_ERR_CUDA;
+    }
+    return FAIR_OK;
 }
 
 // ------------------------------------------------------ normest / gradient ----

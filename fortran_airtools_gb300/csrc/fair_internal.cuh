@@ -261,6 +261,8 @@ int sirt_weights_recip(const DevCSR &A, const DevCSR &AT, bool sart, double *d_M
 // v = 1/v elementwise (IEEE: 1/0 = Inf, 1/Inf = 0).
 int vec_reciprocal(double *v, int64_t n, cudaStream_t s);
 int sirt_iterations(const SirtDev &S, int K, cudaStream_t s);
+// The K iterations of a small FP64 problem in one launch (*ran: launched).
+int sirt_resident(const SirtDev &S, int K, unsigned *gbar, cudaStream_t s, bool *ran);
 // One SIRT pass (1: residual over A, 2: update over A') with the forms
 // already made; enqueues one kernel.
 void sirt_pass(const SirtDev &S, int pass, cudaStream_t s);
@@ -467,7 +469,7 @@ struct fair_csr_s {
     fair::DevBuf w_in, w_out, w_b, w_x, w_x32, w_r, w_M, w_D, w_xn, w_tmp, w_part, w_flag;
     fair::DevBuf w_ord, w_cumul, w_nrA, w_y;
     fair::DevBuf w_adj[19];  // the adjoint's vectors, kept between calls
-    fair::DevBuf w_sched;  // two zeroed counters for dynamic chunk scheduling
+    fair::DevBuf w_sched;  // two zeroed counters for dynamic chunk scheduling; a grid barrier's counter and error
     fair::SweepWork w_sweep;  // Kaczmarz sweep buffers (released after each call)
     // state of fair_sirt_prepare (device-resident SIRT)
     bool sirt_ready = false, sirt_sart = false;

@@ -44,6 +44,7 @@
 #include <mutex>
 
 #include "fair_internal.cuh"
+#include "grid_barrier.cuh"
 
 namespace fair {
 
@@ -854,42 +855,6 @@ __global__ void __launch_bounds__(512, 1) k_lvl_levels_cluster(
     if (lane == 0 && top > 0) atomicMax(nlev, top);
 }
 
-// A barrier of all blocks of a cooperative launch on one counter, gbar[0]
-// (zero at the launch): block 0 adds 2^31 - (blocks - 1), every other block
-// 1, so the counter's top bit flips exactly when the last block arrives -- one
-// reduction per block, nothing to reset (the counter wraps) and, the barriers
-// being counted (phase: the top bit before this one), no value to wait for.
-// The arrival releases the block's writes of the level; the waiting thread
-// reads the counter with acquire semantics. A block that waits more than
-// kGridSpinLimit polls, or sees *gerr set (checked every 1024 polls), sets
-// *gerr and returns false; the sweep then stops, and the host reports the
-// error.
-constexpr unsigned long long kGridSpinLimit = 1ull << 26;
-enum { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
-
-__device__ __forceinline__ bool grid_barrier(unsigned *gbar, int *gerr, unsigned phase) {
-    __shared__ int ok_s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u;
-        int ok = 1;
-        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(gbar), "r"(add) : "memory");
-        for (unsigned long long it = 1;; ++it) {
-            unsigned cur;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(gbar) : "memory");
-            if ((cur >> 31) != phase) break;
-            if ((it & 1023u) == 0 && (it > kGridSpinLimit || *(volatile int *)gerr)) {
-                atomicExch(gerr, 1);
-                ok = 0;
-                break;
-            }
-        }
-        ok_s = ok;
-    }
-    __syncthreads();
-    return ok_s != 0;
-}
-
 // The same on a cooperative grid, a step of the window per block: the scattered
 // table accesses are spread over up to WR SMs, and each thread's columns (the
 // next window's loaded while a window runs) serve both phases from registers.
@@ -1250,6 +1215,8 @@ __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__rest
     }
 }
 
+
+enum { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
 
 // The levels in order on one cluster of gridDim.x blocks (CLUSTER) or one
 // block. Groups of G consecutive warps take the steps of a level in turn; each

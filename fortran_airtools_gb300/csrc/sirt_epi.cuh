@@ -33,9 +33,10 @@ __device__ __forceinline__ double sirt_box(double t, int bmode, double lb, doubl
 struct EpiResidF64 {  // r = (b - Ax) / M
     const double *b, *Mi;  // Mi = 1/M
     double *r;
-    __device__ void operator()(int64_t i, double acc) const {
-        r[i] = __dmul_rn(__dsub_rn(b[i], acc), Mi[i]);
+    static __device__ __forceinline__ double value(double b, double Mi, double acc) {
+        return __dmul_rn(__dsub_rn(b, acc), Mi);
     }
+    __device__ void operator()(int64_t i, double acc) const { r[i] = value(b[i], Mi[i], acc); }
 };
 struct EpiResidLP {  // same, FP32 dot, FP64 weighting, FP32 residual
     const double *b, *Mi;
@@ -50,11 +51,12 @@ struct EpiUpdateF64 {  // x = P(x + omg * (A'r) / D)
     double *x;
     double omg, lb, ub;
     int bmode;
-    __device__ void operator()(int64_t j, double acc) const {
+    __device__ __forceinline__ double value(double xj, double D, double acc) const {  // D: Di[j], if any
         double g = __dmul_rn(omg, acc);
-        if (Di) g = __dmul_rn(g, Di[j]);
-        x[j] = sirt_box(__dadd_rn(x[j], g), bmode, lb, ub);
+        if (Di) g = __dmul_rn(g, D);
+        return sirt_box(__dadd_rn(xj, g), bmode, lb, ub);
     }
+    __device__ void operator()(int64_t j, double acc) const { x[j] = value(x[j], Di ? Di[j] : 0.0, acc); }
 };
 struct EpiUpdateLP {
     const double *Di;
