@@ -425,12 +425,78 @@ __global__ void __launch_bounds__(256, 2) k_sirt_resident_f64(
     }
 }
 
+// The same for more rows: a warp takes the groups w, w + W, ... of every pass, the
+// first from registers (its entries and the second's offsets stay there), each
+// next group's entries and the offsets of the one after it loaded while a
+// group's sums are formed. Two blocks per SM with 128 registers (three with 80
+// spill: fan N = 128, 100 iterations 3.92 ms against 3.51). The launches one by
+// one take 4.24 ms there.
+template <int G>
+__global__ void __launch_bounds__(256, 2) k_sirt_resident_many_f64(
+        const int64_t *rpA, int32_t m, const int32_t *colA, const double *vA, const int64_t *rpT, int32_t n,
+        const int32_t *colT, const double *vT, EpiResidF64 e1, EpiUpdateF64 e2, int K, unsigned *gbar,
+        int *gerr) {
+    using ST = CsrSteps<double, double, double, G>;
+    constexpr int R = 32 / G;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, g = lane / G, gl = lane % G;
+    const int64_t first = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * R;
+    const int64_t step = (((int64_t)gridDim.x * blockDim.x) >> 5) * R;
+    struct Rows {
+        int64_t s, ns;  // this group's row; the next group's
+        int len, nl;
+        typename ST::Raw r0, r1;
+    };
+    auto offsets = [&](const ST &st, int32_t rows, int64_t row, int64_t &s, int &len) {
+        s = 0;
+        len = 0;
+        if (row < rows) {
+            s = __ldg(st.off + row);
+            len = (int)(__ldg(st.off + row + 1) - s);
+        }
+    };
+    auto open = [&](const ST &st, int32_t rows) {
+        Rows q{0, 0, 0, 0, {}, {}};
+        offsets(st, rows, first + g, q.s, q.len);
+        offsets(st, rows, first + step + g, q.ns, q.nl);
+        st.load(q.r0, q.s, st.first(q.s, gl), q.len);
+        st.load(q.r1, q.s, st.first(q.s, gl) + ST::STEP, q.len);
+        return q;
+    };
+    auto pass = [&](const ST &st, Rows q, int32_t rows, const double *v, auto &epi) {
+        for (int64_t row0 = first; row0 < rows; row0 += step) {
+            double acc = steps_part<double, double>(st, q.s, q.len, gl, q.r0, q.r1, v);
+            q.s = q.ns;
+            q.len = q.nl;
+            offsets(st, rows, row0 + 2 * step + g, q.ns, q.nl);
+            st.load(q.r0, q.s, st.first(q.s, gl), q.len);
+            st.load(q.r1, q.s, st.first(q.s, gl) + ST::STEP, q.len);
+            acc = group_sum<double, G>(acc);
+            const double sum = __shfl_sync(FULL, acc, (lane & (R - 1)) * G);
+            if (lane < R && row0 + lane < rows) epi(row0 + lane, sum);
+        }
+    };
+    const ST sa{rpA, colA, vA}, stt{rpT, colT, vT};
+    const Rows qa = open(sa, m), qt = open(stt, n);
+    for (int it = 0; it < K; ++it) {
+        pass(sa, qa, m, e2.x, e1);
+        if (!grid_barrier(gbar, gerr, 0)) return;
+        pass(stt, qt, n, e1.r, e2);
+        if (!grid_barrier(gbar, gerr, 1)) return;
+    }
+}
+
 // Runs the K iterations in one launch (*ran = true) where the problem is small
-// enough: FP64 on the CSR, a warp for every group of rows in at most two
-// blocks of 8 warps per SM (9,728 rows at 8 lanes per row; at 9,200 rows it is
-// still 1.5 times as fast as the launches). gbar: {barrier counter, error}, zero; the counter is
-// zero again after an even number of barriers, the error is the caller's to read
-// behind the launch.
+// enough: FP64 on the CSR, and either a warp for every group of rows in at most
+// two blocks of 8 warps per SM (9,728 rows at 8 lanes per row; at 9,200 rows 1.5
+// times as fast as the launches) or at most 3,100 nonzeros per such warp (100
+// iterations, ms against launches: fan N = 128, 180 angles, 800 per warp, 2.12
+// and 2.81; 360 angles, 1,600 per warp, 3.51 and 4.24; parallel N = 128, 360
+// angles, 3,080 per warp, 5.53 and 6.06; N = 192, 180 angles, 3,470 per warp,
+// 6.18 and 6.13; N = 181, 360 angles, 6,170 per warp, 11.4 and 9.6: the 24 warps
+// per SM of the launches hide more). gbar: {barrier counter, error}, zero; the
+// counter is zero again after an even number of barriers, the error is the
+// caller's to read behind the launch.
 int sirt_resident(const SirtDev &S, int K, unsigned *gbar, cudaStream_t s, bool *ran) {
     *ran = false;
     const DevCSR &A = *S.A, &T = *S.AT;
@@ -440,8 +506,10 @@ int sirt_resident(const SirtDev &S, int K, unsigned *gbar, cudaStream_t s, bool 
         getenv("FAIR_ROWS_BY_GROUP"))
         return FAIR_OK;
     const int64_t groups = ((int64_t)std::max(A.m, T.m) + 32 / G - 1) / (32 / G);
-    const int64_t blocks = (groups + 7) / 8;
-    if (blocks > 2 * (int64_t)sm_count()) return FAIR_OK;
+    const int64_t room = 2 * (int64_t)sm_count();
+    const bool many = (groups + 7) / 8 > room;
+    if (many && A.nnz > 3100 * 8 * room) return FAIR_OK;
+    const int64_t blocks = std::min((groups + 7) / 8, room);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(256);
@@ -469,10 +537,10 @@ int sirt_resident(const SirtDev &S, int K, unsigned *gbar, cudaStream_t s, bool 
         return FAIR_OK;
     };
     switch (G) {
-        case 4: return launch(k_sirt_resident_f64<4>);
-        case 16: return launch(k_sirt_resident_f64<16>);
-        case 32: return launch(k_sirt_resident_f64<32>);
-        default: return launch(k_sirt_resident_f64<8>);
+        case 4: return many ? launch(k_sirt_resident_many_f64<4>) : launch(k_sirt_resident_f64<4>);
+        case 16: return many ? launch(k_sirt_resident_many_f64<16>) : launch(k_sirt_resident_f64<16>);
+        case 32: return many ? launch(k_sirt_resident_many_f64<32>) : launch(k_sirt_resident_f64<32>);
+        default: return many ? launch(k_sirt_resident_many_f64<8>) : launch(k_sirt_resident_f64<8>);
     }
 }
 

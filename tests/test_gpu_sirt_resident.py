@@ -1,4 +1,4 @@
-"""Small FP64 SIRT problems in one launch (every warp's rows in registers, a grid
+"""Small FP64 SIRT problems in one launch (a warp's first rows in registers, a grid
 barrier between passes): bit for bit the passes launched one by one, which
 FAIR_ROWS_BY_GROUP=1 selects, and within 1e-10 of the oracle.
 """
@@ -12,7 +12,9 @@ from conftest import rel_err
 pytestmark = pytest.mark.gpu
 
 # N, angles, bins: one group of rows to just past two blocks per SM (152 SMs x 16 warps x 4 rows)
-SHAPES = [(1, 1, 2), (2, 3, 5), (7, 9, 12), (24, 20, 35), (40, 60, 58), (90, 70, 130), (98, 70, 139)]
+# and several groups per warp
+SHAPES = [(1, 1, 2), (2, 3, 5), (7, 9, 12), (24, 20, 35), (40, 60, 58), (90, 70, 130), (98, 70, 139),
+          (64, 180, 91), (128, 60, 181)]
 
 
 def sirt(fair, A, b, method, K, **kw):
@@ -40,12 +42,13 @@ def test_equals_passes_and_oracle(fair, oracle, monkeypatch, shape, method):
         assert rel_err(y[f], xr[f]) < 1e-10
 
 
+@pytest.mark.parametrize("m", [150, 12001])
 @pytest.mark.parametrize("lanes", [4, 8, 16, 32])
-def test_lanes_per_row_and_long_rows(fair, oracle, monkeypatch, lanes):
+def test_lanes_per_row_and_long_rows(fair, oracle, monkeypatch, lanes, m):
     """Rows from empty to past the entries held in registers."""
     from fortran_airtools_gb300._clib import check, lib
     rng = np.random.default_rng(lanes)
-    m, n = 150, 700
+    n = 700
     lens = rng.integers(0, 300, m)
     lens[:8] = 0
     IA = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
