@@ -330,8 +330,7 @@ int launch(const SweepDev &S, const RowStep *steps, bool smem, size_t smem_bytes
     const DevCSR &A = *S.A;
     if (smem) {
         auto kern = k_sweep<W, CACHE, true>;
-        FAIR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem_bytes));
+        FAIR_CUDA(smem_allow(reinterpret_cast<const void *>(kern), smem_bytes));
         kern<<<1, 32 * W, smem_bytes, s>>>(steps, S.nord, A.col.as<int32_t>(), A.v64.as<double>(),
                                           S.x, A.n, box, dup, only_if_dup);
     } else {
@@ -1499,7 +1498,7 @@ int lvl_cluster_size(int want, int32_t n, size_t room) {
         if (cs > want) continue;
         const size_t smem = XM == XD ? (size_t)8 << part_log2(cs, n) : 0;
         if (XM == XD && smem > room) continue;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        if (smem_allow(reinterpret_cast<const void *>(kern), smem) != cudaSuccess ||
             (cs > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
             cudaGetLastError();
             continue;
@@ -1527,7 +1526,7 @@ int lvl_launch_cluster(int cs, size_t smem, const RowStep *sched, const int64_t 
                        const int *nlev, const int32_t *col, const double *val, double *x,
                        int32_t n, int cb, const Box &box, int G, const int *err, cudaStream_t s) {
     auto kern = k_lvl_sweep<SYNC_CLUSTER, XM, CACHE, NT>;
-    FAIR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FAIR_CUDA(smem_allow(reinterpret_cast<const void *>(kern), smem));
     if (cs > 8) FAIR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(cs);
@@ -1647,8 +1646,7 @@ int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, con
         }
         if ((size_t)8 * n <= room) {
             auto kern = k_lvl_sweep<SYNC_BLOCK, XS, CACHE, NT>;
-            FAIR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(8 * (size_t)n)));
+            FAIR_CUDA(smem_allow(reinterpret_cast<const void *>(kern), 8 * (size_t)n));
             kern<<<1, NT, 8 * (size_t)n, s>>>(sched, lptr, nlev, col, val, S.x, n, 0, box, G, err, nullptr,
                                                nullptr);
             FAIR_CUDA(cudaGetLastError());
@@ -1794,8 +1792,7 @@ int lvl_build(const SweepDev &S, SweepWork &W, SweepWork::Levels &C, const RowSt
         W.tab_blocks = blocks;
         W.uid = 0;
     }
-    FAIR_CUDA(cudaFuncSetAttribute(k_lvl_setup<WR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)setup_smem));
+    FAIR_CUDA(smem_allow(reinterpret_cast<const void *>(k_lvl_setup<WR>), setup_smem));
     k_lvl_setup<WR><<<blocks, kSetupThreads, setup_smem, s>>>(
         steps, W.eoff.as<int64_t>(), nord, A.col.as<int32_t>(), W.tabs.as<unsigned long long>(), A.n, W.uid,
         W.idx.as<int32_t>(), W.rec.as<WinRow>(), W.dpath.as<unsigned char>(), A.v64.as<double>(),
@@ -1818,7 +1815,7 @@ int lvl_build(const SweepDev &S, SweepWork &W, SweepWork::Levels &C, const RowSt
         const bool smem = lv_bytes + 4096 <= optin;
         auto kern = smem ? k_lvl_levels<WR, true> : k_lvl_levels<WR, false>;
         if (smem)
-            FAIR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lv_bytes));
+            FAIR_CUDA(smem_allow(reinterpret_cast<const void *>(kern), lv_bytes));
         kern<<<1, 1024, smem ? lv_bytes : 0, s>>>(W.rec.as<WinRow>(), W.dpath.as<unsigned char>(),
                                                   W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(), A.n,
                                                   W.lvl.as<int32_t>(), otag, C.dnlev.as<int>());

@@ -815,25 +815,6 @@ TlGeo tl_geo(const DevCSR::Tiled &tl) {
     return G;
 }
 
-// Raise a kernel's dynamic shared-memory limit to `bytes` if it is lower
-// (never lowers it: the tiled copies of A and A' launch the same kernels with
-// tiles of different sizes).
-cudaError_t smem_allow(const void *kernel, size_t bytes) {
-    static std::mutex mu;
-    static std::vector<std::pair<const void *, size_t>> set;
-    std::lock_guard<std::mutex> lock(mu);
-    for (auto &k : set)
-        if (k.first == kernel) {
-            if (bytes <= k.second) return cudaSuccess;
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e == cudaSuccess) k.second = bytes;
-            return e;
-        }
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) set.emplace_back(kernel, bytes);
-    return e;
-}
-
 // Launches one pass on the tiled copy (partials, then row sums); errors are
 // left for the caller's cudaGetLastError.
 template <class LD, typename XT, typename ACC, class Epi>
@@ -1765,6 +1746,25 @@ int tl_batch_launch(const TlBatch &T, int prec, int pass, double omg, double lb,
         default:
             return tlb_run<TlFused<uint16_t>, float, float>(T, pass, omg, lb, ub, bmode, ctr, s, dry);
     }
+}
+
+// Raise a kernel's dynamic shared-memory limit to `bytes` if it is lower
+// (never lowers it: the tiled copies of A and A' launch the same kernels with
+// tiles of different sizes, and host threads sweep images of different sizes at once).
+cudaError_t smem_allow(const void *kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::vector<std::pair<const void *, size_t>> set;
+    std::lock_guard<std::mutex> lock(mu);
+    for (auto &k : set)
+        if (k.first == kernel) {
+            if (bytes <= k.second) return cudaSuccess;
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (e == cudaSuccess) k.second = bytes;
+            return e;
+        }
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) set.emplace_back(kernel, bytes);
+    return e;
 }
 
 }  // namespace fair
