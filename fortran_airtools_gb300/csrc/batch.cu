@@ -228,6 +228,7 @@ struct fair_batch_s {
     cudaGraphExec_t gexec = nullptr;
     int g_K = -1, g_cfg[4] = {0, 0, 0, 0};
     const double *g_x = nullptr;  // the shadow conversion of x is a graph node
+    fair::BOpts g_opts{1.0, 0.0, 0.0, 0};  // kernel arguments of the captured passes
     std::mutex mu;
 };
 
@@ -258,6 +259,12 @@ void drop_graph(fair_batch_s *B) {
     if (B->gexec) cudaGraphExecDestroy(B->gexec);
     B->gexec = nullptr;
     B->g_K = -1;
+}
+
+// Equal options, NaN bounds among them.
+bool same_opts(const BOpts &a, const BOpts &b) {
+    return a.bmode == b.bmode && !memcmp(&a.omg, &b.omg, sizeof(double)) &&
+           !memcmp(&a.lb, &b.lb, sizeof(double)) && !memcmp(&a.ub, &b.ub, sizeof(double));
 }
 
 // Descriptor tables of the two passes for vectors d_b, d_x.
@@ -851,7 +858,8 @@ int fair_batch_run_device(fair_batch B, const double *d_b, double *d_x, int32_t 
     std::lock_guard<std::mutex> lk(B->mu);
     FAIR_TRY(batch_bind(B, d_b, d_x));
     if (K == 0) return FAIR_OK;
-    if (!B->gexec || B->g_K != K || B->g_x != d_x || memcmp(B->g_cfg, B->cfg, sizeof(B->cfg)) != 0) {
+    if (!B->gexec || B->g_K != K || B->g_x != d_x || !fair::same_opts(B->g_opts, B->opts) ||
+        memcmp(B->g_cfg, B->cfg, sizeof(B->cfg)) != 0) {
         fair::drop_graph(B);
         FAIR_TRY(fair::batch_pass(B, 1, B->stream, true));  // grids looked up outside the capture
         FAIR_TRY(fair::batch_pass(B, 2, B->stream, true));
@@ -867,6 +875,7 @@ int fair_batch_run_device(fair_batch B, const double *d_b, double *d_x, int32_t 
         if (e != cudaSuccess) { B->gexec = nullptr; return fair::cuda_fail(e, "cudaGraphInstantiate", __FILE__, __LINE__); }
         B->g_K = K;
         B->g_x = d_x;
+        B->g_opts = B->opts;
         memcpy(B->g_cfg, B->cfg, sizeof(B->cfg));
     }
     FAIR_CUDA(cudaGraphLaunch(B->gexec, B->stream));
