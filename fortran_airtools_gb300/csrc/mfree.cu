@@ -283,11 +283,11 @@ __global__ void __launch_bounds__(128) k_mf_project(const MfAngle *__restrict__ 
 }
 
 // xt = the transpose of x viewed as an N x N array (32 x 32 tiles through
-// shared memory, both sides coalesced). *nonfinite becomes epoch (the pass's
-// number, larger than any before) if x holds an Inf or NaN.
+// shared memory, both sides coalesced). flag[0] becomes 1 if x holds an Inf or
+// NaN; the projector behind it takes it back (take_flag).
 template <typename T>
 __global__ void __launch_bounds__(256) k_mf_transpose(const T *__restrict__ x, T *__restrict__ xt,
-                                                      int N, unsigned *nonfinite, unsigned epoch) {
+                                                      int N, unsigned *flag) {
     __shared__ T tile[32][33];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(256) k_mf_transpose(const T *__restrict__ x, T
         if (r < N && c < N) {
             const T v = x[(int64_t)r * N + c];
             tile[k][threadIdx.x] = v;
-            if (sizeof(T) == 4 && !isfinite(v)) atomicMax(nonfinite, epoch);
+            if (sizeof(T) == 4 && !isfinite(v)) atomicExch(flag, 1u);
         }
     }
     __syncthreads();
@@ -303,6 +303,19 @@ __global__ void __launch_bounds__(256) k_mf_transpose(const T *__restrict__ x, T
         const int r = c0 + k, c = r0 + threadIdx.x;
         if (r < N && c < N) xt[(int64_t)r * N + c] = tile[threadIdx.x][k];
     }
+}
+
+// The flag of the transpose before this pass, for every thread of the block;
+// the last block to have read it sets it back to 0 (flag[1] counts them and wraps
+// to 0), so that a pass leaves nothing behind, run or replayed from a graph.
+__device__ __forceinline__ bool take_flag(unsigned *flag) {
+    const bool on = *reinterpret_cast<volatile unsigned *>(flag) != 0;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicInc(flag + 1, gridDim.x - 1) == gridDim.x - 1) atomicExch(flag, 0u);
+    }
+    return on;
 }
 
 // FP32 projector. A warp takes 32 adjacent rays of one angle and walks their
@@ -394,11 +407,10 @@ template <bool FAN, class Epi>
 __global__ void __launch_bounds__(128, 7) k_mf_project32(const MfAngle *__restrict__ ang, int nth, int p,
                                                       int N, const float *__restrict__ x,
                                                       const float *__restrict__ xt,
-                                                      const unsigned *__restrict__ nonfinite, unsigned epoch,
-                                                      Epi epi) {
+                                                      unsigned *flag, Epi epi) {
     const int lane = threadIdx.x & 31, wpa = (p + 31) / 32;
     const int64_t nw = (int64_t)nth * wpa;
-    const bool guard = *nonfinite == epoch;
+    const bool guard = take_flag(flag);
     for (int64_t g = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); g < nw;
          g += (int64_t)gridDim.x * (blockDim.x >> 5)) {
         const int i = (int)(g / wpa), j = (int)(g - (int64_t)i * wpa) * 32 + lane;
@@ -1093,8 +1105,7 @@ struct fair_mf_s {
     fair::DevBuf part;                 // the backprojector's sums per share of the angles
     fair::DevBuf w_in, w_out;          // host-call staging (FP64)
     fair::DevBuf xt;                   // the projector's transposed copy of x
-    fair::DevBuf nonfinite;            // the last pass whose x held an Inf or NaN
-    unsigned epoch = 0;                // passes of the projector
+    fair::DevBuf nonfinite;            // {x of the pass under way holds an Inf or NaN, blocks that know}
     fair::DevBuf v_a, v_b;             // reduced-precision staging
     // SIRT state
     bool ready = false, sart = false;
@@ -1115,8 +1126,8 @@ namespace {
 int mf_grow_xt(fair_mf A) {
     const size_t es = A->prec == FAIR_PREC_F64 ? sizeof(double) : sizeof(float);
     if (!A->nonfinite.p) {
-        FAIR_TRY(A->nonfinite.grow(sizeof(unsigned)));
-        FAIR_CUDA(cudaMemsetAsync(A->nonfinite.p, 0, sizeof(unsigned), A->stream));
+        FAIR_TRY(A->nonfinite.grow(2 * sizeof(unsigned)));
+        FAIR_CUDA(cudaMemsetAsync(A->nonfinite.p, 0, 2 * sizeof(unsigned), A->stream));
     }
     return A->xt.grow(es * (size_t)A->N * A->N);
 }
@@ -1130,17 +1141,16 @@ void mf_project(fair_mf A, const XT *x, Epi epi, cudaStream_t s) {
     unsigned *nf = A->nonfinite.as<unsigned>();
     if (MODE == 0) {  // the rays that walk rows read the transpose (mf_grow_xt)
         const int nb = (N + 31) / 32;
-        ++A->epoch;
-        k_mf_transpose<XT><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(x, A->xt.as<XT>(), N, nf, A->epoch);
+        k_mf_transpose<XT><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(x, A->xt.as<XT>(), N, nf);
         xt = A->xt.as<XT>();
     }
     if constexpr (std::is_same<ACC, float>::value) {
         static_assert(MODE == 0, "FP32 passes read x");
         const int g = grid_for((int64_t)A->nth * ((A->p + 31) / 32) * 32, 128);
         if (A->kind == 1)
-            k_mf_project32<true><<<g, 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, nf, A->epoch, epi);
+            k_mf_project32<true><<<g, 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, nf, epi);
         else
-            k_mf_project32<false><<<g, 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, nf, A->epoch, epi);
+            k_mf_project32<false><<<g, 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, nf, epi);
     } else if (A->kind == 1) {
         k_mf_project<XT, ACC, MODE, true><<<grid_for(m, 128), 128, 0, s>>>(ang, A->nth, A->p, N, x, xt, epi);
     } else {
