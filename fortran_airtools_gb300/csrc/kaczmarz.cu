@@ -124,7 +124,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // warp adds its lanes' integers exactly as three 26-bit limbs with
 // __reduce_add_sync, the warps' sums are aligned to the largest frame, and the
 // total is rounded to double once (round to nearest even). A row of up to
-// 8 x 32 lanes x 2 partials + b stays below 2^63.
+// 8 x 32 lanes x 2 partials + b stays below 2^63; 16 warps' may not (fx_group).
 __device__ __forceinline__ int fx_exp(double v) {
     const int e = (int)((__double_as_longlong(v) >> 52) & 0x7FF);
     return e > 1 ? e : 1;
@@ -439,6 +439,18 @@ __device__ __forceinline__ double fx_to_double_fast(long long total, int E) {
     if (field >= 1 && field <= 2046)
         return __longlong_as_double(bits + ((long long)(E - 1075) << 52));
     return fx_to_double(total, E);
+}
+
+// The sum of the lanes' aligned parts F (|F| < 2^59 + 2^53), rounded once. 16
+// parts can reach 2^63 + 2^53: a total near the ends of 64 bits is formed halved,
+// its lost bit kept as the lowest one, which no rounding to 53 bits looks past.
+__device__ __forceinline__ double fx_group(long long F, int E) {
+    const unsigned l0 = __reduce_add_sync(0xffffffffu, (unsigned)(F & 0x3FFFFFF));
+    const unsigned l1 = __reduce_add_sync(0xffffffffu, (unsigned)((F >> 26) & 0x3FFFFFF));
+    const int l2 = __reduce_add_sync(0xffffffffu, (int)(F >> 52));
+    const long long m = (long long)l1 * (1LL << 26) + (long long)l0;  // < 2^57 + 2^31
+    if ((unsigned)(l2 + 2048) < 4096u - 33u) return fx_to_double_fast((long long)l2 * (1LL << 52) + m, E);
+    return fx_to_double(((long long)l2 * (1LL << 51) + (m >> 1)) | (m & 1LL), E + 1);
 }
 
 // The FP64 sum of the parts that hold an Inf or NaN term.
@@ -1103,12 +1115,13 @@ __device__ __forceinline__ void lvl_load_chunks(const RowStep &st, const int32_t
 __device__ __forceinline__ double step_coef(const FxPart &part, FxPart *parts, double *coef, int G, int wg,
                                             int lane, int bar, double w) {
     if (G > 1) {
-        // by one warp of the group for all: the G parts one per lane, aligned and added by warp reductions. All 16 warps of a block
-        // at it (the conversion and the product are 64 cycles each of a
-        // sub-partition's FP64 pipe, and about 200 integer instructions where
-        // they are done without it) took 730 of a level's 5650 cycles at fan N=128
-        // and 1410 of 8800 at N=512 (sweeps 3.22 and 13.2 ms; one warp: 2.72 and
-        // 12.6 ms); groups take warps of different sub-partitions.
+        // by one warp of the group for all: the G parts one per lane, aligned and
+        // added by warp reductions. All 16 warps of a block at it (the conversion
+        // and the product are 64 cycles each of a sub-partition's FP64 pipe, and
+        // about 200 integer instructions where they are done without it) took 730
+        // of a level's 5650 cycles at fan N=128 and 1410 of 8800 at N=512 (sweeps
+        // 3.22 and 13.2 ms; one warp: 2.72 and 12.6 ms); groups take warps of
+        // different sub-partitions.
         if (lane == 0) parts[wg] = part;
         asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * G) : "memory");
         if (wg == (bar & (G - 1))) {
@@ -1119,7 +1132,7 @@ __device__ __forceinline__ double step_coef(const FxPart &part, FxPart *parts, d
                 r = fx_special(parts, G);
             } else {
                 const int sh = E - e;
-                r = fx_to_double_fast(fx_warp_sum(lane < G && sh < 64 ? parts[lane].s >> sh : 0ll), E);
+                r = fx_group(lane < G && sh < 64 ? parts[lane].s >> sh : 0ll, E);
             }
             if (lane == 0) *coef = __dmul_rn(-r, w);
         }
