@@ -1248,6 +1248,7 @@ static int device_sirt(fair_csr h, const double *d_b, double *d_x, SirtDev &S) {
     S.lb = h->sirt_lb;
     S.ub = h->sirt_ub;
     S.sched = h->w_sched.as<unsigned>();
+    S.shared = true;
     return sirt_prepare_shadow(S, h->stream);
 }
 

@@ -253,6 +253,7 @@ struct SirtDev {
     double lb = 0.0, ub = 0.0;
     unsigned *sched = nullptr;   // chunk-scheduling counters (rows.cuh)
     bool chained = false;        // the pass follows another one on the stream
+    bool shared = false;         // the call returns at once: other streams may have passes of their own
 };
 // The SIRT weights stored as reciprocals 1/M, 1/D: what the epilogues
 // (sirt_epi.cuh) multiply by.

@@ -79,7 +79,17 @@ struct EpiStoreSq {  // y = Ax, partial sum of y^2
 // Fan N = 128 / parallel N = 256 / N = 363 iterations in us, FP64: 3 blocks 42 /
 // 159 / 295, 4 blocks 42 / 164 / 305, 2 blocks 41 / 181 / 344; N = 363 FP32: 5
 // blocks 177, 6 blocks 183, 4 blocks 184.
-constexpr int kOcc64 = 3, kOccLP = 5;
+// The kernels of 16-bit integers, whose conversions lengthen a step, gain from more
+// warps (us per pass of 20 iterations, three streams in turn / one; N = 226, 363,
+// 471: 5 blocks 471 / 821, 3113 / 3675, 3425 / 4075; 6 blocks 464 / 756, 3103 /
+// 3619, 3300 / 3865; 7 with two rounds per chunk, launch_rows, 2754 / 3687, 3006 /
+// 4042 at N = 363 and 471).
+constexpr int kOcc64 = 3, kOccLP = 5, kOccQ = 6, kOccQ2 = 7;
+// whether a form's two-round kernel is one of its own
+template <typename VT, int NG> constexpr bool kTwo = NG == 1 && std::is_integral<VT>::value;
+template <typename VT, bool TWO> constexpr int pk_occ(int ng) {
+    return ng != 1 ? 4 : !std::is_integral<VT>::value ? kOccLP : TWO ? kOccQ2 : kOccQ;
+}
 
 // ---- kernels --------------------------------------------------------------------
 template <int G>
@@ -103,26 +113,26 @@ struct PkArgs {
     const int4 *gside;
     int S, L;
 };
-template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_resid_pk(PkArgs P, int32_t m, const VT *v,
+template <typename VT, int G, int NG, bool TWO>
+__global__ void __launch_bounds__(256, (pk_occ<VT, TWO>(NG))) k_sirt_resid_pk(PkArgs P, int32_t m, const VT *v,
                                                        const float *x, EpiResidLP epi,
                                                        unsigned *sched, int subs) {
     chunk_rows_pk<VT, float, float, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, x, epi, sched, subs);
 }
-template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_update_pk(PkArgs P, int32_t m, const VT *v,
+template <typename VT, int G, int NG, bool TWO>
+__global__ void __launch_bounds__(256, (pk_occ<VT, TWO>(NG))) k_sirt_update_pk(PkArgs P, int32_t m, const VT *v,
                                                         const float *r, EpiUpdateLP epi,
                                                         unsigned *sched, int subs) {
     chunk_rows_pk<VT, float, float, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, r, epi, sched, subs);
 }
-template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_resid_pkf(PkArgs P, int32_t m, const uint4 *rec,
+template <typename VT, int G, int NG, bool TWO>
+__global__ void __launch_bounds__(256, (pk_occ<VT, TWO>(NG))) k_sirt_resid_pkf(PkArgs P, int32_t m, const uint4 *rec,
                                                         const float *x, EpiResidLP epi,
                                                         unsigned *sched, int subs) {
     chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, x, epi, sched, subs);
 }
-template <typename VT, int G, int NG>
-__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_update_pkf(PkArgs P, int32_t m, const uint4 *rec,
+template <typename VT, int G, int NG, bool TWO>
+__global__ void __launch_bounds__(256, (pk_occ<VT, TWO>(NG))) k_sirt_update_pkf(PkArgs P, int32_t m, const uint4 *rec,
                                                          const float *r, EpiUpdateLP epi,
                                                          unsigned *sched, int subs) {
     chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, r, epi, sched, subs);
@@ -338,21 +348,23 @@ int sirt_prepare_shadow(const SirtDev &S, cudaStream_t s) {
 // rows): chunks of 32 rows left one per warp on images up to N = 400, and a pass
 // took as long as 8 rounds in series (N = 363, FP32, us per iteration: 274
 // against 177; N = 1024: 2783 against 2606). FAIR_ROWS_BY_GROUP=0: 32 rows, the
-// same results.
+// same results. On calls that return at once (S.shared) the reduced forms take two
+// rounds where that leaves every warp at least two chunks (kernel K2): a claim
+// and an epilogue of 4 rows cost 5% of the GPU's time once other streams' passes fill
+// the tails (three streams in turn, N = 363 and 471, FP32, us per pass of 20
+// iterations: one round 3156 and 3396, two 2967 and 3159; alone 3592 and 3973,
+// 3741 and 3978; fan N = 289, below the line: 1399 and 1286, alone 1871 and 2018).
 // S.chained: the launch follows another pass of the same call, so it may start
 // (and read its matrix entries) while that one still runs (7 us of the 47 an
 // iteration took at fan N = 128).
 template <auto K, class... A>
-static void launch_rows(const SirtDev &S, int64_t m, int G, cudaStream_t s, A... args) {
+static void launch_cut(const SirtDev &S, int64_t m, int R, int subs, cudaStream_t s, A... args) {
     static const int occ = [] {
         int o = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, K, 256, 0);
         return std::max(o, 1);
     }();
     const int64_t blocks = (int64_t)sm_count() * occ;
-    const int R = 32 / G;
-    const char *bg = getenv("FAIR_ROWS_BY_GROUP");
-    const int subs = bg && bg[0] == '0' ? G : 1;
     const int64_t chunks = (m + subs * R - 1) / (subs * R);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((chunks + 7) / 8, blocks)));
@@ -364,6 +376,15 @@ static void launch_rows(const SirtDev &S, int64_t m, int G, cudaStream_t s, A...
     cfg.attrs = at;
     cfg.numAttrs = S.chained ? 1 : 0;
     cudaLaunchKernelEx(&cfg, K, args..., S.sched, subs);  // errors: the caller's cudaGetLastError
+}
+template <auto K, auto K2 = K, class... A>
+static void launch_rows(const SirtDev &S, int64_t m, int G, cudaStream_t s, A... args) {
+    const int R = 32 / G;
+    const char *bg = getenv("FAIR_ROWS_BY_GROUP");
+    if (bg && bg[0] == '0') return launch_cut<K>(S, m, R, G, s, args...);
+    if (S.shared && S.prec != FAIR_PREC_F64 && m >= (int64_t)2 * sm_count() * kOccLP * 8 * 2 * R)
+        return launch_cut<K2>(S, m, R, 2, s, args...);
+    launch_cut<K>(S, m, R, 1, s, args...);
 }
 
 // All iterations of a small FP64 problem in one cooperative launch: every warp
@@ -577,14 +598,14 @@ static void lp_pass(const SirtDev &S, const DevCSR &M, int pass, const VT *vals,
         switch (code) {
             case 4:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 2>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 2, false>, k_sirt_resid_pkf<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
                 break;
             case 3:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 1>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 1, false>, k_sirt_resid_pkf<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
                 break;
-            case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 2>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
-            case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 1>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
+            case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 2, false>, k_sirt_resid_pk<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
+            case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 1, false>, k_sirt_resid_pk<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
             default: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_lp<VT, g_>>(S, M.m, g_, s, M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(), vals, S.x32, e))) break;
         }
     } else {
@@ -593,14 +614,14 @@ static void lp_pass(const SirtDev &S, const DevCSR &M, int pass, const VT *vals,
         switch (code) {
             case 4:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 2>>(S, M.m, g_, s, P, M.m, fused, r, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 2, false>, k_sirt_update_pkf<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, fused, r, e)))
                 break;
             case 3:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 1>>(S, M.m, g_, s, P, M.m, fused, r, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 1, false>, k_sirt_update_pkf<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, fused, r, e)))
                 break;
-            case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 2>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
-            case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 1>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
+            case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 2, false>, k_sirt_update_pk<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
+            case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 1, false>, k_sirt_update_pk<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
             default: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_lp<VT, g_>>(S, M.m, g_, s, M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(), vals, r, e))) break;
         }
     }
