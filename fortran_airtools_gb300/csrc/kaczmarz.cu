@@ -1890,7 +1890,9 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
         auto fits = [&](int wr) {
             return wr * row_max < (1 << kStampPosBits) && wr * row_max + wr * wr + 24 * wr + 1024 <= optin;
         };
-        const int wr = fits(128) ? 128 : fits(64) ? 64 : 32;
+        // (for the check alone the narrowest, the most windows at once: 2 sweeps in random
+        // order, fan N=73, 84 angles, 15.42 ms in windows of 128, 15.09 in windows of 32)
+        const int wr = want && fits(128) ? 128 : want && fits(64) ? 64 : 32;
         if (!fits(wr)) return FAIR_OK;
         if (W.lens.grow(4 * ((size_t)nord + 1)) || W.eoff.grow(8 * ((size_t)nord + 1)) ||
             W.rec.grow(sizeof(WinRow) * (size_t)nord) || W.lvl.grow(4 * (size_t)nord) ||
