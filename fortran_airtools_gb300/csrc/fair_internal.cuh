@@ -262,7 +262,8 @@ int sirt_weights_recip(const DevCSR &A, const DevCSR &AT, bool sart, double *d_M
 // v = 1/v elementwise (IEEE: 1/0 = Inf, 1/Inf = 0).
 int vec_reciprocal(double *v, int64_t n, cudaStream_t s);
 int sirt_iterations(const SirtDev &S, int K, cudaStream_t s);
-// Raises a kernel's dynamic shared-memory limit to `bytes` if it is lower (tiled.cu).
+// Raises a kernel's dynamic shared-memory limit on the current device to `bytes`
+// if it is lower (tiled.cu).
 cudaError_t smem_allow(const void *kernel, size_t bytes);
 // The K iterations of a small FP64 problem in one launch (*ran: launched).
 int sirt_resident(const SirtDev &S, int K, unsigned *gbar, cudaStream_t s, bool *ran);

@@ -38,6 +38,7 @@
 #include "fair_internal.cuh"
 #include "rows.cuh"
 #include "sirt_epi.cuh"
+#include "smem_limits.h"
 
 namespace fair {
 
@@ -1748,23 +1749,18 @@ int tl_batch_launch(const TlBatch &T, int prec, int pass, double omg, double lb,
     }
 }
 
-// Raise a kernel's dynamic shared-memory limit to `bytes` if it is lower
-// (never lowers it: the tiled copies of A and A' launch the same kernels with
-// tiles of different sizes, and host threads sweep images of different sizes at once).
+// Raise a kernel's dynamic shared-memory limit on the current device to `bytes`
+// if it is lower (never lowers it: the tiled copies of A and A' launch the same
+// kernels with tiles of different sizes, and host threads sweep images of
+// different sizes at once).
 cudaError_t smem_allow(const void *kernel, size_t bytes) {
-    static std::mutex mu;
-    static std::vector<std::pair<const void *, size_t>> set;
-    std::lock_guard<std::mutex> lock(mu);
-    for (auto &k : set)
-        if (k.first == kernel) {
-            if (bytes <= k.second) return cudaSuccess;
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e == cudaSuccess) k.second = bytes;
-            return e;
-        }
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) set.emplace_back(kernel, bytes);
-    return e;
+    static SmemLimits limits;
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)limits.allow(device, kernel, bytes, [&] {
+        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
 }
 
 }  // namespace fair
