@@ -24,6 +24,7 @@
 // 134 + 19 us (the row engine: 280 us); 101 x 101 fan, 180 angles, 3
 // right-hand sides, FP64: 30 + 7 us (82 / 62).
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -165,14 +166,30 @@ __device__ __forceinline__ T boxT(T t, int bmode, T lb, T ub) {
     return t;
 }
 
-// The weights arrive as reciprocals (1/0 = Inf): an FP64 division is a
-// sequence of FP64-pipe instructions, 64 cycles each per warp.
+// Row (M) or column (D) weights that divide. An FP64 division is a sequence of
+// 64-cycle instructions (N = 101 fan, 180 angles, 3 right-hand sides, 9 steps:
+// 2.37 ms), so the product with the weight's reciprocal, formed in FP64 (1/0 = Inf),
+// is taken (2.25 ms; the error against 64-bit sums is the same 1.2e-14 and, in
+// FP32, 1.3e-7), and the division where that reciprocal overflows or is subnormal:
+// inv holds 0 there.
+template <typename T> struct Weights {
+    const T *w, *inv;
+    __device__ __forceinline__ T of(int64_t i, T v, bool zero_if_empty = false) const {
+        const T y = inv[i];
+        unsigned hi;
+        if constexpr (sizeof(T) == 8) hi = (unsigned)__double2hiint(y);
+        else hi = __float_as_uint(y);
+        if (zero_if_empty && hi == (sizeof(T) == 8 ? 0x7FF00000u : 0x7F800000u)) return (T)0;
+        return hi != 0u ? v * y : v / w[i];
+    }
+};
 // forward pass 1: r = (b - A x) / M
 template <typename T, int NR>
 struct EpiFwdResid {
-    const T *b, *Mi;
+    const T *b;
+    Weights<T> M;
     T *r;
-    __device__ void one(int64_t i, int c, T v) const { r[i * NR + c] = (b[i * NR + c] - v) * Mi[i]; }
+    __device__ void one(int64_t i, int c, T v) const { r[i * NR + c] = M.of(i, b[i * NR + c] - v); }
     __device__ void operator()(int64_t i, const T (&acc)[NR]) const {
 #pragma unroll
         for (int c = 0; c < NR; ++c) one(i, c, acc[c]);
@@ -181,13 +198,14 @@ struct EpiFwdResid {
 // forward pass 2: g = A' r (kept when recording), x = P(x + lam g / D)
 template <typename T, int NR>
 struct EpiFwdUpdate {
-    const T *Di, *lam;
+    Weights<T> D;
+    const T *lam;
     T *x, *gsave;
     T lb, ub;
     int bmode;
     __device__ void one(int64_t j, int c, T v) const {
         T u = lam[c] * v;
-        if (Di) u = u * Di[j];
+        if (D.w) u = D.of(j, u);
         if (gsave) gsave[j * NR + c] = v;
         x[j * NR + c] = boxT<T>(x[j * NR + c] + u, bmode, lb, ub);
     }
@@ -199,11 +217,11 @@ struct EpiFwdUpdate {
 // reverse, over A: w = (A t) / M (0 on empty rows), gb += lam w
 template <typename T, int NR>
 struct EpiAdjA {
-    const T *Mi, *lam;
+    Weights<T> M;
+    const T *lam;
     T *w, *gb;
     __device__ void one(int64_t i, int c, T v) const {
-        const T mi = Mi[i];
-        T wi = isinf(mi) ? (T)0 : v * mi;
+        const T wi = M.of(i, v, true);
         w[i * NR + c] = wi;
         gb[i * NR + c] += lam[c] * wi;
     }
@@ -270,7 +288,7 @@ __global__ void __launch_bounds__(256) k_multi_rows(int32_t m, const int64_t *__
 // Elementwise reverse step: gz = gx * [P does not clamp z], t = gz / D,
 // per-block partial sums of gz * g / D for every column (FP64).
 template <typename T, int NR>
-__global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T *gk, const T *Di,
+__global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T *gk, Weights<T> D,
                                                   const T *lam, const T *gx, T *gz, T *t, int bmode,
                                                   T lb, T ub, double *partials) {
     __shared__ double sh[NR][8];
@@ -284,8 +302,7 @@ __global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T
         const int c = (int)(e % NR);
         T g = gk[e];
         T u = lam[c] * g;
-        T d = Di ? Di[j] : (T)1;
-        if (Di) u = u * d;
+        if (D.w) u = D.of(j, u);
         T z = x[e] + u;
         bool pass = true;
         T zc = z;
@@ -293,8 +310,8 @@ __global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T
         if (bmode & 2) pass = pass && (zc > lb);
         T gzv = pass ? gx[e] : (T)0;
         gz[e] = gzv;
-        t[e] = Di ? gzv * d : gzv;
-        part += (double)gzv * (double)(Di ? g * d : g);
+        t[e] = D.w ? D.of(j, gzv) : gzv;
+        part += (double)gzv * (double)(D.w ? D.of(j, g) : g);
     }
     // reduce over the threads sharing a column: lanes c, c+NR, ... then warps
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -332,10 +349,13 @@ __global__ void k_deinterleave(const T *src, int64_t rows, int nrhs, int NRt, in
 }
 
 template <typename T>
-__global__ void k_cast(const double *a, int64_t n, T *o) {
+__global__ void k_weights(const double *a, int64_t n, T *w, T *inv) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        o[i] = (T)a[i];
+         i += (int64_t)gridDim.x * blockDim.x) {
+        w[i] = (T)a[i];
+        const T y = (T)(1.0 / a[i]), least = sizeof(T) == 8 ? (T)DBL_MIN : (T)FLT_MIN;
+        inv[i] = w[i] != (T)0 && (isinf(y) || y < least) ? (T)0 : y;
+    }
 }
 
 int egrid(int64_t n) {
@@ -356,14 +376,14 @@ int mgrid(K kernel, int64_t m, int nr) {
 }
 
 // The handle's buffers (w_adj): kept between calls, each grown to what a call needs.
-enum AdjBuf { AB_B, AB_X, AB_R, AB_GSEG, AB_XSEG, AB_CP, AB_GX, AB_GZ, AB_T, AB_W, AB_GB, AB_LAM, AB_MI,
-              AB_DI, AB_PART, AB_STAGE, AB_SUM, AB_COUNT };
+enum AdjBuf { AB_B, AB_X, AB_R, AB_GSEG, AB_XSEG, AB_CP, AB_GX, AB_GZ, AB_T, AB_W, AB_GB, AB_LAM, AB_M,
+              AB_MI, AB_D, AB_DI, AB_PART, AB_STAGE, AB_SUM, AB_COUNT };
 
 template <typename T, int NR>
 int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_b,
               const double *h_x0, const double *h_gx, const double *h_lam, int nrhs, int c0,
-              int ncols, int K, int bmode, double lb, double ub, const double *d_Mi64,
-              const double *d_Di64, double *h_xK, double *h_gb, double *h_gx0, double *h_glam) {
+              int ncols, int K, int bmode, double lb, double ub, const double *d_M64,
+              const double *d_D64, double *h_xK, double *h_gb, double *h_gx0, double *h_glam) {
     DevCSR &A = h->A, &AT = h->AT;
     cudaStream_t s = h->stream;
     unsigned *sched = h->w_sched.as<unsigned>();
@@ -381,15 +401,15 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
     FAIR_TRY(W[AB_XSEG].grow(sizeof(T) * n * NR * (size_t)C));
     FAIR_TRY(W[AB_GSEG].grow(sizeof(T) * n * NR * (size_t)C));
     FAIR_TRY(W[AB_LAM].grow(sizeof(T) * NR));
-    FAIR_TRY(W[AB_MI].grow(sizeof(T) * m));
-    FAIR_TRY(W[AB_DI].grow(sizeof(T) * n));
+    for (int q : {AB_M, AB_MI}) FAIR_TRY(W[q].grow(sizeof(T) * m));
+    for (int q : {AB_D, AB_DI}) FAIR_TRY(W[q].grow(sizeof(T) * n));
     FAIR_TRY(W[AB_SUM].grow(sizeof(double) * (size_t)ge * NR * (size_t)std::max(K, 1)));
     const int64_t segs = std::max<int64_t>(tiled1 ? A.tlm.nseg : 0, tiled2 ? AT.tlm.nseg : 0);
     FAIR_TRY(W[AB_PART].grow(sizeof(T) * NR * (size_t)segs));
     FAIR_TRY(W[AB_STAGE].grow(sizeof(double) * std::max<int64_t>(m, n) * ncols));
     T *b = W[AB_B].as<T>(), *x = W[AB_X].as<T>(), *r = W[AB_R].as<T>(), *gx = W[AB_GX].as<T>(),
       *gz = W[AB_GZ].as<T>(), *t = W[AB_T].as<T>(), *w = W[AB_W].as<T>(), *gb = W[AB_GB].as<T>(),
-      *lam = W[AB_LAM].as<T>(), *Mi = W[AB_MI].as<T>();
+      *lam = W[AB_LAM].as<T>();
     double *stage = W[AB_STAGE].as<double>(), *sums = W[AB_SUM].as<double>();
     const size_t nNR = (size_t)n * NR, vecb = sizeof(T) * nNR;
     // inputs (stage is reused in stream order)
@@ -406,32 +426,35 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
     T lamh[NR];
     for (int c = 0; c < NR; ++c) lamh[c] = (T)(c < ncols ? h_lam[c0 + c] : 0.0);
     FAIR_CUDA(cudaMemcpyAsync(lam, lamh, sizeof(lamh), cudaMemcpyHostToDevice, s));
-    k_cast<T><<<egrid(m), 256, 0, s>>>(d_Mi64, m, Mi);
-    if (sart) k_cast<T><<<egrid(n), 256, 0, s>>>(d_Di64, n, W[AB_DI].as<T>());
+    auto weights = [&](const double *w64, int64_t rows, int w, int wi) {
+        k_weights<T><<<egrid(rows), 256, 0, s>>>(w64, rows, W[w].as<T>(), W[wi].as<T>());
+        return Weights<T>{W[w].as<T>(), W[wi].as<T>()};
+    };
+    const Weights<T> M = weights(d_M64, m, AB_M, AB_MI);
+    const Weights<T> D = sart ? weights(d_D64, n, AB_D, AB_DI) : Weights<T>{nullptr, nullptr};
     FAIR_CUDA(cudaMemsetAsync(gb, 0, sizeof(T) * m * NR, s));
     FAIR_CUDA(cudaGetLastError());
-    const T *Di = sart ? W[AB_DI].as<T>() : nullptr;
     const T tlb = (T)lb, tub = (T)ub;
     // epi(row, M v) over A (pass 1) or A' (pass 2)
     auto product = [&](int pass, const T *v, const auto &epi) -> int {
         using Epi = std::decay_t<decltype(epi)>;
-        DevCSR &M = pass == 1 ? A : AT;
+        DevCSR &Q = pass == 1 ? A : AT;
         if (pass == 1 ? tiled1 : tiled2) {
             T *part = W[AB_PART].as<T>();
-            FAIR_TRY(tl_multi_partials(M, prec, NR, v, part, sched, s));
-            k_multi_rows<T, NR, Epi><<<egrid((int64_t)M.m * NR * 2), 256, 0, s>>>(
-                M.m, M.tlm.segbase.as<int64_t>(), part, epi);
+            FAIR_TRY(tl_multi_partials(Q, prec, NR, v, part, sched, s));
+            k_multi_rows<T, NR, Epi><<<egrid((int64_t)Q.m * NR * 2), 256, 0, s>>>(
+                Q.m, Q.tlm.segbase.as<int64_t>(), part, epi);
         } else {
             auto k = k_multi<T, NR, Epi>;
-            k<<<mgrid(k, M.m, NR), 256, 0, s>>>(M.rowptr.as<int64_t>(), M.m, M.col.as<int32_t>(),
+            k<<<mgrid(k, Q.m, NR), 256, 0, s>>>(Q.rowptr.as<int64_t>(), Q.m, Q.col.as<int32_t>(),
                                                 pass == 1 ? vA : vAT, v, epi, sched);
         }
         FAIR_CUDA(cudaGetLastError());
         return FAIR_OK;
     };
     auto fwd_step = [&](T *gsave) -> int {
-        FAIR_TRY(product(1, x, EpiFwdResid<T, NR>{b, Mi, r}));
-        return product(2, r, EpiFwdUpdate<T, NR>{Di, lam, x, gsave, tlb, tub, bmode});
+        FAIR_TRY(product(1, x, EpiFwdResid<T, NR>{b, M, r}));
+        return product(2, r, EpiFwdUpdate<T, NR>{D, lam, x, gsave, tlb, tub, bmode});
     };
     // forward with checkpoints
     for (int k = 0; k < K; ++k) {
@@ -459,10 +482,10 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
         for (int k = k1 - 1; k >= k0; --k) {
             const T *xk = W[AB_XSEG].as<T>() + nNR * (k - k0);
             const T *gk = W[AB_GSEG].as<T>() + nNR * (k - k0);
-            k_adj_mask<T, NR><<<ge, 256, 0, s>>>(n, xk, gk, Di, lam, gx, gz, t, bmode, tlb, tub,
+            k_adj_mask<T, NR><<<ge, 256, 0, s>>>(n, xk, gk, D, lam, gx, gz, t, bmode, tlb, tub,
                                                  sums + (size_t)k * ge * NR);
             FAIR_CUDA(cudaGetLastError());
-            FAIR_TRY(product(1, t, EpiAdjA<T, NR>{Mi, lam, w, gb}));
+            FAIR_TRY(product(1, t, EpiAdjA<T, NR>{M, lam, w, gb}));
             FAIR_TRY(product(2, w, EpiAdjAT<T, NR>{gz, lam, gx}));
         }
     }
@@ -491,7 +514,7 @@ int sirt_adjoint(fair_csr h, bool sart, int nrhs, const double *b, const double 
     cudaStream_t s = h->stream;
     FAIR_TRY(h->w_M.grow(sizeof(double) * ((size_t)A.m + 1)));
     FAIR_TRY(h->w_D.grow(sizeof(double) * ((size_t)A.n + 1)));
-    FAIR_TRY(sirt_weights_recip(A, AT, sart, h->w_M.as<double>(), h->w_D.as<double>(), s));
+    FAIR_TRY(sirt_weights(A, AT, sart, h->w_M.as<double>(), h->w_D.as<double>(), s));
     const bool f32 = h->prec == FAIR_PREC_F32;
     if (f32) {
         FAIR_TRY(csr_make_lowprec(A, FAIR_PREC_F32, s));
@@ -504,12 +527,12 @@ int sirt_adjoint(fair_csr h, bool sart, int nrhs, const double *b, const double 
         const int nc = std::min(16, nrhs - c0);
         auto group = [&](auto nr) -> int {
             constexpr int NR = decltype(nr)::value;
-            const double *Mi = h->w_M.as<double>(), *Di = h->w_D.as<double>();
+            const double *M = h->w_M.as<double>(), *D = h->w_D.as<double>();
             if (f32)
                 return run_group<float, NR>(h, A.v32.as<float>(), AT.v32.as<float>(), sart, b, x0, gx, lam,
-                                            nrhs, c0, nc, K, bmode, lb, ub, Mi, Di, xK, gb, gx0, glam);
+                                            nrhs, c0, nc, K, bmode, lb, ub, M, D, xK, gb, gx0, glam);
             return run_group<double, NR>(h, A.v64.as<double>(), AT.v64.as<double>(), sart, b, x0, gx, lam,
-                                         nrhs, c0, nc, K, bmode, lb, ub, Mi, Di, xK, gb, gx0, glam);
+                                         nrhs, c0, nc, K, bmode, lb, ub, M, D, xK, gb, gx0, glam);
         };
         int st;
         if (nc == 1) st = group(std::integral_constant<int, 1>());

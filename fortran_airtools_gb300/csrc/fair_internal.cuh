@@ -225,8 +225,9 @@ int sirt_make_forms(DevCSR &A, DevCSR &AT, int prec, cudaStream_t s, bool all = 
                     bool sliced = true);
 int csr_scale(DevCSR &A, double c, cudaStream_t s);
 int csr_row_norms(const DevCSR &A, int p, double *d_out, cudaStream_t s);
-// The same with the SIRT weights formed from them: 1/norm, or 1/(m norm^2).
-enum RowOut { ROW_NORM = 0, ROW_RECIP = 1, ROW_CIMMINO = 2 };
+// The same with the SIRT weights formed from them: 1/norm, 1/(m norm^2) or
+// m norm^2.
+enum RowOut { ROW_NORM = 0, ROW_RECIP = 1, ROW_CIMMINO = 2, ROW_CIMMINO_M = 3 };
 int csr_row_weights(const DevCSR &A, int p, RowOut out, double *d_out, cudaStream_t s);
 int csr_row_dot(const DevCSR &A, int32_t row, const double *d_x, double *d_out, cudaStream_t s);
 int csr_add_mult_row(const DevCSR &A, int32_t row, double c, double *d_w, int bmode,
@@ -255,6 +256,9 @@ struct SirtDev {
     bool chained = false;        // the pass follows another one on the stream
     bool shared = false;         // the call returns at once: other streams may have passes of their own
 };
+// The SIRT weights M and D (sart: row and column sums).
+int sirt_weights(const DevCSR &A, const DevCSR &AT, bool sart, double *d_M, double *d_D,
+                 cudaStream_t s);
 // The SIRT weights stored as reciprocals 1/M, 1/D: what the epilogues
 // (sirt_epi.cuh) multiply by.
 int sirt_weights_recip(const DevCSR &A, const DevCSR &AT, bool sart, double *d_Mi, double *d_Di,

@@ -327,13 +327,22 @@ int vec_reciprocal(double *v, int64_t n, cudaStream_t s) {
     return FAIR_OK;
 }
 
+int sirt_weights(const DevCSR &A, const DevCSR &AT, bool sart, double *d_M, double *d_D,
+                 cudaStream_t s) {
+    if (sart) {  // AIRMs.f90:1076-1079: row 1-norms, column 1-norms (via the transpose)
+        FAIR_TRY(csr_row_weights(A, 1, ROW_NORM, d_M, s));
+        return csr_row_weights(AT, 1, ROW_NORM, d_D, s);
+    }
+    return csr_row_weights(A, 2, ROW_CIMMINO_M, d_M, s);  // :1072: M = m * row_norms(2)**2
+}
+
 int sirt_weights_recip(const DevCSR &A, const DevCSR &AT, bool sart, double *d_Mi, double *d_Di,
                        cudaStream_t s) {
-    if (sart) {  // AIRMs.f90:1076-1079: row 1-norms, column 1-norms (via the transpose)
+    if (sart) {
         FAIR_TRY(csr_row_weights(A, 1, ROW_RECIP, d_Mi, s));
         return csr_row_weights(AT, 1, ROW_RECIP, d_Di, s);
     }
-    return csr_row_weights(A, 2, ROW_CIMMINO, d_Mi, s);  // :1072: M = m * row_norms(2)**2
+    return csr_row_weights(A, 2, ROW_CIMMINO, d_Mi, s);
 }
 
 int sirt_prepare_shadow(const SirtDev &S, cudaStream_t s) {

@@ -343,11 +343,11 @@ __device__ __forceinline__ double norm_term(double acc, double a, int p) {
     }
 }
 
-// What a row's norm becomes in the output (AIRMs.f90:1072 for ROW_CIMMINO).
+// What a row's norm becomes in the output (AIRMs.f90:1072 for ROW_CIMMINO and _M).
 __device__ __forceinline__ double row_out(double norm, int out, double m) {
     if (out == ROW_NORM) return norm;
-    if (out == ROW_CIMMINO) norm = __dmul_rn(m, __dmul_rn(norm, norm));
-    return __ddiv_rn(1.0, norm);
+    if (out != ROW_RECIP) norm = __dmul_rn(m, __dmul_rn(norm, norm));
+    return out == ROW_CIMMINO_M ? norm : __ddiv_rn(1.0, norm);
 }
 
 // A warp takes `subs` rounds of 4 rows, 8 lanes per row with four loads in
