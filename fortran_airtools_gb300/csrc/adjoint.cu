@@ -326,6 +326,24 @@ __global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T
     }
 }
 
+// glam of the steps of a segment: block k adds its step's partials, ge blocks x NR
+// columns, to out[k][NR].
+template <int NR>
+__global__ void __launch_bounds__(256) k_adj_sums(const double *partials, int ge, double *out) {
+    constexpr int L = 256 / NR;  // threads per column
+    __shared__ double sh[256];
+    const int c = threadIdx.x % NR, l = threadIdx.x / NR;
+    const double *p = partials + (size_t)blockIdx.x * ge * NR;
+    double acc = 0.0;
+    for (int b = l; b < ge; b += L) acc += p[(size_t)b * NR + c];
+    sh[threadIdx.x] = acc;
+    for (int o = L / 2; o > 0; o >>= 1) {
+        __syncthreads();
+        if (l < o) sh[threadIdx.x] += sh[threadIdx.x + o * NR];
+    }
+    if (l == 0) out[(size_t)blockIdx.x * NR + c] = sh[c];
+}
+
 // x0 (column-major n x nrhs, or zeros) into the interleaved layout
 template <typename T>
 __global__ void k_interleave(const double *src, int64_t rows, int nrhs, int NRt, int c0, T *dst) {
@@ -377,7 +395,7 @@ int mgrid(K kernel, int64_t m, int nr) {
 
 // The handle's buffers (w_adj): kept between calls, each grown to what a call needs.
 enum AdjBuf { AB_B, AB_X, AB_R, AB_GSEG, AB_XSEG, AB_CP, AB_GX, AB_GZ, AB_T, AB_W, AB_GB, AB_LAM, AB_M,
-              AB_MI, AB_D, AB_DI, AB_PART, AB_STAGE, AB_SUM, AB_COUNT };
+              AB_MI, AB_D, AB_DI, AB_PART, AB_STAGE, AB_SUM, AB_GL, AB_COUNT };
 
 template <typename T, int NR>
 int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_b,
@@ -403,14 +421,15 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
     FAIR_TRY(W[AB_LAM].grow(sizeof(T) * NR));
     for (int q : {AB_M, AB_MI}) FAIR_TRY(W[q].grow(sizeof(T) * m));
     for (int q : {AB_D, AB_DI}) FAIR_TRY(W[q].grow(sizeof(T) * n));
-    FAIR_TRY(W[AB_SUM].grow(sizeof(double) * (size_t)ge * NR * (size_t)std::max(K, 1)));
+    FAIR_TRY(W[AB_SUM].grow(sizeof(double) * (size_t)ge * NR * (size_t)C));
+    FAIR_TRY(W[AB_GL].grow(sizeof(double) * NR * (size_t)std::max(K, 1)));
     const int64_t segs = std::max<int64_t>(tiled1 ? A.tlm.nseg : 0, tiled2 ? AT.tlm.nseg : 0);
     FAIR_TRY(W[AB_PART].grow(sizeof(T) * NR * (size_t)segs));
     FAIR_TRY(W[AB_STAGE].grow(sizeof(double) * std::max<int64_t>(m, n) * ncols));
     T *b = W[AB_B].as<T>(), *x = W[AB_X].as<T>(), *r = W[AB_R].as<T>(), *gx = W[AB_GX].as<T>(),
       *gz = W[AB_GZ].as<T>(), *t = W[AB_T].as<T>(), *w = W[AB_W].as<T>(), *gb = W[AB_GB].as<T>(),
       *lam = W[AB_LAM].as<T>();
-    double *stage = W[AB_STAGE].as<double>(), *sums = W[AB_SUM].as<double>();
+    double *stage = W[AB_STAGE].as<double>(), *sums = W[AB_SUM].as<double>(), *gl = W[AB_GL].as<double>();
     const size_t nNR = (size_t)n * NR, vecb = sizeof(T) * nNR;
     // inputs (stage is reused in stream order)
     auto put = [&](const double *src, int64_t rows, T *dst) -> int {
@@ -470,7 +489,7 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
         return FAIR_OK;
     };
     if (h_xK) FAIR_TRY(get(x, n, h_xK));
-    // reverse, one segment at a time; the sums of glam stay on the device
+    // reverse, one segment at a time; glam of each step stays on the device
     for (int seg = nseg - 1; seg >= 0; --seg) {
         const int k0 = seg * C, k1 = std::min(K, k0 + C);
         FAIR_CUDA(cudaMemcpyAsync(x, W[AB_CP].as<T>() + nNR * seg, vecb, cudaMemcpyDeviceToDevice, s));
@@ -483,24 +502,25 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
             const T *xk = W[AB_XSEG].as<T>() + nNR * (k - k0);
             const T *gk = W[AB_GSEG].as<T>() + nNR * (k - k0);
             k_adj_mask<T, NR><<<ge, 256, 0, s>>>(n, xk, gk, D, lam, gx, gz, t, bmode, tlb, tub,
-                                                 sums + (size_t)k * ge * NR);
+                                                 sums + (size_t)(k - k0) * ge * NR);
             FAIR_CUDA(cudaGetLastError());
             FAIR_TRY(product(1, t, EpiAdjA<T, NR>{M, lam, w, gb}));
             FAIR_TRY(product(2, w, EpiAdjAT<T, NR>{gz, lam, gx}));
         }
+        k_adj_sums<NR><<<k1 - k0, 256, 0, s>>>(sums, ge, gl + (size_t)k0 * NR);
+        FAIR_CUDA(cudaGetLastError());
     }
     // outputs
     FAIR_TRY(get(gb, m, h_gb));
     FAIR_TRY(get(gx, n, h_gx0));
-    std::vector<double> hsum((size_t)ge * NR * K);
+    std::vector<double> hgl((size_t)NR * K);
     if (K > 0) {
-        FAIR_CUDA(cudaMemcpyAsync(hsum.data(), sums, sizeof(double) * hsum.size(), cudaMemcpyDeviceToHost, s));
+        FAIR_CUDA(cudaMemcpyAsync(hgl.data(), gl, sizeof(double) * hgl.size(), cudaMemcpyDeviceToHost, s));
         FAIR_CUDA(cudaStreamSynchronize(s));
     }
     double acc[NR] = {};
     for (int k = K - 1; k >= 0; --k)
-        for (int bl = 0; bl < ge; ++bl)
-            for (int c = 0; c < NR; ++c) acc[c] += hsum[((size_t)k * ge + bl) * NR + c];
+        for (int c = 0; c < NR; ++c) acc[c] += hgl[(size_t)k * NR + c];
     for (int c = 0; c < ncols; ++c) h_glam[c0 + c] = acc[c];
     return FAIR_OK;
 }
