@@ -527,6 +527,13 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
 
 }  // namespace
 
+void adjoint_release(fair_csr h) {
+    cudaStreamSynchronize(h->stream);
+    h->A.tlm.release();
+    h->AT.tlm.release();
+    for (DevBuf &b : h->w_adj) b.release();
+}
+
 int sirt_adjoint(fair_csr h, bool sart, int nrhs, const double *b, const double *x0, int K,
                  const double *lam, int bmode, double lb, double ub, const double *gx,
                  double *xK, double *gb, double *gx0, double *glam) {
@@ -540,9 +547,16 @@ int sirt_adjoint(fair_csr h, bool sart, int nrhs, const double *b, const double 
         FAIR_TRY(csr_make_lowprec(A, FAIR_PREC_F32, s));
         FAIR_TRY(csr_make_lowprec(AT, FAIR_PREC_F32, s));
     }
-    // the tiled copies of the products (left unbuilt for matrices without an image)
-    FAIR_TRY(csr_make_tiled_multi(A, h->prec, 1, s));
-    FAIR_TRY(csr_make_tiled_multi(AT, h->prec, 2, s));
+    // The tiled copies of the products (left unbuilt for matrices without an image)
+    // where there is memory for them; without it the row engine runs, also when
+    // they leave too little for the vectors.
+    const Reclaim own(nullptr);  // what an allocation here may free is this function's to say
+    if (K > 0) {
+        int st = csr_make_tiled_multi(A, h->prec, 1, s);
+        if (st == FAIR_OK) st = csr_make_tiled_multi(AT, h->prec, 2, s);
+        if (st == FAIR_ERR_ALLOC) adjoint_release(h);
+        else if (st != FAIR_OK) return st;
+    }
     for (int c0 = 0; c0 < nrhs; c0 += 16) {
         const int nc = std::min(16, nrhs - c0);
         auto group = [&](auto nr) -> int {
@@ -554,11 +568,17 @@ int sirt_adjoint(fair_csr h, bool sart, int nrhs, const double *b, const double 
             return run_group<double, NR>(h, A.v64.as<double>(), AT.v64.as<double>(), sart, b, x0, gx, lam,
                                          nrhs, c0, nc, K, bmode, lb, ub, M, D, xK, gb, gx0, glam);
         };
-        int st;
-        if (nc == 1) st = group(std::integral_constant<int, 1>());
-        else if (nc <= 4) st = group(std::integral_constant<int, 4>());
-        else if (nc <= 8) st = group(std::integral_constant<int, 8>());
-        else st = group(std::integral_constant<int, 16>());
+        auto run = [&]() -> int {
+            if (nc == 1) return group(std::integral_constant<int, 1>());
+            if (nc <= 4) return group(std::integral_constant<int, 4>());
+            if (nc <= 8) return group(std::integral_constant<int, 8>());
+            return group(std::integral_constant<int, 16>());
+        };
+        int st = run();
+        if (st == FAIR_ERR_ALLOC) {  // all of a group's allocations come before its work
+            adjoint_release(h);
+            st = run();
+        }
         if (st) return st;
     }
     return FAIR_OK;

@@ -393,6 +393,7 @@ int enqueue_iterations(fair_batch_s *B, int K, cudaStream_t s) {
 // Keep of a problem's matrices only what the batch's passes read.
 void compact(DevCSR &M, int prec, bool tiled) {
     M.drop_sliced();
+    M.tlm.release();  // the adjoint's, of a matrix moved in
     M.dl[0].release();
     M.dl[1].release();
     M.v32.release(); M.v16.release(); M.vq.release();

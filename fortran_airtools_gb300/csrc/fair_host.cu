@@ -36,11 +36,20 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     return FAIR_ERR_CUDA;
 }
 
+static thread_local fair_csr t_reclaim = nullptr;
+Reclaim::Reclaim(fair_csr h) : before(t_reclaim) { t_reclaim = h; }
+Reclaim::~Reclaim() { t_reclaim = before; }
+
 int DevBuf::grow(size_t need) {
     if (need == 0) need = 1;
     if (p && need <= bytes) return FAIR_OK;
     release();
     cudaError_t e = cudaMalloc(&p, need);
+    if (e == cudaErrorMemoryAllocation && t_reclaim) {
+        cudaGetLastError();
+        adjoint_release(t_reclaim);
+        e = cudaMalloc(&p, need);
+    }
     if (e != cudaSuccess) {
         p = nullptr;
         bytes = 0;
@@ -242,10 +251,9 @@ static OptVals read_opts(const fair_opts *o) {
 using namespace fair;
 
 #define ENTER(h)                                                  \
-    do {                                                          \
-        if (!(h)) { set_detail("null handle"); return FAIR_ERR_NULL; } \
-        FAIR_CUDA(cudaSetDevice((h)->device));                    \
-    } while (0)
+    if (!(h)) { set_detail("null handle"); return FAIR_ERR_NULL; } \
+    FAIR_CUDA(cudaSetDevice((h)->device));                        \
+    const Reclaim reclaim_scope(h)
 
 #define NEED_MATRIX(h)                                                   \
     do {                                                                 \

@@ -43,6 +43,18 @@ struct DevBuf {
     template <typename T> T *as() const { return static_cast<T *>(p); }
 };
 
+// While it lives, an allocation of this thread that finds no memory frees what
+// handle h keeps for later adjoint calls and is tried once more (null: no handle).
+struct Reclaim {
+    explicit Reclaim(fair_csr h);
+    Reclaim(const Reclaim &) = delete;
+    Reclaim &operator=(const Reclaim &) = delete;
+    ~Reclaim();
+
+  private:
+    fair_csr before;
+};
+
 // A scratch allocation released when it goes out of scope.
 struct TmpBuf : DevBuf {
     TmpBuf() = default;
@@ -359,6 +371,8 @@ int normest_run(const DevCSR &A, const DevCSR &AT, double *d_v, double *d_vn, do
 int fill_uniform(double *d_v, int64_t n, uint64_t seed, uint64_t ctr, cudaStream_t s);
 
 // Adjoint of unrolled SIRT (adjoint.cu); the handle must hold A and A'.
+// Frees the adjoint's tiled copies and vectors (built anew by the next call).
+void adjoint_release(fair_csr h);
 int sirt_adjoint(fair_csr h, bool sart, int nrhs, const double *b, const double *x0, int K,
                  const double *lam, int bmode, double lb, double ub, const double *gx,
                  double *xK, double *gb, double *gx0, double *glam);
