@@ -395,7 +395,7 @@ int mgrid(K kernel, int64_t m, int nr) {
 
 // The handle's buffers (w_adj): kept between calls, each grown to what a call needs.
 enum AdjBuf { AB_B, AB_X, AB_R, AB_GSEG, AB_XSEG, AB_CP, AB_GX, AB_GZ, AB_T, AB_W, AB_GB, AB_LAM, AB_M,
-              AB_MI, AB_D, AB_DI, AB_PART, AB_STAGE, AB_SUM, AB_GL, AB_COUNT };
+              AB_D, AB_PART, AB_STAGE, AB_SUM, AB_COUNT };
 
 template <typename T, int NR>
 int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_b,
@@ -419,17 +419,18 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
     FAIR_TRY(W[AB_XSEG].grow(sizeof(T) * n * NR * (size_t)C));
     FAIR_TRY(W[AB_GSEG].grow(sizeof(T) * n * NR * (size_t)C));
     FAIR_TRY(W[AB_LAM].grow(sizeof(T) * NR));
-    for (int q : {AB_M, AB_MI}) FAIR_TRY(W[q].grow(sizeof(T) * m));
-    for (int q : {AB_D, AB_DI}) FAIR_TRY(W[q].grow(sizeof(T) * n));
-    FAIR_TRY(W[AB_SUM].grow(sizeof(double) * (size_t)ge * NR * (size_t)C));
-    FAIR_TRY(W[AB_GL].grow(sizeof(double) * NR * (size_t)std::max(K, 1)));
+    FAIR_TRY(W[AB_M].grow(sizeof(T) * m * 2));  // weights, then their reciprocals
+    FAIR_TRY(W[AB_D].grow(sizeof(T) * n * 2));
+    // a segment's partial sums of glam, then glam of every step
+    const size_t seg_sums = (size_t)ge * NR * (size_t)C;
+    FAIR_TRY(W[AB_SUM].grow(sizeof(double) * (seg_sums + (size_t)NR * (size_t)std::max(K, 1))));
     const int64_t segs = std::max<int64_t>(tiled1 ? A.tlm.nseg : 0, tiled2 ? AT.tlm.nseg : 0);
     FAIR_TRY(W[AB_PART].grow(sizeof(T) * NR * (size_t)segs));
     FAIR_TRY(W[AB_STAGE].grow(sizeof(double) * std::max<int64_t>(m, n) * ncols));
     T *b = W[AB_B].as<T>(), *x = W[AB_X].as<T>(), *r = W[AB_R].as<T>(), *gx = W[AB_GX].as<T>(),
       *gz = W[AB_GZ].as<T>(), *t = W[AB_T].as<T>(), *w = W[AB_W].as<T>(), *gb = W[AB_GB].as<T>(),
       *lam = W[AB_LAM].as<T>();
-    double *stage = W[AB_STAGE].as<double>(), *sums = W[AB_SUM].as<double>(), *gl = W[AB_GL].as<double>();
+    double *stage = W[AB_STAGE].as<double>(), *sums = W[AB_SUM].as<double>(), *gl = sums + seg_sums;
     const size_t nNR = (size_t)n * NR, vecb = sizeof(T) * nNR;
     // inputs (stage is reused in stream order)
     auto put = [&](const double *src, int64_t rows, T *dst) -> int {
@@ -445,12 +446,12 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
     T lamh[NR];
     for (int c = 0; c < NR; ++c) lamh[c] = (T)(c < ncols ? h_lam[c0 + c] : 0.0);
     FAIR_CUDA(cudaMemcpyAsync(lam, lamh, sizeof(lamh), cudaMemcpyHostToDevice, s));
-    auto weights = [&](const double *w64, int64_t rows, int w, int wi) {
-        k_weights<T><<<egrid(rows), 256, 0, s>>>(w64, rows, W[w].as<T>(), W[wi].as<T>());
-        return Weights<T>{W[w].as<T>(), W[wi].as<T>()};
+    auto weights = [&](const double *w64, int64_t rows, T *w) {
+        k_weights<T><<<egrid(rows), 256, 0, s>>>(w64, rows, w, w + rows);
+        return Weights<T>{w, w + rows};
     };
-    const Weights<T> M = weights(d_M64, m, AB_M, AB_MI);
-    const Weights<T> D = sart ? weights(d_D64, n, AB_D, AB_DI) : Weights<T>{nullptr, nullptr};
+    const Weights<T> M = weights(d_M64, m, W[AB_M].as<T>());
+    const Weights<T> D = sart ? weights(d_D64, n, W[AB_D].as<T>()) : Weights<T>{nullptr, nullptr};
     FAIR_CUDA(cudaMemsetAsync(gb, 0, sizeof(T) * m * NR, s));
     FAIR_CUDA(cudaGetLastError());
     const T tlb = (T)lb, tub = (T)ub;

@@ -490,7 +490,7 @@ struct fair_csr_s {
     // work buffers reused across calls
     fair::DevBuf w_in, w_out, w_b, w_x, w_x32, w_r, w_M, w_D, w_xn, w_tmp, w_part, w_flag;
     fair::DevBuf w_ord, w_cumul, w_nrA, w_y;
-    fair::DevBuf w_adj[20];  // the adjoint's vectors, kept between calls
+    fair::DevBuf w_adj[18];  // the adjoint's vectors, kept between calls
     fair::DevBuf w_sched;  // two zeroed counters for dynamic chunk scheduling; a grid barrier's counter and error
     fair::SweepWork w_sweep;  // Kaczmarz sweep buffers (released after each call)
     // state of fair_sirt_prepare (device-resident SIRT)
