@@ -1,5 +1,7 @@
-// grid_barrier.cuh -- a barrier of all blocks of a cooperative launch.
+// grid_barrier.cuh -- cooperative launches and a barrier of all their blocks.
 #pragma once
+
+#include <cuda_runtime.h>
 
 namespace fair {
 
@@ -36,6 +38,24 @@ __device__ __forceinline__ bool grid_barrier(unsigned *gbar, int *gerr, unsigned
     }
     __syncthreads();
     return ok_s != 0;
+}
+
+// Launches `kern` cooperatively; false, and nothing launched, where that is refused
+// (its blocks cannot all be resident at once).
+template <class K, class... A>
+bool launch_cooperative(int blocks, int threads, cudaStream_t s, K kern, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
 }
 
 }  // namespace fair

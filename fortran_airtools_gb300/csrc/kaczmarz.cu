@@ -1565,23 +1565,16 @@ int lvl_launch_cluster(int cs, size_t smem, const RowStep *sched, const int64_t 
 // picks x's place (0: global, 1: shared/distributed).
 // The level sweep on a cooperative grid of nb blocks (x in global memory, the
 // software grid barrier between levels); gsync: {barrier counter, unused, error}.
+// *ran = false where the cooperative launch is refused.
 template <int CACHE, int NT>
 int lvl_launch_grid(int nb, const RowStep *sched, const int64_t *lptr, const int *nlev,
                     const int32_t *col, const double *val, double *x, int32_t n, const Box &box,
-                    int G, const int *err, int *gsync, cudaStream_t s) {
+                    int G, const int *err, int *gsync, cudaStream_t s, bool *ran) {
     auto kern = k_lvl_sweep<SYNC_GRID, XG, CACHE, NT>;
     FAIR_CUDA(cudaMemsetAsync(gsync, 0, 4 * sizeof(int), s));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(nb);
-    cfg.blockDim = dim3(NT);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    FAIR_CUDA(cudaLaunchKernelEx(&cfg, kern, sched, lptr, nlev, col, val, x, n, 0, box, G, err,
-                                 (unsigned *)gsync, gsync + 2));
+    *ran = launch_cooperative(nb, NT, s, kern, sched, lptr, nlev, col, val, x, n, 0, box, G, err,
+                              (unsigned *)gsync, gsync + 2);
+    if (!*ran) return FAIR_OK;
     int gerr = 0;
     FAIR_CUDA(cudaMemcpyAsync(&gerr, gsync + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
     FAIR_CUDA(cudaStreamSynchronize(s));
@@ -1646,9 +1639,11 @@ int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, con
         const int cs = cluster(xmem ? 1 : 0);
         int nb = gmode == 0 ? 0 : lvl_grid_blocks<CACHE, NT>(spl, G, std::max(cs, 1));
         if (gmode == 1 && nb == 0) nb = std::min(2 * std::max(cs, 1), sm_count());
+        bool ran = false;
         if (nb > 0 && S.work)
-            return lvl_launch_grid<CACHE, NT>(nb, sched, lptr, nlev, col, val, S.x, n, box, G, err,
-                                              S.work->gsync.as<int>(), s);
+            FAIR_TRY((lvl_launch_grid<CACHE, NT>(nb, sched, lptr, nlev, col, val, S.x, n, box, G, err,
+                                                 S.work->gsync.as<int>(), s, &ran)));
+        if (ran) return FAIR_OK;
     }
     if (xmem) {
         const int cs = cluster(1);
@@ -1677,25 +1672,18 @@ int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, con
                                              err, s);
 }
 
-// The sweep without barriers on a cooperative grid of nb blocks; gsync: {unused, unused, error}.
+// The sweep without barriers on a cooperative grid of nb blocks (*ran = false, x as
+// it was, where that launch is refused); gsync: {unused, unused, error}.
 template <int CACHE, int NT>
 int flow_launch(int nb, const RowStep *sched, int32_t nord, const int32_t *col, const double *val,
                 const int32_t *tag, XPair *xt, double *x, int32_t n, const Box &box, int G, const int *err,
-                int *gsync, cudaStream_t s) {
+                int *gsync, cudaStream_t s, bool *ran) {
     auto kern = k_flow_sweep<CACHE, NT>;
     FAIR_CUDA(cudaMemsetAsync(gsync, 0, 4 * sizeof(int), s));
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)sm_count() * 8));
     k_flow_pack<<<g, 256, 0, s>>>(x, n, xt);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(nb);
-    cfg.blockDim = dim3(NT);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    FAIR_CUDA(cudaLaunchKernelEx(&cfg, kern, sched, nord, col, val, tag, xt, box, G, err, gsync + 2));
+    *ran = launch_cooperative(nb, NT, s, kern, sched, nord, col, val, tag, xt, box, G, err, gsync + 2);
+    if (!*ran) return FAIR_OK;
     k_flow_unpack<<<g, 256, 0, s>>>(xt, n, x);
     FAIR_CUDA(cudaGetLastError());
     int gerr = 0;
@@ -1759,26 +1747,16 @@ bool lvl_levels_grid(SweepWork &W, int32_t nord, int *nlev, int32_t *otag, cudaS
         cudaGetLastError();
         return false;
     }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(WR);
-    cfg.blockDim = dim3(512);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     if (cudaMemsetAsync(nlev, 0, sizeof(int), s) != cudaSuccess ||
-        cudaMemsetAsync(W.bases.p, 0, 2 * WR * sizeof(unsigned long long), s) != cudaSuccess ||
-        cudaLaunchKernelEx(&cfg, kern, (const WinRow *)W.rec.as<WinRow>(),
-                           (const unsigned char *)W.dpath.as<unsigned char>(),
-                           (const int32_t *)W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(),
-                           W.lvl.as<int32_t>(), otag, W.bases.as<unsigned long long>(),
-                           W.gsync.as<unsigned>(), W.gsync.as<int>() + 2, nlev) != cudaSuccess) {
+        cudaMemsetAsync(W.bases.p, 0, 2 * WR * sizeof(unsigned long long), s) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return true;
+    return launch_cooperative(WR, 512, s, kern, (const WinRow *)W.rec.as<WinRow>(),
+                              (const unsigned char *)W.dpath.as<unsigned char>(),
+                              (const int32_t *)W.idx.as<int32_t>(), nord, W.lvtab.as<int32_t>(),
+                              W.lvl.as<int32_t>(), otag, W.bases.as<unsigned long long>(), W.gsync.as<unsigned>(),
+                              W.gsync.as<int>() + 2, nlev);
 }
 
 // Set-up and levels in windows of WR steps. *built = false (and FAIR_OK) when
@@ -1983,9 +1961,8 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
             const int room = (int)std::ceil(spl * 2.0 * Gf / 16.0);
             const int nb = std::min(nb0 > 0 ? nb0 : std::max(room, 1), occ * sm_count());
             FAIR_TRY((flow_launch<2, 512>(nb, sched, S.nord, col, val, W.tag.as<int32_t>(), W.pairs.as<XPair>(), S.x,
-                                          A.n, box, Gf, err, W.gsync.as<int>(), s)));
-            *done = true;
-            return FAIR_OK;
+                                          A.n, box, Gf, err, W.gsync.as<int>(), s, done)));
+            if (*done) return FAIR_OK;
         }
         cudaGetLastError();
     }

@@ -540,15 +540,6 @@ int sirt_resident(const SirtDev &S, int K, unsigned *gbar, cudaStream_t s, bool 
     const bool many = (groups + 7) / 8 > room;
     if (many && A.nnz > 3100 * 8 * room) return FAIR_OK;
     const int64_t blocks = std::min((groups + 7) / 8, room);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(256);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     const EpiResidF64 e1{S.b, S.Minv, (double *)S.r};
     const EpiUpdateF64 e2{S.D, S.x, S.omg, S.lb, S.ub, S.bmode};
     auto launch = [&](auto kern) -> int {
@@ -558,12 +549,11 @@ int sirt_resident(const SirtDev &S, int K, unsigned *gbar, cudaStream_t s, bool 
             cudaGetLastError();
             return FAIR_OK;
         }
-        FAIR_CUDA(cudaLaunchKernelEx(&cfg, kern, (const int64_t *)A.rowptr.as<int64_t>(), A.m,
-                                     (const int32_t *)A.col.as<int32_t>(), (const double *)A.v64.as<double>(),
-                                     (const int64_t *)T.rowptr.as<int64_t>(), T.m,
-                                     (const int32_t *)T.col.as<int32_t>(), (const double *)T.v64.as<double>(), e1,
-                                     e2, K, gbar, (int *)gbar + 1));
-        *ran = true;
+        *ran = launch_cooperative((int)blocks, 256, s, kern, (const int64_t *)A.rowptr.as<int64_t>(), A.m,
+                                  (const int32_t *)A.col.as<int32_t>(), (const double *)A.v64.as<double>(),
+                                  (const int64_t *)T.rowptr.as<int64_t>(), T.m,
+                                  (const int32_t *)T.col.as<int32_t>(), (const double *)T.v64.as<double>(), e1, e2,
+                                  K, gbar, (int *)gbar + 1);
         return FAIR_OK;
     };
     switch (G) {
