@@ -1111,7 +1111,10 @@ __device__ __forceinline__ void lvl_load_chunks(const RowStep &st, const int32_t
 }
 
 // The coefficient -(a.x - b) (omega / nrA) of a group's step from its warps'
-// parts (of shared memory: parts, G each, and coef).
+// parts (of shared memory: parts, G each, and coef). WIDE: G may be 16 (fx_group's
+// test lies on every level's chain: fan N=128 without barriers, G = 8, 19.91 ms with
+// it and 19.79 without).
+template <bool WIDE>
 __device__ __forceinline__ double step_coef(const FxPart &part, FxPart *parts, double *coef, int G, int wg,
                                             int lane, int bar, double w) {
     if (G > 1) {
@@ -1132,7 +1135,8 @@ __device__ __forceinline__ double step_coef(const FxPart &part, FxPart *parts, d
                 r = fx_special(parts, G);
             } else {
                 const int sh = E - e;
-                r = fx_group(lane < G && sh < 64 ? parts[lane].s >> sh : 0ll, E);
+                const long long F = lane < G && sh < 64 ? parts[lane].s >> sh : 0ll;
+                r = WIDE ? fx_group(F, E) : fx_to_double_fast(fx_warp_sum(F), E);
             }
             if (lane == 0) *coef = __dmul_rn(-r, w);
         }
@@ -1199,7 +1203,7 @@ __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__rest
         }
     }
     const FxPart part = fx_warp_part(p0, p1, (wg == 0 && lane == 0) ? -st.b : 0.0);
-    const double c = step_coef(part, parts, coef, G, wg, lane, bar, st.w);
+    const double c = step_coef<true>(part, parts, coef, G, wg, lane, bar, st.w);
 #pragma unroll
     for (int i = 0; i < CACHE; ++i) {
         if (i >= nmine) break;
@@ -1422,7 +1426,7 @@ __device__ __forceinline__ void flow_wait(const FlowChunks<K> &k, const XPair *x
     }
 }
 
-template <int CACHE, int NT>
+template <int CACHE, int NT, bool WIDE>
 __global__ void __launch_bounds__(NT, 1) k_flow_sweep(
         const RowStep *__restrict__ sched, int32_t nord, const int32_t *__restrict__ col,
         const double *__restrict__ val, const int32_t *__restrict__ tag, XPair *xt, Box box, int G,
@@ -1464,7 +1468,7 @@ __global__ void __launch_bounds__(NT, 1) k_flow_sweep(
             p1 = fma(x2[1], f.v[1], p1);
         }
         const FxPart part = fx_warp_part(p0, p1, (wg == 0 && lane == 0) ? -cur.b : 0.0);
-        const double c = step_coef(part, parts[par] + gl * G, &coef[par][gl], G, wg, lane, bar, cur.w);
+        const double c = step_coef<WIDE>(part, parts[par] + gl * G, &coef[par][gl], G, wg, lane, bar, cur.w);
 #pragma unroll
         for (int i = 0; i < CACHE; ++i) {
             if (wg + G * i >= nq) break;
@@ -1674,11 +1678,11 @@ int lvl_launch(const SweepDev &S, const RowStep *sched, const int64_t *lptr, con
 
 // The sweep without barriers on a cooperative grid of nb blocks (*ran = false, x as
 // it was, where that launch is refused); gsync: {unused, unused, error}.
-template <int CACHE, int NT>
+template <int CACHE, int NT, bool WIDE>
 int flow_launch(int nb, const RowStep *sched, int32_t nord, const int32_t *col, const double *val,
                 const int32_t *tag, XPair *xt, double *x, int32_t n, const Box &box, int G, const int *err,
                 int *gsync, cudaStream_t s, bool *ran) {
-    auto kern = k_flow_sweep<CACHE, NT>;
+    auto kern = k_flow_sweep<CACHE, NT, WIDE>;
     FAIR_CUDA(cudaMemsetAsync(gsync, 0, 4 * sizeof(int), s));
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)sm_count() * 8));
     k_flow_pack<<<g, 256, 0, s>>>(x, n, xt);
@@ -1953,15 +1957,17 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
         // 73 ms, two of its four sweeps with barriers)
         const int Gf = Ge == 1 || Ge == 2 || Ge == 4 || Ge == 8 || Ge == 16 ? Ge : std::min(16, 2 * G);
         int occ = 0;
-        auto kern = k_flow_sweep<2, 512>;
+        const bool wide = Gf == 16;
+        auto kern = wide ? k_flow_sweep<2, 512, true> : k_flow_sweep<2, 512, false>;
         const int nb0 = env_int("FAIR_SWEEP_GRID_BLOCKS", 0);
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 512, 0) == cudaSuccess && occ >= 1) {
             // room for two levels' steps in flight: more groups only poll (10 sweeps of fan
             // N=128, G = 8: 32 blocks 20.3 ms, 64 20.9, 152 22.0)
             const int room = (int)std::ceil(spl * 2.0 * Gf / 16.0);
             const int nb = std::min(nb0 > 0 ? nb0 : std::max(room, 1), occ * sm_count());
-            FAIR_TRY((flow_launch<2, 512>(nb, sched, S.nord, col, val, W.tag.as<int32_t>(), W.pairs.as<XPair>(), S.x,
-                                          A.n, box, Gf, err, W.gsync.as<int>(), s, done)));
+            auto launch = wide ? flow_launch<2, 512, true> : flow_launch<2, 512, false>;
+            FAIR_TRY(launch(nb, sched, S.nord, col, val, W.tag.as<int32_t>(), W.pairs.as<XPair>(), S.x, A.n, box, Gf,
+                            err, W.gsync.as<int>(), s, done));
             if (*done) return FAIR_OK;
         }
         cudaGetLastError();
