@@ -1893,16 +1893,25 @@ int lvl_sweep(const SweepDev &S, int dir, const RowStep *steps, const Box &box, 
         if (W.idx.grow(4 * std::max<size_t>(ent, 1))) return FAIR_OK;
         // the sweep without barriers needs a copy of the entries in step order with
         // their tags; the variables that pick a barrier sweep keep to it
-        const bool flow = want && S.order_key != 0 && env_int("FAIR_SWEEP_FLOW", 1) && !getenv("FAIR_SWEEP_CLUSTER") &&
-                          !getenv("FAIR_SWEEP_GRID") && !getenv("FAIR_SWEEP_XMEM") &&
-                          !W.gval.grow(8 * std::max<size_t>(ent, 1)) && !W.tag.grow(4 * std::max<size_t>(ent, 1)) &&
-                          !W.pairs.grow(sizeof(XPair) * (size_t)std::max<int32_t>(A.n, 1));
+        bool flow = want && S.order_key != 0 && env_int("FAIR_SWEEP_FLOW", 1) && !getenv("FAIR_SWEEP_CLUSTER") &&
+                    !getenv("FAIR_SWEEP_GRID") && !getenv("FAIR_SWEEP_XMEM") &&
+                    !W.gval.grow(8 * std::max<size_t>(ent, 1)) && !W.tag.grow(4 * std::max<size_t>(ent, 1)) &&
+                    !W.pairs.grow(sizeof(XPair) * (size_t)std::max<int32_t>(A.n, 1));
         W.flow_slot = -1;
+        W.lev[1 - slot].key = 0;  // its steps would point into the entries written now
         const size_t smem = (size_t)(wr * row_max);
         bool built = false;
-        if (wr == 128) FAIR_TRY(lvl_build<128>(S, W, C, steps, smem, optin, want, flow, &built, s));
-        else if (wr == 64) FAIR_TRY(lvl_build<64>(S, W, C, steps, smem, optin, want, flow, &built, s));
-        else FAIR_TRY(lvl_build<32>(S, W, C, steps, smem, optin, want, flow, &built, s));
+        for (;;) {
+            if (wr == 128) FAIR_TRY(lvl_build<128>(S, W, C, steps, smem, optin, want, flow, &built, s));
+            else if (wr == 64) FAIR_TRY(lvl_build<64>(S, W, C, steps, smem, optin, want, flow, &built, s));
+            else FAIR_TRY(lvl_build<32>(S, W, C, steps, smem, optin, want, flow, &built, s));
+            if (built || !(W.gval.p || W.tag.p || W.pairs.p)) break;
+            // no room for the level table beside the copies: levels without them
+            flow = false;
+            W.gval.release();
+            W.tag.release();
+            W.pairs.release();
+        }
         if (!built || !want) return FAIR_OK;
         FAIR_CUDA(cudaMemsetAsync(W.cnt.p, 0, 4 * ((size_t)nord + 1), s));
         k_lvl_count<<<g, 256, 0, s>>>(W.lvl.as<int32_t>(), nord, W.cnt.as<int32_t>());

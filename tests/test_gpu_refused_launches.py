@@ -32,3 +32,36 @@ for n, nth, p in ((40, 60, 58), (128, 90, 182)):
     fake.fake_no_cooperative(0)
     A.close()
 """)
+
+
+def test_without_room_for_the_sweeps_copies(tmp_path):
+    """Memory for the level schedule but not for the copies of the entries beside
+    it: the sweep with barriers runs, with its own bits."""
+    fake_cuda.run(tmp_path, """
+n, nth, p = 64, 90, 92
+def handle():
+    A = fair.paralleltomo(fair.Data(n=n, p=p, nth=nth, theta=np.pi * np.arange(nth) / nth + 0.01))
+    fair.airms.sirt("cimmino", A, b, 1)
+    return A
+b = np.random.default_rng(0).random(nth * p)
+run = lambda: fair.airms.art("kaczmarz", A, b, [3], opts=fair.airms.options(relaxpar=0.5))
+os.environ["FAIR_SWEEP_FLOW"] = "0"
+A = handle()
+run()
+fake.fake_peak(1)
+barriers = run()
+need = fake.fake_peak(1)
+os.environ["FAIR_SWEEP_LEGACY"] = "1"
+legacy = run()
+del os.environ["FAIR_SWEEP_LEGACY"], os.environ["FAIR_SWEEP_FLOW"]
+flow = run()
+assert not np.array_equal(flow, barriers) and not np.array_equal(legacy, barriers)  # told apart by their bits
+for room in (need, need + 8 * A.nnz, need + 12 * A.nnz):  # the copies: 12 bytes per entry, 16 per pixel
+    fake.fake_limit(room)
+    before = fake.fake_refused()
+    got = run()
+    assert fake.fake_refused() > before
+    assert np.array_equal(got, barriers), room - need
+fake.fake_limit(0)
+assert np.array_equal(run(), flow)
+""")
