@@ -335,9 +335,13 @@ __device__ __forceinline__ bool take_flag(unsigned *flag) {
 // step) -> 0.59 ms (25 and 3); fan beam N = 512, 720 angles: 0.33 -> 0.21 ms.
 // Eight steps' loads in flight and 7 blocks per SM: 592 us, four 608 (8 blocks)
 // and 643 (9); the checked steps one at a time cost another 110 us.
+// Qa is 2^63 where a ray is that close to an axis without lying on it (|sin| or
+// |cos| rounded to 1, an angle held in FP32 such as pi/2): E + Qa and Cb + E are
+// sums modulo 2^64.
 constexpr int kWalkUnroll = 8;  // interior steps whose loads are in flight together
 struct Walk32 {
-    long long E, Fw, Qa, Cb;  // E (see above); what a step takes off it; Qa; the upper candidate's constant
+    long long E, Fw;          // E (see above); what a step takes off it
+    unsigned long long Qa, Cb;  // Qa; the upper candidate's constant
     int H2s;
     float ramp, aa, ab;       // entry = sat((H2s - u) ramp + a)
     int ua;
@@ -349,12 +353,12 @@ __device__ __forceinline__ float mf_walk32(Walk32 w, bool on, const float *__res
     float s0 = 0.f, s1 = 0.f;
     auto entries = [&](float &wa, float &wb) {
         wa = __saturatef(fmaf((float)(w.H2s - (int)(w.E >> 32)), w.ramp, w.aa));
-        wb = __saturatef(fmaf((float)(int)((w.Cb + w.E) >> 32), w.ramp, w.ab));
+        wb = __saturatef(fmaf((float)(int)((w.Cb + (unsigned long long)w.E) >> 32), w.ramp, w.ab));
     };
     auto advance = [&] {
         w.E -= w.Fw;
         if (w.E < 0) {
-            w.E += w.Qa;
+            w.E = (long long)((unsigned long long)w.E + w.Qa);
             --w.ua;
         }
         qt += dqt;
@@ -393,7 +397,7 @@ __device__ __forceinline__ float mf_walk32(Walk32 w, bool on, const float *__res
         w.E -= w.Fw;
         q += dq;
         if (w.E < 0) {
-            w.E += w.Qa;
+            w.E = (long long)((unsigned long long)w.E + w.Qa);
             q -= 4u * (unsigned)su;
         }
     }
@@ -466,16 +470,16 @@ __global__ void __launch_bounds__(128, 7) k_mf_project32(const MfAngle *__restri
                     w.ab = Qa - w.E < A.H2 || Qa - w.E == tub ? 1.f : 0.f;
                     w.E = 0;
                 } else {
-                    w.Qa = Qa << 17;
+                    w.Qa = (unsigned long long)Qa << 17;
                     w.Fw = Fw << 17;
                     w.E = (w.E << 17) - (sq > 0 ? 1 : 0);
                     if (w.E < 0) {
-                        w.E += w.Qa;
+                        w.E = (long long)((unsigned long long)w.E + w.Qa);
                         --w.ua;
                     }
                     w.H2s = A.H2s;
                     w.ramp = A.ramp;
-                    w.Cb = (((long long)A.H2s << 32) | 0xFFFFFFFFLL) - w.Qa + 1;
+                    w.Cb = (((unsigned long long)(unsigned)A.H2s << 32) | 0xFFFFFFFFull) - w.Qa + 1ull;
                 }
                 // steps with both candidates inside for sure: -(G + k Fw)/Qa in [0.1, N - 2.1]
                 const float Gf = (float)G, qf = (float)Qa, ff = (float)Fw, kmax = (float)steps;
@@ -561,7 +565,7 @@ __global__ void __launch_bounds__(128, kBpOcc) k_mf_backproject32(const MfAngle 
         BpAngle &B = cs[buf][sa];
         if (hl < 4) B.Dw[hl] = Dr + hl * 8 * R.C;
         if (hl == 0) {
-            B.c_lo = (unsigned)(R.C << 18);
+            B.c_lo = (unsigned)R.C << 18;
             B.c_mid = (unsigned)(R.C >> 14);
             B.c_hi = (int)(R.C >> kFix);
             B.H2s = R.H2s;
@@ -616,7 +620,7 @@ __global__ void __launch_bounds__(128, kBpOcc) k_mf_backproject32(const MfAngle 
             const int c_hi = B.c_hi, H2s = B.H2s, Hc = B.Hc;
             const float ramp = B.ramp, a0 = B.a0, a1 = B.a1;
             const long long D = B.Dw[wid] - lane * B.S;
-            unsigned lo = (unsigned)(D << 18), mid = (unsigned)(D >> 14);
+            unsigned lo = (unsigned)D << 18, mid = (unsigned)(D >> 14);
             int hi = (int)(D >> kFix);
             auto pixels = [&](auto guard) {
 #pragma unroll
