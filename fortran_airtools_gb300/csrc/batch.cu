@@ -222,8 +222,10 @@ struct fair_batch_s {
     fair::BOpts opts{1.0, 0.0, 0.0, 0};
     // device tables and work vectors
     DevBuf desc1, desc2, c0_1, c0_2, sched, x32, r, w_b, w_x;
-    const double *bound_b = nullptr;
+    const double *bound_b = nullptr;  // what the descriptors hold (null: nothing yet)
     double *bound_x = nullptr;
+    bool bound_sart = false;
+    bool cut = false;           // tb1, tb2 and the chunk tables are those of the problems
     // captured iterations
     cudaGraphExec_t gexec = nullptr;
     int g_K = -1, g_cfg[4] = {0, 0, 0, 0};
@@ -267,10 +269,13 @@ bool same_opts(const BOpts &a, const BOpts &b) {
            !memcmp(&a.lb, &b.lb, sizeof(double)) && !memcmp(&a.ub, &b.ub, sizeof(double));
 }
 
-// Descriptor tables of the two passes for vectors d_b, d_x.
+// Descriptor tables of the two passes for vectors d_b, d_x, written when these or
+// the method changed; the tables that the problems alone settle, when one was added.
 int bind_vectors(fair_batch_s *B, const double *d_b, double *d_x) {
+    if (B->cut && B->bound_b == d_b && B->bound_x == d_x && B->bound_sart == B->sart) return FAIR_OK;
     const int np = (int)B->probs.size();
     const bool red = B->prec != FAIR_PREC_F64;
+    B->bound_b = nullptr;
     std::vector<BPass> t1(np), t2(np);
     std::vector<int64_t> c1(np + 1, 0), c2(np + 1, 0);
     std::vector<TlBatchProb> l1, l2;
@@ -335,12 +340,18 @@ int bind_vectors(fair_batch_s *B, const double *d_b, double *d_x) {
     FAIR_CUDA(cudaStreamSynchronize(s));
     FAIR_CUDA(cudaMemcpy(B->desc1.p, t1.data(), sizeof(BPass) * np, cudaMemcpyHostToDevice));
     FAIR_CUDA(cudaMemcpy(B->desc2.p, t2.data(), sizeof(BPass) * np, cudaMemcpyHostToDevice));
-    FAIR_CUDA(cudaMemcpy(B->c0_1.p, c1.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice));
-    FAIR_CUDA(cudaMemcpy(B->c0_2.p, c2.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice));
+    if (!B->cut) {
+        FAIR_CUDA(cudaMemcpy(B->c0_1.p, c1.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice));
+        FAIR_CUDA(cudaMemcpy(B->c0_2.p, c2.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice));
+        FAIR_TRY(tl_batch_cut(B->tb1, B->prec, l1));
+        FAIR_TRY(tl_batch_cut(B->tb2, B->prec, l2));
+        B->cut = true;
+    }
     FAIR_TRY(tl_batch_bind(B->tb1, B->prec, l1));
     FAIR_TRY(tl_batch_bind(B->tb2, B->prec, l2));
     B->bound_b = d_b;
     B->bound_x = d_x;
+    B->bound_sart = B->sart;
     return FAIR_OK;
 }
 
@@ -591,7 +602,10 @@ int finish_problem(fair_batch_s *B, BatchProb &q) {
         FAIR_TRY(csr_make_tiled(q.AT, B->prec, 2, s));
         FAIR_CUDA(cudaStreamSynchronize(s));
         q.tiled = tl_batch_ready(q.A, B->prec) && tl_batch_ready(q.AT, B->prec);
-        if (!q.tiled) {
+        if (q.tiled) {  // what the units are cut by
+            FAIR_TRY(tl_host_offsets(q.A, s));
+            FAIR_TRY(tl_host_offsets(q.AT, s));
+        } else {
             q.A.tl.release();
             q.AT.tl.release();
         }
@@ -758,6 +772,8 @@ int fair_batch_add(fair_batch B, fair_csr h, int32_t take) {
     B->col_off.push_back(B->col_off.back() + q->A.n);
     B->nnz += q->A.nnz;
     B->ready = false;
+    B->cut = false;
+    B->bound_b = nullptr;
     fair::drop_graph(B);
     return FAIR_OK;
 }
@@ -837,8 +853,6 @@ int fair_batch_prepare(fair_batch B, const char *sirt_method, const fair_opts *o
     const size_t sx = red ? sizeof(float) : sizeof(double);
     FAIR_TRY(B->r.grow(sx * ((size_t)B->row_off.back() + 1)));
     if (red) FAIR_TRY(B->x32.grow(sizeof(float) * ((size_t)B->col_off.back() + 1)));
-    B->bound_b = nullptr;
-    B->bound_x = nullptr;
     B->ready = true;
     return FAIR_OK;
 }
@@ -861,6 +875,7 @@ int fair_batch_run_device(fair_batch B, const double *d_b, double *d_x, int32_t 
     if (K == 0) return FAIR_OK;
     if (!B->gexec || B->g_K != K || B->g_x != d_x || !fair::same_opts(B->g_opts, B->opts) ||
         memcmp(B->g_cfg, B->cfg, sizeof(B->cfg)) != 0) {
+        if (B->gexec) FAIR_CUDA(cudaStreamSynchronize(B->stream));  // it may be under way
         fair::drop_graph(B);
         FAIR_TRY(fair::batch_pass(B, 1, B->stream, true));  // grids looked up outside the capture
         FAIR_TRY(fair::batch_pass(B, 2, B->stream, true));

@@ -158,7 +158,7 @@ struct DevCSR {
             int32_t n = 0;
         } mv[4];
         std::vector<int32_t> hchunk;  // first chunk of each tile (host)
-        std::vector<int64_t> hsoff;   // soff (host, read by mv_units)
+        std::vector<int64_t> hsoff;   // soff (host: tl_host_offsets)
         bool built() const { return T > 0; }
         void release();
     } tl;
@@ -332,6 +332,11 @@ struct TlBatch {
 bool tl_batch_ready(const DevCSR &M, int prec);
 // Frees the parts of M's tiled copy that only its builders read.
 void tl_drop_build(DevCSR &M);
+// The first slots of M's chunks, kept on the host (read back once).
+int tl_host_offsets(DevCSR &M, cudaStream_t s);
+// The tables that the matrices settle (work units, row offsets), and the
+// descriptors with the vectors: the first to be set whenever the matrices change.
+int tl_batch_cut(TlBatch &T, int prec, const std::vector<TlBatchProb> &probs);
 int tl_batch_bind(TlBatch &T, int prec, const std::vector<TlBatchProb> &probs);
 // dry: only the kernel attributes and grids (outside a graph capture).
 int tl_batch_launch(const TlBatch &T, int prec, int pass, double omg, double lb, double ub, int bmode,

@@ -1418,6 +1418,15 @@ __global__ void __launch_bounds__(kMvThreads, (MvCfg<T, NR>::CTAS)) k_tlm_partia
     }
 }
 
+int host_offsets(DevCSR::Tiled &tl, cudaStream_t s) {
+    if (!tl.hsoff.empty()) return FAIR_OK;
+    tl.hsoff.resize((size_t)tl.nchunks + 1);
+    FAIR_CUDA(cudaMemcpyAsync(tl.hsoff.data(), tl.soff.p, sizeof(int64_t) * (tl.nchunks + 1),
+                              cudaMemcpyDeviceToHost, s));
+    FAIR_CUDA(cudaStreamSynchronize(s));
+    return FAIR_OK;
+}
+
 // The work units of the products with LPE lanes per entry: whole rounds of the
 // CTA's warps (one item each), about 6 units per resident CTA (fewer leaves a
 // tail, more reloads the tile too often: a fill costs about one chunk),
@@ -1425,12 +1434,7 @@ __global__ void __launch_bounds__(kMvThreads, (MvCfg<T, NR>::CTAS)) k_tlm_partia
 int mv_units(DevCSR::Tiled &tl, int lpe, int nctas, cudaStream_t s) {
     DevCSR::Tiled::MvUnits &mu = tl.mv[lpe == 1 ? 0 : lpe == 2 ? 1 : lpe == 4 ? 2 : 3];
     if (mu.n > 0) return FAIR_OK;
-    if (tl.hsoff.empty()) {
-        tl.hsoff.resize((size_t)tl.nchunks + 1);
-        FAIR_CUDA(cudaMemcpyAsync(tl.hsoff.data(), tl.soff.p, sizeof(int64_t) * (tl.nchunks + 1),
-                                  cudaMemcpyDeviceToHost, s));
-        FAIR_CUDA(cudaStreamSynchronize(s));
-    }
+    FAIR_TRY(host_offsets(tl, s));
     const int warps = kMvThreads / 32, round = std::max(1, warps / lpe);  // chunks of a round
     int64_t per = tl.nchunks / ((int64_t)nctas * 6) / round * round;
     per = std::max<int64_t>(round, std::min<int64_t>(per, round * 16));
@@ -1663,18 +1667,14 @@ void tl_drop_build(DevCSR &M) {
     tl.tried6 = true;
 }
 
+int tl_host_offsets(DevCSR &M, cudaStream_t s) { return host_offsets(M.tl, s); }
+
 int tl_batch_bind(TlBatch &T, int prec, const std::vector<TlBatchProb> &probs) {
     const int np = (int)probs.size();
     std::vector<TlbDesc> d(np);
-    std::vector<int64_t> ro(np + 1, 0);
-    int64_t cells = 1, chunks = 0;
     for (int p = 0; p < np; ++p) {
         const DevCSR &M = *probs[p].M;
         const DevCSR::Tiled &tl = M.tl;
-        if (!tl_batch_ready(M, prec)) {
-            set_detail("batched tiled pass: a problem without its tiled copy");
-            return FAIR_ERR_STATE;
-        }
         TlbDesc &e = d[p];
         e.P = TlArgs{tl.soff.as<int64_t>(), tl.pslot.as<int32_t>(), tl.units.as<int4>(), tl.nunits, tl_geo(tl)};
         switch (prec) {
@@ -1693,38 +1693,58 @@ int tl_batch_bind(TlBatch &T, int prec, const std::vector<TlBatchProb> &probs) {
         e.x64 = probs[p].x;
         e.x32 = probs[p].x32;
         e.scale = prec == FAIR_PREC_Q16 ? M.qscale : 1.0;
+    }
+    FAIR_TRY(T.desc.grow(sizeof(TlbDesc) * std::max(np, 1)));
+    // a synchronous copy: the host table goes out of scope on return
+    FAIR_CUDA(cudaMemcpy(T.desc.p, d.data(), sizeof(TlbDesc) * np, cudaMemcpyHostToDevice));
+    return FAIR_OK;
+}
+
+int tl_batch_cut(TlBatch &T, int prec, const std::vector<TlBatchProb> &probs) {
+    const int np = (int)probs.size();
+    std::vector<int64_t> ro(np + 1, 0);
+    int64_t cells = 1, chunks = 0;
+    for (int p = 0; p < np; ++p) {
+        const DevCSR &M = *probs[p].M;
+        if (!tl_batch_ready(M, prec)) {
+            set_detail("batched tiled pass: a problem without its tiled copy");
+            return FAIR_ERR_STATE;
+        }
         ro[p + 1] = ro[p] + M.m;
-        cells = std::max<int64_t>(cells, (int64_t)e.P.G.cells() + 1);
-        chunks += tl.nchunks;
+        cells = std::max<int64_t>(cells, (int64_t)tl_geo(M.tl).cells() + 1);
+        chunks += M.tl.nchunks;
     }
     // The units, cut for the batch: whole rounds of the CTA's warps (one chunk
     // each), about 6 units per resident CTA (3 per SM), longest first. A problem's
     // own units, cut to fill the GPU alone, hold 8 chunks here: half the warps of
     // a CTA waited at its barriers (24 fan-beam problems of N <= 352, FP32: 528 us a pass,
-    // 4.5 TB/s; cut together 394 us, 6.1 TB/s).
+    // 4.5 TB/s; cut together 394 us, 6.1 TB/s). In FP64 units of 8 chunks where whole
+    // rounds would be fewer than two per SM, one SM's pipe doing the work of two (4
+    // fan-beam problems of N = 128, 200 angles, 3761 and 1130 chunks: 5 iterations 537
+    // us in whole rounds, 402 in half ones; 3 parallel ones of N = 186, 2374 and 1991
+    // chunks: 522 and 533; 16-bit and FP32 problems of that size: 0 to 3% slower).
     constexpr int round = kTlThreads / 32;
     int64_t per = chunks / ((int64_t)sm_count() * 3 * 6) / round * round;
     per = std::max<int64_t>(round, std::min<int64_t>(per, kUnitChunks));
-    std::vector<std::pair<int64_t, int4>> ul;  // slots, unit
-    std::vector<int64_t> so;
+    if (prec == FAIR_PREC_F64 && chunks < (int64_t)2 * round * sm_count()) per = round / 2;
+    std::vector<int4> ul;
+    std::vector<uint64_t> order;  // slots (inverted), place in ul
     for (int p = 0; p < np; ++p) {
         const DevCSR::Tiled &tl = probs[p].M->tl;
-        so.resize((size_t)tl.nchunks + 1);
-        FAIR_CUDA(cudaMemcpy(so.data(), tl.soff.p, sizeof(int64_t) * so.size(), cudaMemcpyDeviceToHost));
+        const std::vector<int64_t> &so = tl.hsoff;
         for (size_t t = 0; t + 1 < tl.hchunk.size(); ++t)
             for (int64_t c = tl.hchunk[t]; c < tl.hchunk[t + 1]; c += per) {
                 const int64_t e = std::min<int64_t>(c + per, tl.hchunk[t + 1]);
-                ul.emplace_back(so[e] - so[c], make_int4((int)t, (int)c, (int)e, p));
+                order.push_back((uint64_t)(uint32_t)~(uint32_t)std::min<int64_t>((so[e] - so[c]) >> 5, 0xFFFFFFFFll) << 32 |
+                                (uint32_t)ul.size());
+                ul.push_back(make_int4((int)t, (int)c, (int)e, p));
             }
     }
-    std::stable_sort(ul.begin(), ul.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+    std::sort(order.begin(), order.end());
     std::vector<int4> units(ul.size());
-    for (size_t i = 0; i < ul.size(); ++i) units[i] = ul[i].second;
-    FAIR_TRY(T.desc.grow(sizeof(TlbDesc) * std::max(np, 1)));
+    for (size_t i = 0; i < ul.size(); ++i) units[i] = ul[(uint32_t)order[i]];
     FAIR_TRY(T.ulist.grow(sizeof(int4) * std::max<size_t>(units.size(), 1)));
     FAIR_TRY(T.roff.grow(sizeof(int64_t) * (np + 1)));
-    // synchronous copies: the host tables go out of scope on return
-    FAIR_CUDA(cudaMemcpy(T.desc.p, d.data(), sizeof(TlbDesc) * np, cudaMemcpyHostToDevice));
     FAIR_CUDA(cudaMemcpy(T.ulist.p, units.data(), sizeof(int4) * units.size(), cudaMemcpyHostToDevice));
     FAIR_CUDA(cudaMemcpy(T.roff.p, ro.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice));
     T.np = np;
