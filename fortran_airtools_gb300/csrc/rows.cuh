@@ -210,9 +210,14 @@ template <typename VT, typename XT, typename ACC, int G> struct CsrSteps {
     }
 };
 
+// Whether a lane loads entries two steps ahead: FP64 at 4 entries a step (8 leave no
+// registers for it: N = 471, 223 angles, passes of 226 and 235 us; one ahead 152 and
+// 169).
+template <typename ACC, class ST> constexpr bool kTwoAhead = sizeof(ACC) == 8 && ST::N == 4;
+
 // This lane's part of the sum of a row of len entries from s (gl the lane's
 // place among the row's G), its first steps already loaded (r0; r1 in FP64):
-// its entries in order. FP64 gathers a step's x values while the step before
+// its entries in order. FP64 (kTwoAhead) gathers a step's x values while the step before
 // is added and loads entries two steps ahead (its 12 multiply-adds a step leave
 // time for both, and 24 warps per SM fit); the reduced forms, bound by the
 // gathers' L1 wavefronts, load one step ahead and keep 40 warps.
@@ -222,7 +227,7 @@ __device__ __forceinline__ ACC steps_part(const ST &st, int64_t s, int len, int 
     ACC acc = 0;
     ACC xv[ST::N], vv[ST::N];
     int k = st.first(s, gl);
-    if constexpr (sizeof(ACC) == 8) {
+    if constexpr (kTwoAhead<ACC, ST>) {
         st.gather(r0, k, len, x, xv, vv);
         while (k < len) {
             st.load(r0, s, k + 2 * ST::STEP, len);
@@ -277,7 +282,7 @@ __device__ __forceinline__ ACC steps_chunk_sums(const ST &st, int32_t m, const X
         }
         typename ST::Raw r0 = {}, r1 = {};
         st.load(r0, s, st.first(s, gl), len);
-        if constexpr (sizeof(ACC) == 8) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
+        if constexpr (kTwoAhead<ACC, ST>) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
         const ACC acc = group_sum<ACC, G>(steps_part<XT, ACC>(st, s, len, gl, r0, r1, x));
         const ACC r = __shfl_sync(0xffffffffu, acc, ((lane - sub) & (R - 1)) * G);
         if (lane >= sub && lane < sub + R) mine = r;
@@ -325,7 +330,7 @@ __device__ __forceinline__ void rows_stream(const ST &st, int32_t m, const XT *x
     int len = __shfl_sync(FULL, hl, g);
     typename ST::Raw r0 = {}, r1 = {};
     st.load(r0, s, st.first(s, gl), len);
-    if constexpr (sizeof(ACC) == 8) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
+    if constexpr (kTwoAhead<ACC, ST>) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
     pdl_wait();
     while (ch < nchunks) {
         const int next = sched ? (int)next_chunk(sched, ch, nwarps, lane) + nwarps : ch + nwarps;
@@ -339,7 +344,7 @@ __device__ __forceinline__ void rows_stream(const ST &st, int32_t m, const XT *x
             s = __shfl_sync(FULL, hs, from);
             len = __shfl_sync(FULL, hl, from);
             st.load(r0, s, st.first(s, gl), len);
-            if constexpr (sizeof(ACC) == 8) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
+            if constexpr (kTwoAhead<ACC, ST>) st.load(r1, s, st.first(s, gl) + ST::STEP, len);
             acc = group_sum<ACC, G>(acc);
             const ACC r = __shfl_sync(FULL, acc, ((lane - sub) & (R - 1)) * G);
             if (lane >= sub && lane < sub + R) mine = r;

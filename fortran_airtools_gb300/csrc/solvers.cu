@@ -83,7 +83,8 @@ struct EpiStoreSq {  // y = Ax, partial sum of y^2
 // warps (us per pass of 20 iterations, three streams in turn / one; N = 226, 363,
 // 471: 5 blocks 471 / 821, 3113 / 3675, 3425 / 4075; 6 blocks 464 / 756, 3103 /
 // 3619, 3300 / 3865; 7 with two rounds per chunk, launch_rows, 2754 / 3687, 3006 /
-// 4042 at N = 363 and 471).
+// 4042 at N = 363 and 471). The fused records' kernels keep 5 (q16, N = 471: 101 and 86
+// us a pass, 103 and 111 at 7).
 constexpr int kOcc64 = 3, kOccLP = 5, kOccQ = 6, kOccQ2 = 7;
 // whether a form's two-round kernel is one of its own
 template <typename VT, int NG> constexpr bool kTwo = NG == 1 && std::is_integral<VT>::value;
@@ -125,14 +126,14 @@ __global__ void __launch_bounds__(256, (pk_occ<VT, TWO>(NG))) k_sirt_update_pk(P
                                                         unsigned *sched, int subs) {
     chunk_rows_pk<VT, float, float, G, NG>(P.prow, m, P.gidx, P.gside, P.S, P.L, v, r, epi, sched, subs);
 }
-template <typename VT, int G, int NG, bool TWO>
-__global__ void __launch_bounds__(256, (pk_occ<VT, TWO>(NG))) k_sirt_resid_pkf(PkArgs P, int32_t m, const uint4 *rec,
+template <typename VT, int G, int NG>
+__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_resid_pkf(PkArgs P, int32_t m, const uint4 *rec,
                                                         const float *x, EpiResidLP epi,
                                                         unsigned *sched, int subs) {
     chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, x, epi, sched, subs);
 }
-template <typename VT, int G, int NG, bool TWO>
-__global__ void __launch_bounds__(256, (pk_occ<VT, TWO>(NG))) k_sirt_update_pkf(PkArgs P, int32_t m, const uint4 *rec,
+template <typename VT, int G, int NG>
+__global__ void __launch_bounds__(256, (NG == 1 ? kOccLP : 4)) k_sirt_update_pkf(PkArgs P, int32_t m, const uint4 *rec,
                                                          const float *r, EpiUpdateLP epi,
                                                          unsigned *sched, int subs) {
     chunk_rows_pkf<VT, G, NG>(P.prow, m, rec, P.gside, P.S, P.L, r, epi, sched, subs);
@@ -597,11 +598,11 @@ static void lp_pass(const SirtDev &S, const DevCSR &M, int pass, const VT *vals,
         switch (code) {
             case 4:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 2, false>, k_sirt_resid_pkf<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 2>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
                 break;
             case 3:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 1, false>, k_sirt_resid_pkf<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pkf<VT, g_, 1>>(S, M.m, g_, s, P, M.m, fused, S.x32, e)))
                 break;
             case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 2, false>, k_sirt_resid_pk<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
             case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_resid_pk<VT, g_, 1, false>, k_sirt_resid_pk<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, pvals, S.x32, e))) break;
@@ -613,11 +614,11 @@ static void lp_pass(const SirtDev &S, const DevCSR &M, int pass, const VT *vals,
         switch (code) {
             case 4:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 2, false>, k_sirt_update_pkf<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, fused, r, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 2>>(S, M.m, g_, s, P, M.m, fused, r, e)))
                 break;
             case 3:
                 if constexpr (sizeof(VT) == 2)
-                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 1, false>, k_sirt_update_pkf<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, fused, r, e)))
+                    FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pkf<VT, g_, 1>>(S, M.m, g_, s, P, M.m, fused, r, e)))
                 break;
             case 2: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 2, false>, k_sirt_update_pk<VT, g_, 2, kTwo<VT, 2>>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
             case 1: FAIR_G_DISPATCH(G, (launch_rows<k_sirt_update_pk<VT, g_, 1, false>, k_sirt_update_pk<VT, g_, 1, kTwo<VT, 1>>>(S, M.m, g_, s, P, M.m, pvals, r, e))) break;
