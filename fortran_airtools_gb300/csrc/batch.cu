@@ -222,6 +222,7 @@ struct fair_batch_s {
     fair::BOpts opts{1.0, 0.0, 0.0, 0};
     // device tables and work vectors
     DevBuf desc1, desc2, c0_1, c0_2, sched, x32, r, w_b, w_x;
+    DevBuf tune;                // copies of a problem while layouts are timed (until the batch is prepared)
     const double *bound_b = nullptr;  // what the descriptors hold (null: nothing yet)
     double *bound_x = nullptr;
     bool bound_sart = false;
@@ -263,6 +264,59 @@ void drop_graph(fair_batch_s *B) {
     B->g_K = -1;
 }
 
+// A pass over M's packed stream (the CSR in FP64), its vectors not set.
+BPass packed_pass(const DevCSR &M, int prec) {
+    BPass d{};
+    if (prec != FAIR_PREC_F64) {
+        d.ptr = M.prow.as<int64_t>();
+        d.idx = M.gidx.p;
+        d.gside = M.gside.as<int4>();
+        d.val = prec == FAIR_PREC_F32 ? M.pv32.p : prec == FAIR_PREC_F16 ? M.pv16.p : M.pvq.p;
+        d.S = M.pk_S;
+        d.L = M.pk_L;
+        d.scale = prec == FAIR_PREC_Q16 ? M.qscale : 1.0;
+    } else {
+        d.ptr = M.rowptr.as<int64_t>();
+        d.idx = M.col.p;
+        d.val = M.v64.p;
+        d.S = 0;
+        d.L = 7;
+        d.scale = 1.0;
+    }
+    d.rows = M.m;
+    return d;
+}
+
+void launch_packed(int prec, int pass, int G, int NG, bool dry, const BPass *P, const int64_t *c0, int np,
+                   const BOpts &o, unsigned *sched, cudaStream_t s) {
+    switch (prec) {
+        case FAIR_PREC_F64:
+            if (pass == 1) launch_f64<1>(G, dry, P, c0, np, o, sched, s);
+            else launch_f64<2>(G, dry, P, c0, np, o, sched, s);
+            break;
+        case FAIR_PREC_F32:
+            if (pass == 1) launch_pk<float, 1>(G, NG, dry, P, c0, np, o, sched, s);
+            else launch_pk<float, 2>(G, NG, dry, P, c0, np, o, sched, s);
+            break;
+        case FAIR_PREC_F16:
+            if (pass == 1) launch_pk<__half, 1>(G, NG, dry, P, c0, np, o, sched, s);
+            else launch_pk<__half, 2>(G, NG, dry, P, c0, np, o, sched, s);
+            break;
+        default:
+            if (pass == 1) launch_pk<uint16_t, 1>(G, NG, dry, P, c0, np, o, sched, s);
+            else launch_pk<uint16_t, 2>(G, NG, dry, P, c0, np, o, sched, s);
+            break;
+    }
+}
+
+// What a class must gain to leave the default tiles or the tiled copies: the tiles of
+// all problems share the largest one's shared memory, and a first packed problem adds a
+// launch to every pass. (96 fan-beam problems, FP32 / 16-bit / FP64, ms an iteration:
+// every gain taken 9.53 / 2.00 / 5.60, those of 8% and more 9.40 / 1.98 / 5.52; all
+// on the default tiles 9.22 to 9.39 / 1.93 / 5.33.)
+constexpr float kTuneMargin = 0.92f;
+constexpr size_t kTuneBytes = (size_t)320 << 20;  // of one problem's copies: 2.5 times L2
+
 // Equal options, NaN bounds among them.
 bool same_opts(const BOpts &a, const BOpts &b) {
     return a.bmode == b.bmode && !memcmp(&a.omg, &b.omg, sizeof(double)) &&
@@ -296,24 +350,7 @@ int bind_vectors(fair_batch_s *B, const double *d_b, double *d_x) {
         }
         for (int pass = 1; pass <= 2; ++pass) {
             const DevCSR &M = pass == 1 ? q.A : q.AT;
-            BPass d{};
-            if (red) {
-                d.ptr = M.prow.as<int64_t>();
-                d.idx = M.gidx.p;
-                d.gside = M.gside.as<int4>();
-                d.val = B->prec == FAIR_PREC_F32 ? M.pv32.p : B->prec == FAIR_PREC_F16 ? M.pv16.p : M.pvq.p;
-                d.S = M.pk_S;
-                d.L = M.pk_L;
-                d.scale = B->prec == FAIR_PREC_Q16 ? M.qscale : 1.0;
-            } else {
-                d.ptr = M.rowptr.as<int64_t>();
-                d.idx = M.col.p;
-                d.val = M.v64.p;
-                d.S = 0;
-                d.L = 7;
-                d.scale = 1.0;
-            }
-            d.rows = M.m;
+            BPass d = packed_pass(M, B->prec);
             if (pass == 1) {
                 d.xin = xin;
                 d.b = d_b + ro;
@@ -366,27 +403,7 @@ int batch_pass(fair_batch_s *B, int pass, cudaStream_t s, bool dry = false) {
     if (B->ntiled == np) return FAIR_OK;  // no problem on the packed streams / CSR
     const BPass *P = (pass == 1 ? B->desc1 : B->desc2).as<BPass>();
     const int64_t *c0 = (pass == 1 ? B->c0_1 : B->c0_2).as<int64_t>();
-    unsigned *sched = B->sched.as<unsigned>();
-    const int G = B->cfg[pass - 1], NG = B->cfg[pass + 1];
-    const BOpts &o = B->opts;
-    switch (B->prec) {
-        case FAIR_PREC_F64:
-            if (pass == 1) launch_f64<1>(G, dry, P, c0, np, o, sched, s);
-            else launch_f64<2>(G, dry, P, c0, np, o, sched, s);
-            break;
-        case FAIR_PREC_F32:
-            if (pass == 1) launch_pk<float, 1>(G, NG, dry, P, c0, np, o, sched, s);
-            else launch_pk<float, 2>(G, NG, dry, P, c0, np, o, sched, s);
-            break;
-        case FAIR_PREC_F16:
-            if (pass == 1) launch_pk<__half, 1>(G, NG, dry, P, c0, np, o, sched, s);
-            else launch_pk<__half, 2>(G, NG, dry, P, c0, np, o, sched, s);
-            break;
-        default:
-            if (pass == 1) launch_pk<uint16_t, 1>(G, NG, dry, P, c0, np, o, sched, s);
-            else launch_pk<uint16_t, 2>(G, NG, dry, P, c0, np, o, sched, s);
-            break;
-    }
+    launch_packed(B->prec, pass, B->cfg[pass - 1], B->cfg[pass + 1], dry, P, c0, np, B->opts, B->sched.as<unsigned>(), s);
     return FAIR_OK;
 }
 
@@ -455,10 +472,27 @@ int copy_csr(const DevCSR &src, DevCSR &dst, cudaStream_t s) {
     return FAIR_OK;
 }
 
-// Layout 2: times one problem's passes (alone, on scratch vectors) on the
-// packed streams (the CSR in FP64) and on its tiled copies with each candidate
-// tile shape, and keeps the faster layout, with the fastest shape per pass.
-// The problem's weights and transpose are in place.
+// The entries a batched pass over M streams (tiled, else the packed stream or, in
+// FP64, the CSR): the two arrays, the second may be null.
+void streamed(DevCSR &M, int prec, bool tiled, DevBuf *(&out)[2]) {
+    if (tiled) {
+        out[0] = prec == FAIR_PREC_F16 ? &M.tl.r16 : prec == FAIR_PREC_Q16 ? &M.tl.rq : &M.tl.idx;
+        out[1] = prec == FAIR_PREC_F64 ? &M.tl.v64 : prec == FAIR_PREC_F32 ? &M.tl.v32 : nullptr;
+    } else {
+        out[0] = prec == FAIR_PREC_F64 ? &M.col : &M.gidx;
+        out[1] = prec == FAIR_PREC_F64 ? &M.v64 : prec == FAIR_PREC_F32 ? &M.pv32 : prec == FAIR_PREC_F16 ? &M.pv16 : &M.pvq;
+    }
+}
+
+// Layout 2: times one problem's passes (on scratch vectors) on the packed
+// streams (the CSR in FP64) and on its tiled copies with each candidate tile
+// shape, and keeps the faster layout, with the fastest shape per pass. What is
+// timed are the batch's own kernels over several copies of the problem, whose
+// entries come from memory and fill the GPU as those of a full batch do (the
+// single-problem passes, from L2, chose the packed streams for 18 of 96 fan-beam
+// problems of N <= 512 in FP32, 26 of 96 of N <= 256 in 16-bit codes and 38 in FP64,
+// 10.27, 2.39 and 5.92 ms an iteration; these choose none, 9.40, 1.98 and 5.52). The
+// problem's weights and transpose are in place.
 int tune_class(fair_batch_s *B, BatchProb &q, ClassChoice &c) {
     cudaStream_t s = B->stream;
     const int prec = B->prec;
@@ -474,38 +508,90 @@ int tune_class(fair_batch_s *B, BatchProb &q, ClassChoice &c) {
     FAIR_CUDA(cudaMemsetAsync(x.p, 0, sizeof(double) * (size_t)(n + 1), s));
     FAIR_CUDA(cudaMemsetAsync(x32.p, 0, sizeof(float) * (size_t)(n + 1), s));
     FAIR_CUDA(cudaMemsetAsync(sched.p, 0, 4 * sizeof(unsigned), s));
-    SirtDev S;
-    S.prec = prec;
-    S.m = (int32_t)m;
-    S.n = (int32_t)n;
-    S.A = &q.A;
-    S.AT = &q.AT;
-    S.b = b.as<double>();
-    S.Minv = q.M_sart.as<double>();
-    S.D = q.D.as<double>();
-    S.x = x.as<double>();
-    S.x32 = x32.as<float>();
-    S.r = r.p;
-    S.sched = sched.as<unsigned>();
     cudaEvent_t ev[2];
     for (auto &e : ev) FAIR_CUDA(cudaEventCreate(&e));
     struct EvScope {
         cudaEvent_t *e;
         ~EvScope() { cudaEventDestroy(e[0]); cudaEventDestroy(e[1]); }
     } evs{ev};
-    // time of one pass on the layout M is set to (best of two rounds of 5)
-    auto timed = [&](int pass, float *out) -> int {
-        *out = -1.f;
+    TmpBuf desc, c0;
+    TlBatch T;
+    struct TlScope {
+        TlBatch &t;
+        ~TlScope() { t.release(); }
+    } tls{T};
+    // time of a pass over one copy (best of two rounds of 3)
+    auto timed = [&](int pass, bool tiled, float *out) -> int {
+        DevCSR &M = pass == 1 ? q.A : q.AT;
+        DevBuf *src[2];
+        streamed(M, prec, tiled, src);
+        size_t one = 0;
+        for (const DevBuf *d : src) one += d ? (d->bytes + 255) & ~(size_t)255 : 0;
+        int copies = (int)std::min<size_t>(64, std::max<size_t>(1, kTuneBytes / std::max<size_t>(one, 1)));
+        if (copies > 1 && B->tune.grow(kTuneBytes)) copies = 1;
+        std::vector<DevCSR> reps((size_t)copies, M);  // M's buffers, the entries' copies in their place
+        for (int c = 1; c < copies; ++c) {
+            DevBuf *dst[2];
+            streamed(reps[c], prec, tiled, dst);
+            char *at = (char *)B->tune.p + one * (size_t)(c - 1);
+            for (int k = 0; k < 2; ++k)
+                if (src[k]) {
+                    FAIR_CUDA(cudaMemcpyAsync(at, src[k]->p, src[k]->bytes, cudaMemcpyDeviceToDevice, s));
+                    dst[k]->p = at;
+                    at += (src[k]->bytes + 255) & ~(size_t)255;
+                }
+        }
+        const void *xin = pass == 2 ? r.p : red ? x32.p : x.p;
+        const double *Mw = q.M_sart.as<double>(), *D = q.D.as<double>();
+        std::vector<TlBatchProb> tp;
+        std::vector<BPass> bp;
+        std::vector<int64_t> ch{0};
+        for (DevCSR &R : reps) {
+            if (tiled) {
+                tp.push_back(TlBatchProb{&R, xin, b.as<double>(), Mw, r.p, pass == 2 ? D : nullptr, x.as<double>(),
+                                         red ? x32.as<float>() : nullptr});
+                continue;
+            }
+            bp.push_back(packed_pass(R, prec));
+            BPass &d = bp.back();
+            d.xin = xin;
+            d.b = b.as<double>();
+            d.M = Mw;
+            d.r = r.p;
+            d.D = pass == 2 ? D : nullptr;
+            d.x = x.as<double>();
+            d.x32 = red ? x32.as<float>() : nullptr;
+            ch.push_back(ch.back() + ((int64_t)R.m + 31) / 32);
+        }
+        const BOpts o{1.0, 0.0, 0.0, 0};
+        if (tiled) {
+            FAIR_TRY(tl_host_offsets(M, s));
+            for (DevCSR &R : reps) R.tl.hsoff = M.tl.hsoff;
+            FAIR_TRY(tl_batch_cut(T, prec, tp));
+            FAIR_TRY(tl_batch_bind(T, prec, tp));
+        } else {
+            FAIR_TRY(desc.grow(sizeof(BPass) * bp.size()));
+            FAIR_TRY(c0.grow(sizeof(int64_t) * ch.size()));
+            FAIR_CUDA(cudaMemcpy(desc.p, bp.data(), sizeof(BPass) * bp.size(), cudaMemcpyHostToDevice));
+            FAIR_CUDA(cudaMemcpy(c0.p, ch.data(), sizeof(int64_t) * ch.size(), cudaMemcpyHostToDevice));
+        }
+        auto go = [&]() -> int {
+            if (tiled)
+                return tl_batch_launch(T, prec, pass, o.omg, o.lb, o.ub, o.bmode, sched.as<unsigned>(), s, false);
+            launch_packed(prec, pass, 8, 1, false, desc.as<BPass>(), c0.as<int64_t>(), copies, o,
+                          sched.as<unsigned>(), s);
+            return FAIR_OK;
+        };
+        FAIR_TRY(go());  // warm-up
         for (int round = 0; round < 2; ++round) {
-            sirt_pass(S, pass, s);  // warm-up
             cudaEventRecord(ev[0], s);
-            for (int k = 0; k < 5; ++k) sirt_pass(S, pass, s);
+            for (int k = 0; k < 3; ++k) FAIR_TRY(go());
             cudaEventRecord(ev[1], s);
             FAIR_CUDA(cudaEventSynchronize(ev[1]));
             FAIR_CUDA(cudaGetLastError());  // a launch that failed times as nothing
             float ms = 0.f;
             cudaEventElapsedTime(&ms, ev[0], ev[1]);
-            ms /= 5;
+            ms /= 3 * copies;
             *out = round == 0 ? ms : std::min(*out, ms);
         }
         return FAIR_OK;
@@ -518,11 +604,7 @@ int tune_class(fair_batch_s *B, BatchProb &q, ClassChoice &c) {
         pk = q.A.haspk && q.AT.haspk && !(prec == FAIR_PREC_Q16 && (q.A.qsigned || q.AT.qsigned));
     }
     if (pk)
-        for (int pass = 1; pass <= 2; ++pass) {
-            mats[pass - 1]->sirt_lanes[prec] = 8;
-            mats[pass - 1]->sirt_groups[prec] = red ? 1 : 0;
-            FAIR_TRY(timed(pass, &c.ms_packed[pass - 1]));
-        }
+        for (int pass = 1; pass <= 2; ++pass) FAIR_TRY(timed(pass, false, &c.ms_packed[pass - 1]));
     // the tiled copies, each candidate shape
     static const int shapes[2][4][2] = {{{96, 0}, {64, 0}, {128, 0}, {0, 0}},
                                         {{32, 13000}, {32, 6500}, {16, 6500}, {48, 13000}}};
@@ -537,11 +619,9 @@ int tune_class(fair_batch_s *B, BatchProb &q, ClassChoice &c) {
             M.tile_req[1] = shapes[pass - 1][k][1];
             FAIR_TRY(csr_make_tiled(M, prec, pass, s));
             if (!tl_batch_ready(M, prec)) continue;
-            M.sirt_lanes[prec] = 8;
-            M.sirt_groups[prec] = 9;
             float t = -1.f;
-            FAIR_TRY(timed(pass, &t));
-            if (best < 0.f || t < best) {
+            FAIR_TRY(timed(pass, true, &t));
+            if (bk < 0 || t < best * (bk == 0 ? kTuneMargin : 1.f)) {
                 best = t;
                 bk = k;
             }
@@ -554,11 +634,7 @@ int tune_class(fair_batch_s *B, BatchProb &q, ClassChoice &c) {
         M.tile_req[1] = shapes[pass - 1][bk][1];
         c.ms_tiled[pass - 1] = best;
     }
-    for (DevCSR *M : mats) {  // the batch sets the passes' layouts itself
-        M->sirt_lanes[prec] = 8;
-        M->sirt_groups[prec] = red ? 1 : 0;
-    }
-    c.tiled = tl_ok && (!pk || c.ms_tiled[0] + c.ms_tiled[1] < c.ms_packed[0] + c.ms_packed[1]);
+    c.tiled = tl_ok && (!pk || kTuneMargin * (c.ms_tiled[0] + c.ms_tiled[1]) < c.ms_packed[0] + c.ms_packed[1]);
     c.tile[0] = q.A.tile_req[0];
     c.tile[1] = q.AT.tile_req[0];
     c.tile[2] = q.AT.tile_req[1];
@@ -690,7 +766,7 @@ int fair_batch_destroy(fair_batch B) {
         delete p;
     }
     for (DevBuf *d : {&B->desc1, &B->desc2, &B->c0_1, &B->c0_2, &B->sched, &B->x32, &B->r,
-                      &B->w_b, &B->w_x})
+                      &B->w_b, &B->w_x, &B->tune})
         d->release();
     B->tb1.release();
     B->tb2.release();
@@ -853,6 +929,7 @@ int fair_batch_prepare(fair_batch B, const char *sirt_method, const fair_opts *o
     const size_t sx = red ? sizeof(float) : sizeof(double);
     FAIR_TRY(B->r.grow(sx * ((size_t)B->row_off.back() + 1)));
     if (red) FAIR_TRY(B->x32.grow(sizeof(float) * ((size_t)B->col_off.back() + 1)));
+    B->tune.release();
     B->ready = true;
     return FAIR_OK;
 }
