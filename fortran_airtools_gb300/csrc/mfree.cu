@@ -283,8 +283,10 @@ __global__ void __launch_bounds__(128) k_mf_project(const MfAngle *__restrict__ 
 }
 
 // xt = the transpose of x viewed as an N x N array (32 x 32 tiles through
-// shared memory, both sides coalesced). flag[0] becomes 1 if x holds an Inf or
-// NaN; the projector behind it takes it back (take_flag).
+// shared memory, both sides coalesced). *flag becomes 1 if x holds an Inf or NaN, for
+// the projector behind it; the FP32 backprojectors take it back, so that an iteration,
+// run or replayed from a graph, leaves nothing behind (a product of its own is
+// followed by a copy of 0, mf_apply).
 template <typename T>
 __global__ void __launch_bounds__(256) k_mf_transpose(const T *__restrict__ x, T *__restrict__ xt,
                                                       int N, unsigned *flag) {
@@ -295,7 +297,7 @@ __global__ void __launch_bounds__(256) k_mf_transpose(const T *__restrict__ x, T
         if (r < N && c < N) {
             const T v = x[(int64_t)r * N + c];
             tile[k][threadIdx.x] = v;
-            if (sizeof(T) == 4 && !isfinite(v)) atomicExch(flag, 1u);
+            if (sizeof(T) == 4 && !isfinite(v)) *flag = 1u;
         }
     }
     __syncthreads();
@@ -303,19 +305,6 @@ __global__ void __launch_bounds__(256) k_mf_transpose(const T *__restrict__ x, T
         const int r = c0 + k, c = r0 + threadIdx.x;
         if (r < N && c < N) xt[(int64_t)r * N + c] = tile[threadIdx.x][k];
     }
-}
-
-// The flag of the transpose before this pass, for every thread of the block;
-// the last block to have read it sets it back to 0 (flag[1] counts them and wraps
-// to 0), so that a pass leaves nothing behind, run or replayed from a graph.
-__device__ __forceinline__ bool take_flag(unsigned *flag) {
-    const bool on = *reinterpret_cast<volatile unsigned *>(flag) != 0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicInc(flag + 1, gridDim.x - 1) == gridDim.x - 1) atomicExch(flag, 0u);
-    }
-    return on;
 }
 
 // FP32 projector. A warp takes 32 adjacent rays of one angle and walks their
@@ -411,10 +400,10 @@ template <bool FAN, class Epi>
 __global__ void __launch_bounds__(128, 7) k_mf_project32(const MfAngle *__restrict__ ang, int nth, int p,
                                                       int N, const float *__restrict__ x,
                                                       const float *__restrict__ xt,
-                                                      unsigned *flag, Epi epi) {
+                                                      const unsigned *__restrict__ flag, Epi epi) {
     const int lane = threadIdx.x & 31, wpa = (p + 31) / 32;
     const int64_t nw = (int64_t)nth * wpa;
-    const bool guard = take_flag(flag);
+    const bool guard = *flag != 0;
     for (int64_t g = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); g < nw;
          g += (int64_t)gridDim.x * (blockDim.x >> 5)) {
         const int i = (int)(g / wpa), j = (int)(g - (int64_t)i * wpa) * 32 + lane;
@@ -538,7 +527,8 @@ struct __align__(16) BpAngle {
 template <class Epi>
 __global__ void __launch_bounds__(128, kBpOcc) k_mf_backproject32(const MfAngle *__restrict__ ang, int nth, int p,
                                                              int N, const float *__restrict__ y, float *part,
-                                                             Epi epi) {
+                                                             unsigned *flag, Epi epi) {
+    if (blockIdx.x + blockIdx.y + threadIdx.x == 0) *flag = 0;
     __shared__ BpAngle cs[2][kBpBatch];
     __shared__ float2 ys[2][kBpBatch][kBpBins];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -889,7 +879,8 @@ __device__ __forceinline__ long long mad_small(long long d, unsigned l, long lon
 template <typename YT, typename ACC, int MODE, bool TANK, bool UNI, class Epi>
 __global__ void __launch_bounds__(kFanThreads, 7) k_mf_backproject_fan(
         const MfAngle *__restrict__ rays, const MfFanAngle *__restrict__ fa, MfBins B, int nth,
-        int p, int N, const YT *__restrict__ y, ACC *part, Epi epi) {
+        int p, int N, const YT *__restrict__ y, ACC *part, unsigned *flag, Epi epi) {
+    if (sizeof(ACC) == 4 && blockIdx.x + blockIdx.y + threadIdx.x == 0) *flag = 0;
     constexpr int PB = kFanPB, CAP = kFanCap, PAD = kFanPad, NA = kFanThreads;
     __shared__ FanRays<ACC> W[2][2];
     __shared__ int2 win[NA];     // per angle: the sorted keys [x, y) that can meet the tile
@@ -1109,7 +1100,7 @@ struct fair_mf_s {
     fair::DevBuf part;                 // the backprojector's sums per share of the angles
     fair::DevBuf w_in, w_out;          // host-call staging (FP64)
     fair::DevBuf xt;                   // the projector's transposed copy of x
-    fair::DevBuf nonfinite;            // {x of the pass under way holds an Inf or NaN, blocks that know}
+    fair::DevBuf nonfinite;            // whether x of the iteration under way holds an Inf or NaN
     fair::DevBuf v_a, v_b;             // reduced-precision staging
     // SIRT state
     bool ready = false, sart = false;
@@ -1124,15 +1115,19 @@ struct fair_mf_s {
 namespace fair {
 namespace {
 
+int mf_grow_flag(fair_mf A) {
+    if (A->nonfinite.p) return FAIR_OK;
+    FAIR_TRY(A->nonfinite.grow(sizeof(unsigned)));
+    FAIR_CUDA(cudaMemsetAsync(A->nonfinite.p, 0, sizeof(unsigned), A->stream));
+    return FAIR_OK;
+}
+
 // Projector / backprojector launches of either geometry.
 // The transposed copy of x that the projector reads (N^2 elements of the
 // operator's precision), grown before a pass that reads x.
 int mf_grow_xt(fair_mf A) {
     const size_t es = A->prec == FAIR_PREC_F64 ? sizeof(double) : sizeof(float);
-    if (!A->nonfinite.p) {
-        FAIR_TRY(A->nonfinite.grow(2 * sizeof(unsigned)));
-        FAIR_CUDA(cudaMemsetAsync(A->nonfinite.p, 0, 2 * sizeof(unsigned), A->stream));
-    }
+    FAIR_TRY(mf_grow_flag(A));
     return A->xt.grow(es * (size_t)A->N * A->N);
 }
 
@@ -1198,6 +1193,8 @@ int mf_backproject(fair_mf A, const YT *y, Epi epi, cudaStream_t s) {
     const MfAngle *ang = A->ang.as<MfAngle>();
     constexpr bool f32 = std::is_same<ACC, float>::value;
     const int shares = mf_bp_shares(A, f32);
+    FAIR_TRY(mf_grow_flag(A));
+    unsigned *flag = A->nonfinite.as<unsigned>();
     if (shares > 1) FAIR_TRY(A->part.grow(sizeof(ACC) * (size_t)shares * n));
     ACC *part = A->part.as<ACC>();
     if (A->kind == 1) {
@@ -1207,16 +1204,16 @@ int mf_backproject(fair_mf A, const YT *y, Epi epi, cudaStream_t s) {
         const MfFanAngle *fa = A->fang.as<MfFanAngle>();
         if (A->tan_keys && A->uni_b > A->uni_a)
             k_mf_backproject_fan<YT, ACC, MODE, true, true><<<g, kFanThreads, 0, s>>>(
-                ang, fa, B, A->nth, A->p, A->N, y, part, epi);
+                ang, fa, B, A->nth, A->p, A->N, y, part, flag, epi);
         else if (A->tan_keys)
             k_mf_backproject_fan<YT, ACC, MODE, true, false><<<g, kFanThreads, 0, s>>>(
-                ang, fa, B, A->nth, A->p, A->N, y, part, epi);
+                ang, fa, B, A->nth, A->p, A->N, y, part, flag, epi);
         else
             k_mf_backproject_fan<YT, ACC, MODE, false, false><<<g, kFanThreads, 0, s>>>(
-                ang, fa, B, A->nth, A->p, A->N, y, part, epi);
+                ang, fa, B, A->nth, A->p, A->N, y, part, flag, epi);
     } else if constexpr (f32) {
         const dim3 g((unsigned)mf_bp_blocks(A, f32), shares);
-        k_mf_backproject32<<<g, 128, 0, s>>>(ang, A->nth, A->p, A->N, y, part, epi);
+        k_mf_backproject32<<<g, 128, 0, s>>>(ang, A->nth, A->p, A->N, y, part, flag, epi);
     } else {
         const dim3 g((unsigned)std::min<int64_t>(mf_bp_blocks(A, f32), (int64_t)sm_count() * 32), shares);
         if (shares > 1)
@@ -1560,6 +1557,7 @@ static int mf_apply(fair_mf A, bool back, const double *in, double *out) {
         if (back) FAIR_TRY((fair::mf_backproject<float, float, 0>(A, vin, e, s)));
         else fair::mf_project<float, float, 0>(A, vin, e, s);
         FAIR_CUDA(cudaGetLastError());
+        if (!back) FAIR_CUDA(cudaMemsetAsync(A->nonfinite.p, 0, sizeof(unsigned), s));
         FAIR_TRY(fair::vec_to_f64(A->v_b.as<float>(), nout, A->w_out.as<double>(), s));
     }
     FAIR_CUDA(cudaMemcpyAsync(out, A->w_out.p, sizeof(double) * nout, cudaMemcpyDeviceToHost, s));
