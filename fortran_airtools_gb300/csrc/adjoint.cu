@@ -91,7 +91,11 @@ __device__ __forceinline__ void chunk_rows_multi(const int64_t *__restrict__ row
             }
         }
         const int64_t row = base + lane;
-        if (row < m) epi(row, mine);
+        if (row < m) {
+            const T y = epi.at(row);
+#pragma unroll
+            for (int c = 0; c < NR; ++c) epi.one(row, c, mine[c], y);
+        }
     }
     finish_chunks(sched, nwarps, lane);
 }
@@ -153,7 +157,7 @@ __device__ __forceinline__ void chunk_rows_rhs(const int64_t *__restrict__ rowpt
             T v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
 #pragma unroll
             for (int o = 16; o >= NR; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-            if (lane < NR) epi.one(row, c, v);
+            if (lane < NR) epi.one(row, c, v, epi.at(row));
         }
     }
     finish_chunks(sched, nwarps, lane);
@@ -174,8 +178,8 @@ __device__ __forceinline__ T boxT(T t, int bmode, T lb, T ub) {
 // inv holds 0 there.
 template <typename T> struct Weights {
     const T *w, *inv;
-    __device__ __forceinline__ T of(int64_t i, T v, bool zero_if_empty = false) const {
-        const T y = inv[i];
+    __device__ __forceinline__ T at(int64_t i) const { return inv[i]; }
+    __device__ __forceinline__ T of(int64_t i, T y, T v, bool zero_if_empty = false) const {  // y = at(i)
         unsigned hi;
         if constexpr (sizeof(T) == 8) hi = (unsigned)__double2hiint(y);
         else hi = __float_as_uint(y);
@@ -189,11 +193,8 @@ struct EpiFwdResid {
     const T *b;
     Weights<T> M;
     T *r;
-    __device__ void one(int64_t i, int c, T v) const { r[i * NR + c] = M.of(i, b[i * NR + c] - v); }
-    __device__ void operator()(int64_t i, const T (&acc)[NR]) const {
-#pragma unroll
-        for (int c = 0; c < NR; ++c) one(i, c, acc[c]);
-    }
+    __device__ T at(int64_t i) const { return M.at(i); }
+    __device__ void one(int64_t i, int c, T v, T y) const { r[i * NR + c] = M.of(i, y, b[i * NR + c] - v); }
 };
 // forward pass 2: g = A' r (kept when recording), x = P(x + lam g / D)
 template <typename T, int NR>
@@ -203,15 +204,12 @@ struct EpiFwdUpdate {
     T *x, *gsave;
     T lb, ub;
     int bmode;
-    __device__ void one(int64_t j, int c, T v) const {
+    __device__ T at(int64_t j) const { return D.w ? D.at(j) : (T)0; }
+    __device__ void one(int64_t j, int c, T v, T y) const {
         T u = lam[c] * v;
-        if (D.w) u = D.of(j, u);
+        if (D.w) u = D.of(j, y, u);
         if (gsave) gsave[j * NR + c] = v;
         x[j * NR + c] = boxT<T>(x[j * NR + c] + u, bmode, lb, ub);
-    }
-    __device__ void operator()(int64_t j, const T (&acc)[NR]) const {
-#pragma unroll
-        for (int c = 0; c < NR; ++c) one(j, c, acc[c]);
     }
 };
 // reverse, over A: w = (A t) / M (0 on empty rows), gb += lam w
@@ -220,14 +218,11 @@ struct EpiAdjA {
     Weights<T> M;
     const T *lam;
     T *w, *gb;
-    __device__ void one(int64_t i, int c, T v) const {
-        const T wi = M.of(i, v, true);
+    __device__ T at(int64_t i) const { return M.at(i); }
+    __device__ void one(int64_t i, int c, T v, T y) const {
+        const T wi = M.of(i, y, v, true);
         w[i * NR + c] = wi;
         gb[i * NR + c] += lam[c] * wi;
-    }
-    __device__ void operator()(int64_t i, const T (&acc)[NR]) const {
-#pragma unroll
-        for (int c = 0; c < NR; ++c) one(i, c, acc[c]);
     }
 };
 // reverse, over A': gx = gz - lam A' w
@@ -235,11 +230,8 @@ template <typename T, int NR>
 struct EpiAdjAT {
     const T *gz, *lam;
     T *gx;
-    __device__ void one(int64_t j, int c, T v) const { gx[j * NR + c] = gz[j * NR + c] - lam[c] * v; }
-    __device__ void operator()(int64_t j, const T (&acc)[NR]) const {
-#pragma unroll
-        for (int c = 0; c < NR; ++c) one(j, c, acc[c]);
-    }
+    __device__ T at(int64_t) const { return (T)0; }
+    __device__ void one(int64_t j, int c, T v, T) const { gx[j * NR + c] = gz[j * NR + c] - lam[c] * v; }
 };
 
 // (256, 4): up to 64 registers, so the 16 gathers of a block stay in flight
@@ -268,6 +260,7 @@ __global__ void __launch_bounds__(256) k_multi_rows(int32_t m, const int64_t *__
 #pragma unroll
         for (int k = 0; k < V; ++k) acc[k] = 0;
         const int64_t k1 = segbase[i + 1];
+        const T y = epi.at(i);
         for (int64_t k = segbase[i]; k < k1; ++k) {
             const T *p = part + (size_t)k * NR + c0;
             if constexpr (V == 4) {
@@ -281,7 +274,7 @@ __global__ void __launch_bounds__(256) k_multi_rows(int32_t m, const int64_t *__
             }
         }
 #pragma unroll
-        for (int k = 0; k < V; ++k) epi.one(i, c0 + k, acc[k]);
+        for (int k = 0; k < V; ++k) epi.one(i, c0 + k, acc[k], y);
     }
 }
 
@@ -302,7 +295,8 @@ __global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T
         const int c = (int)(e % NR);
         T g = gk[e];
         T u = lam[c] * g;
-        if (D.w) u = D.of(j, u);
+        const T y = D.w ? D.at(j) : (T)0;
+        if (D.w) u = D.of(j, y, u);
         T z = x[e] + u;
         bool pass = true;
         T zc = z;
@@ -310,8 +304,8 @@ __global__ void __launch_bounds__(256) k_adj_mask(int64_t n, const T *x, const T
         if (bmode & 2) pass = pass && (zc > lb);
         T gzv = pass ? gx[e] : (T)0;
         gz[e] = gzv;
-        t[e] = D.w ? D.of(j, gzv) : gzv;
-        part += (double)gzv * (double)(D.w ? D.of(j, g) : g);
+        t[e] = D.w ? D.of(j, y, gzv) : gzv;
+        part += (double)gzv * (double)(D.w ? D.of(j, y, g) : g);
     }
     // reduce over the threads sharing a column: lanes c, c+NR, ... then warps
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -421,8 +415,10 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
     FAIR_TRY(W[AB_LAM].grow(sizeof(T) * NR));
     FAIR_TRY(W[AB_M].grow(sizeof(T) * m * 2));  // weights, then their reciprocals
     FAIR_TRY(W[AB_D].grow(sizeof(T) * n * 2));
-    // a segment's partial sums of glam, then glam of every step
-    const size_t seg_sums = (size_t)ge * NR * (size_t)C;
+    // the partial sums of glam, of all steps where they take no more than a vector (one
+    // launch adds them up then), else of a segment; then glam of every step
+    const bool all_sums = sizeof(double) * ge * (size_t)K <= sizeof(T) * (size_t)n;
+    const size_t seg_sums = (size_t)ge * NR * (size_t)(all_sums ? std::max(K, 1) : C);
     FAIR_TRY(W[AB_SUM].grow(sizeof(double) * (seg_sums + (size_t)NR * (size_t)std::max(K, 1))));
     const int64_t segs = std::max<int64_t>(tiled1 ? A.tlm.nseg : 0, tiled2 ? AT.tlm.nseg : 0);
     FAIR_TRY(W[AB_PART].grow(sizeof(T) * NR * (size_t)segs));
@@ -503,12 +499,13 @@ int run_group(fair_csr h, const T *vA, const T *vAT, bool sart, const double *h_
             const T *xk = W[AB_XSEG].as<T>() + nNR * (k - k0);
             const T *gk = W[AB_GSEG].as<T>() + nNR * (k - k0);
             k_adj_mask<T, NR><<<ge, 256, 0, s>>>(n, xk, gk, D, lam, gx, gz, t, bmode, tlb, tub,
-                                                 sums + (size_t)(k - k0) * ge * NR);
+                                                 sums + (size_t)(all_sums ? k : k - k0) * ge * NR);
             FAIR_CUDA(cudaGetLastError());
             FAIR_TRY(product(1, t, EpiAdjA<T, NR>{M, lam, w, gb}));
             FAIR_TRY(product(2, w, EpiAdjAT<T, NR>{gz, lam, gx}));
         }
-        k_adj_sums<NR><<<k1 - k0, 256, 0, s>>>(sums, ge, gl + (size_t)k0 * NR);
+        if (!all_sums) k_adj_sums<NR><<<k1 - k0, 256, 0, s>>>(sums, ge, gl + (size_t)k0 * NR);
+        else if (k0 == 0) k_adj_sums<NR><<<K, 256, 0, s>>>(sums, ge, gl);
         FAIR_CUDA(cudaGetLastError());
     }
     // outputs
