@@ -359,8 +359,9 @@ __device__ __forceinline__ Span in_box(const double *g, int N, double o0, double
 
 // True when a crossing of the ray's major axis (direction component d, in-box
 // lines s) comes within 2^-28 of a line of the other family: the other
-// coordinate o(k) in fixed point with 46 fractional bits (off by less than
-// 2^-35), lines of the other family at its integers.
+// coordinate o(k) in fixed point with 46 fractional bits (its step rounded: off by
+// at most N (2^-47 + 2^-52) + 2^-46, below 2^-30 up to N = 2^16), lines of the other
+// family at its integers.
 __device__ __forceinline__ bool near_line(const double *g, int N, double o0, double dir, double inv,
                                           double odir, double oo0, Span s) {
     if (s.k1 < s.k0) return false;

@@ -385,8 +385,9 @@ int sweep_warps() {
 //     last | first, not last | shared, not last | shared and last], and the
 //     longest paths between the window's steps (predecessor chains) as one
 //     byte per pair;
-//   k_lvl_levels (one block; k_lvl_levels_cluster for tables that do not fit
-//     shared memory, on a 16-block cluster), windows in order: a step's level
+//   k_lvl_levels_grid (a step of the window per block of a cooperative grid; where
+//     that launch is refused k_lvl_levels_cluster, on a 16-block cluster, or
+//     k_lvl_levels, in one block), windows in order: a step's level
 //     is the largest, over the steps a of its window with a path to it, of
 //     base(a) + the path's length, base(a) = 1 + the table's level over a's
 //     first-touch columns; the last touches write the levels into the table
@@ -1082,13 +1083,6 @@ template <> struct XAcc<XD> {
     }
 };
 
-// One step by a group of G warps: the row's chunks of 32 entries are dealt
-// to the group's warps in turn (chunk q to warp q mod G), CACHE chunks per
-// warp held in registers and the rest loaded in batches of four. Each warp's
-// part of a.x - b is an exact fixed-point sum (fx_warp_part); the G parts meet
-// in shared memory behind the group's named barrier, are added exactly and
-// rounded once; then the coefficient (b - a.x) * (omega / nrA) and the bounded
-// updates.
 // A warp's first CACHE chunks of a step (column and value of entry lane of
 // each chunk; column 0 and value 0 past the row's end).
 template <int CACHE> struct LvlChunks {
@@ -1146,6 +1140,13 @@ __device__ __forceinline__ double step_coef(const FxPart &part, FxPart *parts, d
     return __dmul_rn(-(part.e >= 0x7FF ? part.d : fx_to_double_fast(part.s, part.e)), w);
 }
 
+// One step by a group of G warps: the row's chunks of 32 entries are dealt
+// to the group's warps in turn (chunk q to warp q mod G), CACHE chunks per
+// warp held in registers and the rest loaded in batches of four. Each warp's
+// part of a.x - b is an exact fixed-point sum (fx_warp_part); the G parts meet
+// in shared memory behind the group's named barrier, are added exactly and
+// rounded once; then the coefficient (b - a.x) * (omega / nrA) and the bounded
+// updates.
 template <int XM, int CACHE>
 __device__ __forceinline__ void lvl_row(const RowStep &st, const int32_t *__restrict__ col,
                                         const double *__restrict__ val, const XAcc<XM> &X,
@@ -1797,8 +1798,8 @@ int lvl_build(const SweepDev &S, SweepWork &W, SweepWork::Levels &C, const RowSt
     W.uid += (uint64_t)nwin;
     *built = true;
     if (!want) return FAIR_OK;
-    // on a cluster with the table in global memory; else in one block, the table
-    // in its shared memory where it fits
+    // on a cooperative grid, else on a cluster, the table in global memory; else in one
+    // block, the table in its shared memory where it fits
     const size_t lv_bytes = 4 * (size_t)std::max<int32_t>(A.n, 1);
     if (W.lvtab.grow(lv_bytes)) {
         *built = false;

@@ -12,9 +12,9 @@
 // cycles also when predicated off, and masked multiply-adds in a branch of
 // their own cost every first and last step of a row twice. The row sums are
 // reduced over the G lanes and moved to one lane per row, so that the epilogue
-// of a chunk runs once, with coalesced loads and stores. A matrix with few
-// rows takes smaller chunks (down to the 32/G rows of one round), so that more
-// warps work on it: the same arithmetic per row, the same results.
+// of a chunk runs once, with coalesced loads and stores. A chunk of the SIRT
+// passes is one round of 32/G rows, two on large matrices whose call returns at
+// once (launch_rows, solvers.cu): the same arithmetic per row, the same results.
 //
 // Column/value arrays are allocated with 4 spare entries so that the aligned
 // window never reads past the allocation.

@@ -45,7 +45,11 @@ int fair_spmv_device(fair_csr h, int32_t trans, const void *d_x, void *d_y);
  * it returns gb = dL/db (m x nrhs), gx0 = dL/dx0 (n x nrhs) and glam = dL/dlambda
  * (nrhs); xK (may be NULL) receives x_K. x0 may be NULL (zeros). Checkpoints
  * every ceil(sqrt(K)) steps. FP64 for FAIR_PREC_F64, FP32 values and vectors
- * for FAIR_PREC_F32 (the lambda gradient is summed in FP64). */
+ * for FAIR_PREC_F32 (the lambda gradient is summed in FP64). The handle keeps, for
+ * later calls, tiled copies of A and A' (10 bytes per nonzero and matrix in FP64, 6 in
+ * FP32, where there is memory for them; the products run row by row without) and the
+ * call's vectors, 3 ceil(sqrt(K)) + 8 of up to 16 columns; they are freed when an
+ * allocation of another call on the handle fails, or with it. */
 int fair_sirt_adjoint(fair_csr h, const char *sirt_method, int32_t nrhs, const double *b,
                       const double *x0, int32_t K, const double *lambda, const fair_opts *options,
                       const double *gx, double *xK, double *gb, double *gx0, double *glam);
